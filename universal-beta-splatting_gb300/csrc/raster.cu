@@ -20,9 +20,9 @@
 //     8x8-pixel footprint of every warp and the results turned into per-warp
 //     bitmasks by ballot, so a warp only visits records that can touch its
 //     pixels;
-//   * the backward sums the 7 + channels gradients of a record over a warp with
-//     transpose reductions (14 shuffles for 10 values), each warp writes its
-//     totals into its own list of rows in shared memory with plain stores, and
+//   * the backward sums the 7 + channels gradients of a record over a warp on
+//     the tensor cores (moments of per-pixel values with constant weights, see
+//     moment_products) and a transpose reduction, each warp writes its totals into its own list of rows in shared memory with plain stores, and
 //     per batch the rows of a record are summed and added to its gradient row
 //     with three 16-byte vector atomics (fused path) or one scalar atomic per
 //     value (drop-in arrays).
@@ -78,6 +78,7 @@ struct RasterArgs {
     int32_t n_buckets;          // total (view, tile) buckets
     const int64_t *n_isects_dev; // device-side intersection count (nullptr: n_isects)
     const int32_t *order;        // CTA -> bucket launch order (nullptr: identity)
+    int32_t sub;                 // CTAs per tile side: sub x sub CTAs share a bucket
     // gather mode (fused scene path, packed colours): records are copied per
     // batch from the per-entry tables, addressed by the low word of the
     // sorted (depth, entry) keys, instead of from sorted copies
@@ -117,6 +118,21 @@ __device__ __forceinline__ TileLoc locate_tile(const RasterArgs &a, int bt) {
     l.TW = a.v_dims[lo * 4 + 2];
     l.pix_base = a.v_pix_base[lo];
     return l;
+}
+
+// The bucket of this CTA and its part of the tile: sub x sub consecutive CTAs
+// work on one bucket, each on a square of edge TS pixels.
+struct CtaPart {
+    int bt, x, y; // bucket; first pixel column and row within the tile
+};
+__device__ __forceinline__ CtaPart cta_part(const RasterArgs &a, int TS) {
+    CtaPart p;
+    const int ss = a.sub * a.sub;
+    const int i = (int)blockIdx.x / ss, part = (int)blockIdx.x - i * ss;
+    p.bt = a.order ? a.order[i] : i;
+    p.y = part / a.sub * TS;
+    p.x = (part - part / a.sub * a.sub) * TS;
+    return p;
 }
 
 // Number of valid sorted records: the device count (clamped to the record
@@ -176,28 +192,41 @@ __global__ void pack_records_kernel(int64_t T, int64_t n_prims, const int32_t *_
 // ways.  KE = 0: one shared accumulator row per batch slot (BR x NV floats),
 // which every warp adds its reduced sums to with shared-memory atomics, and a
 // touched flag per slot.  KE > 0: every warp owns a list of KE entry rows
-// (NV floats each) that it fills with plain stores, one row per record it
-// visits, and a byte per batch slot naming the row (0xFF: none); the flush
-// sums the warps' rows of a slot.  Shared float atomics cost about as much as
-// the rest of a visit's reduction, so the small tiles use the lists.
+// (row_pitch floats each, after a dump row) that it fills with plain stores,
+// one row per record it visits, last batch slot first: a slot's row is the
+// number of set bits after it in the warp's mask.  The flush sums the warps'
+// rows of a slot.  Shared float
+// atomics cost about as much as the rest of a visit's reduction, so the small
+// tiles use the lists.
 struct SmemLayout {
     int mask_off, rec_off, col_off, gacc_off, touched_off, total;
 };
+
+// Whether the backward reduces a visit on the tensor cores (see
+// moment_reduce): its 5 + CD rows of sums have to fit the 8 rows one product
+// leaves in a lane's accumulators.
+template <int CD> __host__ __device__ constexpr bool moment_rows() { return CD <= 3; }
+// Floats per entry row: the 6 moments of w, the sums of u and u log2(1 - s)
+// and CD colour sums, or the 7 + CD gradient sums.
+template <int CD> __host__ __device__ constexpr int row_pitch() {
+    return moment_rows<CD>() ? 8 + CD : 7 + CD;
+}
 
 template <int CD, bool PACK, bool BWD>
 __host__ __device__ inline SmemLayout smem_layout(int NT, int RB = 2, int KE = 0) {
     constexpr int NV = 7 + CD; // gradient values per record
     const int nw = NT / 32, BR = RB * NT;
     SmemLayout L;
-    L.mask_off = 16; // after two mbarriers
-    // per-target-warp masks (nw x RB nw words), then one int per warp
-    L.rec_off = (L.mask_off + nw * RB * nw * 4 + nw * 4 + 127) & ~127;
+    L.mask_off = 32; // after two mbarriers and the cold flag of the backward
+    // per-target-warp masks (nw x RB nw words, two sets in the backward), then
+    // one int per warp
+    L.rec_off = (L.mask_off + (BWD ? 2 : 1) * nw * RB * nw * 4 + nw * 4 + 127) & ~127;
     const int colbytes = PACK ? 16 : CD * 4;
     L.col_off = L.rec_off + 2 * BR * (int)sizeof(GeoRec);
     L.gacc_off = (L.col_off + 2 * BR * colbytes + 15) & ~15;
     if (BWD && KE > 0) {
-        L.touched_off = L.gacc_off + nw * KE * NV * 4; // entry rows, then the slot maps
-        L.total = L.touched_off + nw * BR;
+        L.touched_off = L.gacc_off + nw * (KE + 1) * row_pitch<CD>() * 4; // entry rows
+        L.total = L.touched_off;
     } else {
         L.touched_off = L.gacc_off + (BWD ? BR * NV * 4 : 0);
         L.total = L.touched_off + (BWD ? BR * 4 : 0);
@@ -591,24 +620,21 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
 // Per-pixel state of the back-to-front pass.  The reference keeps the colour
 // accumulated behind the current record per channel (buf_k) and forms
 // sum_k (c_k T - buf_k ra) v_k + T_final ra (v_a - bg.v); only the scalar
-// S = sum_k buf_k v_k enters, so it is carried instead of buf, and
-// K = T_final (v_a - bg.v) is folded once per pixel.
+// T_final (v_a - bg.v) - sum_k buf_k v_k enters, so it is carried (KS) instead
+// of buf.  A pixel outside the image has last contributor INT32_MIN.
 template <int CD> struct BwdPair {
-    float2 T, S, K;
+    float2 T, KS;
     float2 vrc[CD];
     int32_t bin0, bin1;
-    bool in0, in1;
 };
 
 template <int CD>
 __device__ __forceinline__ void bwd_pair_init(BwdPair<CD> &s, const RasterArgs &a, int64_t pix0,
                                               int64_t pix1, bool in0, bool in1, const float *bg) {
-    s.in0 = in0;
-    s.in1 = in1;
     const float T0 = 1.0f - a.render_alphas[pix0], T1 = 1.0f - a.render_alphas[pix1];
     s.T = make_float2(T0, T1);
-    s.bin0 = in0 ? a.last_in[pix0] : 0;
-    s.bin1 = in1 ? a.last_in[pix1] : 0;
+    s.bin0 = in0 ? a.last_in[pix0] : INT32_MIN;
+    s.bin1 = in1 ? a.last_in[pix1] : INT32_MIN;
     float bg0 = 0.f, bg1 = 0.f;
 #pragma unroll
     for (int k = 0; k < CD; ++k) {
@@ -618,8 +644,7 @@ __device__ __forceinline__ void bwd_pair_init(BwdPair<CD> &s, const RasterArgs &
             bg1 += bg[k] * s.vrc[k].y;
         }
     }
-    s.K = make_float2(T0 * (a.v_out_a[pix0] - bg0), T1 * (a.v_out_a[pix1] - bg1));
-    s.S = make_float2(0.f, 0.f);
+    s.KS = make_float2(T0 * (a.v_out_a[pix0] - bg0), T1 * (a.v_out_a[pix1] - bg1));
 }
 
 // One back-to-front step of both pixels of a thread against record q
@@ -627,70 +652,82 @@ __device__ __forceinline__ void bwd_pair_init(BwdPair<CD> &s, const RasterArgs &
 // T / (1 - alpha), v_alpha from the colour behind and the final alpha, the
 // sigma chain when opacity (1 - sigma)^beta <= 0.999), packed two-wide (one
 // FP32x2 instruction per step for the pixel pair); valid lanes are inside,
-// at or before their last contributor, with sigma in [0, 1), others evaluate
-// finite dummies (1 - sigma replaced by 1) that selects zero.  A record no
-// lane can use is evaluated too: under 1% of the culled visits are such, and
-// a warp vote to skip them cost more than it saved.  g receives the pair's sums
-//   [w dx, w dy, w dx^2, w dx dy, w dy^2, vis v_alpha, vis v_alpha log2(1-s),
-//    fac v_colour (CD)],  w = v_alpha (1 - sigma)^(beta - 1),
-// turned into [v_xy, v_conic, v_opacity, v_beta, v_colour] per record at
-// the flush (the conic, -opacity beta and opacity ln 2 factors).
-template <int CD>
-__device__ __forceinline__ void grad_pair(const GeoRec &q, const float (&col)[CD], float px,
-                                          float2 npy, int32_t idx, BwdPair<CD> &s,
-                                          float (&g)[7 + CD]) {
+// at or before their last contributor, with sigma in [0, 1).  The others take
+// 1 - sigma = 1 and alpha = 0, which leaves T and KS as they are, and zero
+// v_alpha.  A record no lane can use is evaluated too: under 1% of the culled
+// visits are such, and a warp vote to skip it cost more than it saved.
+// Gives per pixel  w = v_alpha (1 - sigma)^(beta - 1),  u = v_alpha (1 -
+// sigma)^beta,  ul = u log2(1 - sigma)  and  gc_k = alpha T v_colour_k.
+struct PairGeom {
+    float dx;
+    float2 dy;
+};
+// TAME: sigma is not NaN (see tame_record), so [0, 1) is one unsigned compare.
+template <int CD, bool TAME>
+__device__ __forceinline__ PairGeom grad_pair(const GeoRec &q, const float (&col)[CD], float px,
+                                              float2 npy, int32_t idx, BwdPair<CD> &s, float2 &w,
+                                              float2 &u, float2 &ul, float2 (&gc)[CD]) {
     const float dx = q.x - px;
-    const float2 dy = __fadd2_rn(make_float2(q.y, q.y), npy);
+    const float2 dy = make_float2(q.y + npy.x, q.y + npy.y);
     const float A = q.cxx * dx * dx;
     const float B = 2.f * q.cxy * dx;
-    float2 sg = __fmul2_rn(make_float2(q.cyy, q.cyy), dy);
-    sg = __ffma2_rn(sg, dy, make_float2(A, A));
-    sg = __ffma2_rn(make_float2(B, B), dy, sg);
-    const bool v0 = s.in0 && idx <= s.bin0 && !(sg.x < 0.f || sg.x >= 1.f);
-    const bool v1 = s.in1 && idx <= s.bin1 && !(sg.y < 0.f || sg.y >= 1.f);
-    float2 om = __ffma2_rn(sg, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
-    om.x = v0 ? om.x : 1.f;
-    om.y = v1 ? om.y : 1.f;
+    float2 sg;
+    sg.x = fmaf(B, dy.x, fmaf(__fmul_rn(q.cyy, dy.x), dy.x, A));
+    sg.y = fmaf(B, dy.y, fmaf(__fmul_rn(q.cyy, dy.y), dy.y, A));
+    const bool v0 = TAME ? ((idx <= s.bin0) & (__float_as_uint(sg.x) < 0x3f800000u))
+                         : (idx <= s.bin0 && !(sg.x < 0.f || sg.x >= 1.f));
+    const bool v1 = TAME ? ((idx <= s.bin1) & (__float_as_uint(sg.y) < 0x3f800000u))
+                         : (idx <= s.bin1 && !(sg.y < 0.f || sg.y >= 1.f));
+    const float2 om = make_float2(v0 ? 1.f - sg.x : 1.f, v1 ? 1.f - sg.y : 1.f);
     const float2 l = make_float2(__log2f(om.x), __log2f(om.y));
-    const float2 e = __fmul2_rn(l, make_float2(q.beta, q.beta));
-    const float2 vis = make_float2(exp2f(e.x), exp2f(e.y));
-    const float2 ov = __fmul2_rn(make_float2(q.opac, q.opac), vis);
-    const float2 alpha = make_float2(fminf(0.999f, ov.x), fminf(0.999f, ov.y));
-    const float2 oma = __ffma2_rn(alpha, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
-    const float2 ra = make_float2(1.0f / oma.x, 1.0f / oma.y);
-    const float2 Tn = __fmul2_rn(s.T, ra);
-    float2 fac = __fmul2_rn(alpha, Tn);
-    fac.x = v0 ? fac.x : 0.f;
-    fac.y = v1 ? fac.y : 0.f;
-    float2 cv = __fmul2_rn(make_float2(col[0], col[0]), s.vrc[0]);
+    const float2 vis = make_float2(exp2f(l.x * q.beta), exp2f(l.y * q.beta));
+    const float2 ov = make_float2(q.opac * vis.x, q.opac * vis.y);
+    const float2 alpha = make_float2(v0 ? fminf(0.999f, ov.x) : 0.f,
+                                     v1 ? fminf(0.999f, ov.y) : 0.f);
+    const float2 ra = make_float2(1.0f / (1.f - alpha.x), 1.0f / (1.f - alpha.y));
+    s.T = __fmul2_rn(s.T, ra);
+    const float2 fac = __fmul2_rn(alpha, s.T);
+    float2 cv = make_float2(col[0] * s.vrc[0].x, col[0] * s.vrc[0].y);
 #pragma unroll
-    for (int k = 1; k < CD; ++k)
-        cv = __ffma2_rn(make_float2(col[k], col[k]), s.vrc[k], cv);
-#pragma unroll
-    for (int k = 0; k < CD; ++k) {
-        const float2 gc = __fmul2_rn(fac, s.vrc[k]);
-        g[7 + k] = gc.x + gc.y;
+    for (int k = 1; k < CD; ++k) {
+        cv.x = fmaf(col[k], s.vrc[k].x, cv.x);
+        cv.y = fmaf(col[k], s.vrc[k].y, cv.y);
     }
-    const float2 kms = __ffma2_rn(s.S, make_float2(-1.f, -1.f), s.K);
-    float2 va = __ffma2_rn(Tn, cv, __fmul2_rn(ra, kms));
-    va.x = (v0 && ov.x <= 0.999f) ? va.x : 0.f;
-    va.y = (v1 && ov.y <= 0.999f) ? va.y : 0.f;
-    const float2 u = __fmul2_rn(vis, va);
-    const float2 w = __fmul2_rn(u, make_float2(__fdividef(1.f, om.x), __fdividef(1.f, om.y)));
+#pragma unroll
+    for (int k = 0; k < CD; ++k) gc[k] = __fmul2_rn(fac, s.vrc[k]);
+    float2 va = __ffma2_rn(s.T, cv, __fmul2_rn(ra, s.KS));
+    va.x = (v0 & (ov.x <= 0.999f)) ? va.x : 0.f;
+    va.y = (v1 & (ov.y <= 0.999f)) ? va.y : 0.f;
+    u = __fmul2_rn(vis, va);
+    w = make_float2(u.x * __fdividef(1.f, om.x), u.y * __fdividef(1.f, om.y));
+    ul = __fmul2_rn(u, l);
+    s.KS.x = fmaf(-fac.x, cv.x, s.KS.x);
+    s.KS.y = fmaf(-fac.y, cv.y, s.KS.y);
+    PairGeom p;
+    p.dx = dx;
+    p.dy = dy;
+    return p;
+}
+
+// The pair's sums  [w dx, w dy, w dx^2, w dx dy, w dy^2, u, ul, gc (CD)],
+// turned into [v_xy, v_conic, v_opacity, v_beta, v_colour] per record at the
+// flush (the conic, -opacity beta and opacity ln 2 factors).
+template <int CD>
+__device__ __forceinline__ void pair_sums(const PairGeom &p, const float2 &w, const float2 &u,
+                                          const float2 &ul, const float2 (&gc)[CD],
+                                          float (&g)[7 + CD]) {
     const float ws = w.x + w.y;
-    const float2 wdy = __fmul2_rn(w, dy);
-    const float2 wdy2 = __fmul2_rn(wdy, dy);
-    const float2 ul = __fmul2_rn(u, l);
-    g[0] = ws * dx;
+    const float2 wdy = __fmul2_rn(w, p.dy);
+    const float2 wdy2 = __fmul2_rn(wdy, p.dy);
+    g[0] = ws * p.dx;
     g[1] = wdy.x + wdy.y;
-    g[2] = ws * (dx * dx);
-    g[3] = g[1] * dx;
+    g[2] = ws * (p.dx * p.dx);
+    g[3] = g[1] * p.dx;
     g[4] = wdy2.x + wdy2.y;
     g[5] = u.x + u.y;
     g[6] = ul.x + ul.y;
-    s.S = __ffma2_rn(fac, cv, s.S);
-    s.T.x = v0 ? Tn.x : s.T.x;
-    s.T.y = v1 ? Tn.y : s.T.y;
+#pragma unroll
+    for (int k = 0; k < CD; ++k) g[7 + k] = gc[k].x + gc[k].y;
 }
 
 // Factor turning the reduced sum g[u] (u >= 2) of a record into its gradient
@@ -742,34 +779,224 @@ template <int OFF> struct ReduceChunks<OFF, 0> {
                                                Sink &) {}
 };
 
-// MINB > 1: tiles of at most 128 threads, MINB CTAs per SM.  KE > 0: entry
-// lists of KE rows per warp (see smem_layout).
-template <int CD, bool PACK, int RB, int MINB, int KE>
-__global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(RasterArgs a) {
+// ------------------------------------- a visit's sums on the tensor cores
+// The 5 + CD sums a (warp, record) visit needs are linear in per-pixel values
+// with weights that do not depend on the record: the moments of w over the
+// warp's 8x8 pixels (1, x, y, x^2, xy, y^2; the record's own dx, dy follow at
+// the flush from its centre) and plain sums of u, ul and gc.  A lane holds
+// column x = lane / 4, rows y = 2 (lane % 4) + {0, 1}, which is where
+// mma.m16n8k8 (tf32) expects operand A: row g = lane / 4 (and g + 8), k =
+// lane % 4 (and + 4).  So four products contract the values over y straight
+// from the registers they are in: in one, rows x hold w (both pixels) and
+// rows x + 8 the pixel pair's sum of the odd colour (k < 4); in the other rows
+// x hold the pair sums of u (k < 4) and a colour, rows x + 8 those of ul and
+// another colour.  Their
+// constant operands put each sum into a column of its own, chosen so that a
+// lane's four accumulators are four sums still to be added over x (two of
+// them formed by multiplying with x or x^2), which takes a transpose
+// reduction over the lane groups.  tf32 holds 11 significant bits, so every
+// value is split into its leading bits and the exact rest, of which the
+// product reads the leading 11 bits: 22 bits of each value, FP32
+// accumulation; the weights are small multiples of 1/4 and exact.
+// Coordinates are relative to the middle of the 8x8 box.  Measured against
+// the transpose reductions of all 10 sums this replaced (1M primitives at
+// 1080p, 5.6M visits): 211 -> 160 warp instructions per visit, 1.104 -> 0.955
+// ms; finishing a visit while the next is evaluated cost more registers than
+// the latency it hid (0.99 ms), constant weights in operand A (which leaves a
+// second product for x instead of the lane exchanges) more copies (1.32 ms).
+struct MomentBasis {
+    float b0, b1, c0, c1; // operand B of the w and of the u products
+    float f1, f3;         // x and x^2 where a lane's first sum needs them
+    uint32_t m16, m8;     // lane-bit masks of the transpose reduction
+    uint32_t first;       // shared address of this lane's element of the first entry row
+    uint32_t pitch;       // and how far the next row's is; 0 where it has none
+};
+
+// rows: the warp's entry rows, of which the first is a dump.
+template <int CD>
+__device__ __forceinline__ MomentBasis moment_basis(int lane, const float *rows) {
+    const int g = lane >> 2, t = lane & 3;
+    const float y0 = 2.f * t - 3.5f, y1 = y0 + 1.f, x = g - 3.5f;
+    MomentBasis b;
+    // columns: 0 w y, 2 u (ul), 3 colours 0 (1), 4 w y^2, 5 (odd colour), 6 w;
+    // in brackets what rows x + 8 sum
+    b.b0 = g == 0 ? y0 : g == 4 ? y0 * y0 : (g == 5 || g == 6) ? 1.f : 0.f;
+    b.b1 = g == 0 ? y1 : g == 4 ? y1 * y1 : g == 6 ? 1.f : 0.f;
+    b.c0 = g == 2 ? 1.f : 0.f;
+    b.c1 = g == 3 ? 1.f : 0.f;
+    // lane (g, t) holds columns 2t, 2t + 1 of rows g, g + 8
+    b.f1 = (t == 0 || t == 3) ? x : 0.f;
+    b.f3 = t == 3 ? x * x : 0.f;
+    b.m16 = (lane & 16) ? ~0u : 0u;
+    b.m8 = (lane & 8) ? ~0u : 0u;
+    // entry row: [w, wx, wxx, wy, wxy, wyy, u, ul, gc (CD)]; lane (g, t)
+    // ends up with the total of its group's accumulator g / 2
+    const int v = g >> 1;
+    int off = -1;
+    if (t == 0) off = v == 0 ? 3 : v == 1 ? 4 : -1;
+    if (t == 1) off = v == 0 ? 6 : v == 2 ? 7 : CD < 2 ? -1 : v == 1 ? 8 : 9;
+    if (t == 2) off = v == 0 ? 5 : (v == 3 && CD != 2) ? 7 + CD : -1;
+    if (t == 3) off = v < 2 ? v : v == 3 ? 2 : -1;
+    if (g & 1) off = -1;
+    b.first = smem_u32(rows) + 4 * max(off, 0);
+    b.pitch = off < 0 ? 0 : 4 * row_pitch<CD>();
+    return b;
+}
+
+__device__ __forceinline__ void mma_tf32(float (&d)[4], float a0, float a1, float a2, float a3,
+                                         float b0, float b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 "
+        "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)),
+          "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+// The leading 11 significant bits of v.
+__device__ __forceinline__ float tf32_hi(float v) {
+    return __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+}
+// One halving step of a transpose reduction over the lane bit h with mask m.
+__device__ __forceinline__ float tr_step(float a, float b, uint32_t m, int h) {
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    const float send = __uint_as_float((ua & m) | (ub & ~m));
+    const float keep = __uint_as_float((ub & m) | (ua & ~m));
+    return keep + __shfl_xor_sync(0xffffffffu, send, h);
+}
+
+// The products of a visit, and the rest of its sums over the warp into the
+// entry row whose element for this lane is at `row`.
+template <int CD>
+__device__ __forceinline__ void moment_products(const MomentBasis &mb, const float2 &w,
+                                                const float2 &u, const float2 &ul,
+                                                const float2 (&gc)[CD], float (&d)[4]) {
+    static_assert(moment_rows<CD>(), "two colours and an odd one");
+    const float us = u.x + u.y, uh = tf32_hi(us), ls = ul.x + ul.y, lh = tf32_hi(ls);
+    float g0 = 0.f, g1 = 0.f, h0 = 0.f, h1 = 0.f;
+    if constexpr (CD >= 2) {
+        g0 = gc[0].x + gc[0].y;
+        g1 = gc[1].x + gc[1].y;
+        h0 = tf32_hi(g0);
+        h1 = tf32_hi(g1);
+    }
+    d[0] = d[1] = d[2] = d[3] = 0.f;
+    mma_tf32(d, us - uh, ls - lh, g0 - h0, g1 - h1, mb.c0, mb.c1);
+    mma_tf32(d, uh, lh, h0, h1, mb.c0, mb.c1);
+    float g2 = 0.f, h2 = 0.f;
+    if constexpr (CD != 2) {
+        g2 = gc[CD - 1].x + gc[CD - 1].y;
+        h2 = tf32_hi(g2);
+    }
+    const float wx = tf32_hi(w.x), wy = tf32_hi(w.y);
+    // the last element meets zero weights in the columns that are read
+    mma_tf32(d, w.x - wx, g2 - h2, w.y - wy, w.y, mb.b0, mb.b1);
+    mma_tf32(d, wx, h2, wy, g2, mb.b0, mb.b1);
+}
+__device__ __forceinline__ void moment_finish(const MomentBasis &mb, const float (&d)[4],
+                                              uint32_t row) {
+    const float d1 = fmaf(d[0], mb.f1, d[1]), d3 = fmaf(d[0], mb.f3, d[3]);
+    float tot = tr_step(tr_step(d[0], d[2], mb.m16, 16), tr_step(d1, d3, mb.m16, 16), mb.m8, 8);
+    tot += __shfl_xor_sync(0xffffffffu, tot, 4);
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(row), "f"(tot) : "memory");
+}
+
+// Adds an entry row of moments to the sums [w dx, w dy, w dx^2, w dx dy,
+// w dy^2, u, ul, gc] of its record: X, Y is the record's centre relative to
+// the middle of the warp's box, dx = X - x, dy = Y - y.
+template <int CD>
+__device__ __forceinline__ void add_moments(const float *row, float X, float Y,
+                                            float (&sum)[7 + CD]) {
+    const float S = row[0], Sx = row[1], Sxx = row[2], Sy = row[3], Sxy = row[4], Syy = row[5];
+    const float XS = X * S - Sx, YS = Y * S - Sy;
+    sum[0] += XS;
+    sum[1] += YS;
+    sum[2] += X * (XS - Sx) + Sxx;
+    sum[3] += X * YS - (Y * Sx - Sxy);
+    sum[4] += Y * (YS - Sy) + Syy;
+#pragma unroll
+    for (int k = 0; k < 2 + CD; ++k) sum[5 + k] += row[6 + k];
+}
+
+// Values large enough to overflow in a product, infinities and NaN would
+// spread over the sums of a visit in the tensor-core reduction (0 x inf); a
+// batch whose records or pixels hold such values, a negative beta or a
+// non-positive conic diagonal (whose sigma can be -0) is reduced by lane
+// exchanges instead.
+constexpr float kTameLimit = 1e10f;
+template <int CD>
+__device__ __forceinline__ bool tame_record(const GeoRec &q, const float (&col)[CD]) {
+    float m = fabsf(q.x) + fabsf(q.y) + fabsf(q.opac) + fabsf(q.beta) + fabsf(q.cxx) +
+              fabsf(q.cxy) + fabsf(q.cyy);
+#pragma unroll
+    for (int k = 0; k < CD; ++k) m += fabsf(col[k]);
+    return m < kTameLimit && q.beta >= 0.f && q.cxx > 0.f && q.cyy > 0.f;
+}
+template <int CD> __device__ __forceinline__ bool tame_pixels(const BwdPair<CD> &s) {
+    float m = fabsf(s.T.x) + fabsf(s.T.y) + fabsf(s.KS.x) + fabsf(s.KS.y);
+#pragma unroll
+    for (int k = 0; k < CD; ++k) m += fabsf(s.vrc[k].x) + fabsf(s.vrc[k].y);
+    return m < kTameLimit;
+}
+
+// Adds a record's summed values (with the conic applied to the first two) to
+// its gradient row or arrays.
+template <int CD>
+__device__ __forceinline__ void add_record(const RasterArgs &a, const GeoRec &q,
+                                           float (&sum)[7 + CD]) {
     constexpr int NV = 7 + CD;
-    static_assert(KE < 255, "entry rows are named by a byte");
+#pragma unroll
+    for (int u = 0; u < NV; ++u) sum[u] *= record_scale(u, q.opac, q.beta, true);
+    if (NV <= GRAD_ROW && a.v_rows) {
+        // three 16-byte vector atomics per row instead of NV scalar ones
+        float4 *row = reinterpret_cast<float4 *>(a.v_rows + (int64_t)q.gid * GRAD_ROW);
+#pragma unroll
+        for (int c = 0; c < (NV + 3) / 4; ++c) {
+            float4 v;
+            v.x = sum[4 * c];
+            v.y = 4 * c + 1 < NV ? sum[(4 * c + 1) % NV] : 0.f;
+            v.z = 4 * c + 2 < NV ? sum[(4 * c + 2) % NV] : 0.f;
+            v.w = 4 * c + 3 < NV ? sum[(4 * c + 3) % NV] : 0.f;
+            atomicAdd(row + c, v);
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < NV; ++u)
+            if (sum[u] != 0.f) atomicAdd(grad_dst<CD>(a, u, q.gid), sum[u]);
+    }
+}
+
+// TSZ: edge of a CTA's pixels, 8 or 16, or 0 for a whole tile of a.TS; MINB
+// CTAs per SM.  KE > 0: entry lists of KE rows per warp (see smem_layout).
+template <int CD, bool PACK, int TSZ, int RB, int MINB, int KE>
+__global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_kernel(RasterArgs a) {
+    constexpr int NV = 7 + CD;
+    constexpr bool MOM = KE > 0 && moment_rows<CD>(); // tensor-core reduction of the visits
+    constexpr int RP = row_pitch<CD>();
     extern __shared__ __align__(128) unsigned char sm[];
-    const int NT = blockDim.x, nw = NT >> 5, BR = RB * NT;
+    const int TS = TSZ ? TSZ : a.TS;
+    const int NT = TSZ ? TSZ * TSZ / 2 : (int)blockDim.x, nw = NT >> 5, BR = RB * NT;
     const SmemLayout L = smem_layout<CD, PACK, true>(NT, RB, KE);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm);
-    uint32_t *wmask = reinterpret_cast<uint32_t *>(sm + L.mask_off);
-    int32_t *wbin = reinterpret_cast<int32_t *>(sm + L.mask_off + nw * RB * nw * 4);
+    int32_t *cold_flag = reinterpret_cast<int32_t *>(sm + 16); // a value is not tame
+    uint32_t *wmasks = reinterpret_cast<uint32_t *>(sm + L.mask_off); // of even, odd batches
+    int32_t *wbin = reinterpret_cast<int32_t *>(sm + L.mask_off + 2 * nw * RB * nw * 4);
     GeoRec *srec = reinterpret_cast<GeoRec *>(sm + L.rec_off);
     float4 *scol4 = reinterpret_cast<float4 *>(sm + L.col_off);
     float *scol = reinterpret_cast<float *>(sm + L.col_off);
     float *gacc = reinterpret_cast<float *>(sm + L.gacc_off);       // KE > 0: entry rows
     int32_t *touched = reinterpret_cast<int32_t *>(sm + L.touched_off);
-    uint8_t *slot_row = reinterpret_cast<uint8_t *>(sm + L.touched_off); // KE > 0
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int bt = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
+    const CtaPart part = cta_part(a, TS);
+    const int bt = part.bt;
     if (a.masks && !a.masks[bt]) return;
     const TileLoc loc = locate_tile(a, bt);
     const int cam = loc.cam;
     const int ty = loc.tile / loc.TW, tx = loc.tile - ty * loc.TW;
-    const int wpr = a.TS >> 3;
-    const int j = tx * a.TS + (warp % wpr) * 8 + (lane & 7);
-    const int i0 = ty * a.TS + (warp / wpr) * 8 + (lane >> 3) * 2;
+    const int tile_x0 = tx * a.TS + part.x, tile_y0 = ty * a.TS + part.y;
+    const int wpr = TS >> 3;
+    // column lane / 4, rows 2 (lane % 4) + {0, 1} of the warp's 8x8 pixels
+    const int j = tile_x0 + (warp % wpr) * 8 + (lane >> 2);
+    const int i0 = tile_y0 + (warp / wpr) * 8 + (lane & 3) * 2;
     const bool in0 = (i0 < loc.H) && (j < loc.W);
     const bool in1 = (i0 + 1 < loc.H) && (j < loc.W);
     // outside pixels read a clamped pixel, like the reference, and never contribute
@@ -789,12 +1016,9 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
     BwdPair<CD> sp;
     bwd_pair_init<CD>(sp, a, pix0, pix1, in0, in1, bg);
 
-    const int32_t wb = __reduce_max_sync(
-        0xffffffffu, max(in0 ? sp.bin0 : INT32_MIN, in1 ? sp.bin1 : INT32_MIN));
+    const int32_t wb = __reduce_max_sync(0xffffffffu, max(sp.bin0, sp.bin1));
     if (lane == 0) wbin[warp] = wb;
-    if (KE > 0) {
-        for (int t = tid; t < nw * BR; t += NT) slot_row[t] = 0xFF;
-    } else {
+    if (KE == 0) {
         for (int t = tid; t < BR * NV; t += NT) gacc[t] = 0.f;
         for (int t = tid; t < BR; t += NT) touched[t] = 0;
     }
@@ -805,14 +1029,17 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
         mbar_init(&mbar[0], gather ? NT : 1);
         mbar_init(&mbar[1], gather ? NT : 1);
         fence_barrier_init();
+        *cold_flag = 0;
     }
-    __syncthreads();
+    bool cold = __syncthreads_or(MOM && !tame_pixels<CD>(sp));
     int32_t block_bin = INT32_MIN;
     for (int w = 0; w < nw; ++w) block_bin = max(block_bin, wbin[w]);
     const int32_t hi_end = max(rs, min(re, block_bin + 1)); // exclusive upper index
     const int nb = (hi_end - rs + BR - 1) / BR;
 
-    const LaneMasks lm = lane_masks(lane);
+    MomentBasis mb;
+    float *const my_rows = gacc + warp * (KE + 1) * RP;
+    if constexpr (MOM) mb = moment_basis<CD>(lane, my_rows);
     // batch b covers [max(rs, hi_end - (b + 1) BR), hi_end - b BR): back to front
     int issued = 0, waited = 0;
     int32_t ent[RB];
@@ -855,30 +1082,28 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
         const bool ok = mbar_wait_bounded(&mbar[buf], (b >> 1) & 1);
         if (tid == 0 && ok) waited = b + 1;
         const GeoRec *batch = srec + buf * BR;
-        const int32_t gid0 = (tid < cnt) ? batch[tid].gid : 0;
-        const int32_t gid1 = (RB > 1 && tid + NT < cnt) ? batch[tid + NT].gid : 0;
-        // per-slot opacity and beta for the flush (the buffer may be refilled
-        // while other threads still flush)
-        const float op0 = (tid < cnt) ? batch[tid].opac : 0.f;
-        const float be0 = (tid < cnt) ? batch[tid].beta : 0.f;
-        const float op1 = (RB > 1 && tid + NT < cnt) ? batch[tid + NT].opac : 0.f;
-        const float be1 = (RB > 1 && tid + NT < cnt) ? batch[tid + NT].beta : 0.f;
-        const float3 cn0 = (tid < cnt) ? make_float3(batch[tid].cxx, batch[tid].cxy, batch[tid].cyy)
-                                       : make_float3(0.f, 0.f, 0.f);
-        const float3 cn1 = (RB > 1 && tid + NT < cnt)
-                               ? make_float3(batch[tid + NT].cxx, batch[tid + NT].cxy,
-                                             batch[tid + NT].cyy)
-                               : make_float3(0.f, 0.f, 0.f);
-        build_masks<RB>(batch, cnt, lo, NT, nw, wpr, tx * a.TS, ty * a.TS, tid, lane, wmask,
+        uint32_t *wmask = wmasks + (b & 1) * nw * RB * nw;
+        build_masks<RB>(batch, cnt, lo, NT, nw, wpr, tile_x0, tile_y0, tid, lane, wmask,
                         wbin);
         if (!PACK) {
 #pragma unroll
             for (int half = 0; half < RB; ++half) {
                 const int sl = tid + half * NT;
                 if (sl < cnt) {
-                    const float *cp = a.colors + (int64_t)(half ? gid1 : gid0) * CD;
+                    const float *cp = a.colors + (int64_t)batch[sl].gid * CD;
 #pragma unroll
                     for (int k = 0; k < CD; ++k) scol[(buf * BR + sl) * CD + k] = cp[k];
+                }
+            }
+        }
+        if constexpr (MOM) {
+#pragma unroll
+            for (int half = 0; half < RB; ++half) {
+                const int sl = tid + half * NT;
+                if (sl < cnt) {
+                    float col[CD];
+                    load_color<CD, PACK>(scol4, scol, buf * BR + sl, col);
+                    if (!tame_record<CD>(batch[sl], col)) *cold_flag = 1;
                 }
             }
         }
@@ -886,48 +1111,82 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
             if (tid == 0) atomicOr(a.status, DEV_ERR_WAIT_TIMEOUT);
             break;
         }
+        if constexpr (MOM) cold = cold || *cold_flag != 0;
         int rows = 0; // KE > 0: entry rows this warp has filled in this batch
+        uint32_t row = MOM ? mb.first : 0; // this lane's element of the last row filled
+#pragma unroll 1
         for (int k = RB * nw - 1; k >= 0; --k) {
             uint32_t m = wmask[warp * RB * nw + k];
+            if constexpr (MOM) {
+                // as many of the word's records as the list still has rows for
+                uint32_t fit = cold ? 0u : m;
+#pragma unroll 1
+                while (rows + __popc(fit) > KE) fit &= fit - 1;
+                m ^= fit;
+                rows += __popc(fit);
+#pragma unroll 1
+                while (fit) {
+                    const int bit = 31 - __clz(fit);
+                    fit ^= 1u << bit;
+                    const int t = k * 32 + bit;
+                    const GeoRec q = batch[t];
+                    float col[CD];
+                    load_color<CD, PACK>(scol4, scol, buf * BR + t, col);
+                    float2 w, u, ul, gc[CD];
+                    grad_pair<CD, true>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
+                    float d[4];
+                    moment_products<CD>(mb, w, u, ul, gc, d);
+                    row += mb.pitch;
+                    moment_finish(mb, d, row);
+                }
+            }
+#pragma unroll 1
             while (m) {
                 const int bit = 31 - __clz(m);
-                m &= ~(1u << bit);
+                m ^= 1u << bit;
                 const int t = k * 32 + bit;
-                const int32_t idx = lo + t;
                 const GeoRec q = batch[t];
                 float col[CD];
                 load_color<CD, PACK>(scol4, scol, buf * BR + t, col);
+                float2 w, u, ul, gc[CD];
+                const PairGeom pg = grad_pair<CD, false>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
                 float g[NV];
-                grad_pair<CD>(q, col, px, npy, idx, sp, g);
+                pair_sums<CD>(pg, w, u, ul, gc, g);
+                const LaneMasks lm = lane_masks(lane);
                 if constexpr (KE > 0) {
                     const float g0 = g[0], g1 = g[1];
                     g[0] = q.cxx * g0 + q.cxy * g1;
                     g[1] = q.cxy * g0 + q.cyy * g1;
-                    if (rows < KE) {
-                        float *row = gacc + (warp * KE + rows) * NV;
+                    if ((!MOM || cold) && rows < KE) {
+                        float *row = my_rows + (1 + rows) * RP;
                         // every lane of a group holds the same total: all store it
-                        auto put = [row](int u, float tot, bool) { row[u] = tot; };
+                        auto put = [row](int v, float tot, bool) { row[v] = tot; };
                         ReduceChunks<0, NV>::run(g, lm, lane, put);
-                        if (lane == 0) slot_row[warp * BR + t] = (uint8_t)rows;
                         ++rows;
                     } else { // list full: this record's sums go straight to the arrays
-                        auto add = [&](int u, float tot, bool owner) {
+                        auto add = [&](int v, float tot, bool owner) {
                             if (owner && tot != 0.f)
-                                atomicAdd(grad_dst<CD>(a, u, q.gid),
-                                          record_scale(u, q.opac, q.beta, true) * tot);
+                                atomicAdd(grad_dst<CD>(a, v, q.gid),
+                                          record_scale(v, q.opac, q.beta, true) * tot);
                         };
                         ReduceChunks<0, NV>::run(g, lm, lane, add);
                     }
                 } else {
                     float *acc = gacc + t * NV;
-                    auto add = [acc](int u, float tot, bool owner) {
-                        if (owner && tot != 0.f) atomicAdd(&acc[u], tot);
+                    auto add = [acc](int v, float tot, bool owner) {
+                        if (owner && tot != 0.f) atomicAdd(&acc[v], tot);
                     };
                     ReduceChunks<0, NV>::run(g, lm, lane, add);
                     if (lane == 0) touched[t] = 1;
                 }
             }
         }
+        // this thread's slots, read before the barrier: the buffer may be
+        // refilled while other threads still flush
+        GeoRec own[RB];
+#pragma unroll
+        for (int half = 0; half < RB; ++half)
+            if (tid + half * NT < cnt) own[half] = batch[tid + half * NT];
         __syncthreads();
         if constexpr (KE > 0) {
 #pragma unroll
@@ -938,37 +1197,35 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
                 bool any = false;
 #pragma unroll
                 for (int u = 0; u < NV; ++u) sum[u] = 0.f;
+#pragma unroll 1
                 for (int w = 0; w < nw; ++w) {
-                    const int r = slot_row[w * BR + sl];
-                    if (r == 0xFF) continue;
-                    slot_row[w * BR + sl] = 0xFF;
+                    // the slot's row: the set bits after it in the warp's mask
+                    const uint32_t *mw = wmask + w * RB * nw;
+                    const uint32_t after = mw[sl >> 5] >> (sl & 31);
+                    if (!(after & 1u)) continue;
+                    int r = __popc(after) - 1;
+#pragma unroll 1
+                    for (int k = (sl >> 5) + 1; k < RB * nw; ++k) r += __popc(mw[k]);
+                    if (r >= KE) continue; // went straight to the arrays
                     any = true;
-                    const float *row = gacc + (w * KE + r) * NV;
+                    const float *row = gacc + (w * (KE + 1) + 1 + r) * RP;
+                    if (MOM && !cold) {
+                        if constexpr (MOM)
+                            add_moments<CD>(
+                                row, own[half].x - (float)(tile_x0 + (w % wpr) * 8 + 4),
+                                own[half].y - (float)(tile_y0 + (w / wpr) * 8 + 4), sum);
+                    } else {
 #pragma unroll
-                    for (int u = 0; u < NV; ++u) sum[u] += row[u];
+                        for (int u = 0; u < NV; ++u) sum[u] += row[u];
+                    }
                 }
                 if (!any) continue;
-                const int64_t gg = half ? gid1 : gid0;
-                const float op = half ? op1 : op0, be = half ? be1 : be0;
-#pragma unroll
-                for (int u = 0; u < NV; ++u) sum[u] *= record_scale(u, op, be, true);
-                if (NV <= GRAD_ROW && a.v_rows) {
-                    // three 16-byte vector atomics per row instead of NV scalar ones
-                    float4 *row = reinterpret_cast<float4 *>(a.v_rows + gg * GRAD_ROW);
-#pragma unroll
-                    for (int c = 0; c < (NV + 3) / 4; ++c) {
-                        float4 v;
-                        v.x = sum[4 * c];
-                        v.y = 4 * c + 1 < NV ? sum[(4 * c + 1) % NV] : 0.f;
-                        v.z = 4 * c + 2 < NV ? sum[(4 * c + 2) % NV] : 0.f;
-                        v.w = 4 * c + 3 < NV ? sum[(4 * c + 3) % NV] : 0.f;
-                        atomicAdd(row + c, v);
-                    }
-                } else {
-#pragma unroll
-                    for (int u = 0; u < NV; ++u)
-                        if (sum[u] != 0.f) atomicAdd(grad_dst<CD>(a, u, gg), sum[u]);
+                if (MOM && !cold) {
+                    const float s0 = sum[0], s1 = sum[1];
+                    sum[0] = own[half].cxx * s0 + own[half].cxy * s1;
+                    sum[1] = own[half].cxy * s0 + own[half].cyy * s1;
                 }
+                add_record<CD>(a, own[half], sum);
             }
             continue;
         }
@@ -976,17 +1233,15 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_bwd_kernel(
         for (int half = 0; half < RB; ++half) {
             const int sl = tid + half * NT;
             if (sl < cnt && touched[sl]) {
-                const int64_t gg = half ? gid1 : gid0;
-                const float op = half ? op1 : op0, be = half ? be1 : be0;
-                const float3 cn = half ? cn1 : cn0;
+                const GeoRec &r = own[half];
                 float *ga = gacc + sl * NV;
-                const float f2 = -2.f * op * be;
-                const float m0 = f2 * (cn.x * ga[0] + cn.y * ga[1]);
-                const float m1 = f2 * (cn.y * ga[0] + cn.z * ga[1]);
+                const float f2 = -2.f * r.opac * r.beta;
+                const float m0 = f2 * (r.cxx * ga[0] + r.cxy * ga[1]);
+                const float m1 = f2 * (r.cxy * ga[0] + r.cyy * ga[1]);
 #pragma unroll
                 for (int u = 0; u < NV; ++u) {
-                    const float val = u == 0 ? m0 : u == 1 ? m1 : ga[u] * record_scale(u, op, be);
-                    if (val != 0.f) atomicAdd(grad_dst<CD>(a, u, gg), val);
+                    const float val = u == 0 ? m0 : u == 1 ? m1 : ga[u] * record_scale(u, r.opac, r.beta);
+                    if (val != 0.f) atomicAdd(grad_dst<CD>(a, u, r.gid), val);
                     ga[u] = 0.f;
                 }
                 touched[sl] = 0;
@@ -1037,11 +1292,10 @@ static int launch_pack(int64_t T, int64_t n_prims, const int32_t *fl, const floa
 // (16 x 16 pixels and smaller), selected process-wide by
 // ubs_set_blend_variant.  The forward's trade records per staged batch (RB)
 // against CTAs per SM (MINB, the register bound it implies); the backward's
-// the register bound and the accumulation scheme (see smem_layout) --
+// trade the register bound against warps per SM --
 //   forward:  0: RB 2, 8 CTAs/SM;  1: RB 1, 10 CTAs/SM;  2: RB 2, 6 CTAs/SM
-//   backward: 0: RB 1, 8 CTAs/SM, per-warp row lists of 64 entries;
-//             1: the same at 7 CTAs/SM (72 registers);
-//             2: RB 1, 8 CTAs/SM, shared accumulators with shared atomics
+//   backward: 0: 8 CTAs/SM, 6 for small grids (see launch_blend);
+//             1: 7 CTAs/SM (72 registers);  2: 6 CTAs/SM (80 registers)
 // Every variant computes the same images; the backward's gradient sums are
 // the same up to the order of their additions.
 // A warp that visits more than KE_SMALL records of one 128-record batch adds
@@ -1049,50 +1303,77 @@ static int launch_pack(int64_t T, int64_t n_prims, const int32_t *fl, const floa
 // 64 of 5.6M visits do.
 std::atomic<int> g_blend_fwd_variant{0}, g_blend_bwd_variant{0};
 constexpr int kBlendVariants = 3;
-constexpr int KE_SMALL = 64; // backward entry rows per warp in tiles of at most 128 threads
+// Backward grids of fewer blocks than this (of 128 threads) run at 6 CTAs per
+// SM: with few waves the unspilled kernel is faster (1,900 blocks: 67.0 against
+// 69.8 us; 3,600: 258.6 against 250.4 us).
+constexpr int BWD_SMALL_GRID = 152 * 16;
+// Below one wave of 16 x 16 squares each is cut into four one-warp CTAs, which
+// wait for no other warp and spread over more SMs (130 tiles: 82.1 -> 77.2 us;
+// 1,900 tiles: no difference; 8,160: 955 -> 978 us).
+constexpr int BWD_ONE_WAVE = 152 * 6;
+constexpr int KE_SMALL = 64; // backward entry rows per warp
 
 template <int CD, bool BWD>
 static int launch_blend(RasterArgs &a, cudaStream_t st) {
     constexpr bool PACK = CD <= 4;
-    const int NT = a.TS * a.TS / 2; // two pixels per thread
-    // Tiles of at most 128 threads with packed colours run 8 CTAs per SM (7
-    // for the backward of 4 channels; wider colour rows need more registers),
-    // the backward in batches of NT records to fit its shared memory.
+    // A CTA works on at most 16 x 16 pixels (two per thread) where colours are
+    // packed: larger tiles are cut into squares of 16 x 16 (32) or 8 x 8 (24)
+    // whose CTAs share the tile's records (backward; 1M primitives at 1080p,
+    // tiles of 32: 1.85 -> 1.08 ms).  Wider colour rows need more registers
+    // and shared memory and keep one CTA per tile.
+    const bool cut = PACK && BWD;
+    const int64_t cta16 = (int64_t)a.n_buckets * (a.TS / 16) * (a.TS / 16);
+    const int edge = !cut ? a.TS : a.TS % 16 != 0 || cta16 < BWD_ONE_WAVE ? 8 : 16;
+    a.sub = a.TS / edge;
+    const int NT = edge * edge / 2;
     const bool small = PACK && NT <= 128;
     const int variant = (small && CD == 3 && !a.pair_count)
                             ? (BWD ? g_blend_bwd_variant.load() : g_blend_fwd_variant.load())
                             : 0;
     int RB = (small && BWD) ? 1 : 2;
     if (!BWD && variant == 1) RB = 1;
-    const int KE = (BWD && small && !(CD == 3 && variant == 2)) ? KE_SMALL : 0;
+    const int KE = BWD && small ? KE_SMALL : 0;
     const SmemLayout L = smem_layout<CD, PACK, BWD>(NT, RB, KE);
     if (L.total > 227 * 1024)
         return set_error(UBS_ERR_UNSUPPORTED, "raster: tile_size %d with %d channels needs %d B "
                                               "of shared memory", a.TS, CD, L.total);
-    const unsigned nblocks = (unsigned)a.n_buckets;
+    const int64_t nblocks = (int64_t)a.n_buckets * a.sub * a.sub;
     if (nblocks == 0) return UBS_OK;
+    UBS_REQUIRE(nblocks < (1ll << 31), "raster: %lld thread blocks", (long long)nblocks);
     void (*k)(RasterArgs) = nullptr;
-    if constexpr (CD == 3) {
-        if (small && variant == 1)
-            k = BWD ? raster_bwd_kernel<3, true, 1, 7, KE_SMALL>
-                    : raster_fwd_kernel<3, true, false, 1, 10>;
-        else if (small && variant == 2)
-            k = BWD ? raster_bwd_kernel<3, true, 1, 8, 0> : raster_fwd_kernel<3, true, false, 2, 6>;
+    if constexpr (BWD && PACK) {
+        // 8 CTAs of 128 threads per SM bound a thread to 64 registers (24
+        // bytes spilled), 6 leave it 80 and spill nothing
+        constexpr int C16 = CD < 4 ? 8 : 7;
+        const bool few = nblocks < BWD_SMALL_GRID * (128 / NT);
+        const int per_sm = variant == 1 ? 7 : variant == 2 || few ? 6 : C16;
+        if (edge == 8)
+            k = per_sm == 6 ? raster_bwd_kernel<CD, true, 8, 1, 24, KE_SMALL>
+                            : raster_bwd_kernel<CD, true, 8, 1, 28, KE_SMALL>;
+        else
+            k = per_sm == 6   ? raster_bwd_kernel<CD, true, 16, 1, 6, KE_SMALL>
+                : per_sm == 7 ? raster_bwd_kernel<CD, true, 16, 1, 7, KE_SMALL>
+                              : raster_bwd_kernel<CD, true, 16, 1, C16, KE_SMALL>;
+    } else if constexpr (BWD) {
+        k = raster_bwd_kernel<CD, false, 0, 2, 1, 0>;
+    } else {
+        if constexpr (CD == 3) {
+            if (small && variant == 1) k = raster_fwd_kernel<3, true, false, 1, 10>;
+            else if (small && variant == 2) k = raster_fwd_kernel<3, true, false, 2, 6>;
+        }
+        if constexpr (PACK) {
+            if (small && !k)
+                k = a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 8>
+                                 : raster_fwd_kernel<CD, PACK, false, 2, 8>;
+        }
+        if (!k)
+            k = a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 1>
+                             : raster_fwd_kernel<CD, PACK, false, 2, 1>;
     }
-    if constexpr (PACK) {
-        if (small && !k)
-            k = BWD ? raster_bwd_kernel<CD, PACK, 1, (CD < 4 ? 8 : 7), KE_SMALL>
-                    : (a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 8>
-                                    : raster_fwd_kernel<CD, PACK, false, 2, 8>);
-    }
-    if (!k)
-        k = BWD ? raster_bwd_kernel<CD, PACK, 2, 1, 0>
-                : (a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 1>
-                                : raster_fwd_kernel<CD, PACK, false, 2, 1>);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) !=
         cudaSuccess)
         return check_launch("raster smem attribute");
-    UBS_TIMED(BWD ? "raster_bwd" : "raster_fwd", st, k<<<nblocks, NT, L.total, st>>>(a));
+    UBS_TIMED(BWD ? "raster_bwd" : "raster_fwd", st, k<<<(unsigned)nblocks, NT, L.total, st>>>(a));
     note_launch();
     return check_launch(BWD ? "raster_bwd" : "raster_fwd");
 }

@@ -8,8 +8,7 @@ fixes how many CTAs fit on an SM.  It also changes the intersection count
 (smaller tiles: more buckets, fewer wasted pixels per record).  For tiles up
 to 16 x 16 the blend kernels are compiled in variants (ubs_set_blend_variant,
 for the forward and the backward separately: the forward's trade records per
-staged batch against CTAs per SM, the backward's its register bound and how a
-batch's per-record gradient sums are accumulated).  Which point is fastest depends on the
+staged batch against CTAs per SM, the backward's its register bound).  Which point is fastest depends on the
 resolution mix and the scene's footprint sizes, so it is measured: each
 candidate runs the caller's step a few times after a warm-up, timed with CUDA
 events on the launching stream, and the winner is cached under a
