@@ -16,6 +16,7 @@ a time.
     images = views.split(colors)                   # list of [H, W, 3]
 """
 import ctypes
+import gc
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -393,13 +394,21 @@ class GraphedStep:
             before_capture()
         self.graph = torch.cuda.CUDAGraph()
         n0 = L.query("ubs_launch_count")
-        with torch.cuda.graph(self.graph):
-            if optimizer is not None:
-                for v in params.values():
-                    v.grad.zero_()
-            self.loss = self._body()
-            if optimizer is not None:
-                optimizer.launch()
+        # a cycle collection inside the capture may destroy an older graph,
+        # which is not permitted there and fails this capture
+        collecting = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.graph(self.graph):
+                if optimizer is not None:
+                    for v in params.values():
+                        v.grad.zero_()
+                self.loss = self._body()
+                if optimizer is not None:
+                    optimizer.launch()
+        finally:
+            if collecting:
+                gc.enable()
         # library kernels in the graph (each replay launches them all)
         self.launches_per_replay = int(L.query("ubs_launch_count") - n0)
 
