@@ -47,7 +47,7 @@ struct RasterArgs {
     int C, W, H, TS, TW, TH, n_tiles;
     int64_t n_isects, n_prims; // n_prims = C * N
     const int32_t *offsets;
-    const GeoRec *recs;
+    const float4 *recs_a, *recs_b; // first and second halves of the sorted GeoRecs
     const float4 *rcols; // packed colours (channels <= 4) or nullptr
     const float *colors; // [C*N, CD], gathered when rcols == nullptr
     const float *bg;
@@ -82,7 +82,7 @@ struct RasterArgs {
     // gather mode (fused scene path, packed colours): records are copied per
     // batch from the per-entry tables, addressed by the low word of the
     // sorted (depth, entry) keys, instead of from sorted copies
-    const uint64_t *keys;       // nullptr: sorted copies in recs / rcols
+    const uint64_t *keys;       // nullptr: sorted copies in recs_a, recs_b, rcols
     const GeoRec *entry_recs;   // [C*N] one record per (view, primitive) entry
     const float4 *prim_cols;    // [N] packed colour per primitive
     int64_t n_per_view;         // N
@@ -148,8 +148,9 @@ template <int CD, bool PACK>
 __global__ void pack_records_kernel(int64_t T, int64_t n_prims, const int32_t *__restrict__ fl,
                                     const float *__restrict__ m2, const float *__restrict__ cn,
                                     const float *__restrict__ op, const float *__restrict__ be,
-                                    const float *__restrict__ col, GeoRec *__restrict__ recs,
-                                    float4 *__restrict__ rcols, uint32_t *status) {
+                                    const float *__restrict__ col, float4 *__restrict__ recs_a,
+                                    float4 *__restrict__ recs_b, float4 *__restrict__ rcols,
+                                    uint32_t *status) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < T; i += stride) {
         int32_t g = fl[i];
@@ -166,9 +167,8 @@ __global__ void pack_records_kernel(int64_t T, int64_t n_prims, const int32_t *_
         b.y = cn[3 * (int64_t)g + 1];
         b.z = cn[3 * (int64_t)g + 2];
         b.w = __int_as_float(g);
-        float4 *dst = reinterpret_cast<float4 *>(recs + i);
-        dst[0] = a;
-        dst[1] = b;
+        recs_a[i] = a;
+        recs_b[i] = b;
         if (PACK) {
             float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
             const float *cp = col + (int64_t)g * CD;
@@ -232,6 +232,24 @@ __host__ __device__ inline SmemLayout smem_layout(int NT, int RB = 2, int KE = 0
         L.total = L.touched_off + (BWD ? BR * 4 : 0);
     }
     return L;
+}
+
+// Staged records: the first and the second 16 bytes of a buffer pair's GeoRecs
+// and the packed colours are three arrays of `pitch` elements each, one behind
+// the other, so that one slot offset addresses all three and lanes that read
+// or copy neighbouring slots touch neighbouring banks.
+__device__ __forceinline__ GeoRec staged_rec(const float4 *batch, int pitch, int slot) {
+    const float4 a = batch[slot], b = batch[pitch + slot];
+    GeoRec r;
+    r.x = a.x;
+    r.y = a.y;
+    r.opac = a.z;
+    r.beta = a.w;
+    r.cxx = b.x;
+    r.cxy = b.y;
+    r.cyy = b.z;
+    r.gid = __float_as_int(b.w);
+    return r;
 }
 
 // Whether the ellipse {d : d^T Q d < 1} of a record (Q its conic, d = centre -
@@ -299,8 +317,8 @@ __device__ __forceinline__ void load_entries(const RasterArgs &a, int32_t bs, in
 }
 
 template <int RB>
-__device__ __forceinline__ void gather_batch(const RasterArgs &a, GeoRec *srec, float4 *scol4,
-                                             uint64_t *mbar, int BR, int buf, int cnt,
+__device__ __forceinline__ void gather_batch(const RasterArgs &a, float4 *srec, uint64_t *mbar,
+                                             int BR, int buf, int cnt,
                                              const int32_t (&ent)[RB], int64_t lo_e,
                                              int64_t hi_e, int NT, int tid) {
 #pragma unroll
@@ -315,10 +333,10 @@ __device__ __forceinline__ void gather_batch(const RasterArgs &a, GeoRec *srec, 
                 e = min(max(e, lo_e), hi_e);
             }
             const char *src = reinterpret_cast<const char *>(a.entry_recs + e);
-            char *dst = reinterpret_cast<char *>(srec + buf * BR + s);
+            float4 *dst = srec + buf * BR + s;
             cp_async16(dst, src);
-            cp_async16(dst + 16, src + 16);
-            cp_async16(scol4 + buf * BR + s, a.prim_cols + (e - lo_e));
+            cp_async16(dst + 2 * BR, src + 16);
+            cp_async16(dst + 4 * BR, a.prim_cols + (e - lo_e));
         }
     }
     cp_async_arrive(&mbar[buf]);
@@ -326,33 +344,35 @@ __device__ __forceinline__ void gather_batch(const RasterArgs &a, GeoRec *srec, 
 
 // Issues the bulk copies of batch [bs, bs+cnt) into buffer `buf` (thread 0).
 template <bool PACK>
-__device__ __forceinline__ void issue_batch(const RasterArgs &a, GeoRec *srec, float4 *scol4,
-                                            uint64_t *mbar, int BR, int buf, int32_t bs,
-                                            int cnt) {
+__device__ __forceinline__ void issue_batch(const RasterArgs &a, float4 *srec, uint64_t *mbar,
+                                            int BR, int buf, int32_t bs, int cnt) {
     fence_proxy_async_smem();
     const uint32_t bytes = (uint32_t)cnt * (32u + (PACK ? 16u : 0u));
     mbar_arrive_expect_tx(&mbar[buf], bytes);
-    bulk_g2s(srec + buf * BR, a.recs + bs, (uint32_t)cnt * 32u, &mbar[buf]);
-    if (PACK) bulk_g2s(scol4 + buf * BR, a.rcols + bs, (uint32_t)cnt * 16u, &mbar[buf]);
+    float4 *dst = srec + buf * BR;
+    bulk_g2s(dst, a.recs_a + bs, (uint32_t)cnt * 16u, &mbar[buf]);
+    bulk_g2s(dst + 2 * BR, a.recs_b + bs, (uint32_t)cnt * 16u, &mbar[buf]);
+    if (PACK) bulk_g2s(dst + 4 * BR, a.rcols + bs, (uint32_t)cnt * 16u, &mbar[buf]);
 }
 
-// Per-batch culling masks.  Thread tid describes batch slots tid + h NT
-// (h < RB); for every warp w one ballot per slot gives 32 bits of w's
-// RB*nw-word mask (word k covers slots 32k .. 32k+31, so ascending bits are
-// front to back).  limit[w] (backward) drops records past warp w's last
-// contributor.
-template <int RB = 2>
-__device__ __forceinline__ void build_masks(const GeoRec *batch, int cnt, int lo, int NT, int nw,
+// Per-batch culling masks.  Thread tid describes one batch slot of every NT;
+// for every warp w one ballot per slot gives 32 bits of w's RB*nw-word mask
+// (word k covers slots 32k .. 32k+31).  FLIP: the highest bit is the first
+// slot (forward), else the last (backward), so that either finds its next
+// record with one find-leading-one.  limit[w] (backward) drops records past
+// warp w's last contributor.
+template <int RB, bool FLIP>
+__device__ __forceinline__ void build_masks(const float4 *batch, int pitch, int cnt, int lo, int NT, int nw,
                                             int wpr, int tile_x0, int tile_y0, int tid, int lane,
                                             uint32_t *wmask, const int32_t *limit) {
 #pragma unroll
     for (int half = 0; half < RB; ++half) {
-        const int s = tid + half * NT;
+        const int s = (FLIP ? tid ^ 31 : tid) + half * NT;
         const bool valid = s < cnt;
         GeoRec r;
         bool pd = false;
         if (valid) {
-            r = batch[s];
+            r = staged_rec(batch, pitch, s);
             pd = conic_pd(r);
         }
         const int word = s >> 5;
@@ -385,79 +405,86 @@ __device__ __forceinline__ void load_color(const float4 *scol4, const float *sco
 // One front-to-back blend step of a thread's two pixels (column px, rows py0
 // and py0 + 1) over record q (rasterize_to_pixels_fwd.cu:139-171): skip when
 // sigma is outside [0, 1), alpha = min(0.999, opacity (1 - sigma)^beta), stop
-// (exclusively) once the transmittance would reach 1e-4.  The pixel pair is
-// evaluated two-wide with Blackwell's packed FP32x2 instructions (__ffma2_rn,
-// __fadd2_rn, __fmul2_rn: per component the same rounding as the scalar
-// operations); (1 - sigma)^beta is formed as 2^(beta log2(1 - sigma)).  The
-// updates are select-based so that a warp issues them once for both pixels
-// and all lanes; lanes whose record is skipped evaluate dummies (NaN where
+// (exclusively) once the transmittance would reach 1e-4; (1 - sigma)^beta is
+// formed as 2^(beta log2(1 - sigma)).  A pixel that has stopped (or lies
+// outside the image) keeps its transmittance negated, so that no later record
+// passes the 1e-4 test: no predicate per pixel has to be carried, and a step
+// takes one select each for the weight, the transmittance, its sign and the
+// last contributor.  The updates are select-based so that a warp issues them
+// for all lanes; lanes whose record is skipped evaluate dummies (NaN where
 // sigma >= 1) that the selects discard.  Records no lane can use are
 // evaluated the same way rather than skipped after a warp vote: under 1% of
-// the culled visits are such.
+// the culled visits are such.  Packed FP32x2 instructions only where both
+// operands are pairs already: a record's broadcast value would have to be
+// copied into a pair first.  With predicates carried per pixel, packed
+// instructions throughout and a vote per record the kernel took 0.479 ms (1M
+// primitives at 1080p, ALU pipe 69%, 86 warp instructions per visit), this way
+// 0.418 ms (81).
 template <int CD, bool COUNT>
 __device__ __forceinline__ void blend_pair(const GeoRec &q, const float (&col)[CD], float px,
                                            float2 npy, float2 &T, float2 (&acc)[CD],
-                                           int32_t &cur0, int32_t &cur1, bool &d0, bool &d1,
-                                           int32_t idx, uint32_t &n_contrib, int32_t &term0,
-                                           int32_t &term1) {
+                                           int32_t &cur0, int32_t &cur1, int32_t idx,
+                                           uint32_t &n_contrib, int32_t &term0, int32_t &term1) {
     const float dx = q.x - px;
-    const float2 dy = __fadd2_rn(make_float2(q.y, q.y), npy);
+    const float2 dy = make_float2(q.y + npy.x, q.y + npy.y);
     const float A = q.cxx * dx * dx;
     const float B = 2.f * q.cxy * dx;
-    float2 s = __fmul2_rn(make_float2(q.cyy, q.cyy), dy);
-    s = __ffma2_rn(s, dy, make_float2(A, A));
-    s = __ffma2_rn(make_float2(B, B), dy, s);
-    const bool v0 = !d0 && !(s.x < 0.f || s.x >= 1.f);
-    const bool v1 = !d1 && !(s.y < 0.f || s.y >= 1.f);
-    const float2 om = __ffma2_rn(s, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
-    const float2 l = make_float2(__log2f(om.x), __log2f(om.y));
-    const float2 e = __fmul2_rn(l, make_float2(q.beta, q.beta));
-    const float2 p = make_float2(exp2f(e.x), exp2f(e.y));
-    float2 a = __fmul2_rn(make_float2(q.opac, q.opac), p);
-    a.x = fminf(0.999f, a.x);
-    a.y = fminf(0.999f, a.y);
-    const float2 n = __fmul2_rn(T, __ffma2_rn(a, make_float2(-1.f, -1.f), make_float2(1.f, 1.f)));
-    const bool t0 = v0 && n.x <= 1e-4f, t1 = v1 && n.y <= 1e-4f;
-    const bool b0 = v0 && !t0, b1 = v1 && !t1;
-    d0 = d0 || t0;
-    d1 = d1 || t1;
+    float2 s;
+    s.x = fmaf(B, dy.x, fmaf(__fmul_rn(q.cyy, dy.x), dy.x, A));
+    s.y = fmaf(B, dy.y, fmaf(__fmul_rn(q.cyy, dy.y), dy.y, A));
+    const bool v0 = !(s.x < 0.f) & !(s.x >= 1.f);
+    const bool v1 = !(s.y < 0.f) & !(s.y >= 1.f);
+    const float2 p = make_float2(exp2f(__log2f(1.f - s.x) * q.beta),
+                                 exp2f(__log2f(1.f - s.y) * q.beta));
+    const float2 a = make_float2(fminf(0.999f, q.opac * p.x), fminf(0.999f, q.opac * p.y));
+    const float2 n = __fmul2_rn(T, make_float2(1.f - a.x, 1.f - a.y));
     float2 w = __fmul2_rn(a, T);
+    const bool b0 = v0 & !(n.x <= 1e-4f), b1 = v1 & !(n.y <= 1e-4f);
+    if (COUNT) {
+        n_contrib += (uint32_t)b0 + (uint32_t)b1;
+        term0 = v0 && !b0 && T.x > 0.f ? idx : term0;
+        term1 = v1 && !b1 && T.y > 0.f ? idx : term1;
+    }
     w.x = b0 ? w.x : 0.f;
     w.y = b1 ? w.y : 0.f;
 #pragma unroll
-    for (int k = 0; k < CD; ++k) acc[k] = __ffma2_rn(make_float2(col[k], col[k]), w, acc[k]);
+    for (int k = 0; k < CD; ++k) {
+        acc[k].x = fmaf(col[k], w.x, acc[k].x);
+        acc[k].y = fmaf(col[k], w.y, acc[k].y);
+    }
+    T.x = v0 ? -fabsf(T.x) : T.x;
+    T.y = v1 ? -fabsf(T.y) : T.y;
     T.x = b0 ? n.x : T.x;
     T.y = b1 ? n.y : T.y;
     cur0 = b0 ? idx : cur0;
     cur1 = b1 ? idx : cur1;
-    if (COUNT) {
-        n_contrib += (uint32_t)b0 + (uint32_t)b1;
-        term0 = t0 ? idx : term0;
-        term1 = t1 ? idx : term1;
-    }
 }
 
 // --------------------------------------------------------------- forward
-// MINB > 1: tiles of at most 128 threads, MINB CTAs per SM.
-template <int CD, bool PACK, bool COUNT, int RB, int MINB>
-__global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(RasterArgs a) {
+// TSZ: edge of a CTA's pixels, 8 or 16, or 0 for a whole tile of a.TS; MINB
+// CTAs per SM.
+template <int CD, bool PACK, bool COUNT, int TSZ, int RB, int MINB>
+__global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_fwd_kernel(RasterArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
-    const int NT = blockDim.x, nw = NT >> 5, BR = RB * NT;
+    const int TS = TSZ ? TSZ : a.TS;
+    const int NT = TSZ ? TSZ * TSZ / 2 : (int)blockDim.x, nw = NT >> 5, BR = RB * NT;
     const SmemLayout L = smem_layout<CD, PACK, false>(NT, RB);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm);
     uint32_t *wmask = reinterpret_cast<uint32_t *>(sm + L.mask_off);
-    GeoRec *srec = reinterpret_cast<GeoRec *>(sm + L.rec_off);
-    float4 *scol4 = reinterpret_cast<float4 *>(sm + L.col_off);
+    float4 *srec = reinterpret_cast<float4 *>(sm + L.rec_off); // see staged_rec
+    const int pitch = 2 * BR;
     float *scol = reinterpret_cast<float *>(sm + L.col_off);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int bt = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
+    const CtaPart part = cta_part(a, TS);
+    const int bt = part.bt;
     const TileLoc loc = locate_tile(a, bt);
     const int cam = loc.cam;
     const int ty = loc.tile / loc.TW, tx = loc.tile - ty * loc.TW;
-    const int wpr = a.TS >> 3;
-    const int j = tx * a.TS + (warp % wpr) * 8 + (lane & 7);
-    const int i0 = ty * a.TS + (warp / wpr) * 8 + (lane >> 3) * 2;
+    const int tile_x0 = tx * a.TS + part.x, tile_y0 = ty * a.TS + part.y;
+    const int wpr = TS >> 3;
+    const int j = tile_x0 + (warp % wpr) * 8 + (lane & 7);
+    const int i0 = tile_y0 + (warp / wpr) * 8 + (lane >> 3) * 2;
     const bool in0 = (i0 < loc.H) && (j < loc.W);
     const bool in1 = (i0 + 1 < loc.H) && (j < loc.W);
     const int64_t pix0 = loc.pix_base + (int64_t)i0 * loc.W + j;
@@ -484,14 +511,14 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
 
     const float px = (float)j + 0.5f, py0 = (float)i0 + 0.5f, py1 = py0 + 1.f;
     const float2 npy = make_float2(-py0, -py1);
-    float2 T = make_float2(1.0f, 1.0f);
+    // negative once a pixel has stopped
+    float2 T = make_float2(in0 ? 1.0f : -1.0f, in1 ? 1.0f : -1.0f);
     int32_t cur0 = 0, cur1 = 0;
     uint32_t n_contrib = 0;
     int32_t term0 = -1, term1 = -1; // COUNT: record at which a pixel terminated
     float2 acc[CD];
 #pragma unroll
     for (int k = 0; k < CD; ++k) acc[k] = make_float2(0.f, 0.f);
-    bool d0 = !in0, d1 = !in1;
 
     if (nb > 0) {
         const bool gather = PACK && a.keys != nullptr;
@@ -507,12 +534,12 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
         int issued = 0, waited = 0;
         if (gather) {
             load_entries<RB>(a, rs, min(BR, re - rs), NT, tid, ent);
-            gather_batch<RB>(a, srec, scol4, mbar, BR, 0, min(BR, re - rs), ent, lo_e, hi_e, NT,
+            gather_batch<RB>(a, srec, mbar, BR, 0, min(BR, re - rs), ent, lo_e, hi_e, NT,
                              tid);
             if (nb > 1) load_entries<RB>(a, rs + BR, min(BR, re - rs - BR), NT, tid, ent);
             issued = 1;
         } else if (tid == 0) {
-            issue_batch<PACK>(a, srec, scol4, mbar, BR, 0, rs, min(BR, re - rs));
+            issue_batch<PACK>(a, srec, mbar, BR, 0, rs, min(BR, re - rs));
             issued = 1;
         }
         for (int b = 0; b < nb; ++b) {
@@ -522,27 +549,27 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
             if (b + 1 < nb) {
                 const int32_t bn = bs + BR;
                 if (gather) {
-                    gather_batch<RB>(a, srec, scol4, mbar, BR, buf ^ 1, min(BR, re - bn), ent,
+                    gather_batch<RB>(a, srec, mbar, BR, buf ^ 1, min(BR, re - bn), ent,
                                      lo_e, hi_e, NT, tid);
                     if (b + 2 < nb)
                         load_entries<RB>(a, bn + BR, min(BR, re - bn - BR), NT, tid, ent);
                     issued = b + 2;
                 } else if (tid == 0) {
-                    issue_batch<PACK>(a, srec, scol4, mbar, BR, buf ^ 1, bn, min(BR, re - bn));
+                    issue_batch<PACK>(a, srec, mbar, BR, buf ^ 1, bn, min(BR, re - bn));
                     issued = b + 2;
                 }
             }
             const bool ok = mbar_wait_bounded(&mbar[buf], (b >> 1) & 1);
             if (tid == 0 && ok) waited = b + 1;
-            const GeoRec *batch = srec + buf * BR;
-            build_masks<RB>(batch, cnt, 0, NT, nw, wpr, tx * a.TS, ty * a.TS, tid, lane, wmask,
+            const float4 *batch = srec + buf * BR;
+            build_masks<RB, true>(batch, pitch, cnt, 0, NT, nw, wpr, tile_x0, tile_y0, tid, lane, wmask,
                             nullptr);
             if (!PACK) {
 #pragma unroll
                 for (int half = 0; half < RB; ++half) {
                     const int s = tid + half * NT;
                     if (s < cnt) {
-                        const float *cp = a.colors + (int64_t)batch[s].gid * CD;
+                        const float *cp = a.colors + (int64_t)__float_as_int(batch[pitch + s].w) * CD;
 #pragma unroll
                         for (int k = 0; k < CD; ++k) scol[(buf * BR + s) * CD + k] = cp[k];
                     }
@@ -550,30 +577,27 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
             }
             if (__syncthreads_or(!ok)) {
                 if (tid == 0) atomicOr(a.status, DEV_ERR_WAIT_TIMEOUT);
-                d0 = d1 = true;
                 break;
             }
-            if (!__all_sync(0xffffffffu, d0 && d1)) {
-                bool warp_done = false;
-                for (int k = 0; k < RB * nw && !warp_done; ++k) {
-                    uint32_t m = wmask[warp * RB * nw + k];
-                    while (m) {
-                        const int bit = __ffs(m) - 1;
-                        m &= m - 1;
-                        const int t = k * 32 + bit;
-                        const GeoRec q = batch[t];
-                        float col[CD];
-                        load_color<CD, PACK>(scol4, scol, buf * BR + t, col);
-                        blend_pair<CD, COUNT>(q, col, px, npy, T, acc, cur0, cur1, d0, d1,
-                                              bs + t, n_contrib, term0, term1);
-                        if (__all_sync(0xffffffffu, d0 && d1)) {
-                            warp_done = true;
-                            break;
-                        }
-                    }
+            // a warp whose pixels have all stopped looks up once per mask word:
+            // a vote per record costs more than the rest of the word
+#pragma unroll 1
+            for (int k = 0; k < RB * nw; ++k) {
+                if (__all_sync(0xffffffffu, (T.x < 0.f) & (T.y < 0.f))) break;
+                uint32_t m = wmask[warp * RB * nw + k];
+#pragma unroll 1
+                while (m) {
+                    const int bit = 31 - __clz(m);
+                    m ^= 1u << bit;
+                    const int t = k * 32 + 31 - bit;
+                    const GeoRec q = staged_rec(batch, pitch, t);
+                    float col[CD];
+                    load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, t, col);
+                    blend_pair<CD, COUNT>(q, col, px, npy, T, acc, cur0, cur1, bs + t, n_contrib,
+                                          term0, term1);
                 }
             }
-            if (__syncthreads_count(d0 && d1) == NT) break;
+            if (__syncthreads_and((T.x < 0.f) & (T.y < 0.f))) break;
         }
         // no copy may still target this CTA's shared memory at exit
         if (gather) cp_async_wait_all();
@@ -602,6 +626,7 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 512, MINB) raster_fwd_kernel(
         if (lane == 0 && we) atomicAdd(a.pair_count + 1, (unsigned long long)we);
         if (lane == 0 && wb) atomicAdd(a.pair_count + 2, (unsigned long long)wb);
     }
+    T = make_float2(fabsf(T.x), fabsf(T.y));
     if (in0) {
         a.out_a[pix0] = 1.0f - T.x;
 #pragma unroll
@@ -979,8 +1004,8 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
     int32_t *cold_flag = reinterpret_cast<int32_t *>(sm + 16); // a value is not tame
     uint32_t *wmasks = reinterpret_cast<uint32_t *>(sm + L.mask_off); // of even, odd batches
     int32_t *wbin = reinterpret_cast<int32_t *>(sm + L.mask_off + 2 * nw * RB * nw * 4);
-    GeoRec *srec = reinterpret_cast<GeoRec *>(sm + L.rec_off);
-    float4 *scol4 = reinterpret_cast<float4 *>(sm + L.col_off);
+    float4 *srec = reinterpret_cast<float4 *>(sm + L.rec_off); // see staged_rec
+    const int pitch = 2 * BR;
     float *scol = reinterpret_cast<float *>(sm + L.col_off);
     float *gacc = reinterpret_cast<float *>(sm + L.gacc_off);       // KE > 0: entry rows
     int32_t *touched = reinterpret_cast<int32_t *>(sm + L.touched_off);
@@ -1047,14 +1072,14 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
         const int32_t lo = max(rs, hi_end - BR);
         if (gather) {
             load_entries<RB>(a, lo, hi_end - lo, NT, tid, ent);
-            gather_batch<RB>(a, srec, scol4, mbar, BR, 0, hi_end - lo, ent, lo_e, hi_e, NT, tid);
+            gather_batch<RB>(a, srec, mbar, BR, 0, hi_end - lo, ent, lo_e, hi_e, NT, tid);
             if (nb > 1) {
                 const int32_t l1 = max(rs, lo - BR);
                 load_entries<RB>(a, l1, lo - l1, NT, tid, ent);
             }
             issued = 1;
         } else if (tid == 0) {
-            issue_batch<PACK>(a, srec, scol4, mbar, BR, 0, lo, hi_end - lo);
+            issue_batch<PACK>(a, srec, mbar, BR, 0, lo, hi_end - lo);
             issued = 1;
         }
     }
@@ -1067,7 +1092,7 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
             const int32_t hn = hi - BR;
             const int32_t ln = max(rs, hn - BR);
             if (gather) {
-                gather_batch<RB>(a, srec, scol4, mbar, BR, buf ^ 1, hn - ln, ent, lo_e, hi_e, NT,
+                gather_batch<RB>(a, srec, mbar, BR, buf ^ 1, hn - ln, ent, lo_e, hi_e, NT,
                                  tid);
                 if (b + 2 < nb) {
                     const int32_t l2 = max(rs, ln - BR);
@@ -1075,22 +1100,22 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 }
                 issued = b + 2;
             } else if (tid == 0) {
-                issue_batch<PACK>(a, srec, scol4, mbar, BR, buf ^ 1, ln, hn - ln);
+                issue_batch<PACK>(a, srec, mbar, BR, buf ^ 1, ln, hn - ln);
                 issued = b + 2;
             }
         }
         const bool ok = mbar_wait_bounded(&mbar[buf], (b >> 1) & 1);
         if (tid == 0 && ok) waited = b + 1;
-        const GeoRec *batch = srec + buf * BR;
+        const float4 *batch = srec + buf * BR;
         uint32_t *wmask = wmasks + (b & 1) * nw * RB * nw;
-        build_masks<RB>(batch, cnt, lo, NT, nw, wpr, tile_x0, tile_y0, tid, lane, wmask,
+        build_masks<RB, false>(batch, pitch, cnt, lo, NT, nw, wpr, tile_x0, tile_y0, tid, lane, wmask,
                         wbin);
         if (!PACK) {
 #pragma unroll
             for (int half = 0; half < RB; ++half) {
                 const int sl = tid + half * NT;
                 if (sl < cnt) {
-                    const float *cp = a.colors + (int64_t)batch[sl].gid * CD;
+                    const float *cp = a.colors + (int64_t)__float_as_int(batch[pitch + sl].w) * CD;
 #pragma unroll
                     for (int k = 0; k < CD; ++k) scol[(buf * BR + sl) * CD + k] = cp[k];
                 }
@@ -1102,8 +1127,8 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 const int sl = tid + half * NT;
                 if (sl < cnt) {
                     float col[CD];
-                    load_color<CD, PACK>(scol4, scol, buf * BR + sl, col);
-                    if (!tame_record<CD>(batch[sl], col)) *cold_flag = 1;
+                    load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, sl, col);
+                    if (!tame_record<CD>(staged_rec(batch, pitch, sl), col)) *cold_flag = 1;
                 }
             }
         }
@@ -1129,9 +1154,9 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                     const int bit = 31 - __clz(fit);
                     fit ^= 1u << bit;
                     const int t = k * 32 + bit;
-                    const GeoRec q = batch[t];
+                    const GeoRec q = staged_rec(batch, pitch, t);
                     float col[CD];
-                    load_color<CD, PACK>(scol4, scol, buf * BR + t, col);
+                    load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, t, col);
                     float2 w, u, ul, gc[CD];
                     grad_pair<CD, true>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
                     float d[4];
@@ -1145,9 +1170,9 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 const int bit = 31 - __clz(m);
                 m ^= 1u << bit;
                 const int t = k * 32 + bit;
-                const GeoRec q = batch[t];
+                const GeoRec q = staged_rec(batch, pitch, t);
                 float col[CD];
-                load_color<CD, PACK>(scol4, scol, buf * BR + t, col);
+                load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, t, col);
                 float2 w, u, ul, gc[CD];
                 const PairGeom pg = grad_pair<CD, false>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
                 float g[NV];
@@ -1186,7 +1211,7 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
         GeoRec own[RB];
 #pragma unroll
         for (int half = 0; half < RB; ++half)
-            if (tid + half * NT < cnt) own[half] = batch[tid + half * NT];
+            if (tid + half * NT < cnt) own[half] = staged_rec(batch, pitch, tid + half * NT);
         __syncthreads();
         if constexpr (KE > 0) {
 #pragma unroll
@@ -1276,14 +1301,15 @@ size_t raster_ws_bytes(int64_t T, int ch) {
 template <int CD>
 static int launch_pack(int64_t T, int64_t n_prims, const int32_t *fl, const float *m2,
                        const float *cn, const float *op, const float *be, const float *col,
-                       GeoRec *recs, float4 *rcols, uint32_t *status, cudaStream_t st) {
+                       float4 *recs, uint32_t *status, cudaStream_t st) {
     constexpr bool PACK = CD <= 4;
     const int blk = 256;
     const int64_t nblk = (T + blk - 1) / blk;
     const unsigned grid = (unsigned)(nblk < 152 * 16 ? nblk : 152 * 16);
     UBS_TIMED("raster_pack", st,
               pack_records_kernel<CD, PACK><<<grid, blk, 0, st>>>(
-                  T, n_prims, fl, m2, cn, op, be, col, recs, PACK ? rcols : nullptr, status));
+                  T, n_prims, fl, m2, cn, op, be, col, recs, recs + T, PACK ? recs + 2 * T : nullptr,
+                  status));
     note_launch();
     return check_launch("pack_records");
 }
@@ -1308,9 +1334,10 @@ constexpr int kBlendVariants = 3;
 // 69.8 us; 3,600: 258.6 against 250.4 us).
 constexpr int BWD_SMALL_GRID = 152 * 16;
 // Below one wave of 16 x 16 squares each is cut into four one-warp CTAs, which
-// wait for no other warp and spread over more SMs (130 tiles: 82.1 -> 77.2 us;
-// 1,900 tiles: no difference; 8,160: 955 -> 978 us).
-constexpr int BWD_ONE_WAVE = 152 * 6;
+// wait for no other warp and spread over more SMs (130 tiles: backward 82.1 ->
+// 77.2, forward 49.1 -> 37.1 us; 1,900 tiles: no difference; 8,160 tiles:
+// backward 955 -> 978 us).
+constexpr int ONE_WAVE = 152 * 6;
 constexpr int KE_SMALL = 64; // backward entry rows per warp
 
 template <int CD, bool BWD>
@@ -1321,9 +1348,9 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     // whose CTAs share the tile's records (backward; 1M primitives at 1080p,
     // tiles of 32: 1.85 -> 1.08 ms).  Wider colour rows need more registers
     // and shared memory and keep one CTA per tile.
-    const bool cut = PACK && BWD;
+    const bool cut = PACK && !a.pair_count;
     const int64_t cta16 = (int64_t)a.n_buckets * (a.TS / 16) * (a.TS / 16);
-    const int edge = !cut ? a.TS : a.TS % 16 != 0 || cta16 < BWD_ONE_WAVE ? 8 : 16;
+    const int edge = !cut ? a.TS : a.TS % 16 != 0 || cta16 < ONE_WAVE ? 8 : 16;
     a.sub = a.TS / edge;
     const int NT = edge * edge / 2;
     const bool small = PACK && NT <= 128;
@@ -1356,19 +1383,23 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
                               : raster_bwd_kernel<CD, true, 16, 1, C16, KE_SMALL>;
     } else if constexpr (BWD) {
         k = raster_bwd_kernel<CD, false, 0, 2, 1, 0>;
+    } else if (a.pair_count) {
+        k = raster_fwd_kernel<CD, PACK, true, 0, 2, 1>;
     } else {
-        if constexpr (CD == 3) {
-            if (small && variant == 1) k = raster_fwd_kernel<3, true, false, 1, 10>;
-            else if (small && variant == 2) k = raster_fwd_kernel<3, true, false, 2, 6>;
-        }
         if constexpr (PACK) {
-            if (small && !k)
-                k = a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 8>
-                                 : raster_fwd_kernel<CD, PACK, false, 2, 8>;
+            const bool e8 = edge == 8;
+            if (variant == 1)
+                k = e8 ? raster_fwd_kernel<CD, true, false, 8, 1, 32>
+                       : raster_fwd_kernel<CD, true, false, 16, 1, 10>;
+            else if (variant == 2)
+                k = e8 ? raster_fwd_kernel<CD, true, false, 8, 2, 24>
+                       : raster_fwd_kernel<CD, true, false, 16, 2, 6>;
+            else
+                k = e8 ? raster_fwd_kernel<CD, true, false, 8, 2, 32>
+                       : raster_fwd_kernel<CD, true, false, 16, 2, 8>;
+        } else {
+            k = raster_fwd_kernel<CD, false, false, 0, 2, 1>;
         }
-        if (!k)
-            k = a.pair_count ? raster_fwd_kernel<CD, PACK, true, 2, 1>
-                             : raster_fwd_kernel<CD, PACK, false, 2, 1>;
     }
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) !=
         cudaSuccess)
@@ -1445,8 +1476,9 @@ static void fill_common(RasterArgs &a, int32_t C, int64_t N, int32_t ch, int64_t
     a.offsets = offs;
     unsigned char *w = static_cast<unsigned char *>(ws);
     a.status = reinterpret_cast<uint32_t *>(w);
-    a.recs = reinterpret_cast<const GeoRec *>(w + 256);
-    a.rcols = ch <= 4 ? reinterpret_cast<const float4 *>(w + 256 + T * sizeof(GeoRec)) : nullptr;
+    a.recs_a = reinterpret_cast<const float4 *>(w + 256);
+    a.recs_b = a.recs_a + T;
+    a.rcols = ch <= 4 ? a.recs_b + T : nullptr;
     a.colors = colors;
     a.bg = bg;
     a.masks = masks;
@@ -1521,13 +1553,12 @@ int ubs_raster_pack(int32_t C, int64_t N, int32_t channels, int64_t n_isects,
     unsigned char *w = static_cast<unsigned char *>(workspace);
     if (cudaMemsetAsync(w, 0, 256, st) != cudaSuccess) return check_launch("raster_pack memset");
     if (n_isects == 0) return UBS_OK;
-    GeoRec *recs = reinterpret_cast<GeoRec *>(w + 256);
-    float4 *rcols = reinterpret_cast<float4 *>(w + 256 + n_isects * sizeof(GeoRec));
+    float4 *recs = reinterpret_cast<float4 *>(w + 256);
     uint32_t *status = reinterpret_cast<uint32_t *>(w);
     const int64_t P = (int64_t)C * N;
     UBS_CHANNEL_SWITCH(channels, return launch_pack<CDV>(n_isects, P, flatten_ids, means2d,
                                                          conics, opacities, betas, colors, recs,
-                                                         rcols, status, st));
+                                                         status, st));
 }
 
 int ubs_raster_fwd_packed(int32_t C, int64_t N, int32_t channels, int64_t n_isects,
