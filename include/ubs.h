@@ -519,6 +519,25 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
                              float *render_alphas, int32_t *last_ids, int64_t capacity,
                              void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
                              int32_t color_mode, void *stream);
+/* ubs_scene_forward_masked in two parts, so that a caller can read the
+ * intersection count (ubs_scene_stats' two values are the first 16 bytes of
+ * the workspace) as soon as it is known: UBS_SCENE_PART_COUNT runs everything
+ * up to it, UBS_SCENE_PART_BLEND the rest, both the whole frame.  The two parts
+ * of a frame take the same arguments, in this order, on one stream. */
+#define UBS_SCENE_PART_COUNT 1
+#define UBS_SCENE_PART_BLEND 2
+int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const float *mean,
+                            const float *scale, const float *l_triangle, const float *opacity,
+                            const float *beta, const float *rgb, int32_t C,
+                            const float *viewmats, const float *intrinsics,
+                            const float *centers, const float *timestamps,
+                            const int32_t *view_dims, const int32_t *tile_base,
+                            const int64_t *pix_base, int32_t n_buckets, int32_t tile_size,
+                            float eps2d, float near_plane, float far_plane, float radius_clip,
+                            const float *backgrounds, float *render_colors,
+                            float *render_alphas, int32_t *last_ids, int64_t capacity,
+                            void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
+                            int32_t color_mode, int32_t parts, void *stream);
 int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *mean,
                        const float *scale, const float *l_triangle, const float *opacity,
                        const float *beta, const float *rgb, int32_t C, const float *viewmats,

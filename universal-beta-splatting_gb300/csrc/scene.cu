@@ -677,6 +677,26 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
                              float *render_alphas, int32_t *last_ids, int64_t capacity,
                              void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
                              int32_t color_mode, void *stream) {
+    return ubs_scene_forward_parts(
+        dim, N, xyz, mean, scale, l_triangle, opacity, beta, rgb, C, viewmats, intrinsics, centers,
+        timestamps, view_dims, tile_base, pix_base, n_buckets, tile_size, eps2d, near_plane,
+        far_plane, radius_clip, backgrounds, render_colors, render_alphas, last_ids, capacity,
+        workspace, workspace_bytes, prim_mask, color_mode,
+        UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND, stream);
+}
+
+int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const float *mean,
+                            const float *scale, const float *l_triangle, const float *opacity,
+                            const float *beta, const float *rgb, int32_t C,
+                            const float *viewmats, const float *intrinsics,
+                            const float *centers, const float *timestamps,
+                            const int32_t *view_dims, const int32_t *tile_base,
+                            const int64_t *pix_base, int32_t n_buckets, int32_t tile_size,
+                            float eps2d, float near_plane, float far_plane, float radius_clip,
+                            const float *backgrounds, float *render_colors,
+                            float *render_alphas, int32_t *last_ids, int64_t capacity,
+                            void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
+                            int32_t color_mode, int32_t parts, void *stream) {
     SceneArgs a{};
     if (int e = scene_common(a, dim, N, xyz, mean, scale, l_triangle, opacity, beta, rgb, C,
                              viewmats, intrinsics, centers, timestamps, view_dims, tile_base,
@@ -700,53 +720,57 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
                          w.bytes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t CN = (int64_t)C * N;
-    if (cudaMemsetAsync(w.hdr, 0, sizeof(SceneHeader), st) != cudaSuccess ||
-        cudaMemsetAsync(w.bucket_counts, 0, (size_t)n_buckets * kCountReplicas * 4, st) !=
-            cudaSuccess)
-        return check_launch("scene_forward memset");
-    a.recs = w.recs;
-    a.cols_n = w.cols_n;
-    a.radius = w.radius;
-    a.depth = w.depth;
-    a.bucket_counts = w.bucket_counts;
-    a.n_buckets = n_buckets;
-    a.status = &w.hdr->status;
-    a.act = w.act;
-    a.act_b = w.act + act_beta_off(N, dim);
-    a.act_o = w.act + act_opac_off(N, dim);
-    if (CN > 0) {
-        if (int e = launch_scene_act(N, dim, scale, beta, opacity, w.act, st)) return e;
-        UBS_TIMED("scene_prim_fwd", st,
-                  UBS_SCENE_DIM(dim, scene_prim_fwd_kernel<DD><<<grid_for(CN, PRIM_THREADS),
-                                                                PRIM_THREADS, 0, st>>>(a)));
-        note_launch();
-        if (int e = check_launch("scene_prim_fwd")) return e;
-    }
-    // bucket offsets, total and heaviest-first order: one CTA when the
-    // buckets fit it, else a device-wide scan and the order kernel below
+    UBS_REQUIRE(parts >= 1 && parts <= 3, "scene_forward: parts %d", parts);
     const bool one_cta = n_buckets <= SCAN_ORDER_MAX;
-    if (one_cta) {
-        UBS_TIMED("bucket_scan_order", st,
-                  bucket_scan_order_kernel<kCountReplicas><<<1, 1024, 0, st>>>(
-                      w.bucket_counts, n_buckets, w.offsets, &w.hdr->total, w.order, w.cursor,
-                      w.totals));
-        note_launch();
-        if (int e = check_launch("bucket_scan_order")) return e;
-    } else {
-        UBS_TIMED("fold_replicas", st,
-                  fold_replicas_kernel<kCountReplicas><<<grid_for(n_buckets, 256), 256, 0, st>>>(
-                      w.bucket_counts, n_buckets, w.totals));
-        note_launch();
-        if (int e = check_launch("fold_replicas")) return e;
-        if (int e = device_exclusive_scan<int32_t>(w.totals, w.offsets, n_buckets, w.block_sums,
-                                                   &w.hdr->total, st))
-            return e;
-        UBS_TIMED("replica_cursors", st,
-                  replica_cursors_kernel<kCountReplicas><<<grid_for(n_buckets, 256), 256, 0, st>>>(
-                      w.bucket_counts, n_buckets, w.offsets, w.cursor));
-        note_launch();
-        if (int e = check_launch("replica_cursors")) return e;
+    if (parts & UBS_SCENE_PART_COUNT) {
+        if (cudaMemsetAsync(w.hdr, 0, sizeof(SceneHeader), st) != cudaSuccess ||
+            cudaMemsetAsync(w.bucket_counts, 0, (size_t)n_buckets * kCountReplicas * 4, st) !=
+                cudaSuccess)
+            return check_launch("scene_forward memset");
+        a.recs = w.recs;
+        a.cols_n = w.cols_n;
+        a.radius = w.radius;
+        a.depth = w.depth;
+        a.bucket_counts = w.bucket_counts;
+        a.n_buckets = n_buckets;
+        a.status = &w.hdr->status;
+        a.act = w.act;
+        a.act_b = w.act + act_beta_off(N, dim);
+        a.act_o = w.act + act_opac_off(N, dim);
+        if (CN > 0) {
+            if (int e = launch_scene_act(N, dim, scale, beta, opacity, w.act, st)) return e;
+            UBS_TIMED("scene_prim_fwd", st,
+                      UBS_SCENE_DIM(dim, scene_prim_fwd_kernel<DD><<<grid_for(CN, PRIM_THREADS),
+                                                                    PRIM_THREADS, 0, st>>>(a)));
+            note_launch();
+            if (int e = check_launch("scene_prim_fwd")) return e;
+        }
+        // bucket offsets, total and heaviest-first order: one CTA when the
+        // buckets fit it, else a device-wide scan and the order kernel below
+        if (one_cta) {
+            UBS_TIMED("bucket_scan_order", st,
+                      bucket_scan_order_kernel<kCountReplicas><<<1, 1024, 0, st>>>(
+                          w.bucket_counts, n_buckets, w.offsets, &w.hdr->total, w.order, w.cursor,
+                          w.totals));
+            note_launch();
+            if (int e = check_launch("bucket_scan_order")) return e;
+        } else {
+            UBS_TIMED("fold_replicas", st,
+                      fold_replicas_kernel<kCountReplicas><<<grid_for(n_buckets, 256), 256, 0, st>>>(
+                          w.bucket_counts, n_buckets, w.totals));
+            note_launch();
+            if (int e = check_launch("fold_replicas")) return e;
+            if (int e = device_exclusive_scan<int32_t>(w.totals, w.offsets, n_buckets, w.block_sums,
+                                                       &w.hdr->total, st))
+                return e;
+            UBS_TIMED("replica_cursors", st,
+                      replica_cursors_kernel<kCountReplicas><<<grid_for(n_buckets, 256), 256, 0, st>>>(
+                          w.bucket_counts, n_buckets, w.offsets, w.cursor));
+            note_launch();
+            if (int e = check_launch("replica_cursors")) return e;
+        }
     }
+    if (!(parts & UBS_SCENE_PART_BLEND)) return UBS_OK;
     if (CN > 0) {
         UBS_TIMED("scene_emit", st,
                   scene_emit_kernel<<<grid_for(CN, 256), 256, 0, st>>>(

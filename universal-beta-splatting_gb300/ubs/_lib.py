@@ -1,10 +1,11 @@
-"""ctypes binding of the C ABI declared in include/ubs.h.
+"""ctypes binding of the C ABI declared in include/ubs.h, and the loader of
+the host path built on it (csrc/host/native.cpp, the ubs_native module).
 
 The library is the only compute path: there is no CPU or PyTorch fallback.
 If it cannot be built or loaded, or a CUDA device is missing, calls raise.
 """
 import ctypes
-import os
+import importlib.util
 import threading
 
 import torch
@@ -70,6 +71,9 @@ SIGNATURES = {
     "ubs_scene_forward_masked": ([_I32, _I64] + [_P] * 7 + [_I32] + [_P] * 7
                                  + [_I32, _I32, _F, _F, _F, _F] + [_P] * 4
                                  + [_I64, _P, _SZ, _P, _I32, _P], _INT),
+    "ubs_scene_forward_parts": ([_I32, _I64] + [_P] * 7 + [_I32] + [_P] * 7
+                                + [_I32, _I32, _F, _F, _F, _F] + [_P] * 4
+                                + [_I64, _P, _SZ, _P, _I32, _I32, _P], _INT),
     "ubs_scene_backward": ([_I32, _I64] + [_P] * 7 + [_I32] + [_P] * 7 + [_I32, _I32, _F, _F, _F, _F]
                            + [_P] * 5 + [_P] * 7 + [_I32, _I64, _P, _SZ, _P], _INT),
     "ubs_scene_stats": ([_P, _I64P, _U32P, _P], _INT),
@@ -106,6 +110,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 _lock = threading.Lock()
 
 
@@ -123,6 +128,20 @@ def lib():
                     fn.restype = rest
                 _lib = L
     return _lib
+
+
+def native():
+    """The ubs_native extension module (built with the library if needed)."""
+    global _native
+    if _native is None:
+        lib()
+        with _lock:
+            if _native is None:
+                spec = importlib.util.spec_from_file_location("ubs_native", _build.NATIVE_PATH)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                _native = mod
+    return _native
 
 
 def library_path():
@@ -156,6 +175,7 @@ def start_timing():
     """Record CUDA events (on the current stream) around every entry-point call."""
     global _timing
     _timing = []
+    native().timing_start()
 
 
 def stop_timing():
@@ -164,9 +184,10 @@ def stop_timing():
     rec, _timing = _timing or [], None
     torch.cuda.synchronize()
     out = {}
-    for name, e0, e1 in rec:
+    calls = [(name, e0.elapsed_time(e1)) for name, e0, e1 in rec] + native().timing_stop()
+    for name, ms in calls:
         n, t = out.get(name, (0, 0.0))
-        out[name] = (n + 1, t + e0.elapsed_time(e1))
+        out[name] = (n + 1, t + ms)
     return out
 
 

@@ -1,8 +1,9 @@
-"""Build the GB300 rasteriser library (libubs_gb300.so) from csrc/ with nvcc.
+"""Build the GB300 rasteriser library (libubs_gb300.so) from csrc/ with nvcc and
+the host extension module on top of it (ubs_native.so, csrc/host/) with g++.
 
 Translation units are compiled in parallel for sm_103a only and linked into
 one shared library inside the package tree (_build/), which is what the
-ctypes loader in ubs._lib opens.
+ctypes loader in ubs._lib opens; the module links to that library.
 """
 import concurrent.futures as cf
 import hashlib
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(PKG_ROOT, "csrc")
@@ -17,6 +19,8 @@ INCLUDE = os.path.join(os.path.dirname(PKG_ROOT), "include")
 BUILD = os.path.join(PKG_ROOT, "_build")
 LIB_NAME = "libubs_gb300.so"
 LIB_PATH = os.path.join(BUILD, LIB_NAME)
+HOST_SRC = os.path.join(CSRC, "host", "native.cpp")
+NATIVE_PATH = os.path.join(BUILD, "ubs_native.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -44,11 +48,33 @@ def _sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
+def _host_compile(obj):
+    """g++ command of the extension module's object (PyTorch's headers)."""
+    import torch
+    from torch.utils import cpp_extension
+    inc = cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-sign-compare",
+             "-DTORCH_API_INCLUDE_EXTENSION_H",
+             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+            + [a for i in inc for a in ("-isystem", i)] + ["-c", HOST_SRC, "-o", obj])
+
+
+def _host_link(obj, out):
+    from torch.utils import cpp_extension
+    return (["g++", "-shared", obj, "-o", out, "-L" + BUILD, "-l:" + LIB_NAME,
+             "-Wl,-rpath,$ORIGIN"]
+            + ["-L" + d for d in cpp_extension.library_paths("cuda")]
+            + ["-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+               "-lcudart"])
+
+
 def _fingerprint():
+    import torch
     h = hashlib.sha256()
+    h.update(torch.__version__.encode())
     files = _sources() + sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC)
                                 if f.endswith((".cuh", ".h")))
-    files.append(os.path.join(INCLUDE, "ubs.h"))
+    files += [os.path.join(INCLUDE, "ubs.h"), HOST_SRC]
     for f in files:
         h.update(f.encode())
         with open(f, "rb") as fh:
@@ -62,7 +88,7 @@ def build(force=False, verbose=False, jobs=None):
     os.makedirs(BUILD, exist_ok=True)
     stamp = os.path.join(BUILD, "stamp.txt")
     fp = _fingerprint()
-    if not force and os.path.exists(LIB_PATH) and os.path.exists(stamp):
+    if not force and all(map(os.path.exists, (LIB_PATH, NATIVE_PATH, stamp))):
         with open(stamp) as f:
             if f.read().strip() == fp:
                 return LIB_PATH
@@ -74,12 +100,15 @@ def build(force=False, verbose=False, jobs=None):
         objs.append(obj)
         cmds.append([nvcc] + ARCH + _flags(src) + ["-I", INCLUDE, "-c", src, "-o", obj])
 
+    host_obj = os.path.join(BUILD, "native.o")
+    cmds.append(_host_compile(host_obj))
+
     def run(cmd):
         if verbose:
             print(" ".join(cmd), flush=True)
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed:\n%s\n%s" % (" ".join(cmd), r.stderr[-4000:]))
+            raise RuntimeError("build failed:\n%s\n%s" % (" ".join(cmd), r.stderr[-4000:]))
         return r
 
     with cf.ThreadPoolExecutor(max_workers=jobs or min(len(cmds), os.cpu_count() or 4)) as ex:
@@ -87,6 +116,9 @@ def build(force=False, verbose=False, jobs=None):
     tmp = LIB_PATH + ".tmp%d" % os.getpid()
     run([nvcc] + ARCH + ["-shared", "-cudart", "static", "-o", tmp] + objs)
     os.replace(tmp, LIB_PATH)
+    tmp = NATIVE_PATH + ".tmp%d" % os.getpid()
+    run(_host_link(host_obj, tmp))
+    os.replace(tmp, NATIVE_PATH)
     with open(stamp, "w") as f:
         f.write(fp)
     return LIB_PATH

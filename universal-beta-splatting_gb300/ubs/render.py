@@ -15,6 +15,7 @@ a time.
     colors, alphas = r.render(params, views)       # flat [P, 3], [P]
     images = views.split(colors)                   # list of [H, W, 3]
 """
+import contextlib
 import ctypes
 import gc
 from typing import Dict, List, Optional, Sequence
@@ -31,48 +32,28 @@ STATUS_NEG_DEPTH = 2
 class Views:
     """Cameras of one render call, flattened into (view, tile) buckets and one
     pixel buffer.  `cameras` are ubs.scene.Camera objects (viewmat, K, width,
-    height, timestamp).  The per-view tables go to the device in two copies
-    from one pinned staging buffer, on `stream` (default: the current one)."""
+    height, timestamp).  The per-view tables go to the device in one copy from
+    a pinned staging buffer, on `stream` (default: the current one)."""
 
     def __init__(self, cameras: Sequence, tile_size: int = 16, device=None, stream=None):
         if len(cameras) == 0:
             raise ValueError("need at least one view")
         device = torch.device(device or cameras[0].viewmat.device)
         C = len(cameras)
-        fl = torch.empty(C * 24, dtype=torch.float32, pin_memory=torch.cuda.is_available())
-        # int64 pix_base [C+1], then int32 dims [C,4] and tile_base [C+1]
-        ints = torch.empty(2 * (C + 1) + 4 * C + C + 1, dtype=torch.int32,
-                           pin_memory=torch.cuda.is_available())
-        f = fl.view(C, 24)
-        dims, tile_base, pix_base = [], [0], [0]
-        for v, c in enumerate(cameras):
-            vm = c.viewmat.detach().reshape(16).float().cpu()
-            f[v, 0:16] = vm
-            K = c.K.detach().float().cpu()
-            f[v, 16:20] = torch.stack([K[0, 0], K[1, 1], K[0, 2], K[1, 2]])
-            # the camera centre the reference model conditions on: the
-            # camera's own value (computed where its matrices live), so the
-            # view-direction queries round the same way
+        # the camera centre the reference model conditions on: the camera's
+        # own value (computed where its matrices live), so the view-direction
+        # queries round the same way
+        centers = []
+        for c in cameras:
             center = getattr(c, "position", None)
-            if center is None:
-                center = getattr(c, "center", None)
-            if center is not None:
-                f[v, 20:23] = center.detach().reshape(3).float().cpu()
-            else:
-                R, t = vm.view(4, 4)[:3, :3], vm.view(4, 4)[:3, 3]
-                f[v, 20:23] = -R.t() @ t
-            f[v, 23] = float(c.timestamp)
-            tw = (c.width + tile_size - 1) // tile_size
-            th = (c.height + tile_size - 1) // tile_size
-            dims.append([c.width, c.height, tw, th])
-            tile_base.append(tile_base[-1] + tw * th)
-            pix_base.append(pix_base[-1] + c.width * c.height)
-        if tile_base[-1] >= 2 ** 31:
-            raise ValueError("too many tiles in one render call")
-        o = 2 * (C + 1)
-        ints[:o].view(torch.int64)[:] = torch.tensor(pix_base, dtype=torch.int64)
-        ints[o:o + 4 * C] = torch.tensor(dims, dtype=torch.int32).reshape(-1)
-        ints[o + 4 * C:] = torch.tensor(tile_base, dtype=torch.int32)
+            centers.append(getattr(c, "center", None) if center is None else center)
+        on = contextlib.nullcontext() if stream is None else torch.cuda.stream(stream)
+        with on:
+            (staging, self.viewmats, self.intr, self.centers, self.times, self.dims,
+             self.tile_base, self.pix_base, tile_base, pix_base) = L.native().pack_views(
+                 [c.viewmat for c in cameras], [c.K for c in cameras], centers,
+                 [float(c.timestamp) for c in cameras], [c.width for c in cameras],
+                 [c.height for c in cameras], tile_size, device)
         self.C = C
         self.tile_size = tile_size
         self.shapes = [(c.height, c.width) for c in cameras]
@@ -80,23 +61,11 @@ class Views:
         self.n_pixels = pix_base[-1]
         self.pix_base_host = pix_base
         self.device = device
-        if device.type == "cuda":
-            st = stream if stream is not None else torch.cuda.current_stream(device)
-            with torch.cuda.stream(st):
-                fd = fl.to(device, non_blocking=True).view(C, 24)
-                idev = ints.to(device, non_blocking=True)
-                self.viewmats = fd[:, 0:16].contiguous()
-                self.intr = fd[:, 16:20].contiguous()
-                self.centers = fd[:, 20:23].contiguous()
-                self.times = fd[:, 23].contiguous()
-        else:  # host-side tables only (no compute runs on them)
-            fd, idev = fl.clone().view(C, 24), ints.clone()
-            self.viewmats, self.intr = fd[:, 0:16].contiguous(), fd[:, 16:20].contiguous()
-            self.centers, self.times = fd[:, 20:23].contiguous(), fd[:, 23].contiguous()
-        self._staging = (fl, ints)  # pinned buffers must outlive the copies
-        self.pix_base = idev[:o].view(torch.int64)
-        self.dims = idev[o:o + 4 * C].view(C, 4)
-        self.tile_base = idev[o + 4 * C:]
+        self._staging = staging  # the pinned buffer must outlive the copy
+
+    def _tables(self):
+        return [self.viewmats, self.intr, self.centers, self.times, self.dims, self.tile_base,
+                self.pix_base]
 
     def split(self, flat: torch.Tensor) -> List[torch.Tensor]:
         """Per-view [H, W, ...] views of a flat per-pixel buffer."""
@@ -127,17 +96,16 @@ class Renderer:
         self.capacity = capacity
         self.exact_cond_grad = exact_cond_grad
         self.last_isects = None
-        self._pending = None  # (pinned stats, event, capacity) of an unchecked frame
+        self._pending = None  # (stats, capacity) of an unchecked frame
         self.last_ws, self.last_cap = None, None
 
     # ---------------------------------------------------------------- helpers
     def _check_pending(self):
         if self._pending is None:
             return
-        stats, ev, cap = self._pending
+        stats, cap = self._pending
         self._pending = None
-        ev.synchronize()
-        T, status = int(stats[0]), int(stats[1])
+        T, status = stats.wait()
         self.last_isects = T
         if status & STATUS_NEG_DEPTH:
             raise RuntimeError("scene render: a visible primitive has a negative depth")
@@ -245,104 +213,53 @@ class Renderer:
         leaves the verification to `stats()` after the frame(s).
         prim_mask (uint8 [N]) leaves out primitives whose entry is 0;
         color_mode=1 renders depth into channel 0 (one view, no backward)."""
+        return self._forward([p[k] for k in PARAM_ORDER], views, bg, check, prim_mask, color_mode,
+                             False)
+
+    def _forward(self, tensors, views, bg, check, prim_mask, color_mode, grad):
         if check == "none":
             if self.capacity is None:
                 raise RuntimeError("check='none' needs a capacity (render once with check=True)")
         else:
             self._check_pending()
-        N = p["xyz"].shape[0]
-        dev = p["xyz"].device
+        N = tensors[0].shape[0]
         # first frame: a guess from the pixel count (re-run below if too small)
         cap = self.capacity or max(1 << 16, min(16 * N * views.C, 8 * views.n_pixels))
+        native = L.native()
         while True:
-            ws = L.workspace(self.workspace_bytes(views.C, N, views.n_buckets, cap), dev)
-            colors = torch.empty(views.n_pixels, 3, device=dev)
-            alphas = torch.empty(views.n_pixels, device=dev)
-            last = torch.empty(views.n_pixels, dtype=torch.int32, device=dev)
-            st = L.stream(dev)
-            if prim_mask is None and color_mode == 0:
-                L.call("ubs_scene_forward", *self._args(p, views, bg), L.ptr(colors),
-                       L.ptr(alphas), L.ptr(last), cap, L.ptr(ws), ws.numel(), st)
-            else:
-                L.call("ubs_scene_forward_masked", *self._args(p, views, bg), L.ptr(colors),
-                       L.ptr(alphas), L.ptr(last), cap, L.ptr(ws), ws.numel(),
-                       L.ptr(prim_mask, torch.uint8), int(color_mode), st)
+            call = native.SceneCall(self.dim, views._tables(), views.n_buckets, views.n_pixels,
+                                    self.tile_size, self.eps2d, self.near, self.far,
+                                    self.radius_clip, bool(self.exact_cond_grad), cap)
+            colors, alphas, last, ws, stats = native.scene_forward(
+                call, tensors, bg, prim_mask, color_mode, check != "none", grad)
             self.last_ws, self.last_cap = ws, cap
             if check == "none":
                 return colors, alphas, last, ws, cap
-            stats = torch.empty(2, dtype=torch.int64, pin_memory=True)
-            hdr = ws[:16].view(torch.int64)
-            if check:
-                stats.copy_(hdr.cpu())
-                T, status = int(stats[0]), int(stats[1]) & 0xffffffff
-                self.last_isects = T
-                if status & STATUS_NEG_DEPTH:
-                    raise RuntimeError("scene render: a visible primitive has a negative depth")
-                if T > cap:
-                    cap = int(T * 1.25) + 1024
-                    self.capacity = cap
-                    continue
+            if not check:
+                self._pending = (stats, cap)
+                return colors, alphas, last, ws, cap
+            T, status = stats.wait()
+            self.last_isects = T
+            if status & STATUS_NEG_DEPTH:
+                raise RuntimeError("scene render: a visible primitive has a negative depth")
+            if T <= cap:
                 if self.capacity is None:
                     self.capacity = max(int(T * 1.25) + 1024, 1 << 16)
-            else:
-                stats.copy_(hdr, non_blocking=True)
-                ev = torch.cuda.Event()
-                ev.record()
-                self._pending = (stats, ev, cap)
-            return colors, alphas, last, ws, cap
+                return colors, alphas, last, ws, cap
+            cap = int(T * 1.25) + 1024
+            self.capacity = cap
 
     def render(self, params: Dict[str, torch.Tensor], views: Views,
                backgrounds: Optional[torch.Tensor] = None, check=True):
         """Differentiable render of all views: colors [P, 3], alphas [P].
         `check`: True, False or "none", as for forward_raw."""
-        dev = params["xyz"].device
         if backgrounds is None:
-            bg = torch.zeros(views.C, 3, device=dev)
+            bg = torch.zeros(views.C, 3, device=params["xyz"].device)
         else:
             bg = backgrounds.reshape(-1, 3).expand(views.C, 3).contiguous().float()
-        tensors = [params[k] for k in PARAM_ORDER]
-        return _SceneRender.apply(self, views, bg, check, *tensors)
-
-
-def _prep(t, shape_tail=None):
-    t = t.contiguous()
-    if t.dtype != torch.float32:
-        raise TypeError("scene parameters must be float32")
-    return t
-
-
-class _SceneRender(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, renderer, views, bg, check, xyz, mean, scale, l_triangle, opacity, beta, rgb):
-        p = {"xyz": _prep(xyz), "mean": _prep(mean), "scale": _prep(scale),
-             "l_triangle": _prep(l_triangle), "opacity": _prep(opacity.reshape(-1)),
-             "beta": _prep(beta), "rgb": _prep(rgb)}
-        colors, alphas, last, ws, cap = renderer.forward_raw(p, views, bg, check=check)
-        ctx.renderer, ctx.views, ctx.ws, ctx.cap = renderer, views, ws, cap
-        ctx.opacity_shape = opacity.shape
-        ctx.save_for_backward(p["xyz"], p["mean"], p["scale"], p["l_triangle"], p["opacity"],
-                              p["beta"], p["rgb"], bg, alphas, last)
-        ctx.mark_non_differentiable(last)
+        colors, alphas, _, _, _ = self._forward([params[k] for k in PARAM_ORDER], views, bg, check,
+                                                None, 0, True)
         return colors, alphas
-
-    @staticmethod
-    def backward(ctx, v_colors, v_alphas):
-        xyz, mean, scale, ltri, opac, beta, rgb, bg, alphas, last = ctx.saved_tensors
-        r, views = ctx.renderer, ctx.views
-        dev = xyz.device
-        p = {"xyz": xyz, "mean": mean, "scale": scale, "l_triangle": ltri, "opacity": opac,
-             "beta": beta, "rgb": rgb}
-        v_colors = (torch.zeros(views.n_pixels, 3, device=dev) if v_colors is None
-                    else v_colors.contiguous())
-        v_alphas = (torch.zeros(views.n_pixels, device=dev) if v_alphas is None
-                    else v_alphas.contiguous())
-        g = {k: torch.empty_like(p[k]) for k in PARAM_ORDER}
-        L.call("ubs_scene_backward", *r._args(p, views, bg), L.ptr(alphas), L.ptr(last),
-               L.ptr(v_colors), L.ptr(v_alphas), *[L.ptr(g[k]) for k in PARAM_ORDER],
-               int(bool(r.exact_cond_grad)), ctx.cap, L.ptr(ctx.ws), ctx.ws.numel(), L.stream(dev))
-        ctx.ws = None
-        return (None, None, None, None, g["xyz"], g["mean"], g["scale"], g["l_triangle"],
-                g["opacity"].view(ctx.opacity_shape), g["beta"], g["rgb"])
 
 
 class GraphedStep:
