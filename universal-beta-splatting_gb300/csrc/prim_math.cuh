@@ -347,20 +347,20 @@ template <int K> __device__ __forceinline__ void inv_small(const float *A, float
         for (int c = 0; c < K; ++c) out[r * K + c] = aug[r][K + c];
 }
 
-template <int K> struct CondState {
-    float x[K], beta[K], ba[K], i22[K * K], r[3 * K], rb[3 * K], v12[3 * K], v21[3 * K],
-        Lc[K * K], y[K];
+// What conditioning needs of a primitive whatever the query: the regression
+// r = V12 V22^-1 (rb: scaled by the clamped betas), V22^-1 and V22's Cholesky
+// factor.
+template <int K> struct CondFixed {
+    float beta[K], ba[K], i22[K * K], r[3 * K], rb[3 * K], v12[3 * K], v21[3 * K], Lc[K * K];
 };
 
-// m: [D] means, V: [D*D] row-major covariance (D = K + 3)
+// V: [D*D] row-major covariance (D = K + 3)
 template <int K>
-__device__ __forceinline__ void cond_prepare(const float *m, const float *V, const float *b,
-                                             const float *q, CondState<K> &s) {
+__device__ __forceinline__ void cond_fixed(const float *V, const float *b, CondFixed<K> &s) {
     constexpr int D = K + 3;
     float v22[K * K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        s.x[j] = q[j] - m[3 + j];
         s.beta[j] = b[j];
         const float t = b[j] * 0.25f;
         s.ba[j] = (t < 1.f) ? t : 1.f;
@@ -406,28 +406,29 @@ __device__ __forceinline__ void cond_prepare(const float *m, const float *V, con
                 s.Lc[i * K + j] = sum / nz20(s.Lc[j * K + j]);
             }
         }
+}
+
+// x = query - conditional mean and y = L^-1 x.
+template <int K>
+__device__ __forceinline__ void cond_whiten(const float *m, const float *q, const float *Lc,
+                                            float *x, float *y) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) x[j] = q[j] - m[3 + j];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
-        float sum = s.x[i];
+        float sum = x[i];
 #pragma unroll
-        for (int k = 0; k < i; ++k) sum -= s.Lc[i * K + k] * s.y[k];
-        s.y[i] = sum / nz20(s.Lc[i * K + i]);
+        for (int k = 0; k < i; ++k) sum -= Lc[i * K + k] * y[k];
+        y[i] = sum / nz20(Lc[i * K + i]);
     }
 }
 
+// Conditioned covariance (query independent).
 template <int K>
-__device__ __forceinline__ void cond_forward(const float *m, const float *V, float o,
-                                             const float *b, const float *q, float *om, float *oV,
-                                             float *oo) {
+__device__ __forceinline__ void cond_covar(const float *V, const CondFixed<K> &s, float *oV) {
     constexpr int D = K + 3;
-    CondState<K> s;
-    cond_prepare<K>(m, V, b, q, s);
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        float acc = 0.f;
-#pragma unroll
-        for (int c = 0; c < K; ++c) acc += s.rb[r * K + c] * s.x[c];
-        om[r] = m[r] + acc;
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int c2 = 0; c2 < 3; ++c2) {
             float a2 = 0.f;
@@ -435,57 +436,140 @@ __device__ __forceinline__ void cond_forward(const float *m, const float *V, flo
             for (int k = 0; k < K; ++k) a2 += s.rb[r * K + k] * s.v21[k * 3 + c2];
             oV[r * 3 + c2] = V[r * D + c2] - a2;
         }
+}
+
+// Conditioned mean and opacity of one query.
+template <int K>
+__device__ __forceinline__ void cond_query(const float *m, const CondFixed<K> &s, float o,
+                                           const float *x, const float *y, float *om, float *oo) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        float acc = 0.f;
+#pragma unroll
+        for (int c = 0; c < K; ++c) acc += s.rb[r * K + c] * x[c];
+        om[r] = m[r] + acc;
     }
     float oc = 1.f;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        const float d = clamp01_eps(tanhf(s.y[j] * s.y[j]));
+        const float d = clamp01_eps(tanhf(y[j] * y[j]));
         oc *= powf(1.f - d, s.beta[j]);
     }
     *oo = o * oc;
 }
 
-// VJP; gm [D], gV [D*D] (row-major), go, gb [K] are overwritten.
 template <int K>
-__device__ __forceinline__ void cond_backward(const float *m, const float *V, float o,
-                                              const float *b, const float *q, const float *gM,
-                                              const float *gVc, float gO, bool exact, float *gm,
-                                              float *gV, float *go, float *gb) {
-    constexpr int D = K + 3;
+__device__ __forceinline__ void cond_forward(const float *m, const float *V, float o,
+                                             const float *b, const float *q, float *om, float *oV,
+                                             float *oo) {
+    CondFixed<K> s;
+    float x[K], y[K];
+    cond_fixed<K>(V, b, s);
+    cond_whiten<K>(m, q, s.Lc, x, y);
+    cond_covar<K>(V, s, oV);
+    cond_query<K>(m, s, o, x, y, om, oo);
+}
+
+// What the VJP needs of the queries of one primitive: everything after it is
+// linear in these sums, so the gradients of many queries (views) are summed
+// here and pass through the matrix part once.
+template <int K> struct CondGrads {
+    float gM[3], gMx[3 * K]; // sum of v_mean and of v_mean x^T
+    float gVc[9];            // sum of v_covar
+    float go, gb[K];         // opacity and beta of the opacity path
+    float a[K], ay[K * K];   // a = L^-T v_y and the lower triangle of a y^T
+    __device__ __forceinline__ void zero() {
+        go = 0.f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) gM[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 3 * K; ++k) gMx[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) gVc[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k) gb[k] = a[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < K * K; ++k) ay[k] = 0.f;
+    }
+};
+
+template <int K>
+__device__ __forceinline__ void cond_accumulate(const float *Lc, const float *beta, float o,
+                                                const float *x, const float *y, const float *gM,
+                                                const float *gVc, float gO, CondGrads<K> &g) {
     const float upper = 1.0f - 1.1920928955078125e-07f;
-    CondState<K> s;
-    cond_prepare<K>(m, V, b, q, s);
 #pragma unroll
-    for (int k = 0; k < D; ++k) gm[k] = 0.f;
+    for (int r = 0; r < 3; ++r) {
+        g.gM[r] += gM[r];
 #pragma unroll
-    for (int k = 0; k < D * D; ++k) gV[k] = 0.f;
+        for (int c = 0; c < K; ++c) g.gMx[r * K + c] += gM[r] * x[c];
+    }
 #pragma unroll
-    for (int k = 0; k < K; ++k) gb[k] = 0.f;
+    for (int k = 0; k < 9; ++k) g.gVc[k] += gVc[k];
+    // opacity path
+    float dv[K], base[K], oc = 1.f;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) gm[r] = gM[r];
+    for (int j = 0; j < K; ++j) {
+        float d = tanhf(y[j] * y[j]);
+        if (d < 0.f) d = 0.f;
+        if (d > upper) d = upper;
+        dv[j] = d;
+        base[j] = 1.f - d;
+        oc *= powf(base[j], beta[j]);
+    }
+    g.go += gO * oc;
+    const float goc = gO * o;
+    float gy[K], a[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        float gd = 0.f;
+        if (base[j] > 0.f) {
+            g.gb[j] += goc * oc * logf(base[j]);
+            if (dv[j] > 0.f && dv[j] < upper) gd += goc * (-oc * beta[j] / base[j]);
+        }
+        gy[j] = gd * (2.f * y[j] * (1.f - dv[j] * dv[j]));
+    }
+#pragma unroll
+    for (int ii = K - 1; ii >= 0; --ii) {
+        float sum = gy[ii];
+#pragma unroll
+        for (int k = ii + 1; k < K; ++k) sum -= Lc[k * K + ii] * a[k];
+        a[ii] = sum / nz20(Lc[ii * K + ii]);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        g.a[k] += a[k];
+#pragma unroll
+        for (int c = 0; c <= k; ++c) g.ay[k * K + c] += a[k] * y[c];
+    }
+}
+
+// gm [D], gV [D*D] (row-major) and gb [K] are overwritten.
+template <int K>
+__device__ __forceinline__ void cond_finish(const CondFixed<K> &s, const CondGrads<K> &g,
+                                            bool exact, float *gm, float *gV, float *gb) {
+    constexpr int D = K + 3;
     float Gr[3 * K], gx[K];
 #pragma unroll
     for (int c = 0; c < K; ++c) {
-        gx[c] = 0.f;
 #pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            Gr[r * K + c] = gM[r] * s.x[c] -
-                            (gVc[r * 3 + 0] * s.v21[c * 3 + 0] + gVc[r * 3 + 1] * s.v21[c * 3 + 1] +
-                             gVc[r * 3 + 2] * s.v21[c * 3 + 2]);
-        }
-        gx[c] += s.rb[0 * K + c] * gM[0] + s.rb[1 * K + c] * gM[1] + s.rb[2 * K + c] * gM[2];
+        for (int r = 0; r < 3; ++r)
+            Gr[r * K + c] = g.gMx[r * K + c] - (g.gVc[r * 3 + 0] * s.v21[c * 3 + 0] +
+                                                g.gVc[r * 3 + 1] * s.v21[c * 3 + 1] +
+                                                g.gVc[r * 3 + 2] * s.v21[c * 3 + 2]);
+        gx[c] = s.rb[0 * K + c] * g.gM[0] + s.rb[1 * K + c] * g.gM[1] + s.rb[2 * K + c] * g.gM[2];
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) gV[r * D + c] += gVc[r * 3 + c];
+        for (int c = 0; c < 3; ++c) gV[r * D + c] = g.gVc[r * 3 + c];
 #pragma unroll
     for (int rr = 0; rr < K; ++rr)
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-            gV[(3 + rr) * D + c] += -(s.rb[0 * K + rr] * gVc[0 * 3 + c] +
-                                      s.rb[1 * K + rr] * gVc[1 * 3 + c] +
-                                      s.rb[2 * K + rr] * gVc[2 * 3 + c]);
+            gV[(3 + rr) * D + c] = -(s.rb[0 * K + rr] * g.gVc[0 * 3 + c] +
+                                     s.rb[1 * K + rr] * g.gVc[1 * 3 + c] +
+                                     s.rb[2 * K + rr] * g.gVc[2 * 3 + c]);
     float dba[K], G_r[3 * K];
 #pragma unroll
     for (int c = 0; c < K; ++c) {
@@ -501,7 +585,7 @@ __device__ __forceinline__ void cond_backward(const float *m, const float *V, fl
             float acc = 0.f;
 #pragma unroll
             for (int k = 0; k < K; ++k) acc += G_r[r * K + k] * s.i22[c * K + k];
-            gV[r * D + 3 + c] += acc;
+            gV[r * D + 3 + c] = acc;
         }
     float Gi22[K * K];
 #pragma unroll
@@ -511,38 +595,8 @@ __device__ __forceinline__ void cond_backward(const float *m, const float *V, fl
             Gi22[rr * K + c] = s.v12[0 * K + rr] * G_r[0 * K + c] +
                                s.v12[1 * K + rr] * G_r[1 * K + c] +
                                s.v12[2 * K + rr] * G_r[2 * K + c];
-    // opacity path
-    float dv[K], base[K], oc = 1.f;
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-        float d = tanhf(s.y[j] * s.y[j]);
-        if (d < 0.f) d = 0.f;
-        if (d > upper) d = upper;
-        dv[j] = d;
-        base[j] = 1.f - d;
-        oc *= powf(base[j], s.beta[j]);
-    }
-    *go = gO * oc;
-    const float goc = gO * o;
-    float gy[K], a[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        float gd = 0.f;
-        if (base[j] > 0.f) {
-            gb[j] += goc * oc * logf(base[j]);
-            if (dv[j] > 0.f && dv[j] < upper) gd += goc * (-oc * s.beta[j] / base[j]);
-        }
-        gy[j] = gd * (2.f * s.y[j] * (1.f - dv[j] * dv[j]));
-    }
-#pragma unroll
-    for (int ii = K - 1; ii >= 0; --ii) {
-        float sum = gy[ii];
-#pragma unroll
-        for (int k = ii + 1; k < K; ++k) sum -= s.Lc[k * K + ii] * a[k];
-        a[ii] = sum / nz20(s.Lc[ii * K + ii]);
-    }
-#pragma unroll
-    for (int j = 0; j < K; ++j) gx[j] += a[j];
+    for (int j = 0; j < K; ++j) gx[j] += g.a[j];
     float S[K * K], U[K * K], Gm[K * K];
 #pragma unroll
     for (int r = 0; r < K; ++r)
@@ -551,7 +605,7 @@ __device__ __forceinline__ void cond_backward(const float *m, const float *V, fl
             float acc = 0.f;
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const float gl = (c <= k) ? -(a[k] * s.y[c]) : 0.f; // gL = -a y^T, lower
+                const float gl = (c <= k) ? -g.ay[k * K + c] : 0.f; // gL = -a y^T, lower
                 acc += s.Lc[k * K + r] * gl;
             }
             S[r * K + c] = (c > r) ? 0.f : acc;
@@ -588,15 +642,6 @@ __device__ __forceinline__ void cond_backward(const float *m, const float *V, fl
                 Gm[r * K + ii] = sum / nz20(s.Lc[ii * K + ii]);
             }
     }
-#pragma unroll
-    for (int r = 0; r < K; ++r)
-#pragma unroll
-        for (int c = 0; c < K; ++c)
-            gV[(3 + r) * D + 3 + c] += 0.5f * (Gm[r * K + c] + Gm[c * K + r]);
-#pragma unroll
-    for (int j = 0; j < K; ++j) gm[3 + j] += -gx[j];
-#pragma unroll
-    for (int j = 0; j < K; ++j) gb[j] += dba[j] * ((s.beta[j] < 4.f) ? 0.25f : 0.f);
     float tmp[K * K];
 #pragma unroll
     for (int r = 0; r < K; ++r)
@@ -614,8 +659,32 @@ __device__ __forceinline__ void cond_backward(const float *m, const float *V, fl
             float acc = 0.f;
 #pragma unroll
             for (int k = 0; k < K; ++k) acc += s.i22[k * K + r] * tmp[k * K + c];
-            gV[(3 + r) * D + 3 + c] += -acc;
+            gV[(3 + r) * D + 3 + c] = 0.5f * (Gm[r * K + c] + Gm[c * K + r]) - acc;
         }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) gm[r] = g.gM[r];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        gm[3 + j] = -gx[j];
+        gb[j] = g.gb[j] + dba[j] * ((s.beta[j] < 4.f) ? 0.25f : 0.f);
+    }
+}
+
+// VJP of one query; gm [D], gV [D*D] (row-major), go, gb [K] are overwritten.
+template <int K>
+__device__ __forceinline__ void cond_backward(const float *m, const float *V, float o,
+                                              const float *b, const float *q, const float *gM,
+                                              const float *gVc, float gO, bool exact, float *gm,
+                                              float *gV, float *go, float *gb) {
+    CondFixed<K> s;
+    CondGrads<K> g;
+    float x[K], y[K];
+    cond_fixed<K>(V, b, s);
+    cond_whiten<K>(m, q, s.Lc, x, y);
+    g.zero();
+    cond_accumulate<K>(s.Lc, s.beta, o, x, y, gM, gVc, gO, g);
+    cond_finish<K>(s, g, exact, gm, gV, gb);
+    *go = g.go;
 }
 
 // ------------------------------------------------------ D x D covariance

@@ -6,7 +6,7 @@
 // [N, D, D] covariance), cond_mean_convariance_opacity, a [N, 6] gather,
 // fully_fused_projection, isect_tiles (+ host sync), isect_offset_encode and
 // rasterize_to_pixels.  Here the same mathematics runs as:
-//   1. scene_prim_fwd: one thread per (view, primitive) -- activations,
+//   1. scene_prim_fwd: one thread per primitive, looping over views -- activations,
 //      rotation, D x D covariance, conditioning on the view ray (and time),
 //      EWA projection, tile counting into per-(view, tile) buckets;
 //   2. a device-side scan, bucketed emit and per-bucket sort of (depth,
@@ -15,7 +15,7 @@
 //   3. the blend over a flattened (view, tile) work list whose views may have
 //      different resolutions, copying each batch of records from the
 //      per-entry tables by the sorted keys (no sorted copy of the records);
-//   4. scene_prim_bwd: one thread per (view, primitive) recomputes the forward
+//   4. scene_prim_bwd: one thread per primitive recomputes each view's forward
 //      chain and back-propagates blend gradients to the raw parameters.
 // Every launch is stream ordered with fixed grids, so a whole forward or
 // backward can be captured in a CUDA graph.
@@ -139,18 +139,13 @@ __device__ __forceinline__ void view_direction(const float *xyz, const float *ce
     q[2] = __fdiv_rn(d2, nrm);
 }
 
-// Forward state of one (view, primitive), shared by both kernels.
-template <int D> struct PrimFwd {
+// The view-independent state of one primitive, shared by both kernels.
+template <int D> struct PrimFixed {
     static constexpr int K = D - 3;
-    float s[D];        // activated scales
-    float L[D * D];    // covariance factor
-    float V[D * D];    // D x D covariance
-    float m[D];        // means (xyz, angular / temporal)
-    float o;           // activated opacity
-    float b[K];        // activated conditional betas
-    float b0;          // activated spatial beta
-    float q[K];        // query (view direction [, time])
-    float om[3], oV[9], oo; // conditioned mean, covariance, opacity
+    float m[D];  // means (xyz, angular / temporal)
+    float o, b0; // activated opacity and spatial beta
+    float oV[9]; // conditioned covariance
+    CondFixed<K> c;
 };
 
 // One primitive's parameter rows: xyz (3), mean (K), activated scale (D),
@@ -178,18 +173,16 @@ __device__ __forceinline__ const float *stage_rows(const float *__restrict__ src
     return st + lane * W;
 }
 
-// Rows of primitive n: staged for the warp when its 32 entries are 32
-// consecutive primitives of one view (every warp but the one straddling a
-// view boundary or the end), else read in place.  Returns whether staged;
-// the caller syncs the warp before reading staged rows.
+// Rows of primitive n: staged for the warp when its 32 threads are 32
+// consecutive primitives (every warp but the last one), else read in place.
+// Returns whether staged; the caller syncs the warp before reading staged rows.
 template <int D>
-__device__ __forceinline__ bool prim_rows(const SceneArgs &a, int64_t idx, int64_t n, int lane,
-                                          float *stage, PrimRows &r) {
+__device__ __forceinline__ bool prim_rows(const SceneArgs &a, int64_t n, int lane, float *stage,
+                                          PrimRows &r) {
     constexpr int K = D - 3, NL = D * (D - 1) / 2;
     const float *act_s = a.act, *act_b = a.act_b, *act_o = a.act_o;
-    const int64_t w0 = idx - lane, n0 = n - lane;
-    const bool staged = w0 + 32 <= (int64_t)a.C * a.N && n0 >= 0 && n0 + 32 <= a.N;
-    if (__all_sync(0xffffffffu, staged)) {
+    const int64_t n0 = n - lane;
+    if (n0 + 32 <= a.N) { // the same in every lane
         float *st = stage;
         r.xyz = stage_rows<3>(a.xyz, n0, st, lane);
         st += 32 * 3;
@@ -203,7 +196,7 @@ __device__ __forceinline__ bool prim_rows(const SceneArgs &a, int64_t idx, int64
         r.o = act_o[n];
         return true;
     }
-    if (n >= 0 && n < a.N) {
+    if (n < a.N) {
         r.xyz = a.xyz + n * 3;
         r.mean = a.mean + n * K;
         r.s = act_s + n * D;
@@ -214,34 +207,40 @@ __device__ __forceinline__ bool prim_rows(const SceneArgs &a, int64_t idx, int64
     return false;
 }
 
+// Covariance factor and covariance from the rows (activations as the
+// reference's PyTorch kernels round them, scene_act.cu).  L: top-left R
+// diag(s[0:3]) with R = I + A(a01, a02, a12); L[r][r] = s[r] (r >= 3); rest
+// entries row-major below the diagonal.
 template <int D>
-__device__ __forceinline__ void prim_forward(const SceneArgs &a, const PrimRows &rw, int v,
-                                             PrimFwd<D> &f) {
-    constexpr int K = D - 3;
+__device__ __forceinline__ void prim_covar(const PrimRows &rw, float *L, float *V) {
     constexpr int NL = D * (D - 1) / 2;
-    float lt[NL];
-    // activations as the reference's PyTorch kernels round them (scene_act.cu)
+    float lt[NL], sc[D];
 #pragma unroll
     for (int k = 0; k < NL; ++k) lt[k] = rw.lt[k];
 #pragma unroll
-    for (int k = 0; k < D; ++k) f.s[k] = rw.s[k];
-    // L: top-left R diag(s[0:3]) with R = I + A(a01, a02, a12); L[r][r] = s[r] (r >= 3);
-    // rest entries row-major below the diagonal
+    for (int k = 0; k < D; ++k) sc[k] = rw.s[k];
     const float R[9] = {1.f, lt[0], lt[1], -lt[0], 1.f, lt[2], -lt[1], -lt[2], 1.f};
 #pragma unroll
-    for (int k = 0; k < D * D; ++k) f.L[k] = 0.f;
+    for (int k = 0; k < D * D; ++k) L[k] = 0.f;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) f.L[r * D + c] = R[r * 3 + c] * f.s[c];
+        for (int c = 0; c < 3; ++c) L[r * D + c] = R[r * 3 + c] * sc[c];
     int m = 3;
 #pragma unroll
     for (int r = 3; r < D; ++r) {
 #pragma unroll
-        for (int c = 0; c < r; ++c) f.L[r * D + c] = lt[m++];
-        f.L[r * D + r] = f.s[r];
+        for (int c = 0; c < r; ++c) L[r * D + c] = lt[m++];
+        L[r * D + r] = sc[r];
     }
-    covar_from_L<D>(f.L, f.V);
+    covar_from_L<D>(L, V);
+}
+
+template <int D>
+__device__ __forceinline__ void prim_fixed(const PrimRows &rw, PrimFixed<D> &f, float *L) {
+    constexpr int K = D - 3;
+    float V[D * D], b[K];
+    prim_covar<D>(rw, L, V);
 #pragma unroll
     for (int k = 0; k < 3; ++k) f.m[k] = rw.xyz[k];
 #pragma unroll
@@ -249,12 +248,21 @@ __device__ __forceinline__ void prim_forward(const SceneArgs &a, const PrimRows 
     f.o = rw.o;
     f.b0 = rw.b[0];
 #pragma unroll
-    for (int k = 0; k < K; ++k) f.b[k] = rw.b[1 + k];
-    // view direction query (+ timestamp for the 7-D model)
-    const float *cc = a.centers + v * 3;
-    view_direction(f.m, cc, f.q);
-    if (K == 4) f.q[3 % K] = a.times[v];
-    cond_forward<K>(f.m, f.V, f.o, f.b, f.q, f.om, f.oV, &f.oo);
+    for (int k = 0; k < K; ++k) b[k] = rw.b[1 + k];
+    cond_fixed<K>(V, b, f.c);
+    cond_covar<K>(V, f.c, f.oV);
+}
+
+// The view direction query (+ timestamp for the 7-D model) of a view, and what
+// conditioning makes of it.
+template <int D>
+__device__ __forceinline__ void prim_query(const SceneArgs &a, const PrimFixed<D> &f, int v,
+                                           float *x, float *y) {
+    constexpr int K = D - 3;
+    float q[K];
+    view_direction(f.m, a.centers + v * 3, q);
+    if (K == 4) q[3 % K] = a.times[v];
+    cond_whiten<K>(f.m, q, f.c.Lc, x, y);
 }
 
 // conditioned covariance -> world covariance used by the projection: the
@@ -269,68 +277,84 @@ __device__ __forceinline__ M3 upper_sym(const float *oV) {
 
 constexpr int PRIM_THREADS = 128;
 
-template <int D>
-__global__ void __launch_bounds__(PRIM_THREADS, D == 6 ? 8 : 6) scene_prim_fwd_kernel(SceneArgs a) {
+// One thread per primitive and group of views (blockIdx.y, every gridDim.y-th
+// view): what does not depend on the view -- covariance, its conditional
+// block's inverse and Cholesky factor, the conditioned covariance -- is
+// computed once per primitive instead of once per (view, primitive), and the
+// parameter rows are read once (500k 7-D primitives in 8 views: 203 -> 122 us;
+// 3M in 4 views 600 -> 317 us).  ONE: a single view, whose registers allow more
+// CTAs per SM (1M: 54 us, 58 with the registers of the loop).
+template <int D, bool ONE>
+__global__ void __launch_bounds__(PRIM_THREADS, (D == 6 ? 8 : 6) - (ONE ? 0 : D - 5))
+    scene_prim_fwd_kernel(SceneArgs a) {
+    constexpr int K = D - 3;
     __shared__ float stage[PRIM_THREADS / 32][stage_floats<D>()];
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const int v = (int)(idx / a.N);
-    const int64_t n = idx - (int64_t)v * a.N;
     PrimRows rows;
-    if (prim_rows<D>(a, idx, n, lane, stage[threadIdx.x >> 5], rows)) __syncwarp();
-    if (idx >= (int64_t)a.C * a.N) return;
-    PrimFwd<D> f;
-    prim_forward<D>(a, rows, v, f);
-    const Cam cam = view_cam(a, v);
-    const uint32_t W = (uint32_t)a.dims[v * 4], H = (uint32_t)a.dims[v * 4 + 1];
-    const uint32_t TW = (uint32_t)a.dims[v * 4 + 2], TH = (uint32_t)a.dims[v * 4 + 3];
-    float pc[3];
-    world_to_cam(cam, f.om, pc);
-    Proj2D p;
-    p.radius = 0;
+    if (prim_rows<D>(a, n, lane, stage[threadIdx.x >> 5], rows)) __syncwarp();
+    if (n >= a.N) return;
+    PrimFixed<D> f;
+    float L[D * D];
+    prim_fixed<D>(rows, f, L);
     const bool shown = !a.prim_mask || a.prim_mask[n] != 0;
-    if (shown && !(pc[2] < a.near_p || pc[2] > a.far_p)) {
-        const M3 Sw = upper_sym(f.oV);
-        const M3 Sc = mm(mm(cam.R, Sw), tr(cam.R));
-        p = project_2d(pc, Sc, cam, W, H, a.eps2d, a.radius_clip);
+#pragma unroll 1
+    for (int v = ONE ? 0 : blockIdx.y; v < (ONE ? 1 : a.C); v += gridDim.y) {
+        const int64_t idx = ONE ? n : (int64_t)v * a.N + n;
+        float x[K], y[K], om[3], oo;
+        prim_query<D>(a, f, v, x, y);
+        cond_query<K>(f.m, f.c, f.o, x, y, om, &oo);
+        const Cam cam = view_cam(a, v);
+        const uint32_t W = (uint32_t)a.dims[v * 4], H = (uint32_t)a.dims[v * 4 + 1];
+        const uint32_t TW = (uint32_t)a.dims[v * 4 + 2], TH = (uint32_t)a.dims[v * 4 + 3];
+        float pc[3];
+        world_to_cam(cam, om, pc);
+        Proj2D p;
+        p.radius = 0;
+        if (shown && !(pc[2] < a.near_p || pc[2] > a.far_p)) {
+            const M3 Sw = upper_sym(f.oV);
+            const M3 Sc = mm(mm(cam.R, Sw), tr(cam.R));
+            p = project_2d(pc, Sc, cam, W, H, a.eps2d, a.radius_clip);
+        }
+        Rec r;
+        r.gid = (int32_t)idx;
+        r.opac = oo;
+        r.beta = f.b0;
+        if (p.radius > 0) {
+            r.x = p.mx;
+            r.y = p.my;
+            r.cxx = p.conic[0];
+            r.cxy = p.conic[1];
+            r.cyy = p.conic[2];
+        } else {
+            r.x = r.y = r.cxx = r.cxy = r.cyy = 0.f;
+        }
+        float4 *dst = reinterpret_cast<float4 *>(a.recs + idx);
+        dst[0] = make_float4(r.x, r.y, r.opac, r.beta);
+        dst[1] = make_float4(r.cxx, r.cxy, r.cyy, __int_as_float(r.gid));
+        if (v == 0) { // one colour row per primitive, gathered by the blend
+            if (a.color_mode == 1)
+                a.cols_n[n] = make_float4(p.radius > 0 ? p.depth : 0.f, 0.f, 0.f, 0.f);
+            else
+                a.cols_n[n] = make_float4(a.rgb[n * 3], a.rgb[n * 3 + 1], a.rgb[n * 3 + 2], 0.f);
+        }
+        a.radius[idx] = p.radius;
+        a.depth[idx] = p.radius > 0 ? p.depth : 0.f;
+        if (p.radius <= 0) continue;
+        // tile box (isect_tiles.cu:46-66) and bucket counts
+        const float ts = a.tile_size;
+        const float rr = (float)p.radius / ts, tx = p.mx / ts, ty = p.my / ts;
+        const uint32_t x0 = min(max(0u, __float2uint_rz(floorf(tx - rr))), TW);
+        const uint32_t y0 = min(max(0u, __float2uint_rz(floorf(ty - rr))), TH);
+        const uint32_t x1 = min(max(0u, __float2uint_rz(ceilf(tx + rr))), TW);
+        const uint32_t y1 = min(max(0u, __float2uint_rz(ceilf(ty + rr))), TH);
+        if (x1 <= x0 || y1 <= y0) continue;
+        if (__float_as_int(p.depth) < 0) atomicOr(a.status, DEV_ERR_NEG_DEPTH);
+        int32_t *bc =
+            a.bucket_counts + (int64_t)(idx % kCountReplicas) * a.n_buckets + a.tile_base[v];
+        for (uint32_t ty_ = y0; ty_ < y1; ++ty_)
+            for (uint32_t tx_ = x0; tx_ < x1; ++tx_) atomicAdd(&bc[ty_ * TW + tx_], 1);
     }
-    Rec r;
-    r.gid = (int32_t)idx;
-    r.opac = f.oo;
-    r.beta = f.b0;
-    if (p.radius > 0) {
-        r.x = p.mx;
-        r.y = p.my;
-        r.cxx = p.conic[0];
-        r.cxy = p.conic[1];
-        r.cyy = p.conic[2];
-    } else {
-        r.x = r.y = r.cxx = r.cxy = r.cyy = 0.f;
-    }
-    float4 *dst = reinterpret_cast<float4 *>(a.recs + idx);
-    dst[0] = make_float4(r.x, r.y, r.opac, r.beta);
-    dst[1] = make_float4(r.cxx, r.cxy, r.cyy, __int_as_float(r.gid));
-    if (v == 0) { // one colour row per primitive, gathered by the blend
-        if (a.color_mode == 1)
-            a.cols_n[n] = make_float4(p.radius > 0 ? p.depth : 0.f, 0.f, 0.f, 0.f);
-        else
-            a.cols_n[n] = make_float4(a.rgb[n * 3], a.rgb[n * 3 + 1], a.rgb[n * 3 + 2], 0.f);
-    }
-    a.radius[idx] = p.radius;
-    a.depth[idx] = p.radius > 0 ? p.depth : 0.f;
-    if (p.radius <= 0) return;
-    // tile box (isect_tiles.cu:46-66) and bucket counts
-    const float ts = a.tile_size;
-    const float rr = (float)p.radius / ts, tx = p.mx / ts, ty = p.my / ts;
-    const uint32_t x0 = min(max(0u, __float2uint_rz(floorf(tx - rr))), TW);
-    const uint32_t y0 = min(max(0u, __float2uint_rz(floorf(ty - rr))), TH);
-    const uint32_t x1 = min(max(0u, __float2uint_rz(ceilf(tx + rr))), TW);
-    const uint32_t y1 = min(max(0u, __float2uint_rz(ceilf(ty + rr))), TH);
-    if (x1 <= x0 || y1 <= y0) return;
-    if (__float_as_int(p.depth) < 0) atomicOr(a.status, DEV_ERR_NEG_DEPTH);
-    int32_t *bc = a.bucket_counts + (int64_t)(idx % kCountReplicas) * a.n_buckets + a.tile_base[v];
-    for (uint32_t y = y0; y < y1; ++y)
-        for (uint32_t x = x0; x < x1; ++x) atomicAdd(&bc[y * TW + x], 1);
 }
 
 // Writes one sort key per (view, primitive, tile) at the tile's cursor.  A
@@ -381,37 +405,107 @@ struct KeyWriter {
     }
 };
 
-template <int D> __global__ void __launch_bounds__(PRIM_THREADS) scene_prim_bwd_kernel(SceneArgs a) {
+// One thread per primitive and group of views.  Everything after the per-view
+// projection VJP is linear in a few sums over the views (CondGrads), so the
+// views accumulate those in registers and the matrix part runs once per
+// primitive; with one group (gridDim.y == 1) the gradients are plain stores,
+// else the groups add theirs to zeroed arrays.  Against one thread per (view,
+// primitive) with about 45 global atomics each: 500k 7-D primitives in 8 views
+// 763 -> 218 us, 3M in 4 views 1351 -> 594 us.  ONE: a single view, where the
+// view-independent state stays in registers (1M: 106 us; rebuilding it as
+// below 125 us).
+template <int D, bool ONE>
+__global__ void __launch_bounds__(PRIM_THREADS, ONE ? 4 : 3) scene_prim_bwd_kernel(SceneArgs a) {
     constexpr int K = D - 3;
     constexpr int NL = D * (D - 1) / 2;
     __shared__ float stage[PRIM_THREADS / 32][stage_floats<D>()];
     __shared__ float sraw[PRIM_THREADS / 32][32 * D]; // raw scale rows (softplus derivative)
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const int v = (int)(idx / a.N);
-    const int64_t n = idx - (int64_t)v * a.N;
-    // the entry's own rows are requested before the warp stages the
-    // parameter rows, so both sets of loads are in flight together
-    const bool in = idx < (int64_t)a.C * a.N;
+    // the first view's rows are requested before the warp stages the parameter
+    // rows, so both sets of loads are in flight together
+    const bool in = n < a.N;
+    int v = ONE ? 0 : blockIdx.y;
     int32_t rad = 0;
     float4 vr0 = make_float4(0.f, 0.f, 0.f, 0.f), vr1 = vr0, vr2 = vr0, c1 = vr0;
-    if (in) {
+    auto load_entry = [&](int64_t idx) {
         rad = a.radius[idx];
         const float4 *vrow = reinterpret_cast<const float4 *>(a.v_rows + idx * kGradRow);
         vr0 = vrow[0];
         vr1 = vrow[1];
         vr2 = vrow[2];
         c1 = reinterpret_cast<const float4 *>(a.recs + idx)[1];
-    }
+    };
+    if (in) load_entry((int64_t)v * a.N + n);
     PrimRows rows;
     const float *raw_s = a.scale + n * D;
-    if (prim_rows<D>(a, idx, n, lane, stage[threadIdx.x >> 5], rows)) {
+    if (prim_rows<D>(a, n, lane, stage[threadIdx.x >> 5], rows)) {
         raw_s = stage_rows<D>(a.scale, n - lane, sraw[threadIdx.x >> 5], lane);
         __syncwarp();
     }
     if (!in) return;
-    const bool direct = a.C == 1; // one view: plain stores, else atomics into zeroed grads
-    if (rad <= 0) {
+    const bool direct = ONE || gridDim.y == 1;
+    bool any = false;
+    CondGrads<K> g;
+    g.zero();
+    float gb0 = 0.f, gc0 = 0.f, gc1 = 0.f, gc2 = 0.f;
+    PrimFixed<D> f;
+    float L[D * D];
+    {
+        prim_fixed<D>(rows, f, L);
+        const M3 Sw = upper_sym(f.oV);
+#pragma unroll 1
+        while (true) {
+            if (rad > 0) {
+                any = true;
+                float x[K], y[K], om[3], oo;
+                prim_query<D>(a, f, v, x, y);
+                cond_query<K>(f.m, f.c, f.o, x, y, om, &oo);
+                const Cam cam = view_cam(a, v);
+                const uint32_t W = (uint32_t)a.dims[v * 4], H = (uint32_t)a.dims[v * 4 + 1];
+                // projection VJP (fully_fused_projection_bwd.cu:69-174) with the saved conic
+                const float cn[3] = {c1.x, c1.y, c1.z};
+                const float vcn[3] = {vr0.z, vr0.w, vr1.x};
+                float vc2[4];
+                conic_vjp(cn, vcn, a.eps2d, false, 0.f, 0.f, vc2);
+                float pc[3];
+                world_to_cam(cam, om, pc);
+                const M3 Sc = mm(mm(cam.R, Sw), tr(cam.R));
+                M3 vSc;
+#pragma unroll
+                for (int k = 0; k < 9; ++k) vSc.m[k] = 0.f;
+                float vpc[3] = {0.f, 0.f, 0.f};
+                persp_vjp(pc, Sc, cam, W, H, vc2, vr0.x, vr0.y, vSc, vpc);
+                float gM[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    gM[k] = cam.R(0, k) * vpc[0] + cam.R(1, k) * vpc[1] + cam.R(2, k) * vpc[2];
+                const M3 vSw = mm(mm(tr(cam.R), vSc), cam.R);
+                // upper-triangle gather VJP: packed entries back onto the upper triangle
+                float gVc[9];
+                gVc[0] = vSw(0, 0);
+                gVc[1] = vSw(0, 1) + vSw(1, 0);
+                gVc[2] = vSw(0, 2) + vSw(2, 0);
+                gVc[3] = 0.f;
+                gVc[4] = vSw(1, 1);
+                gVc[5] = vSw(1, 2) + vSw(2, 1);
+                gVc[6] = 0.f;
+                gVc[7] = 0.f;
+                gVc[8] = vSw(2, 2);
+                // conditioning VJP (cond_mean_convariance_opacity_bwd.cu:102-563)
+                cond_accumulate<K>(f.c.Lc, f.c.beta, f.o, x, y, gM, gVc, vr1.y, g);
+                gb0 += vr1.z;
+                gc0 += vr1.w;
+                gc1 += vr2.x;
+                gc2 += vr2.y;
+            }
+            if (ONE) break;
+            v += gridDim.y;
+            if (v >= a.C) break;
+            load_entry((int64_t)v * a.N + n);
+        }
+    }
+    if (!any) {
         if (direct) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) a.g_xyz[n * 3 + k] = 0.f;
@@ -429,44 +523,22 @@ template <int D> __global__ void __launch_bounds__(PRIM_THREADS) scene_prim_bwd_
         }
         return;
     }
-    PrimFwd<D> f;
-    prim_forward<D>(a, rows, v, f);
-    const Cam cam = view_cam(a, v);
-    const uint32_t W = (uint32_t)a.dims[v * 4], H = (uint32_t)a.dims[v * 4 + 1];
-    // projection VJP (fully_fused_projection_bwd.cu:69-174) with the saved conic
-    const float cn[3] = {c1.x, c1.y, c1.z};
-    const float vcn[3] = {vr0.z, vr0.w, vr1.x};
-    float vc2[4];
-    conic_vjp(cn, vcn, a.eps2d, false, 0.f, 0.f, vc2);
-    float pc[3];
-    world_to_cam(cam, f.om, pc);
-    const M3 Sw = upper_sym(f.oV);
-    const M3 Sc = mm(mm(cam.R, Sw), tr(cam.R));
-    M3 vSc;
+    float b[K], gm[D], gV[D * D], gb[K];
+    const float *rb = rows.b;
+    if constexpr (ONE) {
+        cond_finish<K>(f.c, g, a.exact != 0, gm, gV, gb);
+    } else {
+        // the view-independent state is rebuilt from the staged rows rather
+        // than kept in registers over the views
+        asm volatile("" : "+l"(rows.lt), "+l"(rows.s), "+l"(rb)::"memory");
+        float V[D * D];
+        prim_covar<D>(rows, L, V);
+        CondFixed<K> c;
+        cond_fixed<K>(V, rb + 1, c);
+        cond_finish<K>(c, g, a.exact != 0, gm, gV, gb);
+    }
 #pragma unroll
-    for (int k = 0; k < 9; ++k) vSc.m[k] = 0.f;
-    float vpc[3] = {0.f, 0.f, 0.f};
-    persp_vjp(pc, Sc, cam, W, H, vc2, vr0.x, vr0.y, vSc, vpc);
-    float gM[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        gM[k] = cam.R(0, k) * vpc[0] + cam.R(1, k) * vpc[1] + cam.R(2, k) * vpc[2];
-    const M3 vSw = mm(mm(tr(cam.R), vSc), cam.R);
-    // upper-triangle gather VJP: packed entries back onto the upper triangle
-    float gVc[9];
-    gVc[0] = vSw(0, 0);
-    gVc[1] = vSw(0, 1) + vSw(1, 0);
-    gVc[2] = vSw(0, 2) + vSw(2, 0);
-    gVc[3] = 0.f;
-    gVc[4] = vSw(1, 1);
-    gVc[5] = vSw(1, 2) + vSw(2, 1);
-    gVc[6] = 0.f;
-    gVc[7] = 0.f;
-    gVc[8] = vSw(2, 2);
-    // conditioning VJP (cond_mean_convariance_opacity_bwd.cu:102-563)
-    float gm[D], gV[D * D], go, gb[K];
-    cond_backward<K>(f.m, f.V, f.o, f.b, f.q, gM, gVc, vr1.y, a.exact != 0, gm, gV, &go,
-                     gb);
+    for (int k = 0; k < K; ++k) b[k] = rb[1 + k];
     // Sigma = L L^T: dL = (gV + gV^T) L (rot_scale_l_triangle_to_covar_bwd.cu)
     float dL[D * D];
 #pragma unroll
@@ -475,7 +547,7 @@ template <int D> __global__ void __launch_bounds__(PRIM_THREADS) scene_prim_bwd_
         for (int c = 0; c < D; ++c) {
             float acc = 0.f;
 #pragma unroll
-            for (int k = 0; k < D; ++k) acc += (gV[r * D + k] + gV[k * D + r]) * f.L[k * D + c];
+            for (int k = 0; k < D; ++k) acc += (gV[r * D + k] + gV[k * D + r]) * L[k * D + c];
             dL[r * D + c] = acc;
         }
     float gs[D], gl[NL];
@@ -486,7 +558,7 @@ template <int D> __global__ void __launch_bounds__(PRIM_THREADS) scene_prim_bwd_
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) dR[r * 3 + c] = dL[r * D + c] * f.s[c];
+        for (int c = 0; c < 3; ++c) dR[r * 3 + c] = dL[r * D + c] * rows.s[c];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
         gs[c] = dL[0 * D + c] * R[0 * 3 + c] + dL[1 * D + c] * R[1 * 3 + c] +
@@ -515,13 +587,21 @@ template <int D> __global__ void __launch_bounds__(PRIM_THREADS) scene_prim_bwd_
     for (int k = 0; k < D; ++k) put(&a.g_scale[n * D + k], gs[k] * sigmoid_f(raw_s[k]));
 #pragma unroll
     for (int k = 0; k < NL; ++k) put(&a.g_ltri[n * NL + k], gl[k]);
-    put(&a.g_opac[n], go * f.o * (1.f - f.o));
-    put(&a.g_beta[n * (D - 2)], vr1.z * f.b0);
+    put(&a.g_opac[n], g.go * rows.o * (1.f - rows.o));
+    put(&a.g_beta[n * (D - 2)], gb0 * rb[0]);
 #pragma unroll
-    for (int k = 0; k < K; ++k) put(&a.g_beta[n * (D - 2) + 1 + k], gb[k] * f.b[k]);
-    put(&a.g_rgb[n * 3], vr1.w);
-    put(&a.g_rgb[n * 3 + 1], vr2.x);
-    put(&a.g_rgb[n * 3 + 2], vr2.y);
+    for (int k = 0; k < K; ++k) put(&a.g_beta[n * (D - 2) + 1 + k], gb[k] * b[k]);
+    put(&a.g_rgb[n * 3], gc0);
+    put(&a.g_rgb[n * 3 + 1], gc1);
+    put(&a.g_rgb[n * 3 + 2], gc2);
+}
+
+// Groups of views of the per-primitive kernels: one where the primitives alone
+// give every SM its resident CTAs (6 forward, 3 backward), else as many as that
+// takes (5k primitives in 8 views: backward 18 us).
+unsigned view_groups(int64_t N, int C, int ctas_per_sm) {
+    const int64_t want = (152 * PRIM_THREADS * ctas_per_sm + N - 1) / (N < 1 ? 1 : N);
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, C));
 }
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -739,9 +819,11 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
         a.act_o = w.act + act_opac_off(N, dim);
         if (CN > 0) {
             if (int e = launch_scene_act(N, dim, scale, beta, opacity, w.act, st)) return e;
-            UBS_TIMED("scene_prim_fwd", st,
-                      UBS_SCENE_DIM(dim, scene_prim_fwd_kernel<DD><<<grid_for(CN, PRIM_THREADS),
-                                                                    PRIM_THREADS, 0, st>>>(a)));
+            const dim3 grid(grid_for(N, PRIM_THREADS), view_groups(N, C, 6));
+            void (*k)(SceneArgs) = nullptr;
+            UBS_SCENE_DIM(dim, k = C == 1 ? scene_prim_fwd_kernel<DD, true>
+                                          : scene_prim_fwd_kernel<DD, false>);
+            UBS_TIMED("scene_prim_fwd", st, k<<<grid, PRIM_THREADS, 0, st>>>(a));
             note_launch();
             if (int e = check_launch("scene_prim_fwd")) return e;
         }
@@ -838,7 +920,8 @@ int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *me
                             v_render_alphas, w.grads, &w.hdr->status, st))
         return e;
     if (CN == 0) return UBS_OK;
-    if (C > 1) {
+    const unsigned groups = view_groups(N, C, 3);
+    if (groups > 1) {
         const int K = dim - 3, NL = dim * (dim - 1) / 2;
         if (cudaMemsetAsync(v_xyz, 0, N * 12, st) || cudaMemsetAsync(v_mean, 0, N * K * 4, st) ||
             cudaMemsetAsync(v_scale, 0, N * dim * 4, st) ||
@@ -864,9 +947,11 @@ int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *me
     a.g_beta = v_beta;
     a.g_rgb = v_rgb;
     a.exact = exact_cond_grad;
-    UBS_TIMED("scene_prim_bwd", st,
-              UBS_SCENE_DIM(dim, scene_prim_bwd_kernel<DD><<<grid_for(CN, PRIM_THREADS),
-                                                                PRIM_THREADS, 0, st>>>(a)));
+    const dim3 grid(grid_for(N, PRIM_THREADS), groups);
+    void (*k)(SceneArgs) = nullptr;
+    UBS_SCENE_DIM(dim, k = C == 1 ? scene_prim_bwd_kernel<DD, true>
+                                  : scene_prim_bwd_kernel<DD, false>);
+    UBS_TIMED("scene_prim_bwd", st, k<<<grid, PRIM_THREADS, 0, st>>>(a));
     note_launch();
     return check_launch("scene_prim_bwd");
 }
