@@ -12,8 +12,7 @@ constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_TILE = SCAN_ITEMS * SCAN_THREADS;
 constexpr int WARP_SEG = 1024;  // longest bucket sorted by one warp in registers
 constexpr int SMALL_SEG = 4096; // longest bucket sorted by one CTA in shared memory
-constexpr int SORT_THREADS = 256;
-constexpr int BIG_THREADS = 1024;
+constexpr int BIG_THREADS = 512;
 constexpr int MERGE_ITEMS = 8;
 constexpr int EMIT_ROUNDS = 4; // (entry, tile) rounds of 32 whose cursor atomics overlap
 
@@ -136,26 +135,6 @@ inline int device_exclusive_scan(const int32_t *in, OutT *out, int64_t n, int64_
 // sorted position, bucket) stores one sorted entry.  The intersection count
 // is read on the device when T_dev is given (clamped to the key capacity
 // cap), else it is cap, so no host round trip is needed.
-
-// In-place bitonic sort of s[0..n2) (n2 a power of two) by the whole CTA.
-__device__ __forceinline__ void block_bitonic(uint64_t *s, int n2) {
-    for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const uint64_t a = s[i], b = s[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        s[i] = b;
-                        s[ixj] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
 
 __device__ __forceinline__ void bucket_range(const int32_t *offsets, int64_t bkt, int64_t n_buckets,
                                              int64_t T, int64_t &lo, int64_t &hi) {
@@ -484,33 +463,239 @@ __device__ __forceinline__ void warp_bitonic(uint64_t (&v)[E], int lane) {
     }
 }
 
-template <int E, typename Writer>
-__device__ __forceinline__ void warp_sort_bucket(const uint64_t *__restrict__ keys, int64_t lo,
-                                                 int n, int64_t bkt, int lane, const Writer &w) {
+// The same network on 32-bit values: a compare-exchange is one minimum or
+// maximum per value instead of a 64-bit comparison and two selects.
+template <int E, int J>
+__device__ __forceinline__ void bitonic32_in_lane(uint32_t (&v)[E], bool up) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int p = e ^ J;
+        if (p > e) {
+            const uint32_t a = v[e], b = v[p];
+            v[e] = up ? min(a, b) : max(a, b);
+            v[p] = up ? max(a, b) : min(a, b);
+        }
+    }
+}
+template <int E, int K, int J> struct Bitonic32RunStage {
+    static __device__ __forceinline__ void run(uint32_t (&v)[E]) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int p = e ^ J;
+            if (p > e) {
+                const uint32_t a = v[e], b = v[p];
+                v[e] = (e & K) == 0 ? min(a, b) : max(a, b);
+                v[p] = (e & K) == 0 ? max(a, b) : min(a, b);
+            }
+        }
+        Bitonic32RunStage<E, K, J / 2>::run(v);
+    }
+};
+template <int E, int K> struct Bitonic32RunStage<E, K, 0> {
+    static __device__ __forceinline__ void run(uint32_t (&)[E]) {}
+};
+template <int E, int K> struct Bitonic32Runs {
+    static __device__ __forceinline__ void run(uint32_t (&v)[E]) {
+        Bitonic32RunStage<E, K, K / 2>::run(v);
+        Bitonic32Runs<E, (2 * K < E ? 2 * K : 0)>::run(v);
+    }
+};
+template <int E> struct Bitonic32Runs<E, 0> {
+    static __device__ __forceinline__ void run(uint32_t (&)[E]) {}
+};
+// The passes of stage k whose distances stay inside a warp (from j down).
+template <int E>
+__device__ __forceinline__ void bitonic32_in_warp(uint32_t (&v)[E], int lane, int j, bool up) {
+#pragma unroll 1
+    for (; j >= E; j >>= 1) { // across lanes
+        const int lj = j / E;
+        const bool keep_min = ((lane & lj) == 0) == up;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const uint32_t o = __shfl_xor_sync(0xffffffffu, v[e], lj);
+            v[e] = keep_min ? min(v[e], o) : max(v[e], o);
+        }
+    }
+    if (E >= 32) bitonic32_in_lane<E, (E >= 32 ? 16 : 1)>(v, up);
+    if (E >= 16) bitonic32_in_lane<E, (E >= 16 ? 8 : 1)>(v, up);
+    if (E >= 8) bitonic32_in_lane<E, (E >= 8 ? 4 : 1)>(v, up);
+    if (E >= 4) bitonic32_in_lane<E, (E >= 4 ? 2 : 1)>(v, up);
+    if (E >= 2) bitonic32_in_lane<E, 1>(v, up);
+}
+// Sorts the values of W warps, E per thread (thread t of the W warps holds
+// elements t E ..); xch: shared memory of W 32 E values (W > 1, whose warps are
+// the whole CTA).
+template <int E, int W>
+__device__ __forceinline__ void bitonic32(uint32_t (&v)[E], int t, uint32_t *xch) {
+    constexpr int N = 32 * E;
+    Bitonic32Runs<E, (E >= 4 ? 2 : 0)>::run(v);
+#pragma unroll 1
+    for (int k = E >= 2 ? E : 2; k <= N; k <<= 1)
+        bitonic32_in_warp<E>(v, t & 31, k >> 1, ((t * E) & k) == 0);
+    if (W > 1) {
+#pragma unroll 1
+        for (int k = 2 * N; k <= W * N; k <<= 1) {
+            const bool up = ((t * E) & k) == 0;
+#pragma unroll 1
+            for (int j = k >> 1; j >= N; j >>= 1) { // across warps
+                const int tj = j / E;
+                const bool keep_min = ((t & tj) == 0) == up;
+                __syncthreads();
+#pragma unroll
+                for (int e = 0; e < E; ++e) xch[e * 32 * W + t] = v[e];
+                __syncthreads();
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const uint32_t o = xch[e * 32 * W + (t ^ tj)];
+                    v[e] = keep_min ? min(v[e], o) : max(v[e], o);
+                }
+            }
+            bitonic32_in_warp<E>(v, t & 31, N >> 1, up);
+        }
+    }
+}
+
+// Shared memory of one warp's sort: its keys and their order.
+constexpr int ORDER_PITCH(int E) { return E + 2; } // 16-bit slots per lane, odd in words
+constexpr size_t WARP_SORT_SMEM = WARP_SEG * sizeof(uint64_t) + 32 * ORDER_PITCH(32) * 2;
+
+// Sorts n <= 32 E W unique keys src[0..n) with W warps (one warp, or all of a
+// CTA's) and hands each to put(position, key).  sk (32 E W keys), si (32 W
+// ORDER_PITCH(E) indices) and, for W > 1, xch are shared memory; src may be
+// where put stores.
+// The network runs on 32-bit composites: the depth bits above the smallest of
+// the bucket (the entry bits where all depths are equal), shifted so that they
+// leave room for the key's index among the n (a 1080p bucket of 500 keys keeps
+// depth to 1 or 2 units in the last place).  Keys that agree in the bits kept
+// come out in index order, so odd-even rounds on the index list exchange
+// neighbours out of order until one finds none (nearly always the first or the
+// second).  Returns false where that does not end soon -- many keys of a few
+// depths -- with sk holding the keys as they came and put not called.
+template <int E, int W, typename Put>
+__device__ __forceinline__ bool sort_keys32(const uint64_t *src, int n, int t, uint64_t *sk,
+                                            uint16_t *si, uint32_t *xch, Put put) {
+    constexpr int T = 32 * W, N = T * E, P = ORDER_PITCH(E);
+    constexpr int IB = N <= 32 ? 5 : N <= 64 ? 6 : N <= 128 ? 7 : N <= 256 ? 8 : N <= 512 ? 9
+                       : N <= 1024 ? 10 : N <= 2048 ? 11 : 12;
+    auto sync = []() {
+        if (W > 1) __syncthreads();
+        else __syncwarp();
+    };
+    auto any = [](bool b) {
+        return W > 1 ? __syncthreads_or(b) != 0 : __any_sync(0xffffffffu, b) != 0;
+    };
+    __shared__ uint32_t range[W > 1 ? 2 * W : 1];
+    // smallest and largest value over the keys
+    auto span = [&](const uint32_t (&c)[E], uint32_t &lo, uint32_t &hi) {
+        lo = ~0u;
+        hi = 0u;
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (e * T + t < n) {
+                lo = min(lo, c[e]);
+                hi = max(hi, c[e]);
+            }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (W > 1) {
+            __syncthreads();
+            if ((t & 31) == 0) {
+                range[t >> 5] = lo;
+                range[W + (t >> 5)] = hi;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                lo = min(lo, range[w]);
+                hi = max(hi, range[W + w]);
+            }
+        }
+    };
+    uint32_t c[E], lo, hi;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = e * T + t;
+        c[e] = 0u;
+        if (i < n) {
+            const uint64_t k = src[i];
+            sk[i] = k;
+            c[e] = (uint32_t)(k >> 32);
+        }
+    }
+    span(c, lo, hi);
+    if (lo == hi) { // the same in every thread
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (e * T + t < n) c[e] = (uint32_t)sk[e * T + t];
+        span(c, lo, hi);
+    }
+    const int shift = max(0, IB - __clz(hi - lo));
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = e * T + t;
+        c[e] = i < n ? ((c[e] - lo) >> shift) << IB | (uint32_t)i : ~0u;
+    }
+    bitonic32<E, W>(c, t, xch);
+#pragma unroll
+    for (int e = 0; e < E; ++e) si[t * P + e] = (uint16_t)(c[e] & (N - 1));
+    sync();
+    auto slot = [](int p) { return p / E * P + p % E; };
+    // odd-even rounds: one without an exchange shows that the sequence is sorted
+    bool sorted = false;
+#pragma unroll 1
+    for (int round = 0; round < 6 && !sorted; ++round) {
+        bool swapped = false;
+#pragma unroll 1
+        for (int odd = 0; odd < 2; ++odd) {
+#pragma unroll 4
+            for (int p = 2 * t + odd; p + 1 < n; p += 2 * T) {
+                const uint16_t a = si[slot(p)], b = si[slot(p + 1)];
+                if (sk[a] > sk[b]) {
+                    si[slot(p)] = b;
+                    si[slot(p + 1)] = a;
+                    swapped = true;
+                }
+            }
+            if (W == 1 || !odd) sync(); // any() is the barrier of several warps
+        }
+        sorted = !any(swapped);
+    }
+    if (!sorted) return false;
+#pragma unroll 4
+    for (int p = t; p < n; p += T) put(p, sk[si[slot(p)]]);
+    return true;
+}
+
+// One warp: the above, and the 64-bit network where it gives up.
+template <int E, typename Put>
+__device__ __forceinline__ void warp_sort_keys(const uint64_t *src, int n, int lane, uint64_t *sk,
+                                               uint16_t *si, Put put) {
+    if (sort_keys32<E, 1>(src, n, lane, sk, si, nullptr, put)) return;
     uint64_t v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int i = lane * E + e;
-        v[e] = i < n ? keys[lo + i] : ~0ull;
+        v[e] = i < n ? sk[i] : ~0ull;
     }
     warp_bitonic<E>(v, lane);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int i = lane * E + e;
-        if (i < n) w(v[e], lo + i, bkt);
+        if (i < n) put(i, v[e]);
     }
 }
 
-// One warp per bucket for buckets of at most WARP_SEG keys (padded to the
-// next power of two >= 32 with all-ones keys, which sort last); longer
-// buckets go to the device-side lists: mid (<= SMALL_SEG) from the front of
-// `lists`, big from the back.  counters = {n_big, n_mid}.
+// One warp per bucket for buckets of at most WARP_SEG keys; longer buckets go
+// to the device-side lists: mid (<= SMALL_SEG) from the front of `lists`, big
+// from the back.  counters = {n_big, n_mid}.
+constexpr int SORT_WARPS = 4;
 template <typename Writer>
-__global__ void __launch_bounds__(256, 3) bucket_sort_warp_kernel(
+__global__ void __launch_bounds__(SORT_WARPS * 32, 5) bucket_sort_warp_kernel(
     int64_t n_buckets, const int32_t *__restrict__ offsets, const int64_t *T_dev, int64_t cap,
-    const uint64_t *__restrict__ keys, int32_t *lists, int32_t *counters, Writer w) {
-    const int lane = threadIdx.x & 31;
-    const int64_t bkt = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const uint64_t *keys, int32_t *lists, int32_t *counters, Writer w) {
+    __shared__ __align__(16) unsigned char sm[SORT_WARPS][WARP_SORT_SMEM];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t bkt = (int64_t)blockIdx.x * SORT_WARPS + warp;
     if (bkt >= n_buckets) return;
     const int64_t T = T_dev ? imin64(*T_dev, cap) : cap;
     int64_t lo, hi;
@@ -525,12 +710,15 @@ __global__ void __launch_bounds__(256, 3) bucket_sort_warp_kernel(
         return;
     }
     const int m = (int)n;
-    if (m <= 32) warp_sort_bucket<1>(keys, lo, m, bkt, lane, w);
-    else if (m <= 64) warp_sort_bucket<2>(keys, lo, m, bkt, lane, w);
-    else if (m <= 128) warp_sort_bucket<4>(keys, lo, m, bkt, lane, w);
-    else if (m <= 256) warp_sort_bucket<8>(keys, lo, m, bkt, lane, w);
-    else if (m <= 512) warp_sort_bucket<16>(keys, lo, m, bkt, lane, w);
-    else warp_sort_bucket<32>(keys, lo, m, bkt, lane, w);
+    uint64_t *sk = reinterpret_cast<uint64_t *>(sm[warp]);
+    uint16_t *si = reinterpret_cast<uint16_t *>(sk + WARP_SEG);
+    auto put = [&](int p, uint64_t k) { w(k, lo + p, bkt); };
+    if (m <= 32) warp_sort_keys<1>(keys + lo, m, lane, sk, si, put);
+    else if (m <= 64) warp_sort_keys<2>(keys + lo, m, lane, sk, si, put);
+    else if (m <= 128) warp_sort_keys<4>(keys + lo, m, lane, sk, si, put);
+    else if (m <= 256) warp_sort_keys<8>(keys + lo, m, lane, sk, si, put);
+    else if (m <= 512) warp_sort_keys<16>(keys + lo, m, lane, sk, si, put);
+    else warp_sort_keys<32>(keys + lo, m, lane, sk, si, put);
 }
 
 // merge path: number of elements taken from a for output diagonal d
@@ -545,82 +733,76 @@ __device__ __forceinline__ int64_t merge_split(const uint64_t *a, int64_t na, co
     return lo;
 }
 
+// In-place bitonic sort of s[0..n2) (n2 a power of two) by the whole CTA.
+__device__ __forceinline__ void block_bitonic(uint64_t *s, int n2) {
+    for (int k = 2; k <= n2; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+                const int ixj = i ^ j;
+                if (ixj > i) {
+                    const uint64_t a = s[i], b = s[ixj];
+                    const bool up = (i & k) == 0;
+                    if ((a > b) == up) {
+                        s[i] = b;
+                        s[ixj] = a;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // Buckets of WARP_SEG < n <= SMALL_SEG keys (the mid list): a fixed grid walks
-// the device-side list with one CTA of MID_WARPS warps per bucket.  Warp c
-// sorts keys [c WARP_SEG, (c + 1) WARP_SEG) in registers (warp_bitonic, 32 per
-// lane), the sorted runs are merged pairwise in shared memory by merge path,
-// and the last merge hands the sorted keys to the writer: two barriers per
-// merge level instead of one per bitonic stage (78 for 4096 keys).
-constexpr int MID_WARPS = SMALL_SEG / WARP_SEG;
-constexpr size_t MID_SMEM = 2 * SMALL_SEG * sizeof(uint64_t);
+// the device-side list with one CTA of MID_WARPS warps per bucket, whose
+// threads run the 32-bit network together, 16 or 32 values each.
+constexpr int MID_WARPS = 4;
+constexpr size_t MID_SMEM = SMALL_SEG * (sizeof(uint64_t) + sizeof(uint32_t)) +
+                            MID_WARPS * 32 * ORDER_PITCH(32) * sizeof(uint16_t);
 template <typename Writer>
-__global__ void __launch_bounds__(MID_WARPS * 32, 3) bucket_sort_mid_kernel(
+__global__ void __launch_bounds__(MID_WARPS * 32, 4) bucket_sort_mid_kernel(
     int64_t n_buckets, const int32_t *__restrict__ offsets, const int64_t *T_dev, int64_t cap,
-    const uint64_t *__restrict__ keys, const int32_t *lists, const int32_t *counters, Writer w) {
-    extern __shared__ __align__(16) uint64_t mid_runs[]; // two buffers of SMALL_SEG
+    const uint64_t *keys, const int32_t *lists, const int32_t *counters, Writer w) {
+    extern __shared__ __align__(16) uint64_t mid_keys[]; // keys, exchange buffer, order
+    uint32_t *xch = reinterpret_cast<uint32_t *>(mid_keys + SMALL_SEG);
+    uint16_t *si = reinterpret_cast<uint16_t *>(xch + SMALL_SEG);
     const int n_mid = counters[1];
     const int64_t T = T_dev ? imin64(*T_dev, cap) : cap;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int item = blockIdx.x; item < n_mid; item += gridDim.x) {
         __syncthreads();
         const int64_t bkt = lists[item];
         int64_t lo, hi;
         bucket_range(offsets, bkt, n_buckets, T, lo, hi);
         const int n = (int)(hi - lo);
-        const int c0 = warp * WARP_SEG;
-        if (c0 < n) {
-            uint64_t v[32];
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                const int i = c0 + lane * 32 + e;
-                v[e] = i < n ? keys[lo + i] : ~0ull;
-            }
-            warp_bitonic<32>(v, lane);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) { // the padding keys sort last: only real keys
-                const int i = c0 + lane * 32 + e;
-                if (i < n) mid_runs[i] = v[e];
-            }
-        }
+        auto put = [&](int p, uint64_t k) { w(k, lo + p, bkt); };
+        const bool done =
+            n <= 2048 ? sort_keys32<16, MID_WARPS>(keys + lo, n, threadIdx.x, mid_keys, si, xch, put)
+                      : sort_keys32<32, MID_WARPS>(keys + lo, n, threadIdx.x, mid_keys, si, xch, put);
+        if (done) continue; // the same in every thread
+        int n2 = 2048;
+        while (n2 < n) n2 <<= 1;
+        for (int i = n + threadIdx.x; i < n2; i += blockDim.x) mid_keys[i] = ~0ull;
         __syncthreads();
-        uint64_t *src = mid_runs, *dst = mid_runs + SMALL_SEG;
-        for (int width = WARP_SEG; width < n; width <<= 1) {
-            const bool last = 2 * width >= n;
-            for (int r0 = 0; r0 < n; r0 += 2 * width) {
-                const int na = min(width, n - r0), nb = min(width, n - r0 - na);
-                const uint64_t *A = src + r0, *Bv = src + r0 + na;
-                const int total = na + nb;
-                for (int o0 = threadIdx.x * MERGE_ITEMS; o0 < total;
-                     o0 += blockDim.x * MERGE_ITEMS) {
-                    int ia = (int)merge_split(A, na, Bv, nb, o0);
-                    int ib = o0 - ia;
-                    const int oend = min(total, o0 + MERGE_ITEMS);
-                    for (int o = o0; o < oend; ++o) {
-                        const bool take_a = ib >= nb || (ia < na && A[ia] < Bv[ib]);
-                        const uint64_t key = take_a ? A[ia++] : Bv[ib++];
-                        if (last) w(key, lo + r0 + o, bkt);
-                        else dst[r0 + o] = key;
-                    }
-                }
-            }
-            __syncthreads();
-            uint64_t *t = src;
-            src = dst;
-            dst = t;
-        }
+        block_bitonic(mid_keys, n2);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) put(i, mid_keys[i]);
     }
 }
 
 // Long buckets (their number is known only on the device): a fixed grid walks
-// the device-side list; each CTA sorts SMALL_SEG chunks in shared memory, then
-// merges runs pairwise in global memory (keys <-> scratch).
+// the device-side list; the warps of a CTA sort runs of WARP_SEG keys in
+// place, which the CTA merges pairwise in global memory (keys <-> scratch).
+constexpr int BIG_WARPS = BIG_THREADS / 32;
+constexpr size_t BIG_SMEM = BIG_WARPS * WARP_SORT_SMEM;
 template <typename Writer>
 __global__ void __launch_bounds__(BIG_THREADS) bucket_sort_big_kernel(
     int64_t n_buckets, const int32_t *__restrict__ offsets, const int64_t *T_dev, int64_t cap,
     uint64_t *keys, uint64_t *scratch, const int32_t *lists, const int32_t *counters, Writer w) {
-    __shared__ uint64_t s[SMALL_SEG];
+    extern __shared__ __align__(16) unsigned char big_sm[];
     const int n_big = counters[0];
     const int64_t T = T_dev ? imin64(*T_dev, cap) : cap;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t *sk = reinterpret_cast<uint64_t *>(big_sm + warp * WARP_SORT_SMEM);
+    uint16_t *si = reinterpret_cast<uint16_t *>(sk + WARP_SEG);
     for (int item = blockIdx.x; item < n_big; item += gridDim.x) {
         __syncthreads();
         const int64_t bkt = lists[n_buckets - 1 - item];
@@ -628,15 +810,13 @@ __global__ void __launch_bounds__(BIG_THREADS) bucket_sort_big_kernel(
         bucket_range(offsets, bkt, n_buckets, T, lo, hi);
         const int64_t n = hi - lo;
         uint64_t *src = keys + lo, *dst = scratch + lo;
-        for (int64_t c0 = 0; c0 < n; c0 += SMALL_SEG) {
-            const int cn = (int)imin64(SMALL_SEG, n - c0);
-            for (int i = threadIdx.x; i < SMALL_SEG; i += blockDim.x) s[i] = i < cn ? src[c0 + i] : ~0ull;
-            __syncthreads();
-            block_bitonic(s, SMALL_SEG);
-            for (int i = threadIdx.x; i < cn; i += blockDim.x) src[c0 + i] = s[i];
-            __syncthreads();
+        for (int64_t c0 = (int64_t)warp * WARP_SEG; c0 < n; c0 += (int64_t)BIG_WARPS * WARP_SEG) {
+            __syncwarp();
+            warp_sort_keys<32>(src + c0, (int)imin64(WARP_SEG, n - c0), lane, sk, si,
+                               [&](int p, uint64_t k) { src[c0 + p] = k; });
         }
-        for (int64_t width = SMALL_SEG; width < n; width <<= 1) {
+        __syncthreads();
+        for (int64_t width = WARP_SEG; width < n; width <<= 1) {
             for (int64_t r0 = 0; r0 < n; r0 += 2 * width) {
                 const int64_t na = imin64(width, n - r0);
                 const int64_t nb = imin64(width, n - r0 - na);
@@ -674,12 +854,13 @@ inline int launch_bucket_sort(int64_t n_buckets, const int32_t *offsets, const i
     if (n_buckets <= 0 || cap <= 0) return UBS_OK;
     if (cudaMemsetAsync(counters, 0, 8, st) != cudaSuccess) return check_launch("sort memset");
     UBS_TIMED("bucket_sort_warp", st,
-              bucket_sort_warp_kernel<Writer><<<grid_for(n_buckets, 8), 256, 0, st>>>(
+              bucket_sort_warp_kernel<Writer>
+              <<<grid_for(n_buckets, SORT_WARPS), SORT_WARPS * 32, 0, st>>>(
                   n_buckets, offsets, T_dev, cap, keys, lists, counters, w));
     note_launch();
     if (cap > WARP_SEG) {
         const int64_t max_mid = cap / (WARP_SEG + 1);
-        const unsigned grid = (unsigned)imin64(imin64(max_mid, n_buckets), 152 * 6);
+        const unsigned grid = (unsigned)imin64(imin64(max_mid, n_buckets), 152 * 8);
         if (cudaFuncSetAttribute(bucket_sort_mid_kernel<Writer>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)MID_SMEM) != cudaSuccess)
@@ -691,10 +872,14 @@ inline int launch_bucket_sort(int64_t n_buckets, const int32_t *offsets, const i
     }
     if (cap > SMALL_SEG) {
         const int64_t max_big = cap / (SMALL_SEG + 1);
-        const unsigned grid = (unsigned)imin64(imin64(max_big, n_buckets), 304);
+        const unsigned grid = (unsigned)imin64(imin64(max_big, n_buckets), 152);
         if (grid > 0) {
+            if (cudaFuncSetAttribute(bucket_sort_big_kernel<Writer>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)BIG_SMEM) != cudaSuccess)
+                return check_launch("bucket_sort_big attribute");
             UBS_TIMED("bucket_sort_big", st,
-                      bucket_sort_big_kernel<Writer><<<grid, BIG_THREADS, 0, st>>>(
+                      bucket_sort_big_kernel<Writer><<<grid, BIG_THREADS, BIG_SMEM, st>>>(
                           n_buckets, offsets, T_dev, cap, keys, scratch, lists, counters, w));
             note_launch();
         }

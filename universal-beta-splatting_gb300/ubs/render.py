@@ -113,6 +113,10 @@ class Renderer:
             self.capacity = max(self.capacity or 0, int(T * 1.25) + 1024)
             raise RuntimeError("scene render: an earlier unchecked frame needed %d intersections "
                                "but had capacity %d; capacity is now %d" % (T, cap, self.capacity))
+        if T > cap - cap // 8:
+            # a scene that grows from frame to frame (training) gets its room
+            # before a frame overflows
+            self.capacity = max(self.capacity or 0, int(T * 1.25) + 1024)
 
     def stats(self):
         """(intersections, status bits) of the last forward's workspace; raises
