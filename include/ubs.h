@@ -520,10 +520,11 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
                              void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
                              int32_t color_mode, void *stream);
 /* ubs_scene_forward_masked in two parts, so that a caller can read the
- * intersection count (ubs_scene_stats' two values are the first 16 bytes of
- * the workspace) as soon as it is known: UBS_SCENE_PART_COUNT runs everything
- * up to it, UBS_SCENE_PART_BLEND the rest, both the whole frame.  The two parts
- * of a frame take the same arguments, in this order, on one stream. */
+ * intersection count as soon as it is known: UBS_SCENE_PART_COUNT runs
+ * everything up to it and, when host_counts is not NULL, writes
+ * ubs_scene_stats' two values there (pinned host memory the device can write);
+ * UBS_SCENE_PART_BLEND runs the rest, both the whole frame.  The two parts of a
+ * frame take the same arguments, in this order, on one stream. */
 #define UBS_SCENE_PART_COUNT 1
 #define UBS_SCENE_PART_BLEND 2
 int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const float *mean,
@@ -537,7 +538,8 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
                             const float *backgrounds, float *render_colors,
                             float *render_alphas, int32_t *last_ids, int64_t capacity,
                             void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
-                            int32_t color_mode, int32_t parts, void *stream);
+                            int32_t color_mode, int32_t parts, int64_t *host_counts,
+                            void *stream);
 int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *mean,
                        const float *scale, const float *l_triangle, const float *opacity,
                        const float *beta, const float *rgb, int32_t C, const float *viewmats,

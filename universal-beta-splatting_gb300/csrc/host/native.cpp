@@ -18,6 +18,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/CachingHostAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 #include <torch/csrc/autograd/function.h>
@@ -252,25 +253,30 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
     Tensor colors = fempty({c->n_pixels, 3}, p[0]), alphas = fempty({c->n_pixels}, p[0]);
     Tensor last = at::empty({c->n_pixels}, p[0].options().dtype(at::kInt));
     void *st = stream_of(p[0]);
-    auto part = [&](int32_t parts) {
+    auto part = [&](int32_t parts, int64_t *counts) {
         UBS_CALL(ubs_scene_forward_parts, c->dim, N, fp(p[0]), fp(p[1]), fp(p[2]), fp(p[3]),
                  fp(p[4]), fp(p[5]), fp(p[6]), c->C, fp(c->viewmats), fp(c->intr), fp(c->centers),
                  fp(c->times), c->dims.const_data_ptr<int32_t>(),
                  c->tile_base.const_data_ptr<int32_t>(), c->pix_base.const_data_ptr<int64_t>(),
                  c->n_buckets, c->tile, c->eps2d, c->near_p, c->far_p, c->clip, fp(b),
                  fpm(colors), fpm(alphas), last.mutable_data_ptr<int32_t>(), c->cap,
-                 c->ws.mutable_data_ptr(), c->ws.nbytes(), m, color_mode, parts, st);
+                 c->ws.mutable_data_ptr(), c->ws.nbytes(), m, color_mode, parts, counts, st);
     };
     py::object fs = py::none();
     if (!stats) {
-        part(UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND);
+        part(UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND, nullptr);
     } else {
-        part(UBS_SCENE_PART_COUNT);
+        // the count kernel writes to the pinned slot itself: a copy would make
+        // the frame wait for the copy engine
         auto s = std::make_shared<FrameStats>();
         s->host = at::empty({2}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
-        s->host.copy_(c->ws.narrow(0, 0, 16).view(at::kLong), /*non_blocking=*/true);
-        s->ev.record(c10::cuda::getCurrentCUDAStream(p[0].device().index()));
-        part(UBS_SCENE_PART_BLEND);
+        part(UBS_SCENE_PART_COUNT, s->host.mutable_data_ptr<int64_t>());
+        const auto cs = c10::cuda::getCurrentCUDAStream(p[0].device().index());
+        s->ev.record(cs);
+        // the slot outlives the kernel's write
+        at::cuda::CachingHostAllocator_recordEvent(s->host.mutable_data_ptr(),
+                                                   s->host.storage().data_ptr().get_context(), cs);
+        part(UBS_SCENE_PART_BLEND, nullptr);
         fs = py::cast(s);
     }
     Tensor ws = c->ws;

@@ -617,7 +617,7 @@ struct SceneWs {
     float4 *cols_n;
     float *grads; // one kGradRow-float gradient row per (view, primitive) entry
     float *act;   // activated parameters (scene_act.cu)
-    size_t bytes;
+    size_t zero_bytes, bytes;
 };
 
 SceneWs scene_ws(void *base, int32_t C, int64_t N, int32_t nb, int64_t cap) {
@@ -630,11 +630,13 @@ SceneWs scene_ws(void *base, int32_t C, int64_t N, int32_t nb, int64_t cap) {
         o = al256(o + bytes);
         return q;
     };
+    // the header and the counters, zeroed together
     w.hdr = reinterpret_cast<SceneHeader *>(take(sizeof(SceneHeader)));
+    w.bucket_counts = reinterpret_cast<int32_t *>(take((size_t)nb * kCountReplicas * 4));
+    w.zero_bytes = o;
     w.recs = reinterpret_cast<Rec *>(take(CN * sizeof(Rec)));
     w.radius = reinterpret_cast<int32_t *>(take(CN * 4));
     w.depth = reinterpret_cast<float *>(take(CN * 4));
-    w.bucket_counts = reinterpret_cast<int32_t *>(take((size_t)nb * kCountReplicas * 4));
     w.offsets = reinterpret_cast<int32_t *>(take((size_t)(nb + 1) * 4));
     w.cursor = reinterpret_cast<int32_t *>(take((size_t)nb * kCountReplicas * 4));
     w.totals = reinterpret_cast<int32_t *>(take((size_t)nb * 4));
@@ -762,7 +764,7 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
         timestamps, view_dims, tile_base, pix_base, n_buckets, tile_size, eps2d, near_plane,
         far_plane, radius_clip, backgrounds, render_colors, render_alphas, last_ids, capacity,
         workspace, workspace_bytes, prim_mask, color_mode,
-        UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND, stream);
+        UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND, nullptr, stream);
 }
 
 int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const float *mean,
@@ -776,7 +778,8 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
                             const float *backgrounds, float *render_colors,
                             float *render_alphas, int32_t *last_ids, int64_t capacity,
                             void *workspace, size_t workspace_bytes, const uint8_t *prim_mask,
-                            int32_t color_mode, int32_t parts, void *stream) {
+                            int32_t color_mode, int32_t parts, int64_t *host_counts,
+                            void *stream) {
     SceneArgs a{};
     if (int e = scene_common(a, dim, N, xyz, mean, scale, l_triangle, opacity, beta, rgb, C,
                              viewmats, intrinsics, centers, timestamps, view_dims, tile_base,
@@ -801,11 +804,9 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t CN = (int64_t)C * N;
     UBS_REQUIRE(parts >= 1 && parts <= 3, "scene_forward: parts %d", parts);
-    const bool one_cta = n_buckets <= SCAN_ORDER_MAX;
+    const bool one_scan = n_buckets <= SCAN_ORDER_MAX;
     if (parts & UBS_SCENE_PART_COUNT) {
-        if (cudaMemsetAsync(w.hdr, 0, sizeof(SceneHeader), st) != cudaSuccess ||
-            cudaMemsetAsync(w.bucket_counts, 0, (size_t)n_buckets * kCountReplicas * 4, st) !=
-                cudaSuccess)
+        if (cudaMemsetAsync(w.hdr, 0, w.zero_bytes, st) != cudaSuccess)
             return check_launch("scene_forward memset");
         a.recs = w.recs;
         a.cols_n = w.cols_n;
@@ -827,15 +828,13 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
             note_launch();
             if (int e = check_launch("scene_prim_fwd")) return e;
         }
-        // bucket offsets, total and heaviest-first order: one CTA when the
+        // bucket offsets, total and heaviest-first order: one cluster when the
         // buckets fit it, else a device-wide scan and the order kernel below
-        if (one_cta) {
-            UBS_TIMED("bucket_scan_order", st,
-                      bucket_scan_order_kernel<kCountReplicas><<<1, 1024, 0, st>>>(
-                          w.bucket_counts, n_buckets, w.offsets, &w.hdr->total, w.order, w.cursor,
-                          w.totals));
-            note_launch();
-            if (int e = check_launch("bucket_scan_order")) return e;
+        if (one_scan) {
+            if (int e = launch_bucket_scan_order<kCountReplicas>(
+                    w.bucket_counts, n_buckets, w.offsets, &w.hdr->total, w.order, w.cursor,
+                    &w.hdr->status, host_counts, st))
+                return e;
         } else {
             UBS_TIMED("fold_replicas", st,
                       fold_replicas_kernel<kCountReplicas><<<grid_for(n_buckets, 256), 256, 0, st>>>(
@@ -850,6 +849,9 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
                           w.bucket_counts, n_buckets, w.offsets, w.cursor));
             note_launch();
             if (int e = check_launch("replica_cursors")) return e;
+            if (host_counts && cudaMemcpyAsync(host_counts, w.hdr, 16, cudaMemcpyDeviceToHost,
+                                               st) != cudaSuccess)
+                return check_launch("scene_forward counts");
         }
     }
     if (!(parts & UBS_SCENE_PART_BLEND)) return UBS_OK;
@@ -863,9 +865,9 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
     }
     const KeyWriter wr{w.keys};
     if (int e = launch_bucket_sort(n_buckets, w.offsets, &w.hdr->total, capacity, w.keys,
-                                   w.scratch, w.big_list, &w.hdr->n_big, wr, st))
+                                   w.scratch, w.big_list, &w.hdr->n_big, wr, st, true))
         return e;
-    if (!one_cta) {
+    if (!one_scan) {
         UBS_TIMED("bucket_order", st,
                   bucket_order_kernel<<<1, 1024, 0, st>>>(w.offsets, &w.hdr->total, capacity,
                                                           n_buckets, w.order));

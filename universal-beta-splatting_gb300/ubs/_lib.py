@@ -73,7 +73,7 @@ SIGNATURES = {
                                  + [_I64, _P, _SZ, _P, _I32, _P], _INT),
     "ubs_scene_forward_parts": ([_I32, _I64] + [_P] * 7 + [_I32] + [_P] * 7
                                 + [_I32, _I32, _F, _F, _F, _F] + [_P] * 4
-                                + [_I64, _P, _SZ, _P, _I32, _I32, _P], _INT),
+                                + [_I64, _P, _SZ, _P, _I32, _I32, _P, _P], _INT),
     "ubs_scene_backward": ([_I32, _I64] + [_P] * 7 + [_I32] + [_P] * 7 + [_I32, _I32, _F, _F, _F, _F]
                            + [_P] * 5 + [_P] * 7 + [_I32, _I64, _P, _SZ, _P], _INT),
     "ubs_scene_stats": ([_P, _I64P, _U32P, _P], _INT),
