@@ -6,118 +6,177 @@
 
 namespace ubs {
 
-// ------------------------------------------------------------------ a2
-__global__ void rotmat_fwd_kernel(int64_t n, const float *__restrict__ l, int64_t stride,
-                                  float *__restrict__ R) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float a0 = l[i * stride], a1 = l[i * stride + 1], a2 = l[i * stride + 2];
-    float *o = R + i * 9;
-    o[0] = 1.f; o[1] = a0; o[2] = a1;
-    o[3] = -a0; o[4] = 1.f; o[5] = a2;
-    o[6] = -a1; o[7] = -a2; o[8] = 1.f;
-}
-__global__ void rotmat_bwd_kernel(int64_t n, const float *__restrict__ g, float *__restrict__ vl) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float *r = g + i * 9;
-    vl[i * 3 + 0] = r[1] - r[3];
-    vl[i * 3 + 1] = r[2] - r[6];
-    vl[i * 3 + 2] = r[5] - r[7];
-}
-
-// ------------------------------------------------- coalesced output rows
-// The per-primitive outputs are [n, w] rows, one per thread; stored directly,
-// every warp store would touch 32 different sectors.  Kernels with rows of
-// up to 49 floats stage a block's rows in shared memory (rows padded to an odd
-// stride, so a thread's own writes are free of bank conflicts) and copy them
-// out with consecutive threads on consecutive floats.
+// ------------------------------------------------------- rows of a block
+// The per-primitive tensors are [n, w] rows, one per thread; accessed directly,
+// every warp access would touch 32 different sectors (the covariance backward
+// read and wrote 96 floats a primitive that way: 80 us for 300k primitives,
+// bound by L1 wavefronts).  Kernels with rows of up to 49 floats pass a block's
+// rows through shared memory (padded to an odd stride, so a thread's accesses to
+// its own row are free of bank conflicts) with consecutive threads on
+// consecutive floats of global memory.  A thread may overwrite its own input row
+// with an output row of at most the same width.
 constexpr int ROW_BLOCK = 128;
 template <int W> struct RowBuf {
     static constexpr int S = W | 1;
     float v[ROW_BLOCK * S];
-    __device__ __forceinline__ float &at(int t, int k) { return v[t * S + k]; }
-    // after a barrier: rows [0, cnt) to dst rows [i0, i0 + cnt)
+    __device__ __forceinline__ float *row(int t) { return v + t * S; }
+    // rows [i0, i0 + cnt) of src; rows_arrived() and a barrier have to follow.
+    // Asynchronous copies: a loop of loads and shared stores would have a load or
+    // two in flight per thread (cond backward, 300k primitives of 6-D: 55 us
+    // that way, 31 this way, 33 with direct reads).
+    __device__ __forceinline__ void load(const float *__restrict__ src, int64_t i0, int cnt) {
+        const float *s = src + i0 * W;
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(v);
+#pragma unroll 4
+        for (int k = 0; k < W; ++k) {
+            const int e = k * ROW_BLOCK + threadIdx.x, t = e / W;
+            if (e < cnt * W)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                 d + 4 * (t * S + (e - t * W))),
+                             "l"(s + e)
+                             : "memory");
+        }
+    }
+    // after a barrier: the first w floats of rows [0, cnt) to dst rows [i0, i0 + cnt)
+    template <int w = W>
     __device__ __forceinline__ void flush(float *__restrict__ dst, int64_t i0, int cnt) const {
-        float *d = dst + i0 * W;
-        for (int e = threadIdx.x; e < cnt * W; e += blockDim.x) {
-            const int t = e / W;
-            d[e] = v[t * S + (e - t * W)];
+        float *d = dst + i0 * w;
+#pragma unroll 4
+        for (int k = 0; k < w; ++k) {
+            const int e = k * ROW_BLOCK + threadIdx.x, t = e / w;
+            if (e < cnt * w) d[e] = v[t * S + (e - t * w)];
         }
     }
 };
+__device__ __forceinline__ void rows_arrived() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+__device__ __forceinline__ int block_rows(int64_t n, int64_t i0) {
+    return (int)(n - i0 < ROW_BLOCK ? n - i0 : ROW_BLOCK);
+}
+
+// ------------------------------------------------------------------ a2
+__global__ void __launch_bounds__(ROW_BLOCK) rotmat_fwd_kernel(int64_t n, const float *__restrict__ l,
+                                                               int64_t stride,
+                                                               float *__restrict__ R) {
+    __shared__ RowBuf<9> rows;
+    const int64_t i0 = (int64_t)blockIdx.x * ROW_BLOCK, i = i0 + threadIdx.x;
+    if (i < n) {
+        const float a0 = l[i * stride], a1 = l[i * stride + 1], a2 = l[i * stride + 2];
+        float *o = rows.row(threadIdx.x);
+        o[0] = 1.f; o[1] = a0; o[2] = a1;
+        o[3] = -a0; o[4] = 1.f; o[5] = a2;
+        o[6] = -a1; o[7] = -a2; o[8] = 1.f;
+    }
+    __syncthreads();
+    rows.flush(R, i0, block_rows(n, i0));
+}
+__global__ void __launch_bounds__(ROW_BLOCK) rotmat_bwd_kernel(int64_t n, const float *__restrict__ g,
+                                                               float *__restrict__ vl) {
+    __shared__ RowBuf<9> rows;
+    const int64_t i0 = (int64_t)blockIdx.x * ROW_BLOCK, i = i0 + threadIdx.x;
+    rows.load(g, i0, block_rows(n, i0));
+    rows_arrived();
+    __syncthreads();
+    if (i < n) {
+        float *r = rows.row(threadIdx.x);
+        const float v0 = r[1] - r[3], v1 = r[2] - r[6], v2 = r[5] - r[7];
+        r[0] = v0;
+        r[1] = v1;
+        r[2] = v2;
+    }
+    __syncthreads();
+    rows.flush<3>(vl, i0, block_rows(n, i0));
+}
 
 // ------------------------------------------------------------------ a3
+// One primitive of covar_fwd_kernel; o may overlay R.
+template <int D, bool ORDERED>
+__device__ __forceinline__ void covar_row(const float *R, const float *s, const float *lt,
+                                          const int32_t *ri, const int32_t *rj, int m_rest,
+                                          bool sp, float *o) {
+    float L[D * D];
+    build_L<D, ORDERED>(R, s, lt, ri, rj, m_rest, L);
+    if (sp) {
+        float v[9];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                v[r * 3 + c] =
+                    L[r * D] * L[c * D] + L[r * D + 1] * L[c * D + 1] + L[r * D + 2] * L[c * D + 2];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) o[k] = v[k];
+    } else {
+        float V[D * D];
+        covar_from_L<D>(L, V);
+#pragma unroll
+        for (int k = 0; k < D * D; ++k) o[k] = V[k];
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(ROW_BLOCK) covar_fwd_kernel(int64_t n, const float *__restrict__ rot,
                                  const float *__restrict__ scale, const float *__restrict__ ltri,
                                  const int32_t *__restrict__ ri_g, const int32_t *__restrict__ rj_g,
                                  int m_rest, int spatial, float *__restrict__ covar) {
     __shared__ int32_t ri[64], rj[64];
+    bool in_order = m_rest == rest_count<D>;
     for (int m = threadIdx.x; m < m_rest && m < 64; m += blockDim.x) {
-        ri[m] = ri_g[m];
-        rj[m] = rj_g[m];
+        const int r = ri_g[m], c = rj_g[m];
+        ri[m] = r;
+        rj[m] = c;
+        in_order = in_order && in_rest_order<D>(m, r, c);
     }
     constexpr bool STAGE = D <= 7;
+    constexpr int full_m = D * (D - 1) / 2;
     __shared__ RowBuf<STAGE ? D * D : 1> full;
-    __shared__ RowBuf<STAGE ? 9 : 1> block3;
-    __syncthreads();
+    __shared__ RowBuf<STAGE ? 9 : 1> sR; // rotations, then 3x3 results
+    __shared__ RowBuf<STAGE ? D : 1> sS;
+    __shared__ RowBuf<STAGE && full_m ? full_m : 1> sL;
     const int t = threadIdx.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + t;
-    const int cnt = (int)(n - i0 < (int64_t)blockDim.x ? n - i0 : (int64_t)blockDim.x);
+    const int cnt = block_rows(n, i0);
+    if constexpr (STAGE) {
+        sR.load(rot, i0, cnt);
+        sS.load(scale, i0, cnt);
+        if (m_rest) sL.load(ltri, i0, cnt);
+    }
+    rows_arrived();
+    const bool ordered = __syncthreads_and(in_order);
     const bool sp = spatial || D == 3;
     if (i < n) {
-        constexpr int full_m = D * (D - 1) / 2;
-        float L[D * D];
-        build_L<D>(rot + i * 9, scale + i * D, ltri + i * full_m + 3, ri, rj, m_rest, L);
-        if (sp) {
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float v = L[r * D] * L[c * D] + L[r * D + 1] * L[c * D + 1] +
-                                    L[r * D + 2] * L[c * D + 2];
-                    if (STAGE) block3.at(t, r * 3 + c) = v;
-                    else covar[i * 9 + r * 3 + c] = v;
-                }
-        } else {
-            float V[D * D];
-            covar_from_L<D>(L, V);
-#pragma unroll
-            for (int k = 0; k < D * D; ++k) {
-                if (STAGE) full.at(t, k) = V[k];
-                else covar[i * D * D + k] = V[k];
-            }
-        }
+        const float *R = STAGE ? sR.row(t) : rot + i * 9, *s = STAGE ? sS.row(t) : scale + i * D;
+        const float *lt = (STAGE ? sL.row(t) : ltri + i * full_m) + 3;
+        float *o = STAGE ? (sp ? sR.row(t) : full.row(t)) : covar + i * (sp ? 9 : D * D);
+        if (ordered) covar_row<D, true>(R, s, lt, ri, rj, m_rest, sp, o);
+        else covar_row<D, false>(R, s, lt, ri, rj, m_rest, sp, o);
     }
     if (!STAGE) return;
     __syncthreads();
-    if (sp) block3.flush(covar, i0, cnt);
-    else full.flush(covar, i0, cnt);
+    if (sp) {
+        if constexpr (STAGE) sR.template flush<9>(covar, i0, cnt);
+    } else {
+        if constexpr (STAGE) full.template flush<D * D>(covar, i0, cnt);
+    }
 }
 
-// One primitive of covar_bwd_kernel: rows go to the shared row buffers when
-// given (strides 9|1, D|1, full_m|1), else straight to global memory.
-template <int D>
-__device__ __forceinline__ void covar_bwd_row(int64_t i, int t, const float *__restrict__ rot,
-                                              const float *__restrict__ scale,
-                                              const float *__restrict__ ltri, const int32_t *ri,
-                                              const int32_t *rj, int m_rest, int spatial,
-                                              const float *__restrict__ v_covar,
-                                              float *__restrict__ v_rot,
-                                              float *__restrict__ v_scale,
-                                              float *__restrict__ v_ltri, float *stR, float *stS,
-                                              float *stL) {
+// One primitive of covar_bwd_kernel: its rows, which the outputs may overlay
+// (gR over R, gs over s, gl over lt).
+template <int D, bool ORDERED>
+__device__ __forceinline__ void covar_bwd_row(const float *Rp, const float *sp, const float *lt,
+                                              const int32_t *ri, const int32_t *rj, int m_rest,
+                                              int spatial, const float *G, float *gR, float *gs,
+                                              float *gl) {
     constexpr int full_m = D * (D - 1) / 2;
     const int dim = (spatial || D == 3) ? 3 : D;
-    const float *R = rot + i * 9;
-    const float *s = scale + i * D;
+    float R[9], s[D];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) R[k] = Rp[k];
+#pragma unroll
+    for (int k = 0; k < D; ++k) s[k] = sp[k];
     float L[D * D];
-    build_L<D>(R, s, ltri + i * full_m + 3, ri, rj, m_rest, L);
-    const float *G = v_covar + i * dim * dim;
-    float *gR = stR ? stR + t * (9 | 1) : v_rot + i * 9;
-    float *gs = stS ? stS + t * (D | 1) : v_scale + i * D;
-    float *gl = stL ? stL + t * (full_m | 1) : v_ltri + i * full_m;
+    build_L<D, ORDERED>(R, s, lt + 3, ri, rj, m_rest, L);
     // dL = (G + G^T) L over the output rows
     float dL[D * D];
 #pragma unroll
@@ -144,6 +203,13 @@ __device__ __forceinline__ void covar_bwd_row(int64_t i, int t, const float *__r
 #pragma unroll
     for (int r = 3; r < D; ++r) gs[r] = (dim == 3) ? 0.f : dL[r * D + r];
     if (dim == 3) return;
+    if constexpr (ORDERED) {
+#pragma unroll
+        for (int r = 3; r < D; ++r)
+#pragma unroll
+            for (int c = 0; c < r; ++c) gl[r * (r - 1) / 2 + c] = dL[r * D + c];
+        return;
+    }
     for (int m = 0; m < m_rest; ++m) {
         const int idx = ri[m] * D + rj[m];
         float v = 0.f;
@@ -162,95 +228,102 @@ __global__ void __launch_bounds__(ROW_BLOCK) covar_bwd_kernel(int64_t n, const f
                                  float *__restrict__ v_rot, float *__restrict__ v_scale,
                                  float *__restrict__ v_ltri) {
     __shared__ int32_t ri[64], rj[64];
+    bool in_order = m_rest == rest_count<D>;
     for (int m = threadIdx.x; m < m_rest && m < 64; m += blockDim.x) {
-        ri[m] = ri_g[m];
-        rj[m] = rj_g[m];
+        const int r = ri_g[m], c = rj_g[m];
+        ri[m] = r;
+        rj[m] = c;
+        in_order = in_order && in_rest_order<D>(m, r, c);
     }
     constexpr int full_m = D * (D - 1) / 2;
     constexpr bool STAGE = D <= 7;
     __shared__ RowBuf<STAGE ? 9 : 1> sR;
     __shared__ RowBuf<STAGE ? D : 1> sS;
     __shared__ RowBuf<STAGE ? full_m : 1> sL;
-    __syncthreads();
+    __shared__ RowBuf<STAGE ? D * D : 1> sG;
     const int t = threadIdx.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + t;
-    const int cnt = (int)(n - i0 < (int64_t)blockDim.x ? n - i0 : (int64_t)blockDim.x);
-    if (i < n)
-        covar_bwd_row<D>(i, t, rot, scale, ltri, ri, rj, m_rest, spatial, v_covar, v_rot, v_scale,
-                         v_ltri, STAGE ? sR.v : nullptr, STAGE ? sS.v : nullptr,
-                         STAGE ? sL.v : nullptr);
+    const int cnt = block_rows(n, i0);
+    const bool sp = spatial || D == 3;
+    if constexpr (STAGE) {
+        sR.load(rot, i0, cnt);
+        sS.load(scale, i0, cnt);
+        if (m_rest) sL.load(ltri, i0, cnt);
+        if (!sp) sG.load(v_covar, i0, cnt);
+    }
+    rows_arrived();
+    const bool ordered = __syncthreads_and(in_order);
+    if (i < n) {
+        const float *R = STAGE ? sR.row(t) : rot + i * 9, *s = STAGE ? sS.row(t) : scale + i * D;
+        const float *lt = STAGE ? sL.row(t) : ltri + i * full_m;
+        const float *G = STAGE && !sp ? sG.row(t) : v_covar + i * (sp ? 9 : D * D);
+        float *gR = STAGE ? sR.row(t) : v_rot + i * 9, *gs = STAGE ? sS.row(t) : v_scale + i * D;
+        float *gl = STAGE ? sL.row(t) : v_ltri + i * full_m;
+        if (ordered) covar_bwd_row<D, true>(R, s, lt, ri, rj, m_rest, spatial, G, gR, gs, gl);
+        else covar_bwd_row<D, false>(R, s, lt, ri, rj, m_rest, spatial, G, gR, gs, gl);
+    }
     if (!STAGE) return;
     __syncthreads();
-    sR.flush(v_rot, i0, cnt);
-    sS.flush(v_scale, i0, cnt);
-    sL.flush(v_ltri, i0, cnt);
+    if constexpr (STAGE) {
+        sR.flush(v_rot, i0, cnt);
+        sS.flush(v_scale, i0, cnt);
+        sL.flush(v_ltri, i0, cnt);
+    }
 }
 
 // ------------------------------------------------------------------ a4
 template <int K>
-__global__ void cond_fwd_kernel(int64_t n, const float *__restrict__ means,
-                                const float *__restrict__ covars, const float *__restrict__ opac,
-                                const float *__restrict__ betas, const float *__restrict__ query,
-                                float *__restrict__ om, float *__restrict__ oV,
-                                float *__restrict__ oo) {
+__global__ void __launch_bounds__(ROW_BLOCK) cond_fwd_kernel(
+    int64_t n, const float *__restrict__ means, const float *__restrict__ covars,
+    const float *__restrict__ opac, const float *__restrict__ betas,
+    const float *__restrict__ query, float *__restrict__ om, float *__restrict__ oV,
+    float *__restrict__ oo) {
     constexpr int D = K + 3;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float m[D], V[D * D], b[K], q[K];
-#pragma unroll
-    for (int k = 0; k < D; ++k) m[k] = means[i * D + k];
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) V[k] = covars[i * D * D + k];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        b[k] = betas[i * K + k];
-        q[k] = query[i * K + k];
+    constexpr bool STAGE = D <= 7;
+    __shared__ RowBuf<STAGE ? D * D : 1> sV; // covariances, then conditioned ones
+    __shared__ RowBuf<STAGE ? D : 1> sM;     // means, then conditioned ones
+    __shared__ RowBuf<STAGE ? K : 1> sB, sQ;
+    const int t = threadIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * ROW_BLOCK, i = i0 + t;
+    const int cnt = block_rows(n, i0);
+    if constexpr (STAGE) {
+        sV.load(covars, i0, cnt);
+        sM.load(means, i0, cnt);
+        sB.load(betas, i0, cnt);
+        sQ.load(query, i0, cnt);
     }
-    cond_forward<K>(m, V, opac[i], b, q, om + i * 3, oV + i * 9, oo + i);
-}
-
-// One primitive of cond_bwd_kernel: the [D, D] and [D] gradient rows go to the
-// shared row buffers when given (strides (D*D)|1 and D|1), else to global memory.
-template <int K>
-__device__ __forceinline__ void cond_bwd_row(int64_t i, int t, const float *__restrict__ means,
-                                             const float *__restrict__ covars,
-                                             const float *__restrict__ opac,
-                                             const float *__restrict__ betas,
-                                             const float *__restrict__ query,
-                                             const float *__restrict__ vm,
-                                             const float *__restrict__ vV,
-                                             const float *__restrict__ vo,
-                                             float *__restrict__ gm, float *__restrict__ gV,
-                                             float *__restrict__ go, float *__restrict__ gb,
-                                             int exact, float *stV, float *stM) {
-    constexpr int D = K + 3;
-    float m[D], V[D * D], b[K], q[K], gM[3], gVc[9];
+    rows_arrived();
+    __syncthreads();
+    if (i < n) {
+        const float *mp = STAGE ? sM.row(t) : means + i * D;
+        const float *Vp = STAGE ? sV.row(t) : covars + i * D * D;
+        const float *bp = STAGE ? sB.row(t) : betas + i * K;
+        const float *qp = STAGE ? sQ.row(t) : query + i * K;
+        float m[D], V[D * D], b[K], q[K];
 #pragma unroll
-    for (int k = 0; k < D; ++k) m[k] = means[i * D + k];
+        for (int k = 0; k < D; ++k) m[k] = mp[k];
 #pragma unroll
-    for (int k = 0; k < D * D; ++k) V[k] = covars[i * D * D + k];
+        for (int k = 0; k < D * D; ++k) V[k] = Vp[k];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        b[k] = betas[i * K + k];
-        q[k] = query[i * K + k];
+        for (int k = 0; k < K; ++k) {
+            b[k] = bp[k];
+            q[k] = qp[k];
+        }
+        float lm[3], lV[9];
+        cond_forward<K>(m, V, opac[i], b, q, lm, lV, oo + i);
+        float *dm = STAGE ? sM.row(t) : om + i * 3, *dV = STAGE ? sV.row(t) : oV + i * 9;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dm[k] = lm[k];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) dV[k] = lV[k];
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) gM[k] = vm[i * 3 + k];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) gVc[k] = vV[i * 9 + k];
-    float lm[D], lV[D * D], lb[K], lo;
-    cond_backward<K>(m, V, opac[i], b, q, gM, gVc, vo[i], exact != 0, lm, lV, &lo, lb);
-    float *dm = stM ? stM + t * (D | 1) : gm + i * D;
-    float *dV = stV ? stV + t * ((D * D) | 1) : gV + i * D * D;
-#pragma unroll
-    for (int k = 0; k < D; ++k) dm[k] = lm[k];
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) dV[k] = lV[k];
-    go[i] = lo;
-#pragma unroll
-    for (int k = 0; k < K; ++k) gb[i * K + k] = lb[k];
+    if (!STAGE) return;
+    __syncthreads();
+    if constexpr (STAGE) {
+        sM.template flush<3>(om, i0, cnt);
+        sV.template flush<9>(oV, i0, cnt);
+    }
 }
-
 
 template <int K>
 __global__ void __launch_bounds__(ROW_BLOCK) cond_bwd_kernel(
@@ -261,17 +334,65 @@ __global__ void __launch_bounds__(ROW_BLOCK) cond_bwd_kernel(
     float *__restrict__ go, float *__restrict__ gb, int exact) {
     constexpr int D = K + 3;
     constexpr bool STAGE = D <= 7;
-    __shared__ RowBuf<STAGE ? D * D : 1> sV;
-    __shared__ RowBuf<STAGE ? D : 1> sM;
+    __shared__ RowBuf<STAGE ? D * D : 1> sV; // covariances, then their gradients
+    __shared__ RowBuf<STAGE ? D : 1> sM;     // means, then their gradients
+    __shared__ RowBuf<STAGE ? K : 1> sB, sQ; // betas, then their gradients; queries
+    __shared__ RowBuf<STAGE ? 9 : 1> sgV;
+    __shared__ RowBuf<STAGE ? 3 : 1> sgM;
     const int t = threadIdx.x;
-    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x, i = i0 + t;
-    const int cnt = (int)(n - i0 < (int64_t)blockDim.x ? n - i0 : (int64_t)blockDim.x);
-    if (i < n) cond_bwd_row<K>(i, t, means, covars, opac, betas, query, vm, vV, vo, gm, gV, go, gb,
-                               exact, STAGE ? sV.v : nullptr, STAGE ? sM.v : nullptr);
+    const int64_t i0 = (int64_t)blockIdx.x * ROW_BLOCK, i = i0 + t;
+    const int cnt = block_rows(n, i0);
+    if constexpr (STAGE) {
+        sV.load(covars, i0, cnt);
+        sM.load(means, i0, cnt);
+        sB.load(betas, i0, cnt);
+        sQ.load(query, i0, cnt);
+        sgV.load(vV, i0, cnt);
+        sgM.load(vm, i0, cnt);
+    }
+    rows_arrived();
+    __syncthreads();
+    if (i < n) {
+        const float *mp = STAGE ? sM.row(t) : means + i * D;
+        const float *Vp = STAGE ? sV.row(t) : covars + i * D * D;
+        const float *bp = STAGE ? sB.row(t) : betas + i * K;
+        const float *qp = STAGE ? sQ.row(t) : query + i * K;
+        const float *gMp = STAGE ? sgM.row(t) : vm + i * 3;
+        const float *gVp = STAGE ? sgV.row(t) : vV + i * 9;
+        float m[D], V[D * D], b[K], q[K], gM[3], gVc[9];
+#pragma unroll
+        for (int k = 0; k < D; ++k) m[k] = mp[k];
+#pragma unroll
+        for (int k = 0; k < D * D; ++k) V[k] = Vp[k];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            b[k] = bp[k];
+            q[k] = qp[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) gM[k] = gMp[k];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) gVc[k] = gVp[k];
+        float lm[D], lV[D * D], lb[K], lo;
+        cond_backward<K>(m, V, opac[i], b, q, gM, gVc, vo[i], exact != 0, lm, lV, &lo, lb);
+        float *dm = STAGE ? sM.row(t) : gm + i * D;
+        float *dV = STAGE ? sV.row(t) : gV + i * D * D;
+        float *db = STAGE ? sB.row(t) : gb + i * K;
+#pragma unroll
+        for (int k = 0; k < D; ++k) dm[k] = lm[k];
+#pragma unroll
+        for (int k = 0; k < D * D; ++k) dV[k] = lV[k];
+#pragma unroll
+        for (int k = 0; k < K; ++k) db[k] = lb[k];
+        go[i] = lo;
+    }
     if (!STAGE) return;
     __syncthreads();
-    sV.flush(gV, i0, cnt);
-    sM.flush(gm, i0, cnt);
+    if constexpr (STAGE) {
+        sV.flush(gV, i0, cnt);
+        sM.flush(gm, i0, cnt);
+        sB.flush(gb, i0, cnt);
+    }
 }
 
 // ------------------------------------------------------------------ a6
@@ -515,7 +636,7 @@ int ubs_l_triangle_to_rotmat_fwd(int64_t n, const float *l_triangle, int64_t row
     UBS_REQUIRE(n >= 0 && row_stride >= 3, "rotmat_fwd: bad sizes");
     if (n == 0) return UBS_OK;
     UBS_TIMED("rotmat_fwd", (cudaStream_t)stream,
-              rotmat_fwd_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(
+              rotmat_fwd_kernel<<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, (cudaStream_t)stream>>>(
                   n, l_triangle, row_stride, rotmats));
     ::ubs::note_launch();
     return finish("rotmat_fwd");
@@ -526,7 +647,7 @@ int ubs_l_triangle_to_rotmat_bwd(int64_t n, const float *v_rotmats, float *v_l_t
     UBS_REQUIRE(n >= 0, "rotmat_bwd: bad sizes");
     if (n == 0) return UBS_OK;
     UBS_TIMED("rotmat_bwd", (cudaStream_t)stream,
-              rotmat_bwd_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(
+              rotmat_bwd_kernel<<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, (cudaStream_t)stream>>>(
                   n, v_rotmats, v_l_triangle));
     ::ubs::note_launch();
     return finish("rotmat_bwd");
@@ -557,7 +678,7 @@ int ubs_rot_scale_l_triangle_to_covar_fwd(int64_t n, int32_t dim, const float *r
     if (n == 0) return UBS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     UBS_TIMED("covar_fwd", st,
-              UBS_DIM_SWITCH(dim, covar_fwd_kernel<DD><<<grid_for(n, 128), 128, 0, st>>>(
+              UBS_DIM_SWITCH(dim, covar_fwd_kernel<DD><<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, st>>>(
                                       n, rot, scale, l_triangle, rest_i, rest_j, m_rest,
                                       spatial_block, covar)));
     ::ubs::note_launch();
@@ -574,7 +695,7 @@ int ubs_rot_scale_l_triangle_to_covar_bwd(int64_t n, int32_t dim, const float *r
     if (n == 0) return UBS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     UBS_TIMED("covar_bwd", st,
-              UBS_DIM_SWITCH(dim, covar_bwd_kernel<DD><<<grid_for(n, 128), 128, 0, st>>>(
+              UBS_DIM_SWITCH(dim, covar_bwd_kernel<DD><<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, st>>>(
                                       n, rot, scale, l_triangle, rest_i, rest_j, m_rest,
                                       spatial_block, v_covar, v_rot, v_scale, v_l_triangle)));
     ::ubs::note_launch();
@@ -601,7 +722,7 @@ int ubs_cond_fwd(int64_t n, int32_t dim, const float *means, const float *covars
     if (n == 0) return UBS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     UBS_TIMED("cond_fwd", st,
-              UBS_K_SWITCH(dim - 3, cond_fwd_kernel<KK><<<grid_for(n, 128), 128, 0, st>>>(
+              UBS_K_SWITCH(dim - 3, cond_fwd_kernel<KK><<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, st>>>(
                                         n, means, covars, opacities, betas, query, out_means,
                                         out_covars, out_opacities)));
     ::ubs::note_launch();
@@ -617,7 +738,7 @@ int ubs_cond_bwd(int64_t n, int32_t dim, const float *means, const float *covars
     if (n == 0) return UBS_OK;
     cudaStream_t st = (cudaStream_t)stream;
     UBS_TIMED("cond_bwd", st,
-              UBS_K_SWITCH(dim - 3, cond_bwd_kernel<KK><<<grid_for(n, 128), 128, 0, st>>>(
+              UBS_K_SWITCH(dim - 3, cond_bwd_kernel<KK><<<grid_for(n, ROW_BLOCK), ROW_BLOCK, 0, st>>>(
                                         n, means, covars, opacities, betas, query, v_out_means,
                                         v_out_covars, v_out_opacities, v_means, v_covars,
                                         v_opacities, v_betas, exact)));

@@ -727,8 +727,18 @@ template <int D> __device__ __forceinline__ void covar_from_L(const float *L, fl
     }
 }
 
-// L: [D*D] row-major factor of rot_scale_l_triangle_to_covar_fwd.cu:8-188
-template <int D>
+// Entry m of the lower triangle below the 3x3 block, row by row: the order of
+// torch.tril_indices(D, D, -1) after its first three.
+template <int D> constexpr int rest_count = D * (D - 1) / 2 - 3;
+template <int D> __device__ __forceinline__ bool in_rest_order(int m, int r, int c) {
+    return c >= 0 && c < r && r >= 3 && r < D && r * (r - 1) / 2 - 3 + c == m;
+}
+
+// L: [D*D] row-major factor of rot_scale_l_triangle_to_covar_fwd.cu:8-188.
+// ORDERED: ri, rj are all entries in the order above, so that each value's place
+// is known at compile time and L stays in registers; for a general list the
+// compiler keeps it in local memory.
+template <int D, bool ORDERED>
 __device__ __forceinline__ void build_L(const float *R, const float *s, const float *lrest,
                                         const int32_t *ri, const int32_t *rj, int m_rest,
                                         float *L) {
@@ -740,6 +750,13 @@ __device__ __forceinline__ void build_L(const float *R, const float *s, const fl
         for (int c = 0; c < 3; ++c) L[r * D + c] = R[r * 3 + c] * s[c];
 #pragma unroll
     for (int r = 3; r < D; ++r) L[r * D + r] = s[r];
+    if constexpr (ORDERED) {
+#pragma unroll
+        for (int r = 3; r < D; ++r)
+#pragma unroll
+            for (int c = 0; c < r; ++c) L[r * D + c] = lrest[r * (r - 1) / 2 - 3 + c];
+        return;
+    }
     for (int m = 0; m < m_rest; ++m) {
         const int r = ri[m], c = rj[m];
         // scatter through a compile-time loop to keep L in registers
