@@ -8,14 +8,17 @@
 // with sxx = E[x^2] - mx^2, sxy = E[xy] - mx my, and the loss reads the mean
 // of the map (optionally cropped by the window radius, fused_ssim's "valid").
 //
-// Two kernels, each over 32 x 32 tiles of one (image, channel); quantities
-// that are filtered with the same window travel in pairs through Blackwell's
-// packed FP32x2 FMA ((x, y), (x^2, y^2), (D1, D2)):
-//  * ssim_map_kernel: the five windowed moments of the tile (separable: a
-//    horizontal then a vertical 11-tap pass over shared memory, the products
-//    formed in registers), the map, the loss partials and -- for the
-//    gradient -- the map's derivatives with the E[.] moments as the free
-//    variables, D0 = d map / d mx, D1 = d map / d E[x^2],
+// Two kernels.  A warp owns a strip of 64 columns and some rows of one (image,
+// channel) and goes down it row by row, two columns per lane: a row (with the
+// halo columns) comes through a ring of shared rows that only this warp uses,
+// the horizontal 11 taps are formed from it in registers, and the vertical ones
+// by ten running sums per quantity, acc[k] = g[9 - k] h + acc[k + 1], of which
+// the last is complete.  No barriers and no pass over shared memory for the
+// vertical window; quantities that are filtered with the same window travel in
+// pairs through Blackwell's packed FP32x2 FMA ((x, y), (x^2, y^2), (D1, D2)):
+//  * ssim_map_kernel: the five windowed moments, the map, the loss partials and
+//    -- for the gradient -- the map's derivatives with the E[.] moments as the
+//    free variables, D0 = d map / d mx, D1 = d map / d E[x^2],
 //    D2 = d map / d E[xy], stored as a D0 plane and a (D1, D2) plane (12 B
 //    per pixel-channel, mostly L2-resident between the two launches);
 //  * ssim_grad_kernel: d loss / d x_p = gb sum_q w(q - p) (D0 + 2 x_p D1 +
@@ -24,21 +27,24 @@
 // Loss sums: one partial per CTA, reduced in a fixed order by the last CTA to
 // finish (a ticket counter that the last CTA resets), so the result is
 // deterministic and the launches can be replayed from a CUDA graph.
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include "ubs_common.cuh"
 
 namespace ubs {
 namespace {
 
-constexpr int SS_T = 32;                // output tile edge
 constexpr int SS_R = 5;                 // window radius (11 taps)
 constexpr int SS_W = 2 * SS_R + 1;
-constexpr int SS_IN = SS_T + 2 * SS_R;  // 42: tile plus halo
-constexpr int SS_IP = SS_IN + 1;        // padded pitch of the halo planes
-constexpr int SS_HP = SS_T + 1;         // padded pitch of the horizontal results
-constexpr int SS_THREADS = 256;
-constexpr int SS_LOADS = (SS_IN * SS_IN + SS_THREADS - 1) / SS_THREADS; // halo loads per thread
+constexpr int SS_C = 64;                // columns of a strip (two per lane)
+constexpr int SS_IN = SS_C + 2 * SS_R;  // 74: with the halo
+constexpr int SS_IP = SS_IN + 2;        // row pitch of the ring (16-byte rows of pairs)
+constexpr int SS_RING = 8;              // rows in flight or in use
+constexpr int SS_WARPS = 4;             // strips of a CTA
+constexpr int SS_THREADS = 32 * SS_WARPS;
+constexpr int SS_CTAS = 4;              // CTAs per SM (map kernel: 80 running sums per lane)
 
 struct SsimArgs {
     const float *img;
@@ -46,16 +52,17 @@ struct SsimArgs {
     float *grad;                 // null: loss only
     int64_t is[4], gs[4], ds[4]; // element strides (image, channel, row, column)
     int32_t n, c, h, w;
-    int32_t tiles_x, tiles_y;
+    int32_t strips_x, strips_y, rows; // strips of `rows` rows
+    int32_t pitch;                    // of the derivative planes (even)
     int32_t valid;               // count only map points >= SS_R from every edge
     float c1, c2;
     float ga, gb;                // d loss / d |x - y| (per pixel), d loss / d map (per point)
     double inv_px, inv_map;      // 1 / pixels, 1 / counted map points
     double wl1, wssim, wconst;   // loss = wl1 mean|x-y| + wssim mean(map) + wconst
-    float g[SS_W];               // normalised 1-D window
-    float *dmap0;                // [n c][h][w] D0 plane (gradient only)
-    float2 *dmap12;              // [n c][h][w] (D1, D2) plane
-    float *partials;             // [n_ctas][2]
+    float g[SS_R + 1];           // normalised 1-D window, first half and centre
+    float *dmap0;                // [n c][h][pitch] D0 plane (gradient only)
+    float2 *dmap12;              // [n c][h][pitch] (D1, D2) plane
+    double *partials;            // [n_ctas][2]
     unsigned *counter;
     float *out;                  // [3]: mean(map), mean|x-y|, loss
 };
@@ -72,82 +79,136 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
     return s; // valid in thread 0
 }
 
-// 4 outputs of an 11-tap window over 14 consecutive values: scalar, and two
-// streams at once with the packed FP32x2 FMA (same rounding per component)
-__device__ __forceinline__ void taps4(const float (&g)[SS_W], const float (&v)[14],
-                                      float (&acc)[4]) {
-#pragma unroll
-    for (int o = 0; o < 4; ++o) acc[o] = 0.f;
-#pragma unroll
-    for (int t = 0; t < SS_W; ++t)
-#pragma unroll
-        for (int o = 0; o < 4; ++o) acc[o] = fmaf(g[t], v[o + t], acc[o]);
+// The 11-tap window over 11 consecutive values: scalar, and two streams at
+// once with the packed FP32x2 FMA (same rounding per component).
+__device__ __forceinline__ float tap(const float (&g)[SS_R + 1], int t) {
+    return g[t <= SS_R ? t : SS_W - 1 - t];
 }
-__device__ __forceinline__ void taps4x2(const float (&g)[SS_W], const float2 (&v)[14],
-                                        float2 (&acc)[4]) {
+__device__ __forceinline__ float2 fma_g(float g, float2 v, float2 c) {
+    return __ffma2_rn(make_float2(g, g), v, c);
+}
+__device__ __forceinline__ float fma_g(float g, float v, float c) { return fmaf(g, v, c); }
+template <class T> __device__ __forceinline__ T zero_of();
+template <> __device__ __forceinline__ float zero_of<float>() { return 0.f; }
+template <> __device__ __forceinline__ float2 zero_of<float2>() { return make_float2(0.f, 0.f); }
+
+__device__ __forceinline__ float2 add_g(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float add_g(float a, float b) { return a + b; }
+// From both ends to the centre: two short chains, whose partial sums stay small
+// until the last two additions.
+template <class T>
+__device__ __forceinline__ T taps(const float (&g)[SS_R + 1], const T *v) {
+    T lo = zero_of<T>(), hi = lo;
 #pragma unroll
-    for (int o = 0; o < 4; ++o) acc[o] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int t = 0; t < SS_W; ++t) {
-        const float2 g2 = make_float2(g[t], g[t]);
-#pragma unroll
-        for (int o = 0; o < 4; ++o) acc[o] = __ffma2_rn(g2, v[o + t], acc[o]);
+    for (int t = 0; t < SS_R; ++t) {
+        lo = fma_g(g[t], v[t], lo);
+        hi = fma_g(g[t], v[SS_W - 1 - t], hi);
     }
+    return add_g(fma_g(g[SS_R], v[SS_R], lo), hi);
+}
+// The vertical window: the running sums take the row's value h, and the one
+// that has now seen its eleven rows (taps in ascending order) is returned.
+template <class T>
+__device__ __forceinline__ T roll(const float (&g)[SS_R + 1], T (&acc)[SS_W - 1], T h) {
+    const T out = fma_g(tap(g, SS_W - 1), h, acc[0]);
+#pragma unroll
+    for (int k = 0; k < SS_W - 2; ++k) acc[k] = fma_g(tap(g, SS_W - 2 - k), h, acc[k + 1]);
+    acc[SS_W - 2] = fma_g(tap(g, 0), h, zero_of<T>());
+    return out;
 }
 
+// A warp's strip: plane, first column, first row, rows.
+struct Strip {
+    int plane, x0, y0, rows;
+};
+__device__ __forceinline__ Strip strip_of(const SsimArgs &a) {
+    const int64_t id = (int64_t)blockIdx.x * SS_WARPS + (threadIdx.x >> 5);
+    const int per = a.strips_x * a.strips_y;
+    Strip s;
+    s.plane = (int)(id / per);
+    const int r = (int)(id - (int64_t)s.plane * per), sy = r / a.strips_x;
+    s.x0 = (r - sy * a.strips_x) * SS_C;
+    s.y0 = sy * a.rows;
+    s.rows = s.plane < a.n * a.c ? min(a.rows, a.h - s.y0) : 0; // past the last strip: none
+    return s;
+}
+// Which of the three columns of a lane's copies of a row (x0 - SS_R + lane + 32 k)
+// lie in the image; the others stay zero in the ring.
+struct Columns {
+    bool in[3];
+    __device__ __forceinline__ Columns(int x0, int w) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int gx = x0 - SS_R + lane + 32 * k;
+            in[k] = gx >= 0 && gx < w && lane + 32 * k < SS_IN;
+        }
+    }
+};
+
 // Asynchronous global -> shared copies of 4 or 8 bytes (no register staging,
-// so every halo load of a thread is in flight at once); src_bytes 0 writes
-// zeros, which is the window's zero padding outside the image.
+// so several rows of a strip are in flight at once).
 template <int BYTES>
-__device__ __forceinline__ void cp_async(void *dst, const void *src, bool in) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src),
-                 "n"(BYTES), "r"(in ? BYTES : 0)
+__device__ __forceinline__ void cp_async(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(dst), "l"(src), "n"(BYTES)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+__device__ __forceinline__ void lds(uint32_t at, float2 &u, float2 &v) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(u.x), "=f"(u.y), "=f"(v.x), "=f"(v.y)
+                 : "r"(at));
+}
+__device__ __forceinline__ void lds(uint32_t at, float &u, float &v) {
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n" : "=f"(u), "=f"(v) : "r"(at));
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+// this warp's row `SS_RING - 1` commits ago has arrived, for every lane
+__device__ __forceinline__ void ring_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SS_RING - 2) : "memory");
+    __syncwarp();
 }
 
 // the CTA's partials -> the last CTA reduces all of them in a fixed order
-__device__ void finish_loss(const SsimArgs &a, float ssim_sum, float l1_sum) {
-    __shared__ float red[SS_THREADS / 32];
+__device__ void finish_loss(const SsimArgs &a, double s, double l) {
     __shared__ bool last;
-    __shared__ double dred[2][SS_THREADS / 32];
-    const float bs = block_sum(ssim_sum, red);
-    const float bl = block_sum(l1_sum, red);
-    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const unsigned n_cta = gridDim.x * gridDim.y * gridDim.z;
+    __shared__ double dred[2][SS_WARPS];
+    auto all = [&](double &s, double &l) { // -> sums over the CTA in thread 0
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            l += __shfl_xor_sync(0xffffffffu, l, o);
+        }
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) {
+            dred[0][threadIdx.x >> 5] = s;
+            dred[1][threadIdx.x >> 5] = l;
+        }
+        __syncthreads();
+        s = l = 0.0;
+        for (int i = 0; i < SS_WARPS; ++i) {
+            s += dred[0][i];
+            l += dred[1][i];
+        }
+    };
+    all(s, l);
     if (threadIdx.x == 0) {
-        a.partials[2 * cta] = bs;
-        a.partials[2 * cta + 1] = bl;
+        a.partials[2 * blockIdx.x] = s;
+        a.partials[2 * blockIdx.x + 1] = l;
         __threadfence();
-        last = atomicAdd(a.counter, 1u) == n_cta - 1;
+        last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double s = 0.0, l = 0.0;
-    for (unsigned i = threadIdx.x; i < n_cta; i += SS_THREADS) {
-        s += (double)__ldcg(a.partials + 2 * i);
-        l += (double)__ldcg(a.partials + 2 * i + 1);
+    s = l = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += SS_THREADS) {
+        s += __ldcg(a.partials + 2 * i);
+        l += __ldcg(a.partials + 2 * i + 1);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        l += __shfl_xor_sync(0xffffffffu, l, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        dred[0][threadIdx.x >> 5] = s;
-        dred[1][threadIdx.x >> 5] = l;
-    }
-    __syncthreads();
+    all(s, l);
     if (threadIdx.x == 0) {
-        double ts = 0.0, tl = 0.0;
-        for (int i = 0; i < SS_THREADS / 32; ++i) {
-            ts += dred[0][i];
-            tl += dred[1][i];
-        }
-        const double ms = ts * a.inv_map, ml = tl * a.inv_px;
+        const double ms = s * a.inv_map, ml = l * a.inv_px;
         a.out[0] = (float)ms;
         a.out[1] = (float)ml;
         a.out[2] = (float)(a.wl1 * ml + a.wssim * ms + a.wconst);
@@ -156,209 +217,240 @@ __device__ void finish_loss(const SsimArgs &a, float ssim_sum, float l1_sum) {
 }
 
 template <bool GRAD>
-__global__ void __launch_bounds__(SS_THREADS, 4) ssim_map_kernel(const SsimArgs a) {
-    __shared__ float2 sxy[SS_IN * SS_IP];          // (x, y) over tile + halo
-    __shared__ float2 hA[SS_IN * SS_HP];           // horizontal (E x, E y)
-    __shared__ float2 hB[SS_IN * SS_HP];           // horizontal (E x^2, E y^2)
-    __shared__ float hP[SS_IN * SS_HP];            // horizontal E xy
-    const int plane = blockIdx.z;
-    const int img = plane / a.c, ch = plane % a.c;
-    const int y0 = blockIdx.y * SS_T, x0 = blockIdx.x * SS_T;
-    const float *X = a.img + img * a.is[0] + ch * a.is[1];
-    const float *Y = a.gt + img * a.gs[0] + ch * a.gs[1];
-    float g[SS_W];
+__global__ void __launch_bounds__(SS_THREADS, SS_CTAS) ssim_map_kernel(const SsimArgs a) {
+    __shared__ __align__(16) float2 ring_[SS_WARPS][SS_RING][SS_IP]; // (x, y)
+    constexpr int ROW = SS_IP * sizeof(float2);
+    float2(*ring)[SS_IP] = ring_[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const Strip st = strip_of(a);
+    float ssim_sum = 0.f, l1_sum = 0.f; // of sums of 8 rows
+    if (st.rows > 0) {
+        const int img = st.plane / a.c, ch = st.plane % a.c;
+        const Columns col(st.x0, a.w);
+        const int n_in = st.rows + 2 * SS_R;
+        // this lane's first column of the next row to fetch
+        const int y_first = max(st.y0 - SS_R, 0);
+        const float *X = a.img + img * a.is[0] + ch * a.is[1] + y_first * a.is[2] +
+                         (st.x0 - SS_R + lane) * a.is[3];
+        const float *Y = a.gt + img * a.gs[0] + ch * a.gs[1] + y_first * a.gs[2] +
+                         (st.x0 - SS_R + lane) * a.gs[3];
+        const int64_t x32 = 32 * a.is[3], y32 = 32 * a.gs[3];
+        const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(ring[0] + lane);
+        for (int e = lane; e < SS_RING * SS_IP; e += 32) ring[0][e] = make_float2(0.f, 0.f);
+        __syncwarp();
+        // row y0 - SS_R + i of both images (zero outside) into its slot
+        auto fetch = [&](int i) {
+            const int gy = st.y0 - SS_R + i;
+            if (i < n_in && gy >= 0) {
+                const uint32_t d = slot0 + i % SS_RING * ROW;
+                if (gy < a.h) {
 #pragma unroll
-    for (int t = 0; t < SS_W; ++t) g[t] = a.g[t];
-
-    // ---- tile and halo of the image and the target (zero outside), as
-    // asynchronous copies into the x and y halves of the pairs
-#pragma unroll
-    for (int k = 0; k < SS_LOADS; ++k) {
-        const int i = threadIdx.x + k * SS_THREADS;
-        if (i < SS_IN * SS_IN) {
-            const int r = i / SS_IN, cc = i - r * SS_IN;
-            const int gy = y0 - SS_R + r, gx = x0 - SS_R + cc;
-            const bool in = gy >= 0 && gy < a.h && gx >= 0 && gx < a.w;
-            const int64_t ox = in ? gy * a.is[2] + gx * a.is[3] : 0;
-            const int64_t oy = in ? gy * a.gs[2] + gx * a.gs[3] : 0;
-            float *d = reinterpret_cast<float *>(&sxy[r * SS_IP + cc]);
-            cp_async<4>(d, X + ox, in);
-            cp_async<4>(d + 1, Y + oy, in);
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-
-    // ---- horizontal pass: (row, 4 outputs) per item; x and y (then x^2
-    // and y^2) share packed FMAs, xy runs scalar
-    for (int it = threadIdx.x; it < SS_IN * (SS_T / 4); it += SS_THREADS) {
-        const int r = it % SS_IN, c0 = (it / SS_IN) * 4;
-        float2 v[14], acc2[4];
-        float p[14], acc[4];
-#pragma unroll
-        for (int j = 0; j < 14; ++j) {
-            v[j] = sxy[r * SS_IP + c0 + j];
-            p[j] = v[j].x * v[j].y;
-        }
-        const int o0 = r * SS_HP + c0;
-        taps4x2(g, v, acc2);
-#pragma unroll
-        for (int o = 0; o < 4; ++o) hA[o0 + o] = acc2[o];
-        taps4(g, p, acc);
-#pragma unroll
-        for (int o = 0; o < 4; ++o) hP[o0 + o] = acc[o];
-#pragma unroll
-        for (int j = 0; j < 14; ++j) v[j] = __fmul2_rn(v[j], v[j]);
-        taps4x2(g, v, acc2);
-#pragma unroll
-        for (int o = 0; o < 4; ++o) hB[o0 + o] = acc2[o];
-    }
-    __syncthreads();
-
-    // ---- vertical pass, map, derivatives: (column, 4 rows) per thread
-    float ssim_sum = 0.f;
-    {
-        const int cx = threadIdx.x % SS_T, r0 = (threadIdx.x / SS_T) * 4;
-        float2 mA[4], mB[4];
-        float mP[4];
-        {
-            float2 v[14];
-#pragma unroll
-            for (int j = 0; j < 14; ++j) v[j] = hA[(r0 + j) * SS_HP + cx];
-            taps4x2(g, v, mA);
-#pragma unroll
-            for (int j = 0; j < 14; ++j) v[j] = hB[(r0 + j) * SS_HP + cx];
-            taps4x2(g, v, mB);
-            float q[14];
-#pragma unroll
-            for (int j = 0; j < 14; ++j) q[j] = hP[(r0 + j) * SS_HP + cx];
-            taps4(g, q, mP);
-        }
-        const int gx = x0 + cx;
-        const int64_t hw = (int64_t)a.h * a.w;
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-            const int gy = y0 + r0 + o;
-            const bool inside = gy < a.h && gx < a.w;
-            bool counted = inside;
-            if (a.valid)
-                counted = counted && gy >= SS_R && gy < a.h - SS_R && gx >= SS_R && gx < a.w - SS_R;
-            const float mx = mA[o].x, my = mA[o].y;
-            const float mxx = mx * mx, myy = my * my, mxy = mx * my;
-            const float vx = mB[o].x - mxx, vy = mB[o].y - myy, cxy = mP[o] - mxy;
-            const float A1 = 2.f * mxy + a.c1, A2 = 2.f * cxy + a.c2;
-            const float B1 = mxx + myy + a.c1, B2 = vx + vy + a.c2;
-            const float s = (A1 * A2) / (B1 * B2);
-            if (counted) ssim_sum += s;
-            if (GRAD && inside) {
-                float d0 = 0.f, d1 = 0.f, d2 = 0.f;
-                if (counted) {
-                    const float iB1 = 1.f / B1, iB2 = 1.f / B2, iBB = iB1 * iB2;
-                    d0 = 2.f * my * (A2 - A1) * iBB - 2.f * mx * s * (iB1 - iB2);
-                    d1 = -s * iB2;
-                    d2 = 2.f * A1 * iBB;
+                    for (int k = 0; k < 3; ++k)
+                        if (col.in[k]) {
+                            cp_async<4>(d + 256 * k, X + k * x32);
+                            cp_async<4>(d + 256 * k + 4, Y + k * y32);
+                        }
+                    X += a.is[2];
+                    Y += a.gs[2];
+                } else {
+                    for (int e = lane; e < SS_IP; e += 32)
+                        ring[i % SS_RING][e] = make_float2(0.f, 0.f);
                 }
-                const int64_t at = (int64_t)plane * hw + (int64_t)gy * a.w + gx;
-                a.dmap0[at] = d0;
-                a.dmap12[at] = make_float2(d1, d2);
             }
+            cp_async_commit();
+        };
+        float g[SS_R + 1];
+#pragma unroll
+        for (int t = 0; t <= SS_R; ++t) g[t] = a.g[t];
+        float2 A[2][SS_W - 1], B[2][SS_W - 1]; // running sums of (x, y), (x^2 + y^2, x y)
+#pragma unroll
+        for (int k = 0; k < SS_W - 1; ++k)
+            A[0][k] = A[1][k] = B[0][k] = B[1][k] = make_float2(0.f, 0.f);
+        const int gx = st.x0 + 2 * lane;
+        const bool col0 = gx < a.w;
+        bool cnt[2]; // columns that count for the mean
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            cnt[c] = a.valid ? gx + c >= SS_R && gx + c < a.w - SS_R : gx + c < a.w;
+        int64_t at = ((int64_t)st.plane * a.h + st.y0) * a.pitch + gx;
+        float s_run = 0.f, l_run = 0.f; // of up to 8 rows
+        float2 mA[2], mB[2];
+        const uint32_t read0 = (uint32_t)__cvta_generic_to_shared(ring[0]) + 16 * lane;
+        // takes row i; what it completes is in mA and mB
+        auto step = [&](int i) {
+            ring_wait();
+            fetch(i + SS_RING - 1); // into the slot that row i - 1 left
+            float2 v[12];
+            const uint32_t row = read0 + i % SS_RING * ROW;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) lds(row + 16 * j, v[2 * j], v[2 * j + 1]);
+            if (i >= SS_R && i < SS_R + st.rows)
+                l_run += fabsf(v[SS_R].x - v[SS_R].y) + fabsf(v[SS_R + 1].x - v[SS_R + 1].y);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) mA[c] = roll(g, A[c], taps(g, v + c));
+#pragma unroll
+            for (int j = 0; j < 12; ++j)
+                v[j] = make_float2(fmaf(v[j].x, v[j].x, v[j].y * v[j].y), v[j].x * v[j].y);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) mB[c] = roll(g, B[c], taps(g, v + c));
+            if (i % 8 == 7) {
+                ssim_sum += s_run;
+                l1_sum += l_run;
+                s_run = l_run = 0.f;
+            }
+        };
+        for (int i = 0; i < SS_RING - 1; ++i) fetch(i);
+        for (int i = 0; i < 2 * SS_R; ++i) step(i);
+        for (int i = 2 * SS_R; i < n_in; ++i) {
+            step(i);
+            const int gy = st.y0 + i - 2 * SS_R;
+            const bool row_counts = !a.valid || (gy >= SS_R && gy < a.h - SS_R);
+            float d0[2], d1[2], d2[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const bool counted = row_counts && cnt[c];
+                const float mx = mA[c].x, my = mA[c].y;
+                const float mxx = mx * mx, myy = my * my, mxy = mx * my;
+                const float vxy = (mB[c].x - mxx) - myy, cxy = mB[c].y - mxy;
+                const float A1 = 2.f * mxy + a.c1, A2 = 2.f * cxy + a.c2;
+                const float B1 = mxx + myy + a.c1, B2 = vxy + a.c2;
+                const float s = (A1 * A2) / (B1 * B2);
+                s_run += counted ? s : 0.f;
+                if (GRAD) {
+                    const float iB1 = 1.f / B1, iB2 = 1.f / B2, iBB = iB1 * iB2;
+                    d0[c] = counted ? 2.f * my * (A2 - A1) * iBB - 2.f * mx * s * (iB1 - iB2) : 0.f;
+                    d1[c] = counted ? -s * iB2 : 0.f;
+                    d2[c] = counted ? 2.f * A1 * iBB : 0.f;
+                }
+            }
+            if (GRAD && col0) { // the pitch is even: a pair fits
+                *reinterpret_cast<float2 *>(a.dmap0 + at) = make_float2(d0[0], d0[1]);
+                *reinterpret_cast<float4 *>(a.dmap12 + at) = make_float4(d1[0], d2[0], d1[1], d2[1]);
+            }
+            at += a.pitch;
         }
-    }
-    // ---- L1 over the tile
-    float l1_sum = 0.f;
-    for (int i = threadIdx.x; i < SS_T * SS_T; i += SS_THREADS) {
-        const int r = i / SS_T, cx = i % SS_T;
-        if (y0 + r >= a.h || x0 + cx >= a.w) continue;
-        const float2 v = sxy[(r + SS_R) * SS_IP + cx + SS_R];
-        l1_sum += fabsf(v.x - v.y);
+        ssim_sum += s_run;
+        l1_sum += l_run;
     }
     finish_loss(a, ssim_sum, l1_sum);
 }
 
-__global__ void __launch_bounds__(SS_THREADS, 4) ssim_grad_kernel(const SsimArgs a) {
-    __shared__ float2 s12[SS_IN * SS_IP];  // (D1, D2) over tile + halo
-    __shared__ float s0[SS_IN * SS_IP];    // D0
-    __shared__ float2 h12[SS_IN * SS_HP];  // horizontal pass of (D1, D2)
-    __shared__ float h0[SS_IN * SS_HP];
-    // tiles in the reverse of the map kernel's order: the derivative planes
-    // it wrote last are the likeliest to still be in L2
-    const int plane = gridDim.z - 1 - blockIdx.z;
-    const int img = plane / a.c, ch = plane % a.c;
-    const int y0 = (gridDim.y - 1 - blockIdx.y) * SS_T, x0 = (gridDim.x - 1 - blockIdx.x) * SS_T;
-    const int64_t hw = (int64_t)a.h * a.w;
-    const float *D0 = a.dmap0 + (int64_t)plane * hw;
-    const float2 *D12 = a.dmap12 + (int64_t)plane * hw;
-    float g[SS_W];
-#pragma unroll
-    for (int t = 0; t < SS_W; ++t) g[t] = a.g[t];
-
-    // ---- the derivative planes over the tile and halo (zero outside), as
-    // asynchronous copies
-#pragma unroll
-    for (int k = 0; k < SS_LOADS; ++k) {
-        const int i = threadIdx.x + k * SS_THREADS;
-        if (i < SS_IN * SS_IN) {
-            const int r = i / SS_IN, cc = i - r * SS_IN;
-            const int gy = y0 - SS_R + r, gx = x0 - SS_R + cc;
-            const bool in = gy >= 0 && gy < a.h && gx >= 0 && gx < a.w;
-            const int64_t at = in ? (int64_t)gy * a.w + gx : 0;
-            cp_async<8>(&s12[r * SS_IP + cc], D12 + at, in);
-            cp_async<4>(&s0[r * SS_IP + cc], D0 + at, in);
-        }
+__global__ void __launch_bounds__(SS_THREADS, SS_CTAS) ssim_grad_kernel(const SsimArgs a) {
+    __shared__ __align__(16) float2 r12_[SS_WARPS][SS_RING][SS_IP]; // (D1, D2)
+    __shared__ __align__(16) float r0_[SS_WARPS][SS_RING][SS_IP];   // D0
+    __shared__ float px_[SS_WARPS][SS_RING][4][32]; // a lane's pixels: x, x, y, y
+    constexpr int ROW12 = SS_IP * sizeof(float2), ROW0 = SS_IP * sizeof(float);
+    float2(*r12)[SS_IP] = r12_[threadIdx.x >> 5];
+    float(*r0)[SS_IP] = r0_[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const float *px = px_[threadIdx.x >> 5][0][0] + lane;
+    const Strip st = strip_of(a);
+    if (st.rows <= 0) return;
+    const int img = st.plane / a.c, ch = st.plane % a.c;
+    const Columns col(st.x0, a.w);
+    const int n_in = st.rows + 2 * SS_R;
+    const int gx = st.x0 + 2 * lane;
+    const bool col0 = gx < a.w, col1 = gx + 1 < a.w;
+    // the next row to fetch: this lane's first column of the derivative
+    // planes, its two columns of the image and the target
+    const int64_t first = ((int64_t)st.plane * a.h + max(st.y0 - SS_R, 0)) * a.pitch + st.x0 - SS_R + lane;
+    const float *D0 = a.dmap0 + first;
+    const float2 *D12 = a.dmap12 + first;
+    const float *X = a.img + img * a.is[0] + ch * a.is[1] + gx * a.is[3] + st.y0 * a.is[2];
+    const float *Y = a.gt + img * a.gs[0] + ch * a.gs[1] + gx * a.gs[3] + st.y0 * a.gs[2];
+    float *Gd = a.grad + img * a.ds[0] + ch * a.ds[1] + gx * a.ds[3] + st.y0 * a.ds[2];
+    const uint32_t slot12 = (uint32_t)__cvta_generic_to_shared(r12[0] + lane);
+    const uint32_t slot0 = (uint32_t)__cvta_generic_to_shared(r0[0] + lane);
+    const uint32_t slot_px = (uint32_t)__cvta_generic_to_shared(px);
+    for (int e = lane; e < SS_RING * SS_IP; e += 32) {
+        r12[0][e] = make_float2(0.f, 0.f);
+        r0[0][e] = 0.f;
     }
-    cp_async_wait_all();
-    __syncthreads();
-    // ---- horizontal pass: (row, 4 outputs) per item, D1 and D2 packed
-    for (int it = threadIdx.x; it < SS_IN * (SS_T / 4); it += SS_THREADS) {
-        const int r = it % SS_IN, c0 = (it / SS_IN) * 4;
+    __syncwarp();
+    // row y0 - SS_R + i of the planes (zero outside) into its slot, with the
+    // pixels of the row that it completes
+    auto fetch = [&](int i) {
+        const int gy = st.y0 - SS_R + i;
+        const int slot = i % SS_RING;
+        if (i < n_in && gy >= 0) {
+            if (gy < a.h) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    if (col.in[k]) {
+                        cp_async<8>(slot12 + slot * ROW12 + 256 * k, D12 + 32 * k);
+                        cp_async<4>(slot0 + slot * ROW0 + 128 * k, D0 + 32 * k);
+                    }
+                D12 += a.pitch;
+                D0 += a.pitch;
+            } else {
+                for (int e = lane; e < SS_IP; e += 32) {
+                    r12[slot][e] = make_float2(0.f, 0.f);
+                    r0[slot][e] = 0.f;
+                }
+            }
+        }
+        if (i >= 2 * SS_R && i < n_in) {
+            const uint32_t d = slot_px + slot * 512;
+            if (col0) {
+                cp_async<4>(d, X);
+                cp_async<4>(d + 256, Y);
+            }
+            if (col1) {
+                cp_async<4>(d + 128, X + a.is[3]);
+                cp_async<4>(d + 384, Y + a.gs[3]);
+            }
+            X += a.is[2];
+            Y += a.gs[2];
+        }
+        cp_async_commit();
+    };
+    float g[SS_R + 1];
+#pragma unroll
+    for (int t = 0; t <= SS_R; ++t) g[t] = a.g[t];
+    float2 S12[2][SS_W - 1], G12[2];
+    float S0[2][SS_W - 1], G0[2];
+#pragma unroll
+    for (int k = 0; k < SS_W - 1; ++k)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            S12[c][k] = make_float2(0.f, 0.f);
+            S0[c][k] = 0.f;
+        }
+    const uint32_t read12 = (uint32_t)__cvta_generic_to_shared(r12[0]) + 16 * lane;
+    const uint32_t read0 = (uint32_t)__cvta_generic_to_shared(r0[0]) + 8 * lane;
+    auto step = [&](int i) {
+        ring_wait();
+        fetch(i + SS_RING - 1);
         {
-            float2 v[14], acc2[4];
+            float2 v[12];
 #pragma unroll
-            for (int j = 0; j < 14; ++j) v[j] = s12[r * SS_IP + c0 + j];
-            taps4x2(g, v, acc2);
+            for (int j = 0; j < 6; ++j)
+                lds(read12 + i % SS_RING * ROW12 + 16 * j, v[2 * j], v[2 * j + 1]);
 #pragma unroll
-            for (int o = 0; o < 4; ++o) h12[r * SS_HP + c0 + o] = acc2[o];
+            for (int c = 0; c < 2; ++c) G12[c] = roll(g, S12[c], taps(g, v + c));
         }
         {
-            float q[14], acc[4];
+            float v[12];
 #pragma unroll
-            for (int j = 0; j < 14; ++j) q[j] = s0[r * SS_IP + c0 + j];
-            taps4(g, q, acc);
+            for (int j = 0; j < 6; ++j)
+                lds(read0 + i % SS_RING * ROW0 + 8 * j, v[2 * j], v[2 * j + 1]);
 #pragma unroll
-            for (int o = 0; o < 4; ++o) h0[r * SS_HP + c0 + o] = acc[o];
+            for (int c = 0; c < 2; ++c) G0[c] = roll(g, S0[c], taps(g, v + c));
         }
-    }
-    __syncthreads();
-    // ---- vertical pass and the gradient: (column, 4 rows) per thread
-    const int cx = threadIdx.x % SS_T, r0 = (threadIdx.x / SS_T) * 4;
-    float2 G12[4];
-    float G0[4];
-    {
-        float2 v[14];
-#pragma unroll
-        for (int j = 0; j < 14; ++j) v[j] = h12[(r0 + j) * SS_HP + cx];
-        taps4x2(g, v, G12);
-    }
-    {
-        float q[14];
-#pragma unroll
-        for (int j = 0; j < 14; ++j) q[j] = h0[(r0 + j) * SS_HP + cx];
-        taps4(g, q, G0);
-    }
-    const float *X = a.img + img * a.is[0] + ch * a.is[1];
-    const float *Y = a.gt + img * a.gs[0] + ch * a.gs[1];
-    float *Gd = a.grad + img * a.ds[0] + ch * a.ds[1];
-    const int gx = x0 + cx;
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-        const int gy = y0 + r0 + o;
-        if (gy >= a.h || gx >= a.w) continue;
-        const float xv = __ldg(X + gy * a.is[2] + gx * a.is[3]);
-        const float yv = __ldg(Y + gy * a.gs[2] + gx * a.gs[3]);
-        const float d = xv - yv;
-        const float sg = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
-        Gd[gy * a.ds[2] + gx * a.ds[3]] =
-            fmaf(a.gb, fmaf(2.f * xv, G12[o].x, fmaf(yv, G12[o].y, G0[o])), a.ga * sg);
+    };
+    for (int i = 0; i < SS_RING - 1; ++i) fetch(i);
+    for (int i = 0; i < 2 * SS_R; ++i) step(i);
+    for (int i = 2 * SS_R; i < n_in; ++i) {
+        step(i);
+        const float *q = px + i % SS_RING * 128;
+        auto grad_of = [&](float x, float y, float2 d12, float d0) {
+            const float d = x - y;
+            const float sg = d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f);
+            return fmaf(a.gb, fmaf(2.f * x, d12.x, fmaf(y, d12.y, d0)), a.ga * sg);
+        };
+        if (col0) Gd[0] = grad_of(q[0], q[64], G12[0], G0[0]);
+        if (col1) Gd[a.ds[3]] = grad_of(q[32], q[96], G12[1], G0[1]);
+        Gd += a.ds[2];
     }
 }
 
@@ -446,6 +538,48 @@ int l1_grid(int64_t n) {
 
 size_t ws_header() { return 256; }
 
+// Rows per strip.  A strip's time is its rows plus the ten halo rows, times a
+// row's time with the warps that share its SM (measured: 0.4 us with 4 warps or
+// fewer, 0.58, 0.76 and 0.94 with 8, 12 and 16), so the strips either fill the
+// SMs evenly -- whole CTAs per SM, a few turns of four where an image is large
+// -- or stay few and long.  Of those the split with the smallest product.  Both
+// kernels, RGB, us (rows: time): 640x480 12: 36, 6: 42, 64: 69; 979x547 24: 47,
+// 10: 58, 108: 103; 1080p 54: 101, 40: 101, 108: 127; 2400x1600 80: 171, 32: 189,
+// 270: 279.
+struct SsimSplit {
+    int32_t strips_x, strips_y, rows;
+    int64_t ctas;
+    int32_t pitch;
+};
+SsimSplit ssim_split(int64_t planes, int32_t h, int32_t w) {
+    constexpr int64_t SMS = 152;
+    constexpr double ROW_US[SS_CTAS + 1] = {0.0, 0.40, 0.58, 0.76, 0.94};
+    SsimSplit s;
+    s.strips_x = (w + SS_C - 1) / SS_C;
+    const int64_t per_row = planes * s.strips_x;
+    double best = 1e300;
+    s.rows = h;
+    for (int64_t per_sm = 1; per_sm <= 64; ++per_sm) {
+        const int64_t fit = std::max<int64_t>(1, SMS * SS_WARPS * per_sm / per_row);
+        const int64_t rows = (h + fit - 1) / fit;
+        const int64_t ctas = (per_row * ((h + rows - 1) / rows) + SS_WARPS - 1) / SS_WARPS;
+        const int64_t used = (ctas + SMS - 1) / SMS;
+        const double cost = (double)(rows + 2 * SS_R) *
+                            ((double)(used / SS_CTAS) * ROW_US[SS_CTAS] + ROW_US[used % SS_CTAS]);
+        if (cost < best) {
+            best = cost;
+            s.rows = (int32_t)rows;
+        }
+    }
+    s.strips_y = (h + s.rows - 1) / s.rows;
+    s.ctas = (per_row * s.strips_y + SS_WARPS - 1) / SS_WARPS;
+    s.pitch = (w + 1) & ~1;
+    return s;
+}
+size_t ssim_partials_bytes(const SsimSplit &s) {
+    return ((size_t)s.ctas * 2 * sizeof(double) + 255) & ~(size_t)255;
+}
+
 } // namespace
 } // namespace ubs
 
@@ -456,11 +590,9 @@ extern "C" {
 size_t ubs_ssim_workspace_bytes(int32_t n_images, int32_t channels, int32_t height,
                                 int32_t width) {
     if (n_images <= 0 || channels <= 0 || height <= 0 || width <= 0) return ws_header();
-    const size_t ctas = (size_t)n_images * channels * ((height + SS_T - 1) / SS_T) *
-                        ((width + SS_T - 1) / SS_T);
-    const size_t part = (ctas * 2 * sizeof(float) + 255) & ~(size_t)255;
-    const size_t maps = (size_t)3 * n_images * channels * height * width * sizeof(float);
-    return ws_header() + part + maps;
+    const SsimSplit sp = ssim_split((int64_t)n_images * channels, height, width);
+    const size_t maps = (size_t)3 * n_images * channels * height * sp.pitch * sizeof(float);
+    return ws_header() + ssim_partials_bytes(sp) + maps;
 }
 
 int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
@@ -492,8 +624,11 @@ int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
     a.c = channels;
     a.h = height;
     a.w = width;
-    a.tiles_x = (width + SS_T - 1) / SS_T;
-    a.tiles_y = (height + SS_T - 1) / SS_T;
+    const SsimSplit sp = ssim_split((int64_t)n_images * channels, height, width);
+    a.strips_x = sp.strips_x;
+    a.strips_y = sp.strips_y;
+    a.rows = sp.rows;
+    a.pitch = sp.pitch;
     a.valid = valid_padding ? 1 : 0;
     a.c1 = (float)(0.01 * 0.01);
     a.c2 = (float)(0.03 * 0.03);
@@ -515,17 +650,15 @@ int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
         gs[i] = std::exp(-d * d / (2.0 * 1.5 * 1.5));
         tot += gs[i];
     }
-    for (int i = 0; i < SS_W; ++i) a.g[i] = (float)(gs[i] / tot);
-    const size_t ctas = (size_t)n_images * channels * a.tiles_x * a.tiles_y;
+    for (int i = 0; i <= SS_R; ++i) a.g[i] = (float)(gs[i] / tot); // symmetric
     a.counter = static_cast<unsigned *>(workspace);
-    a.partials = reinterpret_cast<float *>(static_cast<char *>(workspace) + ws_header());
-    char *maps = static_cast<char *>(workspace) + ws_header() +
-                 ((ctas * 2 * sizeof(float) + 255) & ~(size_t)255);
-    const size_t px_all = (size_t)n_images * channels * height * width;
+    a.partials = reinterpret_cast<double *>(static_cast<char *>(workspace) + ws_header());
+    char *maps = static_cast<char *>(workspace) + ws_header() + ssim_partials_bytes(sp);
+    const size_t px_all = (size_t)n_images * channels * height * sp.pitch;
     a.dmap12 = reinterpret_cast<float2 *>(maps);
     a.dmap0 = reinterpret_cast<float *>(maps + px_all * sizeof(float2));
     a.out = out;
-    const dim3 grid(a.tiles_x, a.tiles_y, n_images * channels);
+    const unsigned grid = (unsigned)sp.ctas;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (grad) {
         UBS_TIMED("ssim_map", st, ssim_map_kernel<true><<<grid, SS_THREADS, 0, st>>>(a));
