@@ -592,7 +592,7 @@ size_t ubs_ssim_workspace_bytes(int32_t n_images, int32_t channels, int32_t heig
     if (n_images <= 0 || channels <= 0 || height <= 0 || width <= 0) return ws_header();
     const SsimSplit sp = ssim_split((int64_t)n_images * channels, height, width);
     const size_t maps = (size_t)3 * n_images * channels * height * sp.pitch * sizeof(float);
-    return ws_header() + ssim_partials_bytes(sp) + maps;
+    return ws_header() + 16 + ssim_partials_bytes(sp) + maps;
 }
 
 int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
@@ -652,8 +652,12 @@ int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
     }
     for (int i = 0; i <= SS_R; ++i) a.g[i] = (float)(gs[i] / tot); // symmetric
     a.counter = static_cast<unsigned *>(workspace);
-    a.partials = reinterpret_cast<double *>(static_cast<char *>(workspace) + ws_header());
-    char *maps = static_cast<char *>(workspace) + ws_header() + ssim_partials_bytes(sp);
+    // 16-byte stores of derivative pairs: aligned here, whatever the caller's
+    // workspace is aligned to
+    char *part = reinterpret_cast<char *>(
+        (reinterpret_cast<uintptr_t>(workspace) + ws_header() + 15) & ~(uintptr_t)15);
+    a.partials = reinterpret_cast<double *>(part);
+    char *maps = part + ssim_partials_bytes(sp);
     const size_t px_all = (size_t)n_images * channels * height * sp.pitch;
     a.dmap12 = reinterpret_cast<float2 *>(maps);
     a.dmap0 = reinterpret_cast<float *>(maps + px_all * sizeof(float2));
