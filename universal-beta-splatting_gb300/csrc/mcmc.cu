@@ -100,6 +100,12 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t z) {
 __device__ __forceinline__ double uniform01(uint64_t seed, uint64_t i) {
     return (double)(splitmix64(seed + (i + 1) * 0x9e3779b97f4a7c15ull) >> 11) * 0x1.0p-53;
 }
+// The same value rounded to float, without the FP64 pipe: 53 bits round once
+// in the conversion, and the power of two is exact (measured, noise for 1M
+// primitives: 37 us through double, 22 this way).
+__device__ __forceinline__ float uniform01f(uint64_t seed, uint64_t i) {
+    return __ull2float_rn(splitmix64(seed + (i + 1) * 0x9e3779b97f4a7c15ull) >> 11) * 0x1.0p-53f;
+}
 
 // The opacity a source sampled `count` times shares with its copies
 // (scene/beta_model.py:553-562): logit(clamp(1 - (1 - o)^(1/(count+1)),
@@ -112,9 +118,39 @@ __device__ __forceinline__ float split_opacity(float raw, int count) {
     return logf(n / (1.f - n));
 }
 
-__device__ __forceinline__ bool is_dead(const float *op, const uint8_t *mask, float thresh,
-                                        int64_t i) {
-    return mask ? mask[i] != 0 : sigmoid_fast(op[i]) <= thresh;
+// The four weights (0: dead or past the end) and dead flags from element `base`
+// (a multiple of four) on; the loads are issued together, in one access each
+// where the alignment allows it.
+__device__ __forceinline__ void load_weights(const float *__restrict__ op,
+                                             const uint8_t *__restrict__ mask, float thresh,
+                                             int relocate, int64_t n, int64_t base,
+                                             double (&ws)[MC_PER], bool (&dead)[MC_PER]) {
+    float o[MC_PER] = {};
+    uint8_t m[MC_PER] = {};
+    const bool masked = relocate && mask;
+    if (base + MC_PER <= n && (reinterpret_cast<uintptr_t>(op) & 15) == 0 &&
+        (!masked || (reinterpret_cast<uintptr_t>(mask) & 3) == 0)) {
+        const float4 q = *reinterpret_cast<const float4 *>(op + base);
+        o[0] = q.x, o[1] = q.y, o[2] = q.z, o[3] = q.w;
+        if (masked) {
+            const uchar4 b = *reinterpret_cast<const uchar4 *>(mask + base);
+            m[0] = b.x, m[1] = b.y, m[2] = b.z, m[3] = b.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < MC_PER; ++k)
+            if (base + k < n) {
+                o[k] = op[base + k];
+                if (masked) m[k] = mask[base + k];
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < MC_PER; ++k) {
+        const bool in = base + k < n;
+        const float v = sigmoid_fast(o[k]);
+        dead[k] = in && relocate && (mask ? m[k] != 0 : v <= thresh);
+        ws[k] = in && !dead[k] ? (double)v : 0.0;
+    }
 }
 
 // ---- 1. weights: block sums and dead counts
@@ -123,22 +159,21 @@ __global__ void __launch_bounds__(MC_THREADS) weights_kernel(const float *__rest
                                                              float thresh, int relocate,
                                                              int64_t n, Ws w) {
     const int64_t base = (int64_t)blockIdx.x * MC_BLOCK + threadIdx.x * MC_PER;
-    double s = 0.0;
-    long long d = 0;
+    double s = 0.0, ws[MC_PER];
+    bool dead[MC_PER];
+    int d = 0;
+    load_weights(op, mask, thresh, relocate, n, base, ws, dead);
 #pragma unroll
     for (int k = 0; k < MC_PER; ++k) {
-        const int64_t i = base + k;
-        if (i >= n) break;
-        const bool dead = relocate && is_dead(op, mask, thresh, i);
-        d += dead;
-        if (!dead) s += (double)sigmoid_fast(op[i]);
+        s += ws[k];
+        d += dead[k];
     }
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, o);
         d += __shfl_xor_sync(0xffffffffu, d, o);
     }
     __shared__ double ss[MC_THREADS / 32];
-    __shared__ long long sd[MC_THREADS / 32];
+    __shared__ int sd[MC_THREADS / 32];
     if ((threadIdx.x & 31) == 0) {
         ss[threadIdx.x >> 5] = s;
         sd[threadIdx.x >> 5] = d;
@@ -146,7 +181,7 @@ __global__ void __launch_bounds__(MC_THREADS) weights_kernel(const float *__rest
     __syncthreads();
     if (threadIdx.x == 0) {
         double ts = 0.0;
-        long long td = 0;
+        int td = 0;
         for (int i = 0; i < MC_THREADS / 32; ++i) {
             ts += ss[i];
             td += sd[i];
@@ -230,18 +265,14 @@ __global__ void __launch_bounds__(MC_THREADS) cdf_kernel(const float *__restrict
                                                          Ws w) {
     const int64_t base = (int64_t)blockIdx.x * MC_BLOCK + threadIdx.x * MC_PER;
     double ws[MC_PER];
-    int dd[MC_PER];
+    bool dd[MC_PER];
+    load_weights(op, mask, thresh, relocate, n, base, ws, dd);
     double s = 0.0;
     int d = 0;
 #pragma unroll
     for (int k = 0; k < MC_PER; ++k) {
-        const int64_t i = base + k;
-        const bool in = i < n;
-        const bool dead = in && relocate && is_dead(op, mask, thresh, i);
-        ws[k] = (in && !dead) ? (double)sigmoid_fast(op[i]) : 0.0;
-        dd[k] = dead;
         s += ws[k];
-        d += dead;
+        d += dd[k];
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double is = s;
@@ -340,13 +371,16 @@ __device__ __forceinline__ void row_col(int64_t e, int wd, int64_t &row, int &co
     }
 }
 
-// ---- 5. relocation: dead slot <- copy of its source, split opacity.
-// Element-parallel (blockIdx.y = tensor; a fixed grid walks the dead list,
-// whose length is known on the device): neighbouring threads touch
+// ---- 5. relocation: dead slot <- copy of its source, split opacity, and the
+// sources lose their Adam moments.  blockIdx.y = tensor * 3 + role (0
+// parameter, 1 exp_avg, 2 exp_avg_sq).  Element-parallel (a fixed grid walks the
+// dead list, whose length is known on the device): neighbouring threads touch
 // neighbouring floats of a row.  With a thread per row the copies of 100k rows
-// took 58 us and the resets 96 us.
-__global__ void __launch_bounds__(MC_THREADS) relocate_copy_kernel(McmcSet t, Ws w) {
-    const int k = blockIdx.y, wd = t.w[k];
+// took 58 us and the resets 96 us; as two launches of this form 36 and 49.
+__global__ void __launch_bounds__(MC_THREADS) relocate_rows_kernel(McmcSet t, Ws w) {
+    const int k = blockIdx.y / 3, role = blockIdx.y % 3, wd = t.w[k];
+    float *dst = role == 0 ? t.p[k] : role == 1 ? t.m[k] : t.v[k];
+    if (!dst) return;
     const int64_t total = (int64_t)w.hdr->n_dead * wd;
     const int64_t stride = (int64_t)gridDim.x * MC_THREADS;
     for (int64_t e = (int64_t)blockIdx.x * MC_THREADS + threadIdx.x; e < total; e += stride) {
@@ -355,31 +389,24 @@ __global__ void __launch_bounds__(MC_THREADS) relocate_copy_kernel(McmcSet t, Ws
         row_col(e, wd, j, c);
         const int32_t s = w.src[j];
         if (s < 0) continue;
-        const float v = t.p[k][(int64_t)s * wd + c];
-        t.p[k][(int64_t)w.dead_list[j] * wd + c] =
-            k == t.opac ? split_opacity(v, w.count[s]) : v;
+        const int64_t from = (int64_t)s * wd + c;
+        if (role) {
+            dst[from] = 0.f;
+            continue;
+        }
+        const float v = dst[from];
+        dst[(int64_t)w.dead_list[j] * wd + c] = k == t.opac ? split_opacity(v, w.count[s]) : v;
     }
 }
 
-// ---- 6. relocation: sources take the split opacity, lose their moments.
-// blockIdx.y = tensor * 2 + moment; the opacity's first plane also carries the
-// opacity over.
-__global__ void __launch_bounds__(MC_THREADS) relocate_sources_kernel(McmcSet t, Ws w) {
-    const int k = blockIdx.y / 2, second = blockIdx.y % 2, wd = t.w[k];
-    float *mom = second ? t.v[k] : t.m[k];
-    const bool carry = k == t.opac && !second;
-    if (!mom && !carry) return;
-    const int64_t total = (int64_t)w.hdr->n_dead * wd;
-    const int64_t stride = (int64_t)gridDim.x * MC_THREADS;
-    for (int64_t e = (int64_t)blockIdx.x * MC_THREADS + threadIdx.x; e < total; e += stride) {
-        int64_t j;
-        int c;
-        row_col(e, wd, j, c);
-        const int32_t s = w.src[j];
-        if (s < 0) continue;
-        if (carry) t.p[k][s] = t.p[k][w.dead_list[j]];
-        if (mom) mom[(int64_t)s * wd + c] = 0.f;
-    }
+// ---- 6. relocation: sources take the split opacity of their copies (in a
+// launch of its own: every copy has read the source's before)
+__global__ void __launch_bounds__(MC_THREADS) relocate_carry_kernel(McmcSet t, Ws w) {
+    float *op = t.p[t.opac];
+    const int64_t n_dead = w.hdr->n_dead;
+    for (int64_t j = (int64_t)blockIdx.x * MC_THREADS + threadIdx.x; j < n_dead;
+         j += (int64_t)gridDim.x * MC_THREADS)
+        if (w.src[j] >= 0) op[w.src[j]] = op[w.dead_list[j]];
 }
 
 // ---- addition: the grown tensors.  blockIdx.y = tensor * 3 + role (0
@@ -459,11 +486,11 @@ __global__ void __launch_bounds__(MC_THREADS) perturb_kernel(int64_t n, int dim,
     } else {
         // Box-Muller on two pairs of uniforms (the fourth normal is unused)
         for (int pr = 0; pr < 2; ++pr) {
-            const double u1 = uniform01(seed, (uint64_t)i * 4 + 2 * pr);
-            const double u2 = uniform01(seed, (uint64_t)i * 4 + 2 * pr + 1);
-            const float r = sqrtf(-2.f * logf(1.f - (float)u1));
+            const float u1 = uniform01f(seed, (uint64_t)i * 4 + 2 * pr);
+            const float u2 = uniform01f(seed, (uint64_t)i * 4 + 2 * pr + 1);
+            const float r = sqrtf(-2.f * logf(1.f - u1));
             float sn, cs;
-            sincospif(2.f * (float)u2, &sn, &cs);
+            sincospif(2.f * u2, &sn, &cs);
             z[2 * pr] = r * cs;
             if (2 * pr + 1 < 3) z[2 * pr + 1] = r * sn;
         }
@@ -514,9 +541,10 @@ int load_set(const ubs_mcmc_tensors *in, McmcSet &out, bool need_params) {
     return UBS_OK;
 }
 
-// Blocks per plane of the element-parallel row kernels: at most four per SM.
+// Blocks per plane of the element-parallel row kernels.
+constexpr int64_t ROWS_GRID = 608; // four per SM
 unsigned rows_grid(int64_t rows) {
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(rows, MC_THREADS), 608));
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(rows, MC_THREADS), ROWS_GRID));
 }
 
 // steps 1-4
@@ -574,10 +602,10 @@ int ubs_mcmc_relocate(const ubs_mcmc_tensors *scene, int64_t n_prims, const uint
                    status, st);
     if (r != UBS_OK) return r;
     const unsigned g = rows_grid(n_prims);
-    UBS_TIMED("mcmc_relocate_copy", st,
-              relocate_copy_kernel<<<dim3(g, t.n), MC_THREADS, 0, st>>>(t, w));
-    UBS_TIMED("mcmc_relocate_sources", st,
-              relocate_sources_kernel<<<dim3(g, 2 * t.n), MC_THREADS, 0, st>>>(t, w));
+    UBS_TIMED("mcmc_relocate_rows", st,
+              relocate_rows_kernel<<<dim3(g, 3 * t.n), MC_THREADS, 0, st>>>(t, w));
+    UBS_TIMED("mcmc_relocate_carry", st,
+              relocate_carry_kernel<<<g, MC_THREADS, 0, st>>>(t, w));
     note_launch(2);
     return check_launch("mcmc_relocate");
 }
