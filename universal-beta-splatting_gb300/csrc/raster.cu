@@ -22,8 +22,9 @@
 //     pixels;
 //   * the backward sums the 7 + channels gradients of a record over a warp on
 //     the tensor cores (moments of per-pixel values with constant weights, see
-//     moment_products) and a transpose reduction, each warp writes its totals into its own list of rows in shared memory with plain stores, and
-//     per batch the rows of a record are summed and added to its gradient row
+//     moment_products) and a transpose reduction, each warp writes its totals
+//     into its own list of rows in shared memory with plain stores, and per
+//     batch the rows of a record are summed and added to its gradient row
 //     with three 16-byte vector atomics (fused path) or one scalar atomic per
 //     value (drop-in arrays).
 #include <atomic>
@@ -185,27 +186,28 @@ __global__ void pack_records_kernel(int64_t T, int64_t n_prims, const int32_t *_
 // Thread layout: every thread owns two vertically adjacent pixels, a warp an
 // 8x8-pixel footprint; a TS x TS tile has (TS/8)^2 warps = TS*TS/2 threads and
 // streams its records in batches of RB*TS*TS/2, RB batch slots per thread in
-// the culling phase (RB = 1 in the backward of tiles up to 16 x 16 with packed
-// colours of at most 4 channels, whose smaller shared footprint lets 8 CTAs
-// share an SM; else 2).
-// The backward accumulates a batch's per-record gradient sums in one of two
-// ways.  KE = 0: one shared accumulator row per batch slot (BR x NV floats),
-// which every warp adds its reduced sums to with shared-memory atomics, and a
-// touched flag per slot.  KE > 0: every warp owns a list of KE entry rows
-// (row_pitch floats each, after a dump row) that it fills with plain stores,
-// one row per record it visits, last batch slot first: a slot's row is the
-// number of set bits after it in the warp's mask.  The flush sums the warps'
-// rows of a slot.  Shared float
-// atomics cost about as much as the rest of a visit's reduction, so the small
-// tiles use the lists.
+// the culling phase (RB = 1 in the backward and for colours of more than 4
+// channels, whose smaller shared footprint lets more CTAs share an SM; else 2).
+// In the backward every warp owns a list of KE entry rows (row_pitch floats
+// each, after a dump row) that it fills with plain stores, one row per record
+// it visits, last batch slot first: a slot's row is the number of set bits
+// after it in the warp's mask.  The flush sums the warps' rows of a slot.
+// (Shared accumulators with float atomics cost about as much as the rest of a
+// visit's reduction: 32 channels 871 against 346 us, 16 channels 122 against
+// 69, 5 channels 124 against 95 together with the squares of launch_blend.)
 struct SmemLayout {
-    int mask_off, rec_off, col_off, gacc_off, touched_off, total;
+    int mask_off, rec_off, col_off, rows_off, total;
 };
 
 // Whether the backward reduces a visit on the tensor cores (see
-// moment_reduce): its 5 + CD rows of sums have to fit the 8 rows one product
-// leaves in a lane's accumulators.
-template <int CD> __host__ __device__ constexpr bool moment_rows() { return CD <= 3; }
+// moment_products), and how many colour sums that takes along with the moments
+// of w and the sums of u and u log2(1 - s): three fit the accumulators.  A
+// fourth colour goes through lane exchanges (690k primitives with depth at
+// 720p: 528 -> 503 us).  Wider rows are mostly colours, whose exchanges
+// dominate either way, and stay on them (the others' sums on the tensor cores:
+// 16 channels 69 -> 68, 8 channels 92 -> 96, 32 channels 346 -> 352 us).
+template <int CD> __host__ __device__ constexpr bool moment_rows() { return CD <= 4; }
+template <int CD> __host__ __device__ constexpr int moment_colours() { return CD <= 3 ? CD : 3; }
 // Floats per entry row: the 6 moments of w, the sums of u and u log2(1 - s)
 // and CD colour sums, or the 7 + CD gradient sums.
 template <int CD> __host__ __device__ constexpr int row_pitch() {
@@ -213,8 +215,7 @@ template <int CD> __host__ __device__ constexpr int row_pitch() {
 }
 
 template <int CD, bool PACK, bool BWD>
-__host__ __device__ inline SmemLayout smem_layout(int NT, int RB = 2, int KE = 0) {
-    constexpr int NV = 7 + CD; // gradient values per record
+__host__ __device__ inline SmemLayout smem_layout(int NT, int RB, int KE) {
     const int nw = NT / 32, BR = RB * NT;
     SmemLayout L;
     L.mask_off = 32; // after two mbarriers and the cold flag of the backward
@@ -223,14 +224,8 @@ __host__ __device__ inline SmemLayout smem_layout(int NT, int RB = 2, int KE = 0
     L.rec_off = (L.mask_off + (BWD ? 2 : 1) * nw * RB * nw * 4 + nw * 4 + 127) & ~127;
     const int colbytes = PACK ? 16 : CD * 4;
     L.col_off = L.rec_off + 2 * BR * (int)sizeof(GeoRec);
-    L.gacc_off = (L.col_off + 2 * BR * colbytes + 15) & ~15;
-    if (BWD && KE > 0) {
-        L.touched_off = L.gacc_off + nw * (KE + 1) * row_pitch<CD>() * 4; // entry rows
-        L.total = L.touched_off;
-    } else {
-        L.touched_off = L.gacc_off + (BWD ? BR * NV * 4 : 0);
-        L.total = L.touched_off + (BWD ? BR * 4 : 0);
-    }
+    L.rows_off = (L.col_off + 2 * BR * colbytes + 15) & ~15;
+    L.total = L.rows_off + (BWD ? nw * (KE + 1) * row_pitch<CD>() * 4 : 0);
     return L;
 }
 
@@ -468,7 +463,7 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_fwd_ke
     extern __shared__ __align__(128) unsigned char sm[];
     const int TS = TSZ ? TSZ : a.TS;
     const int NT = TSZ ? TSZ * TSZ / 2 : (int)blockDim.x, nw = NT >> 5, BR = RB * NT;
-    const SmemLayout L = smem_layout<CD, PACK, false>(NT, RB);
+    const SmemLayout L = smem_layout<CD, PACK, false>(NT, RB, 0);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm);
     uint32_t *wmask = reinterpret_cast<uint32_t *>(sm + L.mask_off);
     float4 *srec = reinterpret_cast<float4 *>(sm + L.rec_off); // see staged_rec
@@ -755,16 +750,12 @@ __device__ __forceinline__ void pair_sums(const PairGeom &p, const float2 &w, co
     for (int k = 0; k < CD; ++k) g[7 + k] = gc[k].x + gc[k].y;
 }
 
-// Factor turning the reduced sum g[u] (u >= 2) of a record into its gradient
-// value u of [v_xy(2), v_conic(3), v_opacity, v_beta, v_colour(CD)]; v_xy is
-// -2 opacity beta (conic [w dx, w dy]) and is formed at the flush.  With
-// the entry lists the first two sums are multiplied by the conic per lane
-// before the reduction, so every value is a factor times its sum
-// (pre_conic = true).
-__device__ __forceinline__ float record_scale(int u, float opac, float beta,
-                                              bool pre_conic = false) {
+// Factor turning the reduced sum u of a record, the first two multiplied by
+// the conic, into its gradient value u of [v_xy(2), v_conic(3), v_opacity,
+// v_beta, v_colour(CD)].
+__device__ __forceinline__ float record_scale(int u, float opac, float beta) {
     const float ob = opac * beta;
-    if (u == 3 || (pre_conic && u < 2)) return -2.f * ob;
+    if (u == 3 || u < 2) return -2.f * ob;
     if (u < 5) return -ob;
     if (u == 6) return opac * 0.6931471805599453f;
     return 1.f;
@@ -840,6 +831,7 @@ struct MomentBasis {
 // rows: the warp's entry rows, of which the first is a dump.
 template <int CD>
 __device__ __forceinline__ MomentBasis moment_basis(int lane, const float *rows) {
+    constexpr int MC = moment_colours<CD>();
     const int g = lane >> 2, t = lane & 3;
     const float y0 = 2.f * t - 3.5f, y1 = y0 + 1.f, x = g - 3.5f;
     MomentBasis b;
@@ -859,8 +851,8 @@ __device__ __forceinline__ MomentBasis moment_basis(int lane, const float *rows)
     const int v = g >> 1;
     int off = -1;
     if (t == 0) off = v == 0 ? 3 : v == 1 ? 4 : -1;
-    if (t == 1) off = v == 0 ? 6 : v == 2 ? 7 : CD < 2 ? -1 : v == 1 ? 8 : 9;
-    if (t == 2) off = v == 0 ? 5 : (v == 3 && CD != 2) ? 7 + CD : -1;
+    if (t == 1) off = v == 0 ? 6 : v == 2 ? 7 : MC < 2 ? -1 : v == 1 ? 8 : 9;
+    if (t == 2) off = v == 0 ? 5 : (v == 3 && (MC & 1)) ? 7 + MC : -1;
     if (t == 3) off = v < 2 ? v : v == 3 ? 2 : -1;
     if (g & 1) off = -1;
     b.first = smem_u32(rows) + 4 * max(off, 0);
@@ -894,10 +886,10 @@ template <int CD>
 __device__ __forceinline__ void moment_products(const MomentBasis &mb, const float2 &w,
                                                 const float2 &u, const float2 &ul,
                                                 const float2 (&gc)[CD], float (&d)[4]) {
-    static_assert(moment_rows<CD>(), "two colours and an odd one");
+    constexpr int MC = moment_colours<CD>();
     const float us = u.x + u.y, uh = tf32_hi(us), ls = ul.x + ul.y, lh = tf32_hi(ls);
     float g0 = 0.f, g1 = 0.f, h0 = 0.f, h1 = 0.f;
-    if constexpr (CD >= 2) {
+    if constexpr (MC >= 2) {
         g0 = gc[0].x + gc[0].y;
         g1 = gc[1].x + gc[1].y;
         h0 = tf32_hi(g0);
@@ -907,8 +899,8 @@ __device__ __forceinline__ void moment_products(const MomentBasis &mb, const flo
     mma_tf32(d, us - uh, ls - lh, g0 - h0, g1 - h1, mb.c0, mb.c1);
     mma_tf32(d, uh, lh, h0, h1, mb.c0, mb.c1);
     float g2 = 0.f, h2 = 0.f;
-    if constexpr (CD != 2) {
-        g2 = gc[CD - 1].x + gc[CD - 1].y;
+    if constexpr (MC & 1) {
+        g2 = gc[MC - 1].x + gc[MC - 1].y;
         h2 = tf32_hi(g2);
     }
     const float wx = tf32_hi(w.x), wy = tf32_hi(w.y);
@@ -969,7 +961,7 @@ __device__ __forceinline__ void add_record(const RasterArgs &a, const GeoRec &q,
                                            float (&sum)[7 + CD]) {
     constexpr int NV = 7 + CD;
 #pragma unroll
-    for (int u = 0; u < NV; ++u) sum[u] *= record_scale(u, q.opac, q.beta, true);
+    for (int u = 0; u < NV; ++u) sum[u] *= record_scale(u, q.opac, q.beta);
     if (NV <= GRAD_ROW && a.v_rows) {
         // three 16-byte vector atomics per row instead of NV scalar ones
         float4 *row = reinterpret_cast<float4 *>(a.v_rows + (int64_t)q.gid * GRAD_ROW);
@@ -990,11 +982,12 @@ __device__ __forceinline__ void add_record(const RasterArgs &a, const GeoRec &q,
 }
 
 // TSZ: edge of a CTA's pixels, 8 or 16, or 0 for a whole tile of a.TS; MINB
-// CTAs per SM.  KE > 0: entry lists of KE rows per warp (see smem_layout).
+// CTAs per SM; KE entry rows per warp (see smem_layout).
 template <int CD, bool PACK, int TSZ, int RB, int MINB, int KE>
 __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_kernel(RasterArgs a) {
     constexpr int NV = 7 + CD;
-    constexpr bool MOM = KE > 0 && moment_rows<CD>(); // tensor-core reduction of the visits
+    constexpr bool MOM = moment_rows<CD>(); // tensor-core reduction of the visits
+    constexpr int MC = moment_colours<CD>();
     constexpr int RP = row_pitch<CD>();
     extern __shared__ __align__(128) unsigned char sm[];
     const int TS = TSZ ? TSZ : a.TS;
@@ -1007,8 +1000,7 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
     float4 *srec = reinterpret_cast<float4 *>(sm + L.rec_off); // see staged_rec
     const int pitch = 2 * BR;
     float *scol = reinterpret_cast<float *>(sm + L.col_off);
-    float *gacc = reinterpret_cast<float *>(sm + L.gacc_off);       // KE > 0: entry rows
-    int32_t *touched = reinterpret_cast<int32_t *>(sm + L.touched_off);
+    float *entry_rows = reinterpret_cast<float *>(sm + L.rows_off);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const CtaPart part = cta_part(a, TS);
@@ -1043,10 +1035,6 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
 
     const int32_t wb = __reduce_max_sync(0xffffffffu, max(sp.bin0, sp.bin1));
     if (lane == 0) wbin[warp] = wb;
-    if (KE == 0) {
-        for (int t = tid; t < BR * NV; t += NT) gacc[t] = 0.f;
-        for (int t = tid; t < BR; t += NT) touched[t] = 0;
-    }
     const bool gather = PACK && a.keys != nullptr;
     const int64_t lo_e = gather ? (int64_t)cam * a.n_per_view : 0;
     const int64_t hi_e = lo_e + a.n_per_view - 1;
@@ -1063,7 +1051,7 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
     const int nb = (hi_end - rs + BR - 1) / BR;
 
     MomentBasis mb;
-    float *const my_rows = gacc + warp * (KE + 1) * RP;
+    float *const my_rows = entry_rows + warp * (KE + 1) * RP;
     if constexpr (MOM) mb = moment_basis<CD>(lane, my_rows);
     // batch b covers [max(rs, hi_end - (b + 1) BR), hi_end - b BR): back to front
     int issued = 0, waited = 0;
@@ -1137,8 +1125,9 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
             break;
         }
         if constexpr (MOM) cold = cold || *cold_flag != 0;
-        int rows = 0; // KE > 0: entry rows this warp has filled in this batch
+        int rows = 0; // entry rows this warp has filled in this batch
         uint32_t row = MOM ? mb.first : 0; // this lane's element of the last row filled
+        float *fourth = my_rows + 8 + MC;  // and that row's fourth colour sum
 #pragma unroll 1
         for (int k = RB * nw - 1; k >= 0; --k) {
             uint32_t m = wmask[warp * RB * nw + k];
@@ -1163,6 +1152,13 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                     moment_products<CD>(mb, w, u, ul, gc, d);
                     row += mb.pitch;
                     moment_finish(mb, d, row);
+                    if constexpr (CD > MC) {
+                        fourth += RP;
+                        float c = gc[MC].x + gc[MC].y;
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+                        *fourth = c; // every lane holds it
+                    }
                 }
             }
 #pragma unroll 1
@@ -1178,31 +1174,22 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 float g[NV];
                 pair_sums<CD>(pg, w, u, ul, gc, g);
                 const LaneMasks lm = lane_masks(lane);
-                if constexpr (KE > 0) {
-                    const float g0 = g[0], g1 = g[1];
-                    g[0] = q.cxx * g0 + q.cxy * g1;
-                    g[1] = q.cxy * g0 + q.cyy * g1;
-                    if ((!MOM || cold) && rows < KE) {
-                        float *row = my_rows + (1 + rows) * RP;
-                        // every lane of a group holds the same total: all store it
-                        auto put = [row](int v, float tot, bool) { row[v] = tot; };
-                        ReduceChunks<0, NV>::run(g, lm, lane, put);
-                        ++rows;
-                    } else { // list full: this record's sums go straight to the arrays
-                        auto add = [&](int v, float tot, bool owner) {
-                            if (owner && tot != 0.f)
-                                atomicAdd(grad_dst<CD>(a, v, q.gid),
-                                          record_scale(v, q.opac, q.beta, true) * tot);
-                        };
-                        ReduceChunks<0, NV>::run(g, lm, lane, add);
-                    }
-                } else {
-                    float *acc = gacc + t * NV;
-                    auto add = [acc](int v, float tot, bool owner) {
-                        if (owner && tot != 0.f) atomicAdd(&acc[v], tot);
+                const float g0 = g[0], g1 = g[1];
+                g[0] = q.cxx * g0 + q.cxy * g1;
+                g[1] = q.cxy * g0 + q.cyy * g1;
+                if ((!MOM || cold) && rows < KE) {
+                    float *row = my_rows + (1 + rows) * RP;
+                    // every lane of a group holds the same total: all store it
+                    auto put = [row](int v, float tot, bool) { row[v] = tot; };
+                    ReduceChunks<0, NV>::run(g, lm, lane, put);
+                    ++rows;
+                } else { // list full: this record's sums go straight to the arrays
+                    auto add = [&](int v, float tot, bool owner) {
+                        if (owner && tot != 0.f)
+                            atomicAdd(grad_dst<CD>(a, v, q.gid),
+                                      record_scale(v, q.opac, q.beta) * tot);
                     };
                     ReduceChunks<0, NV>::run(g, lm, lane, add);
-                    if (lane == 0) touched[t] = 1;
                 }
             }
         }
@@ -1213,64 +1200,43 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
         for (int half = 0; half < RB; ++half)
             if (tid + half * NT < cnt) own[half] = staged_rec(batch, pitch, tid + half * NT);
         __syncthreads();
-        if constexpr (KE > 0) {
-#pragma unroll
-            for (int half = 0; half < RB; ++half) {
-                const int sl = tid + half * NT;
-                if (sl >= cnt) continue;
-                float sum[NV];
-                bool any = false;
-#pragma unroll
-                for (int u = 0; u < NV; ++u) sum[u] = 0.f;
-#pragma unroll 1
-                for (int w = 0; w < nw; ++w) {
-                    // the slot's row: the set bits after it in the warp's mask
-                    const uint32_t *mw = wmask + w * RB * nw;
-                    const uint32_t after = mw[sl >> 5] >> (sl & 31);
-                    if (!(after & 1u)) continue;
-                    int r = __popc(after) - 1;
-#pragma unroll 1
-                    for (int k = (sl >> 5) + 1; k < RB * nw; ++k) r += __popc(mw[k]);
-                    if (r >= KE) continue; // went straight to the arrays
-                    any = true;
-                    const float *row = gacc + (w * (KE + 1) + 1 + r) * RP;
-                    if (MOM && !cold) {
-                        if constexpr (MOM)
-                            add_moments<CD>(
-                                row, own[half].x - (float)(tile_x0 + (w % wpr) * 8 + 4),
-                                own[half].y - (float)(tile_y0 + (w / wpr) * 8 + 4), sum);
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < NV; ++u) sum[u] += row[u];
-                    }
-                }
-                if (!any) continue;
-                if (MOM && !cold) {
-                    const float s0 = sum[0], s1 = sum[1];
-                    sum[0] = own[half].cxx * s0 + own[half].cxy * s1;
-                    sum[1] = own[half].cxy * s0 + own[half].cyy * s1;
-                }
-                add_record<CD>(a, own[half], sum);
-            }
-            continue;
-        }
 #pragma unroll
         for (int half = 0; half < RB; ++half) {
             const int sl = tid + half * NT;
-            if (sl < cnt && touched[sl]) {
-                const GeoRec &r = own[half];
-                float *ga = gacc + sl * NV;
-                const float f2 = -2.f * r.opac * r.beta;
-                const float m0 = f2 * (r.cxx * ga[0] + r.cxy * ga[1]);
-                const float m1 = f2 * (r.cxy * ga[0] + r.cyy * ga[1]);
+            if (sl >= cnt) continue;
+            float sum[NV];
+            bool any = false;
 #pragma unroll
-                for (int u = 0; u < NV; ++u) {
-                    const float val = u == 0 ? m0 : u == 1 ? m1 : ga[u] * record_scale(u, r.opac, r.beta);
-                    if (val != 0.f) atomicAdd(grad_dst<CD>(a, u, r.gid), val);
-                    ga[u] = 0.f;
+            for (int u = 0; u < NV; ++u) sum[u] = 0.f;
+#pragma unroll 1
+            for (int w = 0; w < nw; ++w) {
+                // the slot's row: the set bits after it in the warp's mask
+                const uint32_t *mw = wmask + w * RB * nw;
+                const uint32_t after = mw[sl >> 5] >> (sl & 31);
+                if (!(after & 1u)) continue;
+                int r = __popc(after) - 1;
+#pragma unroll 1
+                for (int k = (sl >> 5) + 1; k < RB * nw; ++k) r += __popc(mw[k]);
+                if (r >= KE) continue; // went straight to the arrays
+                any = true;
+                const float *row = entry_rows + (w * (KE + 1) + 1 + r) * RP;
+                if (MOM && !cold) {
+                    if constexpr (MOM)
+                        add_moments<CD>(
+                            row, own[half].x - (float)(tile_x0 + (w % wpr) * 8 + 4),
+                            own[half].y - (float)(tile_y0 + (w / wpr) * 8 + 4), sum);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < NV; ++u) sum[u] += row[u];
                 }
-                touched[sl] = 0;
             }
+            if (!any) continue;
+            if (MOM && !cold) {
+                const float s0 = sum[0], s1 = sum[1];
+                sum[0] = own[half].cxx * s0 + own[half].cxy * s1;
+                sum[1] = own[half].cxy * s0 + own[half].cyy * s1;
+            }
+            add_record<CD>(a, own[half], sum);
         }
     }
     // no copy may still target this CTA's shared memory at exit
@@ -1282,16 +1248,6 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
 }
 
 // ------------------------------------------------------------- host side
-static bool channels_supported(int ch) {
-    switch (ch) {
-    case 1: case 2: case 3: case 4: case 5: case 8: case 9:
-    case 16: case 17: case 32: case 33:
-        return true;
-    default:
-        return false;
-    }
-}
-
 size_t raster_ws_bytes(int64_t T, int ch) {
     size_t b = 256 + (size_t)T * sizeof(GeoRec);
     if (ch <= 4) b += (size_t)T * 16;
@@ -1340,30 +1296,38 @@ constexpr int BWD_SMALL_GRID = 152 * 16;
 constexpr int ONE_WAVE = 152 * 6;
 constexpr int KE_SMALL = 64; // backward entry rows per warp
 
+// Shared memory of a CTA over a whole tile with an accumulator row and a flag
+// per batch slot.
+template <int CD, bool BWD> static int whole_tile_bytes(int ts) {
+    const int NT = ts * ts / 2;
+    return smem_layout<CD, false, BWD>(NT, 2, 0).rows_off + (BWD ? 2 * NT * (7 + CD + 1) * 4 : 0);
+}
+
 template <int CD, bool BWD>
 static int launch_blend(RasterArgs &a, cudaStream_t st) {
     constexpr bool PACK = CD <= 4;
-    // A CTA works on at most 16 x 16 pixels (two per thread) where colours are
-    // packed: larger tiles are cut into squares of 16 x 16 (32) or 8 x 8 (24)
-    // whose CTAs share the tile's records (backward; 1M primitives at 1080p,
-    // tiles of 32: 1.85 -> 1.08 ms).  Wider colour rows need more registers
-    // and shared memory and keep one CTA per tile.
-    const bool cut = PACK && !a.pair_count;
+    // A CTA works on at most 16 x 16 pixels (two per thread): larger tiles are
+    // cut into squares of 16 x 16 (32) or 8 x 8 (24) whose CTAs share the tile's
+    // records (backward; 1M primitives at 1080p, tiles of 32: 1.85 -> 1.08 ms).
+    const bool cut = !a.pair_count;
     const int64_t cta16 = (int64_t)a.n_buckets * (a.TS / 16) * (a.TS / 16);
     const int edge = !cut ? a.TS : a.TS % 16 != 0 || cta16 < ONE_WAVE ? 8 : 16;
     a.sub = a.TS / edge;
     const int NT = edge * edge / 2;
-    const bool small = PACK && NT <= 128;
+    const bool small = NT <= 128;
     const int variant = (small && CD == 3 && !a.pair_count)
                             ? (BWD ? g_blend_bwd_variant.load() : g_blend_fwd_variant.load())
                             : 0;
-    int RB = (small && BWD) ? 1 : 2;
-    if (!BWD && variant == 1) RB = 1;
-    const int KE = BWD && small ? KE_SMALL : 0;
-    const SmemLayout L = smem_layout<CD, PACK, BWD>(NT, RB, KE);
-    if (L.total > 227 * 1024)
+    // wide colour rows: one batch slot per thread (forward, 32 channels: 209 ->
+    // 176, 16 channels: 46 -> 42 us)
+    const int RB = BWD || variant == 1 || (!PACK && cut) ? 1 : 2;
+    const SmemLayout L = smem_layout<CD, PACK, BWD>(NT, RB, KE_SMALL);
+    // wide colours: what a CTA over the whole tile would need stays the limit on
+    // tile size and channels
+    const int whole = PACK ? L.total : whole_tile_bytes<CD, BWD>(a.TS);
+    if (whole > 227 * 1024)
         return set_error(UBS_ERR_UNSUPPORTED, "raster: tile_size %d with %d channels needs %d B "
-                                              "of shared memory", a.TS, CD, L.total);
+                                              "of shared memory", a.TS, CD, whole);
     const int64_t nblocks = (int64_t)a.n_buckets * a.sub * a.sub;
     if (nblocks == 0) return UBS_OK;
     UBS_REQUIRE(nblocks < (1ll << 31), "raster: %lld thread blocks", (long long)nblocks);
@@ -1382,7 +1346,10 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
                 : per_sm == 7 ? raster_bwd_kernel<CD, true, 16, 1, 7, KE_SMALL>
                               : raster_bwd_kernel<CD, true, 16, 1, C16, KE_SMALL>;
     } else if constexpr (BWD) {
-        k = raster_bwd_kernel<CD, false, 0, 2, 1, 0>;
+        // registers allow 4 CTAs of 128 threads per SM, 2 of the widest
+        constexpr int C16 = CD <= 17 ? 4 : 2;
+        k = edge == 8 ? raster_bwd_kernel<CD, false, 8, 1, 4 * C16, KE_SMALL>
+                      : raster_bwd_kernel<CD, false, 16, 1, C16, KE_SMALL>;
     } else if (a.pair_count) {
         k = raster_fwd_kernel<CD, PACK, true, 0, 2, 1>;
     } else {
@@ -1398,7 +1365,9 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
                 k = e8 ? raster_fwd_kernel<CD, true, false, 8, 2, 32>
                        : raster_fwd_kernel<CD, true, false, 16, 2, 8>;
         } else {
-            k = raster_fwd_kernel<CD, false, false, 0, 2, 1>;
+            constexpr int C16 = CD <= 9 ? 6 : CD <= 17 ? 5 : 3;
+            k = edge == 8 ? raster_fwd_kernel<CD, false, false, 8, 1, 4 * C16>
+                          : raster_fwd_kernel<CD, false, false, 16, 1, C16>;
         }
     }
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) !=
