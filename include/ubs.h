@@ -296,6 +296,10 @@ size_t ubs_l1_loss_workspace_bytes(int64_t n);
 int ubs_l1_loss(const float *x, const float *y, float *grad, int64_t n, double weight,
                 float *out, void *workspace, size_t workspace_bytes, void *stream);
 
+/* out[i] = x[i] * *by for a device scalar: a loss's stored gradient times the
+ * incoming one.  out may be x. */
+int ubs_scale(const float *x, const float *by, float *out, int64_t n, void *stream);
+
 /* --------------------------------------------------- MCMC densification ---
  * BetaModel.relocate_gs / add_new_gs (scene/beta_model.py:553-658) and the
  * position noise of train.py:164-171, on the device with no host

@@ -385,10 +385,27 @@ py::tuple pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tens
 }
 
 // ------------------------------------------------------------------- losses
-// The stored gradient of a loss times the incoming scalar.
+// The stored gradient of a loss times the incoming scalar.  One kernel over
+// dense float32 tensors of one device; anything else (a gradient that is itself
+// differentiated, what saved-tensor hooks may return) multiplies in general.
 variable_list scaled(const variable_list &s, variable_list &g, size_t n) {
     variable_list o(n);
-    if (g[0].defined()) o[0] = s[0] * g[0];
+    if (!g[0].defined()) return o;
+    const Tensor &x = s[0], &by = g[0];
+    const auto plain = [](const Tensor &t) {
+        const c10::DispatchKeySet k = t.key_set();
+        return t.layout() == at::kStrided && t.is_cuda() && t.scalar_type() == at::kFloat &&
+               !k.has(c10::DispatchKey::Python) && !k.has(c10::DispatchKey::FuncTorchBatched) &&
+               !k.has(c10::DispatchKey::Batched) && !t.is_neg() && !t._fw_grad(0).defined();
+    };
+    if (at::GradMode::is_enabled() || !plain(x) || !plain(by) || by.dim() != 0 ||
+        x.device() != by.device() || !x.is_non_overlapping_and_dense()) {
+        o[0] = x * by;
+        return o;
+    }
+    const c10::cuda::CUDAGuard guard(x.device());
+    o[0] = at::empty_like(x);
+    UBS_CALL(ubs_scale, fp(x), fp(by), fpm(o[0]), x.numel(), stream_of(x));
     return o;
 }
 

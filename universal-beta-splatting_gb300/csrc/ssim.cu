@@ -527,6 +527,36 @@ __global__ void __launch_bounds__(L1_THREADS) l1_kernel(const float *__restrict_
     }
 }
 
+// out = x times a device scalar (the stored gradient of a loss times the incoming
+// one): four 16-byte accesses per thread in flight.  Bound by memory; 8 views of
+// 1352x1014 (33M floats): 40 us, against 81 of the general broadcast product.
+constexpr int SCALE_THREADS = 256, SCALE_UNROLL = 4;
+__global__ void __launch_bounds__(SCALE_THREADS) scale_kernel(const float *__restrict__ x,
+                                                              const float *__restrict__ by,
+                                                              float *__restrict__ out, int64_t n) {
+    const float f = *by;
+    const int64_t i0 = (int64_t)blockIdx.x * (SCALE_THREADS * SCALE_UNROLL) + threadIdx.x;
+    int64_t done = 0;
+    if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+        const int64_t n4 = n >> 2;
+        float4 v[SCALE_UNROLL];
+#pragma unroll
+        for (int k = 0; k < SCALE_UNROLL; ++k)
+            if (i0 + k * SCALE_THREADS < n4)
+                v[k] = reinterpret_cast<const float4 *>(x)[i0 + k * SCALE_THREADS];
+#pragma unroll
+        for (int k = 0; k < SCALE_UNROLL; ++k)
+            if (i0 + k * SCALE_THREADS < n4)
+                reinterpret_cast<float4 *>(out)[i0 + k * SCALE_THREADS] =
+                    make_float4(v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f);
+        done = n4 << 2;
+    }
+    // what is left: everything, or up to three floats
+    for (int64_t i = done + (int64_t)blockIdx.x * SCALE_THREADS + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * SCALE_THREADS)
+        out[i] = x[i] * f;
+}
+
 int l1_grid(int64_t n) {
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
@@ -673,6 +703,18 @@ int ubs_ssim_loss(const float *img, const int64_t *img_strides, const float *gt,
         note_launch();
     }
     return check_launch("ssim_loss");
+}
+
+int ubs_scale(const float *x, const float *by, float *out, int64_t n, void *stream) {
+    UBS_REQUIRE(n >= 0 && (n == 0 || (x && by && out)), "scale: bad arguments");
+    if (n == 0) return UBS_OK;
+    constexpr int64_t per = 4LL * SCALE_THREADS * SCALE_UNROLL;
+    UBS_REQUIRE((n + per - 1) / per < (1LL << 31), "scale: too many values");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    UBS_TIMED("loss_scale", st,
+              scale_kernel<<<(unsigned)((n + per - 1) / per), SCALE_THREADS, 0, st>>>(x, by, out, n));
+    note_launch();
+    return check_launch("scale");
 }
 
 size_t ubs_l1_loss_workspace_bytes(int64_t n) {
