@@ -52,10 +52,10 @@ constexpr int kCountReplicas = 8;
 
 struct CountWs {
     IsectHeader *hdr;
-    int32_t *bucket_counts; // [C*n_tiles]
     int32_t *replicas;      // [kCountReplicas][C*n_tiles]
+    int32_t *bucket_counts; // [C*n_tiles], frames of more than SCAN_ORDER_MAX buckets
     int64_t *block_sums;    // [n_scan_blocks]
-    size_t bytes;
+    size_t zero_bytes, bytes;
 };
 static CountWs count_ws_layout(void *base, int32_t C, int64_t N, int32_t n_tiles) {
     CountWs w{};
@@ -63,11 +63,12 @@ static CountWs count_ws_layout(void *base, int32_t C, int64_t N, int32_t n_tiles
     const int64_t nb = (int64_t)C * n_tiles;
     const int64_t nblocks = (std::max<int64_t>(nb, (int64_t)C * N) + SCAN_TILE - 1) / SCAN_TILE;
     size_t off = 256;
-    w.hdr = reinterpret_cast<IsectHeader *>(p);
+    w.hdr = reinterpret_cast<IsectHeader *>(p); // zeroed together with the replicas
+    w.replicas = reinterpret_cast<int32_t *>(p + off);
+    w.zero_bytes = off + nb * kCountReplicas * 4;
+    off = align256(w.zero_bytes);
     w.bucket_counts = reinterpret_cast<int32_t *>(p + off);
     off = align256(off + nb * 4);
-    w.replicas = reinterpret_cast<int32_t *>(p + off);
-    off = align256(off + nb * kCountReplicas * 4);
     w.block_sums = reinterpret_cast<int64_t *>(p + off);
     off = align256(off + (nblocks + 1) * 8);
     w.bytes = off;
@@ -245,6 +246,35 @@ __global__ void offset_encode_kernel(int64_t T, const int64_t *__restrict__ ids,
     offsets[b] = (int32_t)lo;
 }
 
+// The emit's cursors start at the bucket offsets, the sort's two list counters
+// at zero: one launch instead of a copy and a memset.
+__global__ void init_cursor_kernel(const int32_t *__restrict__ offsets, int64_t nb,
+                                   int32_t *__restrict__ cursor, int32_t *__restrict__ counters) {
+    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < 2) counters[b] = 0;
+    if (b < nb) cursor[b] = offsets[b];
+}
+
+// Two words of host memory that this thread's calls have the device write their
+// counts to (a copy to pageable memory goes through the driver's staging and a
+// second wait); null if there is none to be had.
+struct HostCounts {
+    int64_t *p = nullptr;
+    HostCounts() {
+        if (cudaHostAlloc(&p, 16, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+    }
+    ~HostCounts() {
+        if (p) cudaFreeHost(p);
+    }
+};
+static int64_t *host_counts() {
+    static thread_local HostCounts h;
+    return h.p;
+}
+
 } // namespace ubs
 
 using namespace ubs;
@@ -279,8 +309,7 @@ int ubs_isect_count(int32_t C, int64_t N, const float *means2d, const int32_t *r
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t CN = (int64_t)C * N;
     const int64_t nb = (int64_t)C * n_tiles;
-    if (cudaMemsetAsync(w.hdr, 0, sizeof(IsectHeader), st) != cudaSuccess ||
-        cudaMemsetAsync(w.replicas, 0, nb * kCountReplicas * 4, st) != cudaSuccess)
+    if (cudaMemsetAsync(w.hdr, 0, w.zero_bytes, st) != cudaSuccess)
         return check_launch("isect_count memset");
     if (CN > 0)
         UBS_TIMED("isect_count", st,
@@ -290,18 +319,33 @@ int ubs_isect_count(int32_t C, int64_t N, const float *means2d, const int32_t *r
                       tiles_per_gauss, w.replicas, &w.hdr->status));
     ::ubs::note_launch();
     if (int e = check_launch("isect_count")) return e;
-    UBS_TIMED("isect_count_fold", st,
-              fold_count_replicas_kernel<<<grid_for(nb, 256), 256, 0, st>>>(w.replicas, nb,
-                                                                           w.bucket_counts));
-    ::ubs::note_launch();
-    if (int e = check_launch("isect_count fold")) return e;
-    if (int e = device_exclusive_scan<int32_t>(w.bucket_counts, isect_offsets, nb, w.block_sums,
-                                               &w.hdr->total, st))
-        return e;
-    IsectHeader h;
-    if (cudaMemcpyAsync(&h, w.hdr, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+    // up to SCAN_ORDER_MAX buckets (65,536: 16.8M pixels of 16x16 tiles, 4.2M of 8x8)
+    // one launch folds, scans and reports; more take a fold, three scan launches
+    // and a copy
+    int64_t *host = nb <= SCAN_ORDER_MAX ? host_counts() : nullptr;
+    if (nb <= SCAN_ORDER_MAX) {
+        if (int e = launch_bucket_scan_order<kCountReplicas>(w.replicas, (int32_t)nb, isect_offsets,
+                                                             &w.hdr->total, nullptr, nullptr,
+                                                             &w.hdr->status, host, st))
+            return e;
+    } else {
+        UBS_TIMED("isect_count_fold", st,
+                  fold_count_replicas_kernel<<<grid_for(nb, 256), 256, 0, st>>>(
+                      w.replicas, nb, w.bucket_counts));
+        ::ubs::note_launch();
+        if (int e = check_launch("isect_count fold")) return e;
+        if (int e = device_exclusive_scan<int32_t>(w.bucket_counts, isect_offsets, nb, w.block_sums,
+                                                   &w.hdr->total, st))
+            return e;
+    }
+    IsectHeader h{};
+    if (!host && cudaMemcpyAsync(&h, w.hdr, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return check_launch("isect_count readback");
+    if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch("isect_count readback");
+    if (host) {
+        h.total = host[0];
+        h.status = (uint32_t)host[1];
+    }
     if (h.status & DEV_ERR_NEG_DEPTH)
         return set_error(UBS_ERR_DEVICE, "isect_count: a visible primitive has a negative depth");
     if (h.total >= (1ll << 31))
@@ -347,9 +391,11 @@ int ubs_isect_emit(int32_t C, int64_t N, const float *means2d, const int32_t *ra
     ::ubs::note_launch();
         return check_launch("isect_emit_ordered");
     }
-    if (cudaMemcpyAsync(w.cursor, isect_offsets, nb * 4, cudaMemcpyDeviceToDevice, st) !=
-        cudaSuccess)
-        return check_launch("isect_emit init");
+    UBS_TIMED("isect_emit_init", st,
+              init_cursor_kernel<<<grid_for(std::max<int64_t>(nb, 2), 256), 256, 0, st>>>(
+                  isect_offsets, nb, w.cursor, &w.cw.hdr->n_big));
+    ::ubs::note_launch();
+    if (int e = check_launch("isect_emit init")) return e;
     UBS_TIMED("isect_emit", st,
               isect_emit_bucket_kernel<<<grid_for(CN, 256), 256, 0, st>>>(
                   CN, N, m2, radii, depths, ts, (uint32_t)tile_width, (uint32_t)tile_height,
@@ -358,7 +404,7 @@ int ubs_isect_emit(int32_t C, int64_t N, const float *means2d, const int32_t *ra
     if (int e = check_launch("isect emit")) return e;
     const IdsWriter wr{isect_ids, flatten_ids, (int32_t)n_tiles, tile_bits};
     return launch_bucket_sort(nb, isect_offsets, nullptr, n_isects, w.keys, w.scratch, w.big_list,
-                              &w.cw.hdr->n_big, wr, st);
+                              &w.cw.hdr->n_big, wr, st, true);
 }
 
 int ubs_isect_offset_encode(int64_t n_isects, const int64_t *isect_ids, int32_t C,

@@ -266,6 +266,7 @@ static __global__ void __launch_bounds__(1024) bucket_order_kernel(const int32_t
 // 0 .. r - 1).  One CTA took 24 us for the 8,160 buckets of a 1080p frame and
 // 111 us for 30,000.
 // host (optional, memory the host reads): the total and the status word.
+// order and cursor are optional too: without them this is the scan alone.
 constexpr int SCAN_CTAS = 8;                    // cluster size above SCAN_SMALL buckets
 constexpr int SCAN_SMALL = 1024;                // up to here one CTA
 constexpr int SCAN_PER = 8;                     // buckets per thread at most
@@ -375,12 +376,15 @@ __global__ void __launch_bounds__(1024) bucket_scan_order_kernel(
     __syncthreads();
     pos[tid] = x - in_bin + (wid ? btot[wid - 1] : 0) + before;
     __syncthreads();
+    if (order) {
 #pragma unroll
-    for (int k = 0; k < SCAN_PER; ++k)
-        if (c[k] >= 0) order[atomicAdd(&pos[bin_of(c[k])], 1)] = c0 + tid * per + k;
+        for (int k = 0; k < SCAN_PER; ++k)
+            if (c[k] >= 0) order[atomicAdd(&pos[bin_of(c[k])], 1)] = c0 + tid * per + k;
+    }
     for (int i = tid; i < m; i += 1024) {
         int32_t o = cnt[i];
         offsets[c0 + i] = o;
+        if (!cursor) continue;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             cursor[(int64_t)r * n + c0 + i] = o;
