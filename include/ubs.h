@@ -528,9 +528,13 @@ int ubs_scene_forward_masked(int32_t dim, int64_t N, const float *xyz, const flo
  * everything up to it and, when host_counts is not NULL, writes
  * ubs_scene_stats' two values there (pinned host memory the device can write);
  * UBS_SCENE_PART_BLEND runs the rest, both the whole frame.  The two parts of a
- * frame take the same arguments, in this order, on one stream. */
+ * frame take the same arguments, in this order, on one stream.
+ * UBS_SCENE_HOST_IMAGE, added to the part that blends: render_colors is pinned
+ * host memory, which the blend then stores to in whole rows of a tile, so that
+ * the image arrives while the frame is computed. */
 #define UBS_SCENE_PART_COUNT 1
 #define UBS_SCENE_PART_BLEND 2
+#define UBS_SCENE_HOST_IMAGE 4
 int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const float *mean,
                             const float *scale, const float *l_triangle, const float *opacity,
                             const float *beta, const float *rgb, int32_t C,

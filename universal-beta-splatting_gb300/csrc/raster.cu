@@ -56,6 +56,7 @@ struct RasterArgs {
     const uint8_t *masks;
     // forward outputs
     float *out_c;
+    bool rows_out; // out_c is host memory (three packed colours)
     float *out_a;
     int32_t *last_ids;
     // backward inputs / outputs
@@ -459,7 +460,14 @@ __device__ __forceinline__ void blend_pair(const GeoRec &q, const float (&col)[C
 // --------------------------------------------------------------- forward
 // TSZ: edge of a CTA's pixels, 8 or 16, or 0 for a whole tile of a.TS; MINB
 // CTAs per SM.
-template <int CD, bool PACK, bool COUNT, int TSZ, int RB, int MINB>
+// ROWS: out_c is host memory.  A CTA's pixels go through shared memory, so that
+// consecutive threads store consecutive floats of an image row: the link takes
+// whole sectors at the rate of a copy while the other CTAs compute.  1M primitives
+// at 1080p, to pinned memory: 446 us + 132 for the copy; storing each pixel from
+// its thread 492 us, and 515 for a nearly empty frame; so 446, and 155 against 189
+// for the nearly empty frame.  An instance of its own: as a run-time branch it
+// cost the device path 4%.
+template <int CD, bool PACK, bool COUNT, int TSZ, int RB, int MINB, bool ROWS = false>
 __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_fwd_kernel(RasterArgs a) {
     extern __shared__ __align__(128) unsigned char sm[];
     const int TS = TSZ ? TSZ : a.TS;
@@ -623,6 +631,32 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_fwd_ke
         if (lane == 0 && wb) atomicAdd(a.pair_count + 2, (unsigned long long)wb);
     }
     T = make_float2(fabsf(T.x), fabsf(T.y));
+    if constexpr (ROWS) {
+        if (in0) {
+            a.out_a[pix0] = 1.0f - T.x;
+            a.last_ids[pix0] = cur0;
+        }
+        if (in1) {
+            a.out_a[pix1] = 1.0f - T.y;
+            a.last_ids[pix1] = cur1;
+        }
+        float *stage = reinterpret_cast<float *>(srec); // no copy is under way
+        const int at = ((i0 - tile_y0) * TS + j - tile_x0) * CD;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < CD; ++k) {
+            stage[at + k] = bg ? acc[k].x + T.x * bg[k] : acc[k].x;
+            stage[at + TS * CD + k] = bg ? acc[k].y + T.y * bg[k] : acc[k].y;
+        }
+        __syncthreads();
+        const int cols = min(TS, loc.W - tile_x0) * CD, rows = min(TS, loc.H - tile_y0);
+        float *out = a.out_c + (loc.pix_base + (int64_t)tile_y0 * loc.W + tile_x0) * CD;
+        for (int e = tid; e < TS * TS * CD; e += NT) {
+            const int r = e / (TS * CD), c = e - r * (TS * CD);
+            if (r < rows && c < cols) out[(int64_t)r * loc.W * CD + c] = stage[e];
+        }
+        return;
+    }
     if (in0) {
         a.out_a[pix0] = 1.0f - T.x;
 #pragma unroll
@@ -1332,7 +1366,7 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     a.sub = a.TS / edge;
     const int NT = edge * edge / 2;
     const bool small = NT <= 128;
-    const int variant = (small && CD == 3 && !a.pair_count)
+    const int variant = (small && CD == 3 && !a.pair_count && !a.rows_out)
                             ? (BWD ? g_blend_bwd_variant.load() : g_blend_fwd_variant.load())
                             : 0;
     // wide colour rows: one batch slot per thread (forward, 32 channels: 209 ->
@@ -1372,7 +1406,10 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     } else {
         if constexpr (PACK) {
             const bool e8 = edge == 8;
-            if (variant == 1)
+            if (CD == 3 && a.rows_out)
+                k = e8 ? raster_fwd_kernel<3, true, false, 8, 2, 32, true>
+                       : raster_fwd_kernel<3, true, false, 16, 2, 8, true>;
+            else if (variant == 1)
                 k = e8 ? raster_fwd_kernel<CD, true, false, 8, 1, 32>
                        : raster_fwd_kernel<CD, true, false, 16, 1, 10>;
             else if (variant == 2)
@@ -1486,7 +1523,7 @@ int scene_blend(int fwd, int32_t C, int64_t CN, int32_t n_buckets, int32_t tile_
                 const int32_t *dims, const int64_t *pix_base, float *out_c, float *out_a,
                 int32_t *last_ids, const float *render_alphas, const int32_t *last_in,
                 const float *v_out_c, const float *v_out_a, float *v_rows, uint32_t *status,
-                cudaStream_t st) {
+                cudaStream_t st, bool rows_out) {
     RasterArgs a{};
     a.C = C;
     a.TS = tile_size;
@@ -1507,6 +1544,7 @@ int scene_blend(int fwd, int32_t C, int64_t CN, int32_t n_buckets, int32_t tile_
     a.order = order;
     if (fwd) {
         a.out_c = out_c;
+        a.rows_out = rows_out;
         a.out_a = out_a;
         a.last_ids = last_ids;
         return launch_blend<3, false>(a, st);

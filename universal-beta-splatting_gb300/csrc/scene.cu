@@ -39,7 +39,7 @@ int scene_blend(int fwd, int32_t C, int64_t CN, int32_t n_buckets, int32_t tile_
                 const int32_t *dims, const int64_t *pix_base, float *out_c, float *out_a,
                 int32_t *last_ids, const float *render_alphas, const int32_t *last_in,
                 const float *v_out_c, const float *v_out_a, float *v_rows, uint32_t *status,
-                cudaStream_t st);
+                cudaStream_t st, bool rows_out);
 
 // scene_act.cu (compiled with IEEE math): activated scales, betas and
 // opacities, act = [N, D] | [N, D - 2] | [N] at the 16-byte aligned section
@@ -803,7 +803,8 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
                          w.bytes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t CN = (int64_t)C * N;
-    UBS_REQUIRE(parts >= 1 && parts <= 3, "scene_forward: parts %d", parts);
+    const bool host_image = parts & UBS_SCENE_HOST_IMAGE;
+    UBS_REQUIRE(parts >= 1 && parts <= 7 && (parts & 3), "scene_forward: parts %d", parts);
     const bool one_scan = n_buckets <= SCAN_ORDER_MAX;
     if (parts & UBS_SCENE_PART_COUNT) {
         if (cudaMemsetAsync(w.hdr, 0, w.zero_bytes, st) != cudaSuccess)
@@ -877,7 +878,7 @@ int ubs_scene_forward_parts(int32_t dim, int64_t N, const float *xyz, const floa
     return scene_blend(1, C, CN, n_buckets, tile_size, w.offsets, w.order, &w.hdr->total, capacity,
                        w.keys, w.recs, w.cols_n, backgrounds, tile_base, view_dims, pix_base,
                        render_colors, render_alphas, last_ids, nullptr, nullptr, nullptr, nullptr,
-                       nullptr, &w.hdr->status, st);
+                       nullptr, &w.hdr->status, st, host_image);
 }
 
 int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *mean,
@@ -919,7 +920,7 @@ int ubs_scene_backward(int32_t dim, int64_t N, const float *xyz, const float *me
                             capacity, w.keys, w.recs, w.cols_n, backgrounds, tile_base,
                             view_dims, pix_base,
                             nullptr, nullptr, nullptr, render_alphas, last_ids, v_render_colors,
-                            v_render_alphas, w.grads, &w.hdr->status, st))
+                            v_render_alphas, w.grads, &w.hdr->status, st, false))
         return e;
     if (CN == 0) return UBS_OK;
     const unsigned groups = view_groups(N, C, 3);

@@ -207,7 +207,7 @@ class Renderer:
             float(self.radius_clip), L.ptr(bg)]
 
     def forward_raw(self, p: Dict[str, torch.Tensor], views: Views, bg, check=True,
-                    prim_mask=None, color_mode=0):
+                    prim_mask=None, color_mode=0, image=None):
         """Run the forward kernels; returns (colors, alphas, last_ids, workspace, capacity).
 
         check=True reads the intersection count back (synchronising) and
@@ -216,11 +216,14 @@ class Renderer:
         issues nothing but the kernels (safe inside CUDA graph capture) and
         leaves the verification to `stats()` after the frame(s).
         prim_mask (uint8 [N]) leaves out primitives whose entry is 0;
-        color_mode=1 renders depth into channel 0 (one view, no backward)."""
+        color_mode=1 renders depth into channel 0 (one view, no backward).
+        image (pinned float32 host tensor of 3 * n_pixels values) takes the
+        colours and is returned as such; it is complete once the current stream
+        has been waited for."""
         return self._forward([p[k] for k in PARAM_ORDER], views, bg, check, prim_mask, color_mode,
-                             False)
+                             False, image)
 
-    def _forward(self, tensors, views, bg, check, prim_mask, color_mode, grad):
+    def _forward(self, tensors, views, bg, check, prim_mask, color_mode, grad, image=None):
         if check == "none":
             if self.capacity is None:
                 raise RuntimeError("check='none' needs a capacity (render once with check=True)")
@@ -235,7 +238,7 @@ class Renderer:
                                     self.tile_size, self.eps2d, self.near, self.far,
                                     self.radius_clip, bool(self.exact_cond_grad), cap)
             colors, alphas, last, ws, stats = native.scene_forward(
-                call, tensors, bg, prim_mask, color_mode, check != "none", grad)
+                call, tensors, bg, prim_mask, color_mode, check != "none", grad, image)
             self.last_ws, self.last_cap = ws, cap
             if check == "none":
                 return colors, alphas, last, ws, cap

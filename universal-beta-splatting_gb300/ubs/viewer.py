@@ -123,6 +123,11 @@ class FrameRenderer:
         """One frame on the device: (image [H, W, 3], raw, visible) where raw
         is what the image was made from (RGB [H, W, 3], alpha or depth
         [H, W, 1]) and visible the count of rendered primitives (device)."""
+        return self._frame(params, c2w, K, width, height, state)
+
+    def _frame(self, params, c2w, K, width, height, state, image=None):
+        """frame(), with the image of mode "RGB" written to pinned host memory
+        when image is given."""
         dev = self.device
         c2w = torch.as_tensor(np.asarray(c2w), dtype=torch.float32)
         K = torch.as_tensor(np.asarray(K), dtype=torch.float32)
@@ -144,7 +149,8 @@ class FrameRenderer:
             color_mode = 0
         p = {k: params[k].detach() for k in PARAM_NAMES}
         colors, alphas, _, _, _ = r.forward_raw(p, views, bg, check=True, prim_mask=mask,
-                                                color_mode=color_mode)
+                                                color_mode=color_mode,
+                                                image=image if mode == "RGB" else None)
         H, W = int(height), int(width)
         if mode == "RGB":
             raw = colors.view(H, W, 3)
@@ -172,19 +178,21 @@ class FrameRenderer:
         """One frame as a float32 [H, W, 3] host array: params are the raw
         scene tensors (xyz, mean, scale, l_triangle, opacity, beta, rgb), c2w
         the camera-to-world matrix and K the intrinsics of the viewer camera."""
-        img, _, visible = self.frame(params, c2w, K, width, height, state)
         H, W = int(height), int(width)
         # the frame and the visible count to pinned host memory, one wait
         slot = self._ring
-        self._ring ^= 1
         need = H * W * 3 + 1
         buf = self._host[slot]
         if buf is None or buf.numel() < need:
             buf = torch.empty(need, dtype=torch.float32, pin_memory=True)
             self._host[slot] = buf
-        buf[:H * W * 3].view(H, W, 3).copy_(img, non_blocking=True)
+        host = buf[:H * W * 3]
+        img, _, visible = self._frame(params, c2w, K, width, height, state, image=host)
+        if img.data_ptr() != host.data_ptr():
+            host.view(H, W, 3).copy_(img, non_blocking=True)
         buf[H * W * 3:].copy_(visible.float().view(1), non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
+        self._ring ^= 1
         self.rendered_count = int(buf[H * W * 3].item())
         out = buf[:H * W * 3].view(H, W, 3).numpy()
         return out.copy() if copy else out
