@@ -54,14 +54,14 @@ def cond_mean_convariance_opacity(
     assert covars.shape == (N, D, D), covars.shape
     assert opacities.numel() == N and betas.shape == (N, D - 3) and query.shape == (N, D - 3)
     # the mode at forward time applies
-    return L.native().cond(means, covars, opacities, betas, query, _COND_GRAD_MODE == "exact")
+    return L.op("cond", means, covars, opacities, betas, query, _COND_GRAD_MODE == "exact")
 
 
 # --------------------------------------------------------------------- a2
 def l_triangle_to_rotmat(l_triangle: Tensor) -> Tensor:
     """R = I + A from the 3 skew entries (_wrapper.py:34-36)."""
     assert l_triangle.shape[1] == 3, l_triangle.shape
-    return L.native().rotmat(l_triangle)
+    return L.op("rotmat", l_triangle)
 
 
 # --------------------------------------------------------------------- a3
@@ -74,7 +74,7 @@ def rot_scale_l_triangle_to_covar(
     spatial_block: bool = False,
 ) -> Tensor:
     """Sigma = L L^T (_wrapper.py:39-55)."""
-    return L.native().covar(rot, scale, l_triangle, rest_i, rest_j, bool(spatial_block))
+    return L.op("covar", rot, scale, l_triangle, rest_i, rest_j, bool(spatial_block))
 
 
 # --------------------------------------------------------------------- a6
@@ -112,16 +112,16 @@ def fully_fused_projection(
     else:
         assert quats is not None and scales is not None, "covars or quats+scales is required"
         assert quats.size() == (N, 4) and scales.size() == (N, 3)
-    return L.native().projection(
-        means, covars, quats, scales, viewmats, Ks, int(width), int(height), float(eps2d),
-        float(near_plane), float(far_plane), float(radius_clip), bool(calc_compensations))
+    return L.op("projection", means, covars, quats, scales, viewmats, Ks, int(width), int(height),
+                float(eps2d), float(near_plane), float(far_plane), float(radius_clip),
+                bool(calc_compensations))
 
 
 # --------------------------------------------------------------- a7 / a8
 def _isect(means2d, radii, depths, tile_size, tile_width, tile_height, sort=True):
     """Intersections plus the (camera, tile) offsets the count step yields."""
-    return L.native().isect(means2d, radii, depths, int(tile_size), int(tile_width),
-                            int(tile_height), bool(sort))
+    return L.op("isect", means2d, radii, depths, int(tile_size), int(tile_width), int(tile_height),
+                bool(sort))
 
 
 @torch.no_grad()
@@ -156,7 +156,7 @@ def isect_tiles(
 def isect_offset_encode(isect_ids: Tensor, n_cameras: int, tile_width: int,
                         tile_height: int) -> Tensor:
     """First sorted intersection of every (camera, tile) (_wrapper.py:347-363)."""
-    return L.native().offset_encode(isect_ids, int(n_cameras), int(tile_width), int(tile_height))
+    return L.op("offset_encode", isect_ids, int(n_cameras), int(tile_width), int(tile_height))
 
 
 # ------------------------------------------------------------ a9 / a10
@@ -220,8 +220,8 @@ def rasterize_to_pixels(
         if backgrounds is not None:
             backgrounds = torch.cat(
                 [backgrounds, torch.zeros(*backgrounds.shape[:-1], padded, device=device)], -1)
-    render_colors, render_alphas = L.native().raster(
-        means2d, conics, colors, opacities, betas, backgrounds, masks, int(image_width),
+    render_colors, render_alphas = L.op(
+        "raster", means2d, conics, colors, opacities, betas, backgrounds, masks, int(image_width),
         int(image_height), int(tile_size), isect_offsets, flatten_ids)
     if padded > 0:
         render_colors = render_colors[..., :-padded]

@@ -4,6 +4,7 @@ the host path built on it (csrc/host/native.cpp, the ubs_native module).
 The library is the only compute path: there is no CPU or PyTorch fallback.
 If it cannot be built or loaded, or a CUDA device is missing, calls raise.
 """
+import contextlib
 import ctypes
 import importlib.util
 import threading
@@ -143,6 +144,92 @@ def native():
                 spec.loader.exec_module(mod)
                 _native = mod
     return _native
+
+
+# torch.jit.trace records the tensor operations that a call dispatches.  Of an
+# operator here those are its allocations: the kernels are launched beside the
+# dispatcher.  So an operator is recorded as one node that makes the call again.
+def tracing():
+    """Whether torch.jit.trace is recording on this thread."""
+    return torch._C._get_tracing_state() is not None
+
+
+@contextlib.contextmanager
+def untraced():
+    """Nothing done inside is recorded."""
+    state = torch._C._get_tracing_state()
+    torch._C._set_tracing_state(None)
+    try:
+        yield
+    finally:
+        torch._C._set_tracing_state(state)
+
+
+class _Recorded(torch.autograd.Function):
+    """fn(*tensors) -> tuple of tensors, as one node of a traced program (the
+    allocations recorded on the way are dead code)."""
+
+    @staticmethod
+    def forward(ctx, fn, *tensors):
+        with torch.enable_grad():
+            ins = [t.detach().requires_grad_(need)
+                   for t, need in zip(tensors, ctx.needs_input_grad[1:])]
+            outs = fn(*ins)
+            res = tuple(o.detach() for o in outs)
+        ctx.ins, ctx.outs = ins, outs
+        ctx.mark_non_differentiable(*[r for o, r in zip(outs, res) if not o.requires_grad])
+        ctx.save_for_backward(*res)  # released with the graph, like an operator's own
+        return res
+
+    @staticmethod
+    def backward(ctx, *grads):
+        ctx.saved_tensors  # raises once the graph has been released
+        outs = [(o, g) for o, g in zip(ctx.outs, grads) if o.requires_grad]
+        ins = [t for t in ctx.ins if t.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in outs], ins, [g for _, g in outs],
+                                       retain_graph=True, allow_unused=True))
+        return (None,) + tuple(next(got) if t.requires_grad else None for t in ctx.ins)
+
+
+class _Call:
+    """A call with a name: torch.jit.trace compares two recordings by text."""
+
+    def __init__(self, name, fn):
+        self.name, self.fn = name, fn
+
+    def __call__(self, *tensors):
+        return self.fn(*tensors)
+
+    def __repr__(self):
+        return "ubs::" + self.name
+
+
+def recorded(name, fn, *tensors):
+    """fn(*tensors), a tuple of tensors; under torch.jit.trace one node."""
+    return _Recorded.apply(_Call(name, fn), *tensors) if tracing() else fn(*tensors)
+
+
+def op(name, *args):
+    """Operator `name` of the ubs_native module."""
+    f = getattr(native(), name)
+    if not tracing():
+        return f(*args)
+    at = [i for i, a in enumerate(args) if isinstance(a, torch.Tensor)]
+    rest = [None if isinstance(a, torch.Tensor) else a for a in args]
+    given = []  # per result of the call: is it a tensor (else None)?
+
+    def fn(*tensors):
+        full = list(rest)
+        for i, t in zip(at, tensors):
+            full[i] = t
+        r = f(*full)
+        r = (r,) if isinstance(r, torch.Tensor) else r
+        given[:] = [t is not None for t in r]
+        return tuple(t for t in r if t is not None)
+
+    outs = iter(recorded(name, fn, *[args[i] for i in at]))
+    res = tuple(next(outs) if g else None for g in given)
+    return res if len(res) > 1 else res[0]
 
 
 def library_path():

@@ -33,7 +33,7 @@ def _check(img, gt, channels_last):
 
 def _apply(img, gt, channels_last, valid, weights, index):
     _check(img, gt, channels_last)
-    return L.native().ssim_loss(img, gt.detach(), channels_last, valid, *weights, index)
+    return L.op("ssim_loss", img, gt.detach(), channels_last, valid, *weights, index)
 
 
 def l1_ssim_loss(img, gt, lambda_dssim=0.2, channels_last=False, padding="same"):
@@ -64,4 +64,4 @@ def l1_loss(img, gt):
         raise ValueError("shapes differ: %s vs %s" % (tuple(img.shape), tuple(gt.shape)))
     if not (img.is_contiguous() and gt.is_contiguous()):
         raise ValueError("l1_loss needs contiguous tensors")
-    return L.native().l1_loss(img, gt.detach())
+    return L.op("l1_loss", img, gt.detach())

@@ -48,7 +48,7 @@ class Views:
             center = getattr(c, "position", None)
             centers.append(getattr(c, "center", None) if center is None else center)
         on = contextlib.nullcontext() if stream is None else torch.cuda.stream(stream)
-        with on:
+        with on, L.untraced():  # the tables are constants of a traced program
             (staging, self.viewmats, self.intr, self.centers, self.times, self.dims,
              self.tile_base, self.pix_base, tile_base, pix_base) = L.native().pack_views(
                  [c.viewmat for c in cameras], [c.K for c in cameras], centers,
@@ -264,9 +264,9 @@ class Renderer:
             bg = torch.zeros(views.C, 3, device=params["xyz"].device)
         else:
             bg = backgrounds.reshape(-1, 3).expand(views.C, 3).contiguous().float()
-        colors, alphas, _, _, _ = self._forward([params[k] for k in PARAM_ORDER], views, bg, check,
-                                                None, 0, True)
-        return colors, alphas
+        return L.recorded("scene_render",
+                          lambda bg, *p: self._forward(p, views, bg, check, None, 0, True)[:2], bg,
+                          *[params[k] for k in PARAM_ORDER])
 
 
 class GraphedStep:
