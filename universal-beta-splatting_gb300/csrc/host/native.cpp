@@ -109,9 +109,41 @@ Tensor grad_or_zeros(const Tensor &g, at::IntArrayRef s, const Tensor &like) {
 // its outputs (undefined where none arrived).
 struct OpNode : public torch::autograd::Node {
     using Backward = std::function<variable_list(OpNode &, const variable_list &, variable_list &)>;
+    // what a kernel that reads a saved tensor relies on
+    struct Kind {
+        c10::SmallVector<int64_t, 4> sizes;
+        at::ScalarType type;
+        at::Device device;
+    };
     std::string op;
     std::vector<SavedVariable> saved;
+    std::vector<std::optional<Kind>> kinds;
     Backward bwd;
+
+    // The saved tensors for a kernel.  Saved-tensor hooks may return anything:
+    // other strides are copied to C order, another size, type or device raises.
+    variable_list for_kernel(const variable_list &s) const {
+        variable_list o;
+        o.reserve(s.size());
+        for (size_t i = 0; i < s.size(); ++i) {
+            TORCH_CHECK_VALUE(s[i].defined() == kinds[i].has_value(), op, ": saved tensor ", i,
+                              " is missing");
+            if (s[i].defined()) {
+                const Kind &k = *kinds[i];
+                TORCH_CHECK_VALUE(s[i].device() == k.device, op, ": expected a saved tensor on ",
+                                  k.device, ", got device ", s[i].device());
+                TORCH_CHECK_TYPE(s[i].scalar_type() == k.type, op, ": expected a saved tensor of ",
+                                 k.type, ", got ", s[i].scalar_type());
+                TORCH_CHECK_VALUE(s[i].sizes() == at::IntArrayRef(k.sizes), op,
+                                  ": expected a saved tensor of size ", at::IntArrayRef(k.sizes),
+                                  ", got ", s[i].sizes());
+                o.push_back(s[i].contiguous());
+            } else {
+                o.emplace_back();
+            }
+        }
+        return o;
+    }
 
     variable_list apply(variable_list &&grads) override {
         std::lock_guard<std::mutex> lk(mutex_);
@@ -159,8 +191,16 @@ void attach(const char *op, at::ArrayRef<Tensor> inputs, at::ArrayRef<Tensor> ou
     node->set_next_edges(std::move(edges));
     for (const Tensor &t : outputs) torch::autograd::create_gradient_edge(const_cast<Tensor &>(t), node);
     node->saved.reserve(saved.size() + saved_outputs.size());
-    for (const Tensor &t : saved) node->saved.emplace_back(t, /*is_output=*/false);
-    for (const Tensor &t : saved_outputs) node->saved.emplace_back(t, /*is_output=*/true);
+    node->kinds.reserve(saved.size() + saved_outputs.size());
+    auto save = [&](const Tensor &t, bool is_output) {
+        node->saved.emplace_back(t, is_output);
+        node->kinds.emplace_back();
+        if (t.defined())
+            node->kinds.back() = OpNode::Kind{{t.sizes().begin(), t.sizes().end()},
+                                              t.scalar_type(), t.device()};
+    };
+    for (const Tensor &t : saved) save(t, false);
+    for (const Tensor &t : saved_outputs) save(t, true);
     node->bwd = std::move(bwd);
 }
 
@@ -314,8 +354,9 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
         p.push_back(b);
         p.push_back(last);
         attach("SceneRenderBackward", params, {colors, alphas}, p, {alphas},
-               [c, opacity_shape](OpNode &, const variable_list &s, variable_list &g) {
+               [c, opacity_shape](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
+                   const variable_list s = node.for_kernel(saved);
                    TORCH_CHECK(c->ws.defined(), "scene_backward: the frame's workspace was "
                                                 "released by an earlier backward");
                    const c10::cuda::CUDAGuard guard(s[0].device());
@@ -534,8 +575,9 @@ std::tuple<Tensor, Tensor, Tensor> cond(const Tensor &means_, const Tensor &cova
     const std::vector<Tensor> diff{means_, covars_, opac_, betas_};
     if (wants_grad(diff))
         attach("CondMeanConvarianceOpacityBackward", diff, {om, oV, oo}, s, {},
-               [exact](OpNode &, const variable_list &s, variable_list &g) {
+               [exact](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
+                   const variable_list s = node.for_kernel(saved);
                    const c10::cuda::CUDAGuard guard(s[0].device());
                    const int64_t N = s[0].size(0), D = s[0].size(1);
                    const Tensor vm = grad_or_zeros(g[0], {N, 3}, s[0]);
@@ -594,9 +636,10 @@ Tensor covar(const Tensor &rot_, const Tensor &scale_, const Tensor &lt_, const 
     }
     if (wants_grad({rot_, scale_, lt_}))
         attach("RotScaleLTriangleToCovarBackward", {rot_, scale_, lt_}, {out}, s, {},
-               [spatial_block](OpNode &, const variable_list &s, variable_list &g) {
+               [spatial_block](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
                    if (!g[0].defined()) return variable_list(3);
+                   const variable_list s = node.for_kernel(saved);
                    const c10::cuda::CUDAGuard guard(s[0].device());
                    const int64_t N = s[1].size(0), D = s[1].size(1);
                    const Tensor v = f32(g[0]);
@@ -648,8 +691,9 @@ py::tuple projection(const Tensor &means_, const OptTensor &covars_, const OptTe
         }
         s.push_back(radii);
         attach("FullyFusedProjectionBackward", diff, outs, s, so,
-               [=](OpNode &node, const variable_list &s, variable_list &g) {
+               [=](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
+                   const variable_list s = node.for_kernel(saved);
                    const c10::cuda::CUDAGuard guard(s[0].device());
                    const int64_t C = s[4].size(0), N = s[0].size(0);
                    const Tensor vm = grad_or_zeros(g[0], {C, N, 2}, s[0]);
@@ -768,8 +812,9 @@ std::tuple<Tensor, Tensor> raster(const Tensor &means2d_, const Tensor &conics_,
         s.push_back(last);
         auto held = std::make_shared<Tensor>(ws); // released by the backward
         attach("RasterizeToPixelsBackward", in, {rc, ra}, s, {ra},
-               [=](OpNode &node, const variable_list &s, variable_list &g) {
+               [=](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
+                   const variable_list s = node.for_kernel(saved);
                    TORCH_CHECK(held->defined(), "rasterize_to_pixels: the records were released "
                                                 "by an earlier backward");
                    const c10::cuda::CUDAGuard guard(s[0].device());
