@@ -572,8 +572,8 @@ int ubs_scene_stats(const void *workspace, int64_t *n_isects, uint32_t *status, 
  * register bound --
  *   forward:  0 (default): 256-record batches, 8 CTAs per SM;
  *             1: 128-record batches, 10 CTAs per SM; 2: 256-record, 6 CTAs per SM
- *   backward: 0 (default): 128-record batches, 8 CTAs per SM (6 in small
- *             grids); 1: 7 CTAs per SM; 2: 6 CTAs per SM
+ *   backward: 0 (default): 128-record batches, 8 CTAs per SM; 1: 7 CTAs per
+ *             SM; 2: 6 CTAs per SM
  * (for 16 x 16 tiles; an 8 x 8 tile's batches are a quarter of that).
  * Process-wide: it applies to every later launch from any thread (an
  * autotuner sets it between measured steps, outside stream capture).  Images

@@ -20,13 +20,11 @@
 //     8x8-pixel footprint of every warp and the results turned into per-warp
 //     bitmasks by ballot, so a warp only visits records that can touch its
 //     pixels;
-//   * the backward sums the 7 + channels gradients of a record over a warp on
-//     the tensor cores (moments of per-pixel values with constant weights, see
-//     moment_products) and a transpose reduction, each warp writes its totals
-//     into its own list of rows in shared memory with plain stores, and per
-//     batch the rows of a record are summed and added to its gradient row
-//     with three 16-byte vector atomics (fused path) or one scalar atomic per
-//     value (drop-in arrays).
+//   * the backward sums the 7 + channels gradients of a record over a warp with
+//     a transpose reduction, each warp writes its totals into its own list of
+//     rows in shared memory with plain stores, and per batch the rows of a
+//     record are summed and added to its gradient row with three 16-byte vector
+//     atomics (fused path) or one scalar atomic per value (drop-in arrays).
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -190,10 +188,10 @@ __global__ void pack_records_kernel(int64_t T, int64_t n_prims, const int32_t *_
 // streams its records in batches of RB*TS*TS/2, RB batch slots per thread in
 // the culling phase (RB = 1 in the backward and for colours of more than 4
 // channels, whose smaller shared footprint lets more CTAs share an SM; else 2).
-// In the backward every warp owns a list of KE entry rows (row_pitch floats
-// each, after a dump row) that it fills with plain stores, one row per record
-// it visits, last batch slot first: a slot's row is the number of set bits
-// after it in the warp's mask.  The flush sums the warps' rows of a slot.
+// In the backward every warp owns a list of KE entry rows (7 + CD gradient sums
+// each) that it fills with plain stores, one row per record it visits, last
+// batch slot first: a slot's row is the number of set bits after it in the
+// warp's mask.  The flush sums the warps' rows of a slot.
 // (Shared accumulators with float atomics cost about as much as the rest of a
 // visit's reduction: 32 channels 871 against 346 us, 16 channels 122 against
 // 69, 5 channels 124 against 95 together with the squares of launch_blend.)
@@ -201,33 +199,18 @@ struct SmemLayout {
     int mask_off, rec_off, col_off, rows_off, total;
 };
 
-// Whether the backward reduces a visit on the tensor cores (see
-// moment_products), and how many colour sums that takes along with the moments
-// of w and the sums of u and u log2(1 - s): three fit the accumulators.  A
-// fourth colour goes through lane exchanges (690k primitives with depth at
-// 720p: 528 -> 503 us).  Wider rows are mostly colours, whose exchanges
-// dominate either way, and stay on them (the others' sums on the tensor cores:
-// 16 channels 69 -> 68, 8 channels 92 -> 96, 32 channels 346 -> 352 us).
-template <int CD> __host__ __device__ constexpr bool moment_rows() { return CD <= 4; }
-template <int CD> __host__ __device__ constexpr int moment_colours() { return CD <= 3 ? CD : 3; }
-// Floats per entry row: the 6 moments of w, the sums of u and u log2(1 - s)
-// and CD colour sums, or the 7 + CD gradient sums.
-template <int CD> __host__ __device__ constexpr int row_pitch() {
-    return moment_rows<CD>() ? 8 + CD : 7 + CD;
-}
-
 template <int CD, bool PACK, bool BWD>
 __host__ __device__ inline SmemLayout smem_layout(int NT, int RB, int KE) {
     const int nw = NT / 32, BR = RB * NT;
     SmemLayout L;
-    L.mask_off = 32; // after two mbarriers and the cold flag of the backward
+    L.mask_off = 16; // after two mbarriers
     // per-target-warp masks (nw x RB nw words, two sets in the backward), then
     // one int per warp
     L.rec_off = (L.mask_off + (BWD ? 2 : 1) * nw * RB * nw * 4 + nw * 4 + 127) & ~127;
     const int colbytes = PACK ? 16 : CD * 4;
     L.col_off = L.rec_off + 2 * BR * (int)sizeof(GeoRec);
     L.rows_off = (L.col_off + 2 * BR * colbytes + 15) & ~15;
-    L.total = L.rows_off + (BWD ? nw * (KE + 1) * row_pitch<CD>() * 4 : 0);
+    L.total = L.rows_off + (BWD ? nw * KE * (7 + CD) * 4 : 0);
     return L;
 }
 
@@ -717,8 +700,7 @@ struct PairGeom {
     float dx;
     float2 dy;
 };
-// TAME: sigma is not NaN (see tame_record), so [0, 1) is one unsigned compare.
-template <int CD, bool TAME>
+template <int CD>
 __device__ __forceinline__ PairGeom grad_pair(const GeoRec &q, const float (&col)[CD], float px,
                                               float2 npy, int32_t idx, BwdPair<CD> &s, float2 &w,
                                               float2 &u, float2 &ul, float2 (&gc)[CD]) {
@@ -729,10 +711,8 @@ __device__ __forceinline__ PairGeom grad_pair(const GeoRec &q, const float (&col
     float2 sg;
     sg.x = fmaf(B, dy.x, fmaf(__fmul_rn(q.cyy, dy.x), dy.x, A));
     sg.y = fmaf(B, dy.y, fmaf(__fmul_rn(q.cyy, dy.y), dy.y, A));
-    const bool v0 = TAME ? ((idx <= s.bin0) & (__float_as_uint(sg.x) < 0x3f800000u))
-                         : (idx <= s.bin0 && !(sg.x < 0.f || sg.x >= 1.f));
-    const bool v1 = TAME ? ((idx <= s.bin1) & (__float_as_uint(sg.y) < 0x3f800000u))
-                         : (idx <= s.bin1 && !(sg.y < 0.f || sg.y >= 1.f));
+    const bool v0 = idx <= s.bin0 && !(sg.x < 0.f || sg.x >= 1.f);
+    const bool v1 = idx <= s.bin1 && !(sg.y < 0.f || sg.y >= 1.f);
     const float2 om = make_float2(v0 ? 1.f - sg.x : 1.f, v1 ? 1.f - sg.y : 1.f);
     const float2 l = make_float2(__log2f(om.x), __log2f(om.y));
     const float2 vis = make_float2(exp2f(l.x * q.beta), exp2f(l.y * q.beta));
@@ -830,165 +810,6 @@ template <int OFF> struct ReduceChunks<OFF, 0> {
                                                Sink &) {}
 };
 
-// ------------------------------------- a visit's sums on the tensor cores
-// The 5 + CD sums a (warp, record) visit needs are linear in per-pixel values
-// with weights that do not depend on the record: the moments of w over the
-// warp's 8x8 pixels (1, x, y, x^2, xy, y^2; the record's own dx, dy follow at
-// the flush from its centre) and plain sums of u, ul and gc.  A lane holds
-// column x = lane / 4, rows y = 2 (lane % 4) + {0, 1}, which is where
-// mma.m16n8k8 (tf32) expects operand A: row g = lane / 4 (and g + 8), k =
-// lane % 4 (and + 4).  So four products contract the values over y straight
-// from the registers they are in: in one, rows x hold w (both pixels) and
-// rows x + 8 the pixel pair's sum of the odd colour (k < 4); in the other rows
-// x hold the pair sums of u (k < 4) and a colour, rows x + 8 those of ul and
-// another colour.  Their
-// constant operands put each sum into a column of its own, chosen so that a
-// lane's four accumulators are four sums still to be added over x (two of
-// them formed by multiplying with x or x^2), which takes a transpose
-// reduction over the lane groups.  tf32 holds 11 significant bits, so every
-// value is split into its leading bits and the exact rest, of which the
-// product reads the leading 11 bits: 22 bits of each value, FP32
-// accumulation; the weights are small multiples of 1/4 and exact.
-// Coordinates are relative to the middle of the 8x8 box.  Measured against
-// the transpose reductions of all 10 sums this replaced (1M primitives at
-// 1080p, 5.6M visits): 211 -> 160 warp instructions per visit, 1.104 -> 0.955
-// ms; finishing a visit while the next is evaluated cost more registers than
-// the latency it hid (0.99 ms), constant weights in operand A (which leaves a
-// second product for x instead of the lane exchanges) more copies (1.32 ms).
-struct MomentBasis {
-    float b0, b1, c0, c1; // operand B of the w and of the u products
-    float f1, f3;         // x and x^2 where a lane's first sum needs them
-    uint32_t m16, m8;     // lane-bit masks of the transpose reduction
-    uint32_t first;       // shared address of this lane's element of the first entry row
-    uint32_t pitch;       // and how far the next row's is; 0 where it has none
-};
-
-// rows: the warp's entry rows, of which the first is a dump.
-template <int CD>
-__device__ __forceinline__ MomentBasis moment_basis(int lane, const float *rows) {
-    constexpr int MC = moment_colours<CD>();
-    const int g = lane >> 2, t = lane & 3;
-    const float y0 = 2.f * t - 3.5f, y1 = y0 + 1.f, x = g - 3.5f;
-    MomentBasis b;
-    // columns: 0 w y, 2 u (ul), 3 colours 0 (1), 4 w y^2, 5 (odd colour), 6 w;
-    // in brackets what rows x + 8 sum
-    b.b0 = g == 0 ? y0 : g == 4 ? y0 * y0 : (g == 5 || g == 6) ? 1.f : 0.f;
-    b.b1 = g == 0 ? y1 : g == 4 ? y1 * y1 : g == 6 ? 1.f : 0.f;
-    b.c0 = g == 2 ? 1.f : 0.f;
-    b.c1 = g == 3 ? 1.f : 0.f;
-    // lane (g, t) holds columns 2t, 2t + 1 of rows g, g + 8
-    b.f1 = (t == 0 || t == 3) ? x : 0.f;
-    b.f3 = t == 3 ? x * x : 0.f;
-    b.m16 = (lane & 16) ? ~0u : 0u;
-    b.m8 = (lane & 8) ? ~0u : 0u;
-    // entry row: [w, wx, wxx, wy, wxy, wyy, u, ul, gc (CD)]; lane (g, t)
-    // ends up with the total of its group's accumulator g / 2
-    const int v = g >> 1;
-    int off = -1;
-    if (t == 0) off = v == 0 ? 3 : v == 1 ? 4 : -1;
-    if (t == 1) off = v == 0 ? 6 : v == 2 ? 7 : MC < 2 ? -1 : v == 1 ? 8 : 9;
-    if (t == 2) off = v == 0 ? 5 : (v == 3 && (MC & 1)) ? 7 + MC : -1;
-    if (t == 3) off = v < 2 ? v : v == 3 ? 2 : -1;
-    if (g & 1) off = -1;
-    b.first = smem_u32(rows) + 4 * max(off, 0);
-    b.pitch = off < 0 ? 0 : 4 * row_pitch<CD>();
-    return b;
-}
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], float a0, float a1, float a2, float a3,
-                                         float b0, float b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 "
-        "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)),
-          "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
-}
-// The leading 11 significant bits of v.
-__device__ __forceinline__ float tf32_hi(float v) {
-    return __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-}
-// One halving step of a transpose reduction over the lane bit h with mask m.
-__device__ __forceinline__ float tr_step(float a, float b, uint32_t m, int h) {
-    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-    const float send = __uint_as_float((ua & m) | (ub & ~m));
-    const float keep = __uint_as_float((ub & m) | (ua & ~m));
-    return keep + __shfl_xor_sync(0xffffffffu, send, h);
-}
-
-// The products of a visit, and the rest of its sums over the warp into the
-// entry row whose element for this lane is at `row`.
-template <int CD>
-__device__ __forceinline__ void moment_products(const MomentBasis &mb, const float2 &w,
-                                                const float2 &u, const float2 &ul,
-                                                const float2 (&gc)[CD], float (&d)[4]) {
-    constexpr int MC = moment_colours<CD>();
-    const float us = u.x + u.y, uh = tf32_hi(us), ls = ul.x + ul.y, lh = tf32_hi(ls);
-    float g0 = 0.f, g1 = 0.f, h0 = 0.f, h1 = 0.f;
-    if constexpr (MC >= 2) {
-        g0 = gc[0].x + gc[0].y;
-        g1 = gc[1].x + gc[1].y;
-        h0 = tf32_hi(g0);
-        h1 = tf32_hi(g1);
-    }
-    d[0] = d[1] = d[2] = d[3] = 0.f;
-    mma_tf32(d, us - uh, ls - lh, g0 - h0, g1 - h1, mb.c0, mb.c1);
-    mma_tf32(d, uh, lh, h0, h1, mb.c0, mb.c1);
-    float g2 = 0.f, h2 = 0.f;
-    if constexpr (MC & 1) {
-        g2 = gc[MC - 1].x + gc[MC - 1].y;
-        h2 = tf32_hi(g2);
-    }
-    const float wx = tf32_hi(w.x), wy = tf32_hi(w.y);
-    // the last element meets zero weights in the columns that are read
-    mma_tf32(d, w.x - wx, g2 - h2, w.y - wy, w.y, mb.b0, mb.b1);
-    mma_tf32(d, wx, h2, wy, g2, mb.b0, mb.b1);
-}
-__device__ __forceinline__ void moment_finish(const MomentBasis &mb, const float (&d)[4],
-                                              uint32_t row) {
-    const float d1 = fmaf(d[0], mb.f1, d[1]), d3 = fmaf(d[0], mb.f3, d[3]);
-    float tot = tr_step(tr_step(d[0], d[2], mb.m16, 16), tr_step(d1, d3, mb.m16, 16), mb.m8, 8);
-    tot += __shfl_xor_sync(0xffffffffu, tot, 4);
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(row), "f"(tot) : "memory");
-}
-
-// Adds an entry row of moments to the sums [w dx, w dy, w dx^2, w dx dy,
-// w dy^2, u, ul, gc] of its record: X, Y is the record's centre relative to
-// the middle of the warp's box, dx = X - x, dy = Y - y.
-template <int CD>
-__device__ __forceinline__ void add_moments(const float *row, float X, float Y,
-                                            float (&sum)[7 + CD]) {
-    const float S = row[0], Sx = row[1], Sxx = row[2], Sy = row[3], Sxy = row[4], Syy = row[5];
-    const float XS = X * S - Sx, YS = Y * S - Sy;
-    sum[0] += XS;
-    sum[1] += YS;
-    sum[2] += X * (XS - Sx) + Sxx;
-    sum[3] += X * YS - (Y * Sx - Sxy);
-    sum[4] += Y * (YS - Sy) + Syy;
-#pragma unroll
-    for (int k = 0; k < 2 + CD; ++k) sum[5 + k] += row[6 + k];
-}
-
-// Values large enough to overflow in a product, infinities and NaN would
-// spread over the sums of a visit in the tensor-core reduction (0 x inf); a
-// batch whose records or pixels hold such values, a negative beta or a
-// non-positive conic diagonal (whose sigma can be -0) is reduced by lane
-// exchanges instead.
-constexpr float kTameLimit = 1e10f;
-template <int CD>
-__device__ __forceinline__ bool tame_record(const GeoRec &q, const float (&col)[CD]) {
-    float m = fabsf(q.x) + fabsf(q.y) + fabsf(q.opac) + fabsf(q.beta) + fabsf(q.cxx) +
-              fabsf(q.cxy) + fabsf(q.cyy);
-#pragma unroll
-    for (int k = 0; k < CD; ++k) m += fabsf(col[k]);
-    return m < kTameLimit && q.beta >= 0.f && q.cxx > 0.f && q.cyy > 0.f;
-}
-template <int CD> __device__ __forceinline__ bool tame_pixels(const BwdPair<CD> &s) {
-    float m = fabsf(s.T.x) + fabsf(s.T.y) + fabsf(s.KS.x) + fabsf(s.KS.y);
-#pragma unroll
-    for (int k = 0; k < CD; ++k) m += fabsf(s.vrc[k].x) + fabsf(s.vrc[k].y);
-    return m < kTameLimit;
-}
-
 // Adds a record's summed values (with the conic applied to the first two) to
 // its gradient row or arrays.
 template <int CD>
@@ -1021,15 +842,11 @@ __device__ __forceinline__ void add_record(const RasterArgs &a, const GeoRec &q,
 template <int CD, bool PACK, int TSZ, int RB, int MINB, int KE>
 __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_kernel(RasterArgs a) {
     constexpr int NV = 7 + CD;
-    constexpr bool MOM = moment_rows<CD>(); // tensor-core reduction of the visits
-    constexpr int MC = moment_colours<CD>();
-    constexpr int RP = row_pitch<CD>();
     extern __shared__ __align__(128) unsigned char sm[];
     const int TS = TSZ ? TSZ : a.TS;
     const int NT = TSZ ? TSZ * TSZ / 2 : (int)blockDim.x, nw = NT >> 5, BR = RB * NT;
     const SmemLayout L = smem_layout<CD, PACK, true>(NT, RB, KE);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm);
-    int32_t *cold_flag = reinterpret_cast<int32_t *>(sm + 16); // a value is not tame
     uint32_t *wmasks = reinterpret_cast<uint32_t *>(sm + L.mask_off); // of even, odd batches
     int32_t *wbin = reinterpret_cast<int32_t *>(sm + L.mask_off + 2 * nw * RB * nw * 4);
     float4 *srec = reinterpret_cast<float4 *>(sm + L.rec_off); // see staged_rec
@@ -1046,9 +863,8 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
     const int ty = loc.tile / loc.TW, tx = loc.tile - ty * loc.TW;
     const int tile_x0 = tx * a.TS + part.x, tile_y0 = ty * a.TS + part.y;
     const int wpr = TS >> 3;
-    // column lane / 4, rows 2 (lane % 4) + {0, 1} of the warp's 8x8 pixels
-    const int j = tile_x0 + (warp % wpr) * 8 + (lane >> 2);
-    const int i0 = tile_y0 + (warp / wpr) * 8 + (lane & 3) * 2;
+    const int j = tile_x0 + (warp % wpr) * 8 + (lane & 7);
+    const int i0 = tile_y0 + (warp / wpr) * 8 + (lane >> 3) * 2;
     const bool in0 = (i0 < loc.H) && (j < loc.W);
     const bool in1 = (i0 + 1 < loc.H) && (j < loc.W);
     // outside pixels read a clamped pixel, like the reference, and never contribute
@@ -1077,17 +893,15 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
         mbar_init(&mbar[0], gather ? NT : 1);
         mbar_init(&mbar[1], gather ? NT : 1);
         fence_barrier_init();
-        *cold_flag = 0;
     }
-    bool cold = __syncthreads_or(MOM && !tame_pixels<CD>(sp));
+    __syncthreads();
     int32_t block_bin = INT32_MIN;
     for (int w = 0; w < nw; ++w) block_bin = max(block_bin, wbin[w]);
     const int32_t hi_end = max(rs, min(re, block_bin + 1)); // exclusive upper index
     const int nb = (hi_end - rs + BR - 1) / BR;
 
-    MomentBasis mb;
-    float *const my_rows = entry_rows + warp * (KE + 1) * RP;
-    if constexpr (MOM) mb = moment_basis<CD>(lane, my_rows);
+    float *const my_rows = entry_rows + warp * KE * NV;
+    const LaneMasks lm = lane_masks(lane);
     // batch b covers [max(rs, hi_end - (b + 1) BR), hi_end - b BR): back to front
     int issued = 0, waited = 0;
     int32_t ent[RB];
@@ -1144,58 +958,14 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 }
             }
         }
-        if constexpr (MOM) {
-#pragma unroll
-            for (int half = 0; half < RB; ++half) {
-                const int sl = tid + half * NT;
-                if (sl < cnt) {
-                    float col[CD];
-                    load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, sl, col);
-                    if (!tame_record<CD>(staged_rec(batch, pitch, sl), col)) *cold_flag = 1;
-                }
-            }
-        }
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicOr(a.status, DEV_ERR_WAIT_TIMEOUT);
             break;
         }
-        if constexpr (MOM) cold = cold || *cold_flag != 0;
         int rows = 0; // entry rows this warp has filled in this batch
-        uint32_t row = MOM ? mb.first : 0; // this lane's element of the last row filled
-        float *fourth = my_rows + 8 + MC;  // and that row's fourth colour sum
 #pragma unroll 1
         for (int k = RB * nw - 1; k >= 0; --k) {
             uint32_t m = wmask[warp * RB * nw + k];
-            if constexpr (MOM) {
-                // as many of the word's records as the list still has rows for
-                uint32_t fit = cold ? 0u : m;
-#pragma unroll 1
-                while (rows + __popc(fit) > KE) fit &= fit - 1;
-                m ^= fit;
-                rows += __popc(fit);
-#pragma unroll 1
-                while (fit) {
-                    const int bit = 31 - __clz(fit);
-                    fit ^= 1u << bit;
-                    const int t = k * 32 + bit;
-                    const GeoRec q = staged_rec(batch, pitch, t);
-                    float col[CD];
-                    load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, t, col);
-                    float2 w, u, ul, gc[CD];
-                    grad_pair<CD, true>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
-                    float d[4];
-                    moment_products<CD>(mb, w, u, ul, gc, d);
-                    row += mb.pitch;
-                    moment_finish(mb, d, row);
-                    if constexpr (CD > MC) {
-                        fourth += RP;
-                        float c = gc[MC].x + gc[MC].y;
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-                        *fourth = c; // every lane holds it
-                    }
-                }
-            }
 #pragma unroll 1
             while (m) {
                 const int bit = 31 - __clz(m);
@@ -1205,15 +975,14 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 float col[CD];
                 load_color<CD, PACK>(batch + 2 * pitch, scol + buf * BR * CD, t, col);
                 float2 w, u, ul, gc[CD];
-                const PairGeom pg = grad_pair<CD, false>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
+                const PairGeom pg = grad_pair<CD>(q, col, px, npy, lo + t, sp, w, u, ul, gc);
                 float g[NV];
                 pair_sums<CD>(pg, w, u, ul, gc, g);
-                const LaneMasks lm = lane_masks(lane);
                 const float g0 = g[0], g1 = g[1];
                 g[0] = q.cxx * g0 + q.cxy * g1;
                 g[1] = q.cxy * g0 + q.cyy * g1;
-                if ((!MOM || cold) && rows < KE) {
-                    float *row = my_rows + (1 + rows) * RP;
+                if (rows < KE) {
+                    float *row = my_rows + rows * NV;
                     // every lane of a group holds the same total: all store it
                     auto put = [row](int v, float tot, bool) { row[v] = tot; };
                     ReduceChunks<0, NV>::run(g, lm, lane, put);
@@ -1254,24 +1023,11 @@ __global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_ke
                 for (int k = (sl >> 5) + 1; k < RB * nw; ++k) r += __popc(mw[k]);
                 if (r >= KE) continue; // went straight to the arrays
                 any = true;
-                const float *row = entry_rows + (w * (KE + 1) + 1 + r) * RP;
-                if (MOM && !cold) {
-                    if constexpr (MOM)
-                        add_moments<CD>(
-                            row, own[half].x - (float)(tile_x0 + (w % wpr) * 8 + 4),
-                            own[half].y - (float)(tile_y0 + (w / wpr) * 8 + 4), sum);
-                } else {
+                const float *row = entry_rows + (w * KE + r) * NV;
 #pragma unroll
-                    for (int u = 0; u < NV; ++u) sum[u] += row[u];
-                }
+                for (int u = 0; u < NV; ++u) sum[u] += row[u];
             }
-            if (!any) continue;
-            if (MOM && !cold) {
-                const float s0 = sum[0], s1 = sum[1];
-                sum[0] = own[half].cxx * s0 + own[half].cxy * s1;
-                sum[1] = own[half].cxy * s0 + own[half].cyy * s1;
-            }
-            add_record<CD>(a, own[half], sum);
+            if (any) add_record<CD>(a, own[half], sum);
         }
     }
     // no copy may still target this CTA's shared memory at exit
@@ -1327,8 +1083,7 @@ static int launch_pack(int64_t T, int64_t n_prims, const int32_t *fl, const floa
 // against CTAs per SM (MINB, the register bound it implies); the backward's
 // trade the register bound against warps per SM --
 //   forward:  0: RB 2, 8 CTAs/SM;  1: RB 1, 10 CTAs/SM;  2: RB 2, 6 CTAs/SM
-//   backward: 0: 8 CTAs/SM, 6 for small grids (see launch_blend);
-//             1: 7 CTAs/SM (72 registers);  2: 6 CTAs/SM (80 registers)
+//   backward: 0: 8 CTAs/SM (64 registers);  1: 7 CTAs/SM (72);  2: 6 CTAs/SM (80)
 // Every variant computes the same images; the backward's gradient sums are
 // the same up to the order of their additions.
 // A warp that visits more than KE_SMALL records of one 128-record batch adds
@@ -1336,14 +1091,12 @@ static int launch_pack(int64_t T, int64_t n_prims, const int32_t *fl, const floa
 // 64 of 5.6M visits do.
 std::atomic<int> g_blend_fwd_variant{0}, g_blend_bwd_variant{0};
 constexpr int kBlendVariants = 3;
-// Backward grids of fewer blocks than this (of 128 threads) run at 6 CTAs per
-// SM: with few waves the unspilled kernel is faster (1,900 blocks: 67.0 against
-// 69.8 us; 3,600: 258.6 against 250.4 us).
-constexpr int BWD_SMALL_GRID = 152 * 16;
 // Below one wave of 16 x 16 squares each is cut into four one-warp CTAs, which
-// wait for no other warp and spread over more SMs (130 tiles: backward 82.1 ->
-// 77.2, forward 49.1 -> 37.1 us; 1,900 tiles: no difference; 8,160 tiles:
-// backward 955 -> 978 us).
+// wait for no other warp and spread over more SMs (130 tiles: backward 93.4 ->
+// 72.6, forward 39.2 -> 37.2 us).  Above it the forward stages each record for
+// fewer pixels (1,900 tiles 33.1 -> 37.1, 8,160 tiles 419 -> 453 us), while the
+// backward is undecided (1,900 tiles 67.0 -> 62.5, 8,160 tiles 1007 -> 962, with a
+// fourth colour 528 -> 549 us).
 constexpr int ONE_WAVE = 152 * 6;
 constexpr int KE_SMALL = 64; // backward entry rows per warp
 
@@ -1359,7 +1112,7 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     constexpr bool PACK = CD <= 4;
     // A CTA works on at most 16 x 16 pixels (two per thread): larger tiles are
     // cut into squares of 16 x 16 (32) or 8 x 8 (24) whose CTAs share the tile's
-    // records (backward; 1M primitives at 1080p, tiles of 32: 1.85 -> 1.08 ms).
+    // records (backward; 1M primitives at 1080p, tiles of 32: 1.85 -> 1.10 ms).
     const bool cut = !a.pair_count;
     const int64_t cta16 = (int64_t)a.n_buckets * (a.TS / 16) * (a.TS / 16);
     const int edge = !cut ? a.TS : a.TS % 16 != 0 || cta16 < ONE_WAVE ? 8 : 16;
@@ -1384,18 +1137,16 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     UBS_REQUIRE(nblocks < (1ll << 31), "raster: %lld thread blocks", (long long)nblocks);
     void (*k)(RasterArgs) = nullptr;
     if constexpr (BWD && PACK) {
-        // 8 CTAs of 128 threads per SM bound a thread to 64 registers (24
-        // bytes spilled), 6 leave it 80 and spill nothing
-        constexpr int C16 = CD < 4 ? 8 : 7;
-        const bool few = nblocks < BWD_SMALL_GRID * (128 / NT);
-        const int per_sm = variant == 1 ? 7 : variant == 2 || few ? 6 : C16;
+        // none of these bounds spills; 1M primitives at 1080p (8,160 blocks): 8
+        // CTAs per SM 1008 us, 7 1014, 6 1034; 1,900 blocks: 67.0, 67.1, 69.3
+        const int per_sm = variant == 1 ? 7 : variant == 2 ? 6 : 8;
         if (edge == 8)
             k = per_sm == 6 ? raster_bwd_kernel<CD, true, 8, 1, 24, KE_SMALL>
                             : raster_bwd_kernel<CD, true, 8, 1, 28, KE_SMALL>;
         else
             k = per_sm == 6   ? raster_bwd_kernel<CD, true, 16, 1, 6, KE_SMALL>
                 : per_sm == 7 ? raster_bwd_kernel<CD, true, 16, 1, 7, KE_SMALL>
-                              : raster_bwd_kernel<CD, true, 16, 1, C16, KE_SMALL>;
+                              : raster_bwd_kernel<CD, true, 16, 1, 8, KE_SMALL>;
     } else if constexpr (BWD) {
         // registers allow 4 CTAs of 128 threads per SM, 2 of the widest
         constexpr int C16 = CD <= 17 ? 4 : 2;
