@@ -278,8 +278,10 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
                         const Tensor &bg, const OptTensor &mask, int32_t color_mode, bool stats,
                         bool grad, const OptTensor &image) {
     TORCH_CHECK_VALUE(params.size() == kParams, "seven scene parameters expected");
-    no_tangents("scene render", params);
-    const bool attached = grad && wants_grad(params);
+    std::vector<Tensor> in = params;
+    in.push_back(bg); // a node's input, as in the operators; its gradient is undefined
+    if (grad) no_tangents("scene render", in);
+    const bool attached = grad && wants_grad(in);
     const at::NoGradGuard no_grad;
     std::vector<Tensor> p(kParams);
     for (int i = 0; i < kParams; ++i) p[i] = scene_param(params[i]);
@@ -353,7 +355,7 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
         const std::vector<int64_t> opacity_shape = params[4].sizes().vec();
         p.push_back(b);
         p.push_back(last);
-        attach("SceneRenderBackward", params, {colors, alphas}, p, {alphas},
+        attach("SceneRenderBackward", in, {colors, alphas}, p, {alphas},
                [c, opacity_shape](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
                    const variable_list s = node.for_kernel(saved);
@@ -362,7 +364,7 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
                    const c10::cuda::CUDAGuard guard(s[0].device());
                    const Tensor vc = grad_or_zeros(g[0], {c->n_pixels, 3}, s[0]);
                    const Tensor va = grad_or_zeros(g[1], {c->n_pixels}, s[0]);
-                   variable_list o(kParams);
+                   variable_list o(kParams + 1);
                    for (int i = 0; i < kParams; ++i) o[i] = at::empty_like(s[i]);
                    UBS_CALL(ubs_scene_backward, c->dim, s[0].size(0), fp(s[0]), fp(s[1]), fp(s[2]),
                             fp(s[3]), fp(s[4]), fp(s[5]), fp(s[6]), c->C, fp(c->viewmats),
@@ -571,10 +573,9 @@ std::tuple<Tensor, Tensor, Tensor> cond(const Tensor &means_, const Tensor &cova
         UBS_CALL(ubs_cond_fwd, N, (int32_t)D, fp(s[0]), fp(s[1]), fp(s[2]), fp(s[3]), fp(s[4]),
                  fpm(om), fpm(oV), fpm(oo), stream_of(s[0]));
     }
-    // no gradient through the query, as in the reference
-    const std::vector<Tensor> diff{means_, covars_, opac_, betas_};
-    if (wants_grad(diff))
-        attach("CondMeanConvarianceOpacityBackward", diff, {om, oV, oo}, s, {},
+    // no gradient through the query, as in the reference (but a node)
+    if (wants_grad(in))
+        attach("CondMeanConvarianceOpacityBackward", in, {om, oV, oo}, s, {},
                [exact](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
                    const variable_list s = node.for_kernel(saved);
@@ -584,7 +585,8 @@ std::tuple<Tensor, Tensor, Tensor> cond(const Tensor &means_, const Tensor &cova
                    const Tensor vV = grad_or_zeros(g[1], {N, 3, 3}, s[0]);
                    const Tensor vo = grad_or_zeros(g[2], {N, 1}, s[0]);
                    variable_list o{fempty({N, D}, s[0]), fempty({N, D, D}, s[0]),
-                                   fempty(s[2].sizes(), s[0]), fempty({N, D - 3}, s[0])};
+                                   fempty(s[2].sizes(), s[0]), fempty({N, D - 3}, s[0]),
+                                   Tensor()};
                    UBS_CALL(ubs_cond_bwd, N, (int32_t)D, fp(s[0]), fp(s[1]), fp(s[2]), fp(s[3]),
                             fp(s[4]), fp(vm), fp(vV), fp(vo), fpm(o[0]), fpm(o[1]), fpm(o[2]),
                             fpm(o[3]), (int32_t)exact, stream_of(s[0]));
@@ -682,15 +684,14 @@ py::tuple projection(const Tensor &means_, const OptTensor &covars_, const OptTe
                  radii.mutable_data_ptr<int32_t>(), fpm(m2), fpm(dep), fpm(con), fpm(comp),
                  stream_of(s[0]));
     }
-    const std::vector<Tensor> diff{in[0], in[1], in[2], in[3], in[4]};
-    if (wants_grad(diff)) {
+    if (wants_grad(in)) {
         std::vector<Tensor> outs{m2, dep, con}, so{con};
         if (with_comps) {
             outs.push_back(comp);
             so.push_back(comp);
         }
         s.push_back(radii);
-        attach("FullyFusedProjectionBackward", diff, outs, s, so,
+        attach("FullyFusedProjectionBackward", in, outs, s, so,
                [=](OpNode &node, const variable_list &saved, variable_list &g) {
                    const at::NoGradGuard no_grad;
                    const variable_list s = node.for_kernel(saved);
@@ -700,7 +701,7 @@ py::tuple projection(const Tensor &means_, const OptTensor &covars_, const OptTe
                    const Tensor vd = grad_or_zeros(g[1], {C, N}, s[0]);
                    const Tensor vc = grad_or_zeros(g[2], {C, N, 3}, s[0]);
                    const Tensor vk = with_comps ? grad_or_zeros(g[3], {C, N}, s[0]) : Tensor();
-                   variable_list o(5);
+                   variable_list o(6); // none for the intrinsics
                    o[0] = fempty({N, 3}, s[0]);
                    if (s[1].defined()) {
                        o[1] = at::empty_like(s[1]);
