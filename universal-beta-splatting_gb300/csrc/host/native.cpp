@@ -386,12 +386,15 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
 }
 
 // Camera tables of a Views object: one pinned staging buffer and one copy to
-// the device.  Sections: pix_base int64 [C + 1], dims int32 [C, 4], tile_base
+// the device, on `stream` (its id and device; default: the current one).  The
+// cameras' own tensors are read on the current stream, which they were made on.
+// Sections: pix_base int64 [C + 1], dims int32 [C, 4], tile_base
 // int32 [C + 1], viewmats [C, 16], intrinsics [C, 4], centers [C, 3], times.
 py::tuple pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tensor> &Ks,
                      const std::vector<OptTensor> &centers, const std::vector<double> &times,
                      const std::vector<int64_t> &widths, const std::vector<int64_t> &heights,
-                     int64_t tile, const at::Device &device) {
+                     int64_t tile, const at::Device &device,
+                     const std::optional<std::pair<int64_t, int64_t>> &stream) {
     const at::NoGradGuard no_grad;
     const int64_t C = (int64_t)viewmats.size();
     const int64_t words = 2 * (C + 1) + 4 * C + (C + 1) + 24 * C;
@@ -435,6 +438,10 @@ py::tuple pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tens
     }
     Tensor dev;
     if (device.is_cuda()) {
+        c10::cuda::OptionalCUDAStreamGuard on;
+        if (stream)
+            on.reset_stream(c10::Stream::unpack3(
+                stream->first, (c10::DeviceIndex)stream->second, c10::DeviceType::CUDA));
         const c10::cuda::OptionalCUDAGuard guard(device);
         dev = staging.to(at::TensorOptions().device(device), /*non_blocking=*/true);
     } else {
@@ -868,7 +875,9 @@ PYBIND11_MODULE(ubs_native, m) {
     m.def("scene_forward", &scene_forward, py::arg("call"), py::arg("params"), py::arg("bg"),
           py::arg("mask"), py::arg("color_mode"), py::arg("stats"), py::arg("grad"),
           py::arg("image") = py::none());
-    m.def("pack_views", &pack_views);
+    m.def("pack_views", &pack_views, py::arg("viewmats"), py::arg("Ks"), py::arg("centers"),
+          py::arg("times"), py::arg("widths"), py::arg("heights"), py::arg("tile"),
+          py::arg("device"), py::arg("stream") = py::none());
     m.def("l1_loss", &l1_loss);
     m.def("ssim_loss", &ssim_loss);
     m.def("cond", &cond);

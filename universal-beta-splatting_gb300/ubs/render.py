@@ -15,7 +15,6 @@ a time.
     colors, alphas = r.render(params, views)       # flat [P, 3], [P]
     images = views.split(colors)                   # list of [H, W, 3]
 """
-import contextlib
 import ctypes
 import gc
 from typing import Dict, List, Optional, Sequence
@@ -47,13 +46,13 @@ class Views:
         for c in cameras:
             center = getattr(c, "position", None)
             centers.append(getattr(c, "center", None) if center is None else center)
-        on = contextlib.nullcontext() if stream is None else torch.cuda.stream(stream)
-        with on, L.untraced():  # the tables are constants of a traced program
+        with L.untraced():  # the tables are constants of a traced program
             (staging, self.viewmats, self.intr, self.centers, self.times, self.dims,
              self.tile_base, self.pix_base, tile_base, pix_base) = L.native().pack_views(
                  [c.viewmat for c in cameras], [c.K for c in cameras], centers,
                  [float(c.timestamp) for c in cameras], [c.width for c in cameras],
-                 [c.height for c in cameras], tile_size, device)
+                 [c.height for c in cameras], tile_size, device,
+                 None if stream is None else (stream.stream_id, stream.device_index))
         self.C = C
         self.tile_size = tile_size
         self.shapes = [(c.height, c.width) for c in cameras]
