@@ -5,6 +5,7 @@
 
 #include <cooperative_groups.h>
 
+#include "bucket_math.h"
 #include "ubs_common.cuh"
 
 namespace ubs {
@@ -17,8 +18,6 @@ constexpr int SMALL_SEG = 4096; // longest bucket sorted by one CTA in shared me
 constexpr int BIG_THREADS = 512;
 constexpr int MERGE_ITEMS = 8;
 constexpr int EMIT_ROUNDS = 4; // (entry, tile) rounds of 32 whose cursor atomics overlap
-
-__host__ __device__ __forceinline__ int64_t imin64(int64_t a, int64_t b) { return a < b ? a : b; }
 
 // ------------------------------------------------------------------- scan
 // Exclusive scan of int32 counts.  Per block: SCAN_TILE items; block-local
@@ -64,7 +63,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_blocks_kernel(const int32_t
     const int64_t off = warp_tot[warp] + (inc - run);
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k)
-        if (base + k < n) out[base + k] = (OutT)(v[k] + off);
+        if (base + k < n) out[base + k] = scan_value<OutT>(v[k] + off);
 }
 
 static __global__ void __launch_bounds__(SCAN_THREADS) scan_sums_kernel(int64_t *sums, int64_t nblocks,
@@ -109,7 +108,7 @@ template <typename OutT>
 __global__ void scan_add_kernel(OutT *out, int64_t n, const int64_t *__restrict__ sums) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    out[i] = (OutT)((int64_t)out[i] + sums[i / SCAN_TILE]);
+    out[i] = scan_value<OutT>((int64_t)out[i] + sums[i / SCAN_TILE]);
 }
 
 template <typename OutT>
@@ -140,9 +139,7 @@ inline int device_exclusive_scan(const int32_t *in, OutT *out, int64_t n, int64_
 
 __device__ __forceinline__ void bucket_range(const int32_t *offsets, int64_t bkt, int64_t n_buckets,
                                              int64_t T, int64_t &lo, int64_t &hi) {
-    lo = imin64(offsets[bkt], T);
-    hi = (bkt + 1 < n_buckets) ? imin64(offsets[bkt + 1], T) : T;
-    if (hi < lo) hi = lo;
+    bucket_bounds(offsets[bkt], bkt + 1 < n_buckets ? offsets[bkt + 1] : INT32_MAX, T, lo, hi);
 }
 
 // Warp-flattened emission of sort keys: every lane holds the tile rectangle
@@ -352,7 +349,7 @@ __global__ void __launch_bounds__(1024) bucket_scan_order_kernel(
     }
 #pragma unroll
     for (int k = 0; k < SCAN_PER; ++k) {
-        if (c[k] >= 0) cnt[tid * per + k] = (int32_t)off;
+        if (c[k] >= 0) cnt[tid * per + k] = bucket_start(off);
         off += max(c[k], 0);
     }
     // heaviest-first order: exclusive scan of the bins, then a scatter
@@ -388,7 +385,7 @@ __global__ void __launch_bounds__(1024) bucket_scan_order_kernel(
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             cursor[(int64_t)r * n + c0 + i] = o;
-            o += counts[(int64_t)r * n + c0 + i];
+            o = bucket_start((int64_t)o + counts[(int64_t)r * n + c0 + i]);
         }
     }
     cluster.sync(); // no CTA leaves while another reads its histogram
@@ -438,7 +435,7 @@ __global__ void replica_cursors_kernel(const int32_t *__restrict__ counts, int32
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         cursor[(int64_t)r * n + b] = off;
-        off += counts[(int64_t)r * n + b];
+        off = bucket_start((int64_t)off + counts[(int64_t)r * n + b]);
     }
 }
 
