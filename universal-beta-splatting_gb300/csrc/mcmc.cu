@@ -102,9 +102,12 @@ __device__ __forceinline__ double uniform01(uint64_t seed, uint64_t i) {
 }
 // The same value rounded to float, without the FP64 pipe: 53 bits round once
 // in the conversion, and the power of two is exact (measured, noise for 1M
-// primitives: 37 us through double, 22 this way).
+// primitives: 37 us through double, 22 this way).  The values that would round
+// to 1 (one in 2^25) give the float below it: 1 - u stays positive.
 __device__ __forceinline__ float uniform01f(uint64_t seed, uint64_t i) {
-    return __ull2float_rn(splitmix64(seed + (i + 1) * 0x9e3779b97f4a7c15ull) >> 11) * 0x1.0p-53f;
+    const float u =
+        __ull2float_rn(splitmix64(seed + (i + 1) * 0x9e3779b97f4a7c15ull) >> 11) * 0x1.0p-53f;
+    return fminf(u, 1.f - 0x1.0p-24f);
 }
 
 // The opacity a source sampled `count` times shares with its copies
