@@ -598,10 +598,10 @@ __global__ void __launch_bounds__(PRIM_THREADS, ONE ? 4 : 3) scene_prim_bwd_kern
 
 // Groups of views of the per-primitive kernels: one where the primitives alone
 // give every SM its resident CTAs (6 forward, 3 backward), else as many as that
-// takes (5k primitives in 8 views: backward 18 us).
+// takes (5k primitives in 8 views: backward 18 us); at most a grid's 65,535 rows.
 unsigned view_groups(int64_t N, int C, int ctas_per_sm) {
     const int64_t want = (152 * PRIM_THREADS * ctas_per_sm + N - 1) / (N < 1 ? 1 : N);
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, C));
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>({want, C, 65535}));
 }
 
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
