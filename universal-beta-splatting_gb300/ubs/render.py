@@ -26,6 +26,7 @@ from . import _lib as L
 PARAM_ORDER = ("xyz", "mean", "scale", "l_triangle", "opacity", "beta", "rgb")
 STATUS_OVERFLOW = 4
 STATUS_NEG_DEPTH = 2
+MAX_CAPACITY = 2 ** 31 - 1  # intersections of one call (their positions are int32)
 
 
 class Views:
@@ -114,8 +115,8 @@ class Renderer:
                                "but had capacity %d; capacity is now %d" % (T, cap, self.capacity))
         if T > cap - cap // 8:
             # a scene that grows from frame to frame (training) gets its room
-            # before a frame overflows
-            self.capacity = max(self.capacity or 0, int(T * 1.25) + 1024)
+            # before a frame overflows, as far as a capacity goes
+            self.capacity = max(self.capacity or 0, min(int(T * 1.25) + 1024, MAX_CAPACITY))
 
     def stats(self):
         """(intersections, status bits) of the last forward's workspace; raises
