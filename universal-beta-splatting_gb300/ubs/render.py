@@ -15,8 +15,10 @@ a time.
     colors, alphas = r.render(params, views)       # flat [P, 3], [P]
     images = views.split(colors)                   # list of [H, W, 3]
 """
+import contextlib
 import ctypes
-import gc
+import threading
+import weakref
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -269,6 +271,40 @@ class Renderer:
                           *[params[k] for k in PARAM_ORDER])
 
 
+class _Graphs:
+    """Destroying a graph is not permitted while another is being captured and
+    fails that capture; a step in a reference cycle can die at any time, inside
+    a later step's capture too (a cycle collection there).  The graphs of steps
+    that die during a capture, on whatever thread, are kept until the last
+    capture has ended."""
+
+    def __init__(self):
+        self._lock = threading.RLock()  # a collection may run while it is held
+        self._captures, self._kept = 0, []
+
+    def release(self, graph):
+        with self._lock:
+            if self._captures:
+                self._kept.append(graph)
+
+    @contextlib.contextmanager
+    def capturing(self):
+        with self._lock:
+            self._captures += 1
+        try:
+            yield
+        finally:
+            kept = []
+            with self._lock:
+                self._captures -= 1
+                if not self._captures:
+                    kept, self._kept = self._kept, kept
+            del kept  # destroyed here
+
+
+_GRAPHS = _Graphs()
+
+
 class GraphedStep:
     """One training step -- fused render of `views`, `loss_fn(colors, alphas)`,
     backward to every parameter -- captured once into a CUDA graph and then
@@ -318,21 +354,15 @@ class GraphedStep:
             before_capture()
         self.graph = torch.cuda.CUDAGraph()
         n0 = L.query("ubs_launch_count")
-        # a cycle collection inside the capture may destroy an older graph,
-        # which is not permitted there and fails this capture
-        collecting = gc.isenabled()
-        gc.disable()
-        try:
-            with torch.cuda.graph(self.graph):
-                if optimizer is not None:
-                    for v in params.values():
-                        v.grad.zero_()
-                self.loss = self._body()
-                if optimizer is not None:
-                    optimizer.launch()
-        finally:
-            if collecting:
-                gc.enable()
+        # the graph outlives this object until no step is being captured
+        weakref.finalize(self, _GRAPHS.release, self.graph).atexit = False
+        with _GRAPHS.capturing(), torch.cuda.graph(self.graph):
+            if optimizer is not None:
+                for v in params.values():
+                    v.grad.zero_()
+            self.loss = self._body()
+            if optimizer is not None:
+                optimizer.launch()
         # library kernels in the graph (each replay launches them all)
         self.launches_per_replay = int(L.query("ubs_launch_count") - n0)
 
