@@ -178,9 +178,22 @@ class FrameRenderer:
         """One frame as a float32 [H, W, 3] host array: params are the raw
         scene tensors (xyz, mean, scale, l_triangle, opacity, beta, rgb), c2w
         the camera-to-world matrix and K the intrinsics of the viewer camera."""
+        # the slot is this frame's from the start (another thread's takes the
+        # other one); a frame that fails gives it back, so that the last image
+        # stays valid
+        slot = self._ring
+        self._ring ^= 1
+        try:
+            out = self._render(slot, params, c2w, K, width, height, state)
+        except BaseException:
+            self._ring = slot
+            raise
+        return out.copy() if copy else out
+
+    def _render(self, slot, params, c2w, K, width, height, state):
+        """render() into ring slot `slot`."""
         H, W = int(height), int(width)
         # the frame and the visible count to pinned host memory, one wait
-        slot = self._ring
         need = H * W * 3 + 1
         buf = self._host[slot]
         if buf is None or buf.numel() < need:
@@ -192,10 +205,8 @@ class FrameRenderer:
             host.view(H, W, 3).copy_(img, non_blocking=True)
         buf[H * W * 3:].copy_(visible.float().view(1), non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
-        self._ring ^= 1
         self.rendered_count = int(buf[H * W * 3].item())
-        out = buf[:H * W * 3].view(H, W, 3).numpy()
-        return out.copy() if copy else out
+        return host.view(H, W, 3).numpy()
 
 
 def view(model, camera_state, render_tab_state, center=None):
