@@ -19,6 +19,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CachingHostAllocator.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 #include <torch/csrc/autograd/function.h>
@@ -26,7 +27,7 @@
 #include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/utils/pybind.h>
 
-#include <array>
+#include <algorithm>
 #include <functional>
 #include <memory>
 #include <mutex>
@@ -89,11 +90,16 @@ float *fpm(Tensor &t) { return t.defined() ? t.mutable_data_ptr<float>() : nullp
 Tensor fempty(at::IntArrayRef s, const Tensor &like) {
     return at::empty(s, like.options().dtype(at::kFloat));
 }
+// Zeroes the first n bytes of t on its current stream.
+void zero(Tensor &t, size_t n) {
+    n = std::min<size_t>(n, t.nbytes());
+    if (n)
+        C10_CUDA_CHECK(cudaMemsetAsync(t.mutable_data_ptr(), 0, n,
+                                       static_cast<cudaStream_t>(stream_of(t))));
+}
 Tensor fzeros(at::IntArrayRef s, const Tensor &like) {
     Tensor t = fempty(s, like);
-    if (t.numel())
-        cudaMemsetAsync(t.mutable_data_ptr(), 0, t.nbytes(),
-                        static_cast<cudaStream_t>(stream_of(t)));
+    zero(t, t.nbytes());
     return t;
 }
 Tensor bytes(size_t n, const Tensor &like) {
@@ -500,7 +506,7 @@ Tensor l1_loss(const Tensor &x, const Tensor &y) {
         out = fempty({2}, x);
         Tensor ws = bytes(ubs_l1_loss_workspace_bytes(n), x);
         void *st = stream_of(x);
-        cudaMemsetAsync(ws.mutable_data_ptr(), 0, 256, static_cast<cudaStream_t>(st));
+        zero(ws, 256);
         if (grad) g = at::empty_like(x);
         UBS_CALL(ubs_l1_loss, fp(x), fp(y), fpm(g), n, 1.0, fpm(out), ws.mutable_data_ptr(),
                  ws.nbytes(), st);
@@ -546,8 +552,7 @@ Tensor ssim_loss(const Tensor &img, const Tensor &gt, bool channels_last, bool v
         void *st = stream_of(img);
         // the ticket counter (first bytes) starts at zero; the rest is written
         // before it is read
-        cudaMemsetAsync(ws.mutable_data_ptr(), 0, std::min<size_t>(256, ws.nbytes()),
-                        static_cast<cudaStream_t>(st));
+        zero(ws, 256);
         UBS_CALL(ubs_ssim_loss, img.const_data_ptr<float>(), si, gt.const_data_ptr<float>(), sg,
                  want ? grad.mutable_data_ptr<float>() : nullptr, want ? sd : nullptr, (int32_t)n,
                  (int32_t)c, (int32_t)h, (int32_t)w, (int32_t)valid, w0, w1, w2, fpm(out),
