@@ -12,6 +12,9 @@
 // few microseconds, and the count is copied as soon as the scan has produced
 // it, so that the host prepares what follows while the frame still renders.
 //
+// The calls run without Python's lock, as ctypes and PyTorch's operators do: a
+// full launch queue blocks the calling thread alone.
+//
 // Nothing is kept between calls: every call allocates its outputs and
 // workspace from PyTorch's caching allocator on the current stream, and reads
 // the current stream when it runs.
@@ -226,10 +229,7 @@ struct FrameStats {
     Tensor host; // pinned int64 [2]
     at::cuda::CUDAEvent ev;
     std::pair<int64_t, int64_t> wait() {
-        {
-            py::gil_scoped_release nogil;
-            ev.synchronize();
-        }
+        ev.synchronize();
         const int64_t *p = host.const_data_ptr<int64_t>();
         return {p[0], p[1] & 0xffffffff};
     }
@@ -280,9 +280,10 @@ Tensor scene_param(const Tensor &t) {
 // waited for; tiles of 16 pixels and more are stored there by the blend itself,
 // smaller ones copied (their 96-byte rows use the link badly: a nearly empty
 // 1080p frame 191 us against 46 + 135).
-py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<Tensor> &params,
-                        const Tensor &bg, const OptTensor &mask, int32_t color_mode, bool stats,
-                        bool grad, const OptTensor &image) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, std::shared_ptr<FrameStats>>
+scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<Tensor> &params,
+              const Tensor &bg, const OptTensor &mask, int32_t color_mode, bool stats, bool grad,
+              const OptTensor &image) {
     TORCH_CHECK_VALUE(params.size() == kParams, "seven scene parameters expected");
     std::vector<Tensor> in = params;
     in.push_back(bg); // a node's input, as in the operators; its gradient is undefined
@@ -330,22 +331,21 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
                  host && (parts & UBS_SCENE_PART_BLEND) ? parts | UBS_SCENE_HOST_IMAGE : parts,
                  counts, st);
     };
-    py::object fs = py::none();
+    std::shared_ptr<FrameStats> fs; // none without stats
     if (!stats) {
         part(UBS_SCENE_PART_COUNT | UBS_SCENE_PART_BLEND, nullptr);
     } else {
         // the count kernel writes to the pinned slot itself: a copy would make
         // the frame wait for the copy engine
-        auto s = std::make_shared<FrameStats>();
-        s->host = at::empty({2}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
-        part(UBS_SCENE_PART_COUNT, s->host.mutable_data_ptr<int64_t>());
+        fs = std::make_shared<FrameStats>();
+        fs->host = at::empty({2}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+        part(UBS_SCENE_PART_COUNT, fs->host.mutable_data_ptr<int64_t>());
         const auto cs = c10::cuda::getCurrentCUDAStream(p[0].device().index());
-        s->ev.record(cs);
+        fs->ev.record(cs);
         // the slot outlives the kernel's write
-        at::cuda::CachingHostAllocator_recordEvent(s->host.mutable_data_ptr(),
-                                                   s->host.storage().data_ptr().get_context(), cs);
+        at::cuda::CachingHostAllocator_recordEvent(fs->host.mutable_data_ptr(),
+                                                   fs->host.storage().data_ptr().get_context(), cs);
         part(UBS_SCENE_PART_BLEND, nullptr);
-        fs = py::cast(s);
     }
     if (image) {
         if (!host) image->view({c->n_pixels, 3}).copy_(colors, /*non_blocking=*/true);
@@ -388,7 +388,7 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
                    return o;
                });
     }
-    return py::make_tuple(colors, alphas, last, ws, fs);
+    return {colors, alphas, last, ws, fs};
 }
 
 // Camera tables of a Views object: one pinned staging buffer and one copy to
@@ -396,11 +396,12 @@ py::tuple scene_forward(const std::shared_ptr<SceneCall> &c, const std::vector<T
 // cameras' own tensors are read on the current stream, which they were made on.
 // Sections: pix_base int64 [C + 1], dims int32 [C, 4], tile_base
 // int32 [C + 1], viewmats [C, 16], intrinsics [C, 4], centers [C, 3], times.
-py::tuple pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tensor> &Ks,
-                     const std::vector<OptTensor> &centers, const std::vector<double> &times,
-                     const std::vector<int64_t> &widths, const std::vector<int64_t> &heights,
-                     int64_t tile, const at::Device &device,
-                     const std::optional<std::pair<int64_t, int64_t>> &stream) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, std::vector<int64_t>,
+           std::vector<int64_t>>
+pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tensor> &Ks,
+           const std::vector<OptTensor> &centers, const std::vector<double> &times,
+           const std::vector<int64_t> &widths, const std::vector<int64_t> &heights, int64_t tile,
+           const at::Device &device, const std::optional<std::pair<int64_t, int64_t>> &stream) {
     const at::NoGradGuard no_grad;
     const int64_t C = (int64_t)viewmats.size();
     const int64_t words = 2 * (C + 1) + 4 * C + (C + 1) + 24 * C;
@@ -465,8 +466,7 @@ py::tuple pack_views(const std::vector<Tensor> &viewmats, const std::vector<Tens
     Tensor d_in = take(4 * C).view(at::kFloat).view({C, 4});
     Tensor d_ce = take(3 * C).view(at::kFloat).view({C, 3});
     Tensor d_ti = take(C).view(at::kFloat);
-    return py::make_tuple(staging, d_vm, d_in, d_ce, d_ti, d_dims, d_tb, d_pix, tile_base,
-                          pix_base);
+    return {staging, d_vm, d_in, d_ce, d_ti, d_dims, d_tb, d_pix, tile_base, pix_base};
 }
 
 // ------------------------------------------------------------------- losses
@@ -669,7 +669,7 @@ Tensor covar(const Tensor &rot_, const Tensor &scale_, const Tensor &lt_, const 
     return out;
 }
 
-py::tuple projection(const Tensor &means_, const OptTensor &covars_, const OptTensor &quats_,
+std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> projection(const Tensor &means_, const OptTensor &covars_, const OptTensor &quats_,
                      const OptTensor &scales_, const Tensor &viewmats_, const Tensor &Ks_,
                      int32_t W, int32_t H, double eps2d, double near_p, double far_p, double clip,
                      bool with_comps) {
@@ -731,8 +731,7 @@ py::tuple projection(const Tensor &means_, const OptTensor &covars_, const OptTe
                    return o;
                });
     }
-    return py::make_tuple(radii, m2, dep, con,
-                          with_comps ? py::cast(comp) : py::object(py::none()));
+    return {radii, m2, dep, con, with_comps ? OptTensor(comp) : std::nullopt};
 }
 
 // (tiles_per_gauss, isect_ids, flatten_ids, isect_offsets)
@@ -751,12 +750,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> isect(const Tensor &means2d_, const T
     Tensor tpg = at::empty({C, N}, ints), off = at::empty({C, th, tw}, ints);
     Tensor ws = bytes(ubs_isect_count_workspace_bytes((int32_t)C, N, nt), m2);
     int64_t T = 0;
-    {
-        const py::gil_scoped_release nogil;
-        UBS_CALL(ubs_isect_count, (int32_t)C, N, fp(m2), rad.const_data_ptr<int32_t>(), fp(dep), ts,
-                 tw, th, tpg.mutable_data_ptr<int32_t>(), off.mutable_data_ptr<int32_t>(), &T,
-                 ws.mutable_data_ptr(), ws.nbytes(), st);
-    }
+    UBS_CALL(ubs_isect_count, (int32_t)C, N, fp(m2), rad.const_data_ptr<int32_t>(), fp(dep), ts, tw,
+             th, tpg.mutable_data_ptr<int32_t>(), off.mutable_data_ptr<int32_t>(), &T,
+             ws.mutable_data_ptr(), ws.nbytes(), st);
     Tensor ids = at::empty({T}, m2.options().dtype(at::kLong)), fl = at::empty({T}, ints);
     if (T > 0) {
         Tensor w2 = bytes(ubs_isect_sort_workspace_bytes((int32_t)C, N, nt, T), m2);
@@ -875,23 +871,24 @@ PYBIND11_MODULE(ubs_native, m) {
         .def(py::init(&scene_call), py::arg("dim"), py::arg("tables"), py::arg("n_buckets"),
              py::arg("n_pixels"), py::arg("tile"), py::arg("eps2d"), py::arg("near"),
              py::arg("far"), py::arg("clip"), py::arg("exact"), py::arg("cap"));
+    using NoGil = py::call_guard<py::gil_scoped_release>;
     py::class_<FrameStats, std::shared_ptr<FrameStats>>(m, "FrameStats")
-        .def("wait", &FrameStats::wait);
-    m.def("scene_forward", &scene_forward, py::arg("call"), py::arg("params"), py::arg("bg"),
-          py::arg("mask"), py::arg("color_mode"), py::arg("stats"), py::arg("grad"),
+        .def("wait", &FrameStats::wait, NoGil());
+    m.def("scene_forward", &scene_forward, NoGil(), py::arg("call"), py::arg("params"),
+          py::arg("bg"), py::arg("mask"), py::arg("color_mode"), py::arg("stats"), py::arg("grad"),
           py::arg("image") = py::none());
-    m.def("pack_views", &pack_views, py::arg("viewmats"), py::arg("Ks"), py::arg("centers"),
-          py::arg("times"), py::arg("widths"), py::arg("heights"), py::arg("tile"),
-          py::arg("device"), py::arg("stream") = py::none());
-    m.def("l1_loss", &l1_loss);
-    m.def("ssim_loss", &ssim_loss);
-    m.def("cond", &cond);
-    m.def("rotmat", &rotmat);
-    m.def("covar", &covar);
-    m.def("projection", &projection);
-    m.def("isect", &isect);
-    m.def("offset_encode", &offset_encode);
-    m.def("raster", &raster);
+    m.def("pack_views", &pack_views, NoGil(), py::arg("viewmats"), py::arg("Ks"),
+          py::arg("centers"), py::arg("times"), py::arg("widths"), py::arg("heights"),
+          py::arg("tile"), py::arg("device"), py::arg("stream") = py::none());
+    m.def("l1_loss", &l1_loss, NoGil());
+    m.def("ssim_loss", &ssim_loss, NoGil());
+    m.def("cond", &cond, NoGil());
+    m.def("rotmat", &rotmat, NoGil());
+    m.def("covar", &covar, NoGil());
+    m.def("projection", &projection, NoGil());
+    m.def("isect", &isect, NoGil());
+    m.def("offset_encode", &offset_encode, NoGil());
+    m.def("raster", &raster, NoGil());
     m.def("timing_start", &timing_start);
     m.def("timing_stop", &timing_stop);
 }
