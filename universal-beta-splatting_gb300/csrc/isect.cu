@@ -145,16 +145,6 @@ __global__ void isect_count_kernel(int64_t CN, int64_t N, const float2 *__restri
         for (uint32_t x = b.x0; x < b.x1; ++x) atomicAdd(&bc[y * tw + x], 1);
 }
 
-__global__ void fold_count_replicas_kernel(const int32_t *__restrict__ replicas, int64_t nb,
-                                           int32_t *__restrict__ counts) {
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    int32_t c = 0;
-#pragma unroll
-    for (int r = 0; r < kCountReplicas; ++r) c += replicas[r * nb + b];
-    counts[b] = c;
-}
-
 // ------------------------------------------------------------------- emit
 __global__ void isect_emit_bucket_kernel(int64_t CN, int64_t N, const float2 *__restrict__ means2d,
                                          const int32_t *__restrict__ radii,
@@ -330,7 +320,7 @@ int ubs_isect_count(int32_t C, int64_t N, const float *means2d, const int32_t *r
             return e;
     } else {
         UBS_TIMED("isect_count_fold", st,
-                  fold_count_replicas_kernel<<<grid_for(nb, 256), 256, 0, st>>>(
+                  fold_replicas_kernel<kCountReplicas><<<grid_for(nb, 256), 256, 0, st>>>(
                       w.replicas, nb, w.bucket_counts));
         ::ubs::note_launch();
         if (int e = check_launch("isect_count fold")) return e;

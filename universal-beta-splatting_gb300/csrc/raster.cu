@@ -837,14 +837,13 @@ __device__ __forceinline__ void add_record(const RasterArgs &a, const GeoRec &q,
     }
 }
 
-// TSZ: edge of a CTA's pixels, 8 or 16, or 0 for a whole tile of a.TS; MINB
-// CTAs per SM; KE entry rows per warp (see smem_layout).
-template <int CD, bool PACK, int TSZ, int RB, int MINB, int KE>
-__global__ void __launch_bounds__(TSZ ? TSZ * TSZ / 2 : 512, MINB) raster_bwd_kernel(RasterArgs a) {
+// TS: edge of a CTA's pixels, 8 or 16; MINB CTAs per SM; KE entry rows per warp
+// (see smem_layout).
+template <int CD, bool PACK, int TS, int RB, int MINB, int KE>
+__global__ void __launch_bounds__(TS * TS / 2, MINB) raster_bwd_kernel(RasterArgs a) {
     constexpr int NV = 7 + CD;
     extern __shared__ __align__(128) unsigned char sm[];
-    const int TS = TSZ ? TSZ : a.TS;
-    const int NT = TSZ ? TSZ * TSZ / 2 : (int)blockDim.x, nw = NT >> 5, BR = RB * NT;
+    constexpr int NT = TS * TS / 2, nw = NT >> 5, BR = RB * NT;
     const SmemLayout L = smem_layout<CD, PACK, true>(NT, RB, KE);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(sm);
     uint32_t *wmasks = reinterpret_cast<uint32_t *>(sm + L.mask_off); // of even, odd batches
@@ -1094,17 +1093,17 @@ constexpr int kBlendVariants = 3;
 // Below one wave of 16 x 16 squares each is cut into four one-warp CTAs, which
 // wait for no other warp and spread over more SMs (130 tiles: backward 93.4 ->
 // 72.6, forward 39.2 -> 37.2 us).  Above it the forward stages each record for
-// fewer pixels (1,900 tiles 33.1 -> 37.1, 8,160 tiles 419 -> 453 us), while the
-// backward is undecided (1,900 tiles 67.0 -> 62.5, 8,160 tiles 1007 -> 962, with a
-// fourth colour 528 -> 549 us).
+// fewer pixels (1,900 tiles 33.1 -> 37.1, 8,160 tiles 419 -> 453 us); the backward
+// would gain there with three colours (67.0 -> 62.5, 1007 -> 962 us) and lose with
+// four (3,600 tiles 528 -> 549 us).
 constexpr int ONE_WAVE = 152 * 6;
 constexpr int KE_SMALL = 64; // backward entry rows per warp
 
-// Shared memory of a CTA over a whole tile with an accumulator row and a flag
-// per batch slot.
-template <int CD, bool BWD> static int whole_tile_bytes(int ts) {
-    const int NT = ts * ts / 2;
-    return smem_layout<CD, false, BWD>(NT, 2, 0).rows_off + (BWD ? 2 * NT * (7 + CD + 1) * 4 : 0);
+// Most colour channels of a tile size.  The limit dates from kernels whose CTAs
+// worked on whole tiles (the squares of today need at most 81 KB of shared
+// memory); what it refuses stays refused.
+constexpr int max_channels(int ts, bool bwd) {
+    return ts <= 16 ? 33 : ts == 24 ? (bwd ? 17 : 33) : (bwd ? 9 : 17);
 }
 
 template <int CD, bool BWD>
@@ -1126,12 +1125,10 @@ static int launch_blend(RasterArgs &a, cudaStream_t st) {
     // 176, 16 channels: 46 -> 42 us)
     const int RB = BWD || variant == 1 || (!PACK && cut) ? 1 : 2;
     const SmemLayout L = smem_layout<CD, PACK, BWD>(NT, RB, KE_SMALL);
-    // wide colours: what a CTA over the whole tile would need stays the limit on
-    // tile size and channels
-    const int whole = PACK ? L.total : whole_tile_bytes<CD, BWD>(a.TS);
-    if (whole > 227 * 1024)
-        return set_error(UBS_ERR_UNSUPPORTED, "raster: tile_size %d with %d channels needs %d B "
-                                              "of shared memory", a.TS, CD, whole);
+    if (CD > max_channels(a.TS, BWD))
+        return set_error(UBS_ERR_UNSUPPORTED, "raster: tile_size %d takes up to %d channels in the "
+                                              "%s (a whole tile's shared memory), got %d", a.TS,
+                         max_channels(a.TS, BWD), BWD ? "backward" : "forward", CD);
     const int64_t nblocks = (int64_t)a.n_buckets * a.sub * a.sub;
     if (nblocks == 0) return UBS_OK;
     UBS_REQUIRE(nblocks < (1ll << 31), "raster: %lld thread blocks", (long long)nblocks);

@@ -415,13 +415,13 @@ inline int launch_bucket_scan_order(const int32_t *counts, int32_t n, int32_t *o
 
 // Larger frames (more than SCAN_ORDER_MAX buckets): the replicas' sums ...
 template <int R>
-__global__ void fold_replicas_kernel(const int32_t *__restrict__ counts, int32_t n,
+__global__ void fold_replicas_kernel(const int32_t *__restrict__ counts, int64_t n,
                                      int32_t *__restrict__ totals) {
     const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n) return;
     int32_t c = 0;
 #pragma unroll
-    for (int r = 0; r < R; ++r) c += counts[(int64_t)r * n + b];
+    for (int r = 0; r < R; ++r) c += counts[r * n + b];
     totals[b] = c;
 }
 // ... and, after their exclusive scan, the replicas' cursors.

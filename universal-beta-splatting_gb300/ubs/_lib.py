@@ -319,13 +319,6 @@ def ptr(t, dtype=None):
     return ctypes.c_void_p(t.data_ptr())
 
 
-def strided_ptr(t):
-    """Device pointer of a CUDA tensor whose strides the callee is given."""
-    if not t.is_cuda:
-        raise ValueError("expected a CUDA tensor, got device %s" % t.device)
-    return ctypes.c_void_p(t.data_ptr())
-
-
 def stream(device=None):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 

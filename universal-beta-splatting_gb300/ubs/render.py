@@ -201,13 +201,6 @@ class Renderer:
             out.append((ids, fl, (starts[b0:b1] - a).to(torch.int32).view(th, tw)))
         return out
 
-    def _args(self, p, views, bg):
-        return [self.dim, p["xyz"].shape[0]] + [L.ptr(p[k]) for k in PARAM_ORDER] + [
-            views.C, L.ptr(views.viewmats), L.ptr(views.intr), L.ptr(views.centers),
-            L.ptr(views.times), L.ptr(views.dims), L.ptr(views.tile_base), L.ptr(views.pix_base),
-            views.n_buckets, self.tile_size, float(self.eps2d), float(self.near), float(self.far),
-            float(self.radius_clip), L.ptr(bg)]
-
     def forward_raw(self, p: Dict[str, torch.Tensor], views: Views, bg, check=True,
                     prim_mask=None, color_mode=0, image=None):
         """Run the forward kernels; returns (colors, alphas, last_ids, workspace, capacity).
