@@ -4,7 +4,6 @@ the host path built on it (csrc/host/native.cpp, the ubs_native module).
 The library is the only compute path: there is no CPU or PyTorch fallback.
 If it cannot be built or loaded, or a CUDA device is missing, calls raise.
 """
-import contextlib
 import ctypes
 import importlib.util
 import threading
@@ -149,18 +148,24 @@ def native():
 # torch.jit.trace records the tensor operations that a call dispatches.  Of an
 # operator here those are its allocations: the kernels are launched beside the
 # dispatcher.  So an operator is recorded as one node that makes the call again.
+_trace = torch._C._get_tracing_state
+
+
 def tracing():
     """Whether torch.jit.trace is recording on this thread."""
-    return torch._C._get_tracing_state() is not None
+    return _trace() is not None
 
 
-@contextlib.contextmanager
-def untraced():
-    """Nothing done inside is recorded."""
-    state = torch._C._get_tracing_state()
+def untraced(name, *args):
+    """Function `name` of the ubs_native module, unrecorded: its results are
+    constants of a traced program."""
+    f = getattr(_native or native(), name)
+    state = _trace()
+    if state is None:
+        return f(*args)
     torch._C._set_tracing_state(None)
     try:
-        yield
+        return f(*args)
     finally:
         torch._C._set_tracing_state(state)
 
@@ -205,14 +210,15 @@ class _Call:
 
 
 def recorded(name, fn, *tensors):
-    """fn(*tensors), a tuple of tensors; under torch.jit.trace one node."""
-    return _Recorded.apply(_Call(name, fn), *tensors) if tracing() else fn(*tensors)
+    """fn(*tensors), a tuple of tensors, as one node of the program that
+    torch.jit.trace records."""
+    return _Recorded.apply(_Call(name, fn), *tensors)
 
 
 def op(name, *args):
     """Operator `name` of the ubs_native module."""
-    f = getattr(native(), name)
-    if not tracing():
+    f = getattr(_native or native(), name)
+    if _trace() is None:
         return f(*args)
     at = [i for i, a in enumerate(args) if isinstance(a, torch.Tensor)]
     rest = [None if isinstance(a, torch.Tensor) else a for a in args]

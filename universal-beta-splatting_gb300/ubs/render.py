@@ -49,13 +49,12 @@ class Views:
         for c in cameras:
             center = getattr(c, "position", None)
             centers.append(getattr(c, "center", None) if center is None else center)
-        with L.untraced():  # the tables are constants of a traced program
-            (staging, self.viewmats, self.intr, self.centers, self.times, self.dims,
-             self.tile_base, self.pix_base, tile_base, pix_base) = L.native().pack_views(
-                 [c.viewmat for c in cameras], [c.K for c in cameras], centers,
-                 [float(c.timestamp) for c in cameras], [c.width for c in cameras],
-                 [c.height for c in cameras], tile_size, device,
-                 None if stream is None else (stream.stream_id, stream.device_index))
+        (staging, self.viewmats, self.intr, self.centers, self.times, self.dims, self.tile_base,
+         self.pix_base, tile_base, pix_base) = L.untraced(
+             "pack_views", [c.viewmat for c in cameras], [c.K for c in cameras], centers,
+             [float(c.timestamp) for c in cameras], [c.width for c in cameras],
+             [c.height for c in cameras], tile_size, device,
+             None if stream is None else (stream.stream_id, stream.device_index))
         self.C = C
         self.tile_size = tile_size
         self.shapes = [(c.height, c.width) for c in cameras]
@@ -259,9 +258,12 @@ class Renderer:
             bg = torch.zeros(views.C, 3, device=params["xyz"].device)
         else:
             bg = backgrounds.reshape(-1, 3).expand(views.C, 3).contiguous().float()
-        return L.recorded("scene_render",
-                          lambda bg, *p: self._forward(p, views, bg, check, None, 0, True)[:2], bg,
-                          *[params[k] for k in PARAM_ORDER])
+        tensors = [params[k] for k in PARAM_ORDER]
+        if L.tracing():
+            return L.recorded("scene_render", lambda bg, *p: self._forward(
+                p, views, bg, check, None, 0, True)[:2], bg, *tensors)
+        colors, alphas, _, _, _ = self._forward(tensors, views, bg, check, None, 0, True)
+        return colors, alphas
 
 
 class _Graphs:
