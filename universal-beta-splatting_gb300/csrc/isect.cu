@@ -18,6 +18,7 @@
 // Because the per-bucket keys are unique the result is bit-identical to the
 // reference's stable radix sort, independent of scatter order.
 #include <algorithm>
+#include <mutex>
 
 #include "sort_common.cuh"
 
@@ -247,17 +248,31 @@ __global__ void init_cursor_kernel(const int32_t *__restrict__ offsets, int64_t 
 
 // Two words of host memory that this thread's calls have the device write their
 // counts to (a copy to pageable memory goes through the driver's staging and a
-// second wait); null if there is none to be had.
+// second wait); null if there is none to be had.  A thread that ends leaves its
+// words to the next one: freeing them is a call that fails another thread's
+// graph capture, and there are never more than threads at one time.
+static std::mutex left_mu;
+static int64_t *left = nullptr; // the words of ended threads, the first holding the next's address
 struct HostCounts {
     int64_t *p = nullptr;
     HostCounts() {
+        {
+            std::lock_guard<std::mutex> lk(left_mu);
+            if ((p = left)) {
+                left = reinterpret_cast<int64_t *>(p[0]);
+                return;
+            }
+        }
         if (cudaHostAlloc(&p, 16, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
         }
     }
     ~HostCounts() {
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        std::lock_guard<std::mutex> lk(left_mu);
+        p[0] = reinterpret_cast<int64_t>(left);
+        left = p;
     }
 };
 static int64_t *host_counts() {
